@@ -91,6 +91,30 @@ def test_sgemm_true_float32(cuda_device, M):
     assert torch.equal(out, big[:M])
 
 
+# the three tile heights (16: few rows; 32, 64: by the tiles on the busiest SM), whole and ragged
+@pytest.mark.parametrize("M,N,K", [(16, 64, 64), (17, 4100, 68), (32, 12288, 16), (65, 66, 132),
+                                   (300, 8200, 80), (64, 64, 1)])
+def test_sgemm_tiles_and_alignments_agree(cuda_device, M, N, K):
+    from binfer_b200.csrc import ops
+    a = torch.randn(M, K, device=cuda_device)
+    w = torch.randn(N, K, device=cuda_device)
+    out = torch.full((M, N), 7.0, device=cuda_device)
+    ops.sgemm_nt(a, w, out)
+    ref = a.double() @ w.double().T
+    # runs of 64 terms: each rounding is at most half a unit of a partial sum
+    bound = (64 + K / 64) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    # rows off the 16-byte boundaries are read term by term: the same sums
+    off = torch.randn(M, K + 1, device=cuda_device)
+    off[:, 1:] = a
+    other = torch.full((M, N), 7.0, device=cuda_device)
+    ops.sgemm_nt(off[:, 1:], w, other)
+    assert torch.equal(out, other)
+    one = torch.full((1, N), 7.0, device=cuda_device)
+    ops.sgemm_nt(a[M - 1:], w, one)
+    assert torch.equal(one[0], out[M - 1])
+
+
 # ------------------------------------------------------- q/k norm, rotation, cache write
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("nh,nkv,d,rot,norm", [(3, 1, 16, 16, True), (4, 2, 48, 24, True),
