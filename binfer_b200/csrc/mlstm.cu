@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(MLSTM_COLS * MLSTM_GROUPS) mlstm_scan_kernel(
     const A* __restrict__ proj, long long stride, const float* __restrict__ gates,
     float* __restrict__ state, long long slot_stride, int state_size,
     const int* __restrict__ q_start, const int* __restrict__ state_slots, int num_slots,
-    float* __restrict__ o_raw, int H, int dk, int dv, float q_scale, int* __restrict__ err) {
+    float* __restrict__ o_raw, int H, int dk, int dv, float q_scale, int* __restrict__ err,
+    int n_max) {
   constexpr int NT = MLSTM_COLS * MLSTM_GROUPS;
   extern __shared__ float sh[];
   float* qs = sh;                    // dk
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(MLSTM_COLS * MLSTM_GROUPS) mlstm_scan_kernel(
   const int col = blockIdx.x * MLSTM_COLS + lane;
   const int head = blockIdx.y, b = blockIdx.z;
   const int t0 = q_start[b], t1 = q_start[b + 1];
+  if (t1 - t0 > n_max) return;                     // (longer portions: chunk_scan.cu)
   const int slot = state_slots[b];
   if (slot < 0 || slot >= num_slots) {
     if (threadIdx.x == 0) atomicOr(err, BF_ERR_SLOT);
@@ -200,7 +202,8 @@ __global__ void __launch_bounds__(128) mlstm_scan2_kernel(
     const A* __restrict__ proj, long long stride, const float* __restrict__ gates,
     float* __restrict__ state, long long slot_stride, int state_size,
     const int* __restrict__ q_start, const int* __restrict__ state_slots, int num_slots,
-    float* __restrict__ o_raw, int H, int dk, int dv, float q_scale, int* __restrict__ err) {
+    float* __restrict__ o_raw, int H, int dk, int dv, float q_scale, int* __restrict__ err,
+    int n_max) {
   constexpr int PAD = R == 8 ? 4 : 0;              // keeps the lanes' 16-byte reads off each
   constexpr int PITCH = 32 * (R + PAD);            // other's banks
   __shared__ __align__(16) float qs[MLSTM2_CH * PITCH];   // row r at (r / R) (R + PAD) + r % R
@@ -211,6 +214,7 @@ __global__ void __launch_bounds__(128) mlstm_scan2_kernel(
   const int colw = blockIdx.x * MLSTM2_COLS + warp * 8;    // the warp's first column
   const int head = blockIdx.y, b = blockIdx.z;
   const int t0 = q_start[b], t1 = q_start[b + 1];
+  if (t1 - t0 > n_max) return;                     // (longer portions: chunk_scan.cu)
   const int slot = state_slots[b];
   if (slot < 0 || slot >= num_slots) {
     if (threadIdx.x == 0) atomicOr(err, BF_ERR_SLOT);
@@ -425,9 +429,11 @@ __global__ void __launch_bounds__(128) mlstm_scan2_kernel(
 BF_EXPORT int bf_mlstm_scan(const void* proj, long long stride, const float* gates, float* state,
                             long long slot_stride, int state_size, const int* q_start,
                             const int* state_slots, int num_slots, float* o_raw, int B, int H,
-                            int dk, int dv, float q_scale, int act_dtype, int* err,
+                            int dk, int dv, float q_scale, int act_dtype, int* err, int n_max,
                             cudaStream_t stream) {
+  // n_max > 0: requests that bring more tokens are left alone
   if (B <= 0) return 0;
+  if (n_max <= 0) n_max = 0x7fffffff;
   if (dk > 64 * MLSTM_GROUPS || dk <= 0 || dv <= 0) return (int)cudaErrorInvalidValue;
   if (dk % 8 == 0 && stride % 8 == 0 && ((uintptr_t)proj & 15) == 0 && (H * dk) % 8 == 0 &&
       ((uintptr_t)state & 15) == 0 && slot_stride % 4 == 0 && state_size % 4 == 0) {
@@ -435,7 +441,7 @@ BF_EXPORT int bf_mlstm_scan(const void* proj, long long stride, const float* gat
 #define GO2(A, J)                                                                             \
   mlstm_scan2_kernel<A, J><<<grid2, 128, 0, stream>>>(                                        \
       (const A*)proj, stride, gates, state, slot_stride, state_size, q_start, state_slots,   \
-      num_slots, o_raw, H, dk, dv, q_scale, err)
+      num_slots, o_raw, H, dk, dv, q_scale, err, n_max)
     if (act_dtype == BF_DTYPE_F32) {
       if (dk <= 128) GO2(float, 4); else GO2(float, 8);
     } else {
@@ -450,7 +456,7 @@ BF_EXPORT int bf_mlstm_scan(const void* proj, long long stride, const float* gat
 #define GO(A, J)                                                                              \
   mlstm_scan_kernel<A, J><<<grid, threads, smem, stream>>>(                                   \
       (const A*)proj, stride, gates, state, slot_stride, state_size, q_start, state_slots,   \
-      num_slots, o_raw, H, dk, dv, q_scale, err)
+      num_slots, o_raw, H, dk, dv, q_scale, err, n_max)
   const int rows = (dk + MLSTM_GROUPS - 1) / MLSTM_GROUPS;
   if (act_dtype == BF_DTYPE_F32) {
     if (rows <= 16) GO(float, 16); else if (rows <= 32) GO(float, 32); else GO(float, 64);

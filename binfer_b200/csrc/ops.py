@@ -691,19 +691,67 @@ def conv_state_shift(proj: torch.Tensor, state: torch.Tensor, state_slots: torch
 # ------------------------------------------------------------------------- retention
 RETENTION_MAX_QK_DIM = 1024
 
+# Portions of at most this many tokens are walked token by token also where the products over
+# chunks may run: their five kernels take 40 to 55 us whatever the portion, the walk 0.14 to 0.5 us a
+# token.  One portion, walk / products: 64 heads of 128 x 64: 39 / 51 us at 130 tokens, 76 / 65 at
+# 300, 459 / 226 at 2,000; mLSTM, 8 heads of 256 x 512: 40 / 83 at 64, 150 / 107 at 300, 982 / 396 at
+# 2,048.
+CHUNK_SCAN_MIN = 160
+# tokens a chunk (of 64 / 128: 226 / 228 us and 396 / 390 for the two above; 64 takes half the
+# products inside a chunk, 128 half the states between them)
+CHUNK_SCAN_TOKENS = 64
+# most scratch that a step's chunks may take; a step that needs more is walked
+CHUNK_SCAN_MAX_BYTES = 768 << 20
+
+
+def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_heads: int, dk: int,
+                   dv: int, state: torch.Tensor, mlstm: int) -> Optional[torch.Tensor]:
+    """Scratch for the products over chunks, or None where a step's recurrence is walked: single
+    tokens and short portions, and sizes or addresses that are no whole 16-byte pieces."""
+    if (not chunked or max_q <= CHUNK_SCAN_MIN or dk % 4 or dv % 4 or state.stride(0) % 4
+            or state.data_ptr() % 16 or B > 65535 or heads > 65535):
+        return None
+    fn = lib().bf_chunk_scan_scratch
+    fn.restype = _c_ll
+    n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
+           _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm))
+    if n > CHUNK_SCAN_MAX_BYTES:
+        return None
+    return torch.empty(n, dtype=torch.uint8, device=state.device)
+
+
+def _walk_limit(scratch: Optional[torch.Tensor], B: int) -> int:
+    """For the kernels that walk: the longest portion they take (0: any, -1: none, the step's only
+    request has chunks)."""
+    return 0 if scratch is None else -1 if B == 1 else CHUNK_SCAN_MIN
+
+
+def _chunk_scan_linear(name, qk, vf, decays, tok_decay, state, q_start, state_slots, o_raw, scratch,
+                       B, heads, qk_heads, dk, dv, err) -> None:
+    _run(name + "_chunks", lib().bf_chunk_scan_linear, _ptr(qk), _ptr(vf), _ptr(decays),
+         _ptr(tok_decay), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
+         _c_int(state.shape[0]), _ptr(o_raw), _ptr(scratch), _c_int(vf.shape[0]), _c_int(B),
+         _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv), _c_int(CHUNK_SCAN_TOKENS),
+         _c_int(CHUNK_SCAN_MIN), _ptr(err), _stream())
+    global _launches
+    _launches += 4          # five kernels
+
 
 def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decays: torch.Tensor,
                    inv_freq: Optional[torch.Tensor], positions: torch.Tensor,
                    state: torch.Tensor, q_start: torch.Tensor, state_slots: torch.Tensor,
                    o_raw: torch.Tensor, B: int, heads: int, dk: int, dv: int, k_scale: float,
-                   err: torch.Tensor, max_q: int = 0, silu: bool = False) -> None:
+                   err: torch.Tensor, max_q: int = 0, silu: bool = False,
+                   chunked: bool = False) -> None:
     """The recurrence ``S <- decay_h S + k v^T, o = S^T q`` over every request's tokens of the
     step.  ``proj`` rows hold q (``heads dk`` numbers from column ``q_off``), k (from
     ``k_off``) and v (``heads dv`` from ``v_off``); q and k are turned by the position
     (``inv_freq`` float32, None: not) and k multiplied by ``k_scale``.  ``state`` float32
     ``[slots, heads * dv * dk]`` (a column block of the slots' storage); ``o_raw`` float32
     ``[T, heads dv]``.  ``max_q``: the most tokens one request brings to the step, if the
-    caller knows it (0: not known).  ``silu``: q, k and v pass silu first."""
+    caller knows it (0: not known).  ``silu``: q, k and v pass silu first.  ``chunked``: portions of
+    more than ``CHUNK_SCAN_MIN`` tokens may run as products over chunks (``chunk_scan.cu``), whose
+    order of sums depends on where the portion begins."""
     _want(decays, torch.float32, "decays"); _want(o_raw, torch.float32, "o_raw")
     if proj.stride(1) != 1 or dk > RETENTION_MAX_QK_DIM:
         raise KernelError(f"retention_scan: contiguous rows and a key size of at most "
@@ -720,25 +768,30 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
     # two kernels
     qk = torch.empty((T, 2, heads, dk), dtype=torch.float32, device=proj.device)
     vf = torch.empty((T, heads, dv), dtype=torch.float32, device=proj.device)
+    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, heads, dk, dv, state, 0)
     _run("retention_scan", lib().bf_retention_scan, _ptr(proj), _c_ll(proj.stride(0)),
          _c_ll(q_off), _c_ll(k_off), _c_ll(v_off), _ptr(decays), _ptr(inv_freq), _c_int(rot_half),
          _ptr(positions), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
          _c_int(state.shape[0]), _ptr(o_raw), _ptr(qk), _ptr(vf), _c_int(T), _c_int(B),
          _c_int(max_q if max_q > 0 else T), _c_int(heads), _c_int(dk), _c_int(dv), _c_float(k_scale), _c_int(_dtype_code(proj)), _ptr(err),
-         _c_int(1 if silu else 0), _stream())
+         _c_int(1 if silu else 0), _c_int(_walk_limit(scratch, B)), _stream())
     global _launches
     _launches += 1          # two kernels: the rotation and the scan
+    if scratch is not None:
+        _chunk_scan_linear("retention_scan", qk, vf, decays, None, state, q_start, state_slots,
+                           o_raw, scratch, B, heads, heads, dk, dv, err)
 
 
 def linear_scan(qk: torch.Tensor, vf: torch.Tensor, tok_decay: torch.Tensor, state: torch.Tensor,
                 q_start: torch.Tensor, state_slots: torch.Tensor, o_raw: torch.Tensor, B: int,
                 heads: int, qk_heads: int, dk: int, dv: int, err: torch.Tensor,
-                max_q: int = 0) -> None:
+                max_q: int = 0, chunked: bool = False) -> None:
     """The recurrence ``S <- decay[t, h] S + k v^T, o = S^T q`` over every request's tokens of
     the step, on inputs that are float already: ``qk [T, 2, qk_heads, dk]`` (q, then k; head h
     reads head ``h // (heads / qk_heads)``), ``vf [T, heads, dv]``, ``tok_decay [T, heads]``.
     ``state`` float32 ``[slots, heads * dv * dk]`` (a column block of the slots' storage);
-    ``o_raw`` float32 ``[T, heads dv]``.  ``max_q``: the most tokens one request brings."""
+    ``o_raw`` float32 ``[T, heads dv]``.  ``max_q``: the most tokens one request brings.
+    ``chunked``: as for :func:`retention_scan`."""
     for name, t in (("qk", qk), ("vf", vf), ("tok_decay", tok_decay), ("o_raw", o_raw)):
         _want(t, torch.float32, name)
         if not t.is_contiguous():
@@ -752,10 +805,17 @@ def linear_scan(qk: torch.Tensor, vf: torch.Tensor, tok_decay: torch.Tensor, sta
     if (state.dtype != torch.float32 or state.stride(1) != 1
             or state.shape[1] != heads * dk * dv):
         raise KernelError("linear_scan: state must be float32 [slots, heads * dk * dv]")
+    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, qk_heads, dk, dv, state, 0)
+    if scratch is not None:
+        _chunk_scan_linear("linear_scan", qk, vf, None, tok_decay, state, q_start, state_slots,
+                           o_raw, scratch, B, heads, qk_heads, dk, dv, err)
+        if _walk_limit(scratch, B) < 0:
+            return
     _run("linear_scan", lib().bf_linear_scan, _ptr(qk), _ptr(vf), _ptr(tok_decay), _ptr(state),
          _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
          _ptr(o_raw), _c_int(T), _c_int(B), _c_int(max_q if max_q > 0 else T), _c_int(heads),
-         _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err), _stream())
+         _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err), _c_int(_walk_limit(scratch, B)),
+         _stream())
 
 
 def mamba2_encode(proj: torch.Tensor, xbc_off: int, dt_off: int, conv_w: Optional[torch.Tensor],
@@ -1240,11 +1300,13 @@ def mlstm_state_size(dk: int, dv: int) -> int:
 
 def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
                q_start: torch.Tensor, state_slots: torch.Tensor, o_raw: torch.Tensor, B: int,
-               heads: int, dk: int, dv: int, q_scale: float, err: torch.Tensor) -> None:
+               heads: int, dk: int, dv: int, q_scale: float, err: torch.Tensor, max_q: int = 0,
+               chunked: bool = False) -> None:
     """The recurrence over every request's tokens of this step.  ``proj`` rows hold
     ``[q: heads dk | k: heads dk | v: heads dv | ...]``; ``state`` is float32
     ``[slots, heads, mlstm_state_size]``; ``o_raw`` float32 ``[T, heads dv]`` receives the
-    memory's output before its norm and gate."""
+    memory's output before its norm and gate.  ``max_q``: the most tokens one request brings, if
+    the caller knows it.  ``chunked`` (bfloat16): as for :func:`retention_scan`."""
     _want(gates, torch.float32, "gates"); _want(state, torch.float32, "state")
     _want(o_raw, torch.float32, "o_raw")
     if proj.stride(1) != 1 or dk > MLSTM_MAX_QK_DIM:
@@ -1252,11 +1314,26 @@ def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
                           f"{MLSTM_MAX_QK_DIM}")
     if state.shape[1:] != (heads, mlstm_state_size(dk, dv)):
         raise KernelError("mlstm_scan: state must be [slots, heads, mlstm_state_size(dk, dv)]")
+    T = proj.shape[0]
+    takes = (chunked and proj.dtype == torch.bfloat16 and proj.stride(0) % 4 == 0
+             and proj.data_ptr() % 8 == 0 and state.stride(1) == state.shape[2])
+    scratch = _chunk_scratch(takes, max_q or T, T, B, heads, heads, dk, dv, state, 1)
+    if scratch is not None:
+        _run("mlstm_scan_chunks", lib().bf_chunk_scan_mlstm, _ptr(proj), _c_ll(proj.stride(0)),
+             _ptr(gates), _ptr(state), _c_ll(state.stride(0)), _c_int(state.shape[2]),
+             _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]), _ptr(o_raw),
+             _ptr(scratch), _c_int(T), _c_int(B), _c_int(heads), _c_int(dk), _c_int(dv),
+             _c_float(q_scale), _c_int(CHUNK_SCAN_TOKENS), _c_int(CHUNK_SCAN_MIN), _ptr(err),
+             _stream())
+        global _launches
+        _launches += 4          # five kernels
+        if _walk_limit(scratch, B) < 0:
+            return
     _run("mlstm_scan", lib().bf_mlstm_scan, _ptr(proj), _c_ll(proj.stride(0)), _ptr(gates),
          _ptr(state), _c_ll(state.stride(0)), _c_int(state.shape[2]), _ptr(q_start),
          _ptr(state_slots), _c_int(state.shape[0]), _ptr(o_raw), _c_int(B), _c_int(heads),
          _c_int(dk), _c_int(dv), _c_float(q_scale), _c_int(_dtype_code(proj)), _ptr(err),
-         _stream())
+         _c_int(_walk_limit(scratch, B)), _stream())
 
 
 def mlstm_out(o_raw: torch.Tensor, proj: torch.Tensor, g_off: int, norm_w: torch.Tensor,

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(RET_THREADS) retention_scan_kernel(
     float* __restrict__ state, long long state_stride, const int* __restrict__ q_start,
     const int* __restrict__ state_slots, int n_slots, float* __restrict__ o_raw, int H, int dk,
     int dv, int ks_rt, int stage, int* __restrict__ err, const float* __restrict__ tok_decay,
-    int QH) {
+    int QH, int n_max) {
   extern __shared__ __align__(16) float sh[];
   const int KS = KST ? KST : ks_rt;
   const int cols = RET_THREADS / KS * CV;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(RET_THREADS) retention_scan_kernel(
   const int cg = tid / KS, part = tid % KS;
   const int col = col0 + cg * CV;           // the lane's first column
   const int t0 = q_start[b], n = q_start[b + 1] - t0;
-  if (n <= 0) return;
+  if (n <= 0 || n > n_max) return;          // (longer portions: chunk_scan.cu)
   int slot = state_slots[b];
   if (slot < 0 || slot >= n_slots) {
     if (tid == 0) atomicOr(err, BF_ERR_SLOT);
@@ -308,7 +308,10 @@ static int ret_launch_scan(const float* vf, const float* qk, const float* decays
                            const float* tok_decay, int QH, float* state, long long state_stride,
                            const int* q_start, const int* state_slots, int n_slots,
                            float* o_raw, int B, int max_q, int H, int dk, int dv, int* err,
-                           cudaStream_t stream) {
+                           int n_max, cudaStream_t stream) {
+  // n_max: requests that bring more tokens are left alone (0: none are)
+  if (n_max > 0 && max_q > n_max) max_q = n_max;
+  if (n_max <= 0) n_max = 0x7fffffff;
   const int R = dk <= 256 ? 8 : 32;
   int KS = 1;
   while (KS * R < dk) KS <<= 1;
@@ -359,7 +362,7 @@ static int ret_launch_scan(const float* vf, const float* qk, const float* decays
     }                                                                                          \
     kern<<<grid, RET_THREADS, st * per_token, stream>>>(                                       \
         vf, qk, decays, state, state_stride, q_start, state_slots, n_slots, o_raw, H, dk, dv,  \
-        KS, st, err, tok_decay, QH);                                                           \
+        KS, st, err, tok_decay, QH, n_max);                                                           \
   }
 #define RET_GO(RR, CC, KK)                                                                    \
   {                                                                                            \
@@ -381,7 +384,8 @@ BF_EXPORT int bf_retention_scan(
     const float* decays, const float* inv_freq, int rot_half, const int* positions, float* state,
     long long state_stride, const int* q_start, const int* state_slots, int n_slots, float* o_raw,
     float* qk, float* vf, int T, int B, int max_q, int H, int dk, int dv, float k_scale,
-    int act_dtype, int* err, int act, cudaStream_t stream) {
+    int act_dtype, int* err, int act, int n_max, cudaStream_t stream) {
+  // n_max < 0: the encoding alone; > 0: the walk of portions of at most so many tokens
   // qk: scratch, float [T][2][H][dk]; vf: scratch, float [T][H][dv]; max_q: the most tokens one request brings (a hint that
   // sizes the staging buffers: single tokens leave room for more blocks an SM)
   if (B <= 0 || T <= 0) return 0;
@@ -398,10 +402,10 @@ BF_EXPORT int bf_retention_scan(
           (const __nv_bfloat16*)proj, stride, q_off, k_off, inv_freq, rot_half, positions, qk, T,
           H, dk, k_scale, act, v_off, dv, vf);
     const int e = bf_launch_status();
-    if (e) return e;
+    if (e || n_max < 0) return e;
   }
   return ret_launch_scan(vf, qk, decays, nullptr, H, state, state_stride, q_start, state_slots,
-                         n_slots, o_raw, B, max_q, H, dk, dv, err, stream);
+                         n_slots, o_raw, B, max_q, H, dk, dv, err, n_max, stream);
 }
 
 // The scan alone, on q, k and v that are float already: qk [T][2][qk_heads][dk] (q, then k),
@@ -409,14 +413,14 @@ BF_EXPORT int bf_retention_scan(
 BF_EXPORT int bf_linear_scan(const float* qk, const float* vf, const float* tok_decay,
                              float* state, long long state_stride, const int* q_start,
                              const int* state_slots, int n_slots, float* o_raw, int T, int B,
-                             int max_q, int H, int qk_heads, int dk, int dv, int* err,
+                             int max_q, int H, int qk_heads, int dk, int dv, int* err, int n_max,
                              cudaStream_t stream) {
   if (B <= 0 || T <= 0) return 0;
   if (dk <= 0 || dv <= 0 || dk > 1024 || !qk || !vf || !tok_decay || qk_heads <= 0 ||
       H % qk_heads)
     return (int)cudaErrorInvalidValue;
   return ret_launch_scan(vf, qk, nullptr, tok_decay, qk_heads, state, state_stride, q_start,
-                         state_slots, n_slots, o_raw, B, max_q, H, dk, dv, err, stream);
+                         state_slots, n_slots, o_raw, B, max_q, H, dk, dv, err, n_max, stream);
 }
 
 // One warp per (token, head).

@@ -83,7 +83,9 @@ class MLSTMMixer(Mixer):
         ops.mlstm_gates(x, self.w_gates, self.gate_bias, gates, self.heads, self.spec.gate_cap)
         o_raw = torch.empty((T, self.v_size), dtype=torch.float32, device=x.device)
         ops.mlstm_scan(proj, gates, view.state, ctx.q_start, ctx.state_slots, o_raw, ctx.B,
-                       self.heads, self.dk, self.dv, self.dk ** -0.5, ctx.err)
+                       self.heads, self.dk, self.dv, self.dk ** -0.5, ctx.err,
+                       max_q=1 if ctx.decode_only else ctx.max_q_len,
+                       chunked=x.dtype == torch.bfloat16)
         out = torch.empty((T, self.v_size), dtype=x.dtype, device=x.device)
         ops.mlstm_out(o_raw, proj, 2 * self.qk_size + self.v_size, self.norm_w, out, self.heads,
                       self.dv, self.spec.norm_eps)

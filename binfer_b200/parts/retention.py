@@ -98,7 +98,8 @@ class RetentionMixer(Mixer):
                            ctx.positions, view.state, ctx.q_start, ctx.state_slots, o_raw, ctx.B,
                            self.heads, self.dk, self.dv, self.k_scale, ctx.err,
                            max_q=1 if ctx.decode_only else ctx.max_q_len,
-                           silu=self.spec.activation == "silu")
+                           silu=self.spec.activation == "silu",
+                           chunked=proj.dtype == torch.bfloat16)
         g_off = 2 * self.qk_size + self.v_size
         if self.plain_out:
             ops.retention_out(o_raw, proj, g_off, out, self.heads, self.dv, self.spec.norm_eps,

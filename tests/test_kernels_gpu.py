@@ -1079,3 +1079,110 @@ def test_gemm_bf16_cluster_many_k_steps_many_launches(cuda_device, N, K, bn, c):
         assert ops.gemm_bf16_cluster(x, w, out, err, bn, c)
         same &= (out == first).all()
     assert bool(same) and int(err.item()) == 0
+
+
+# ------------------------------------------------------------ recurrences in chunks of tokens
+def _walk64(q, k, v, decay, S):
+    """``S <- decay S + k v^T, o = S^T q`` in float64: (o, S)."""
+    out = torch.empty_like(v)
+    for t in range(v.shape[0]):
+        S = S * decay[t][:, None, None] + k[t][:, :, None] * v[t][:, None, :]
+        out[t] = (q[t][:, None, :] @ S)[:, 0]
+    return out, S
+
+
+# portions at the edges of a chunk of 64 and of the shortest portion that has chunks, beside
+# portions that are walked; sizes below, at and between tiles of 64; shared q and k; a fixed decay;
+# decays that are zero
+@pytest.mark.parametrize("lens,H,G,dk,dv,decays", [
+    ([161, 1, 192, 160, 257], 4, 2, 32, 24, "spread"), ([193, 320], 3, 3, 20, 68, "zeros"),
+    ([300], 2, 1, 128, 64, "slow"), ([170, 3], 2, 2, 68, 132, "fixed")])
+def test_linear_scan_in_chunks(cuda_device, lens, H, G, dk, dv, decays):
+    from binfer_b200.csrc import ops
+    torch.manual_seed(len(lens) + dk)
+    T, B, dev = sum(lens), len(lens), cuda_device
+    qk = torch.randn(T, 2, G, dk, device=dev)
+    v = torch.randn(T, H, dv, device=dev)
+    d = torch.rand(T, H, device=dev)
+    if decays == "slow":
+        d = 1.0 - 0.01 * d
+    elif decays == "zeros":
+        d[torch.rand(T, H, device=dev) < 0.1] = 0.0
+    elif decays == "fixed":
+        d = d[:1].expand(T, H).contiguous()
+    state = torch.randn(B + 1, H * dk * dv, device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev).flip(0).contiguous()
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    out = torch.full((T, H * dv), 7.0, device=dev)
+    got, err = state.clone(), _err(dev)
+    ops.linear_scan(qk, v, d, got, qs, slots, out, B, H, G, dk, dv, err, max_q=max(lens),
+                    chunked=True)
+    assert int(err.item()) == 0 and torch.equal(got[B], state[B])
+    for b in range(B):
+        a, e, s = int(qs[b]), int(qs[b + 1]), int(slots[b])
+        q, k = (qk[a:e, i].double().repeat_interleave(H // G, 1) for i in (0, 1))
+        S0 = state[s].double().view(H, dv, dk).transpose(1, 2)
+        o, S = _walk64(q, k, v[a:e].double(), d[a:e].double(), S0)
+        # the same recurrence over absolute values bounds what a relative error of every factor and
+        # sum can come to: sums of runs of 16 and of up to 12 + 4 runs, a weight (two roundings),
+        # one update per chunk
+        bound_o, bound_S = _walk64(q.abs(), k.abs(), v[a:e].double().abs(), d[a:e].double(), S0.abs())
+        c = (64 + 4 * len(lens)) * 2.0 ** -24
+        assert bool(((out[a:e].view(-1, H, dv).double() - o).abs() <= c * bound_o + 1e-30).all())
+        have = got[s].double().view(H, dv, dk).transpose(1, 2)
+        assert bool(((have - S).abs() <= c * bound_S + 1e-30).all())
+    # a bad slot is flagged, and every state that no request owns left alone
+    bad, keep = slots.clone(), got.clone()
+    bad[0] = B + 5
+    ops.linear_scan(qk, v, d, keep, qs, bad, out, B, H, G, dk, dv, err, max_q=max(lens),
+                    chunked=True)
+    assert int(err.item()) == 2 and torch.equal(keep[int(slots[0])], got[int(slots[0])])
+    err.zero_()
+
+
+@pytest.mark.parametrize("lens,H,dk,dv", [([161, 1, 192, 160, 257], 2, 24, 40),
+                                          ([193], 3, 64, 100), ([320, 5], 1, 256, 64)])
+def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
+    """Against the walking kernel and both against float64: the products are no further off."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(len(lens) + dk)
+    T, B, dev = sum(lens), len(lens), cuda_device
+    proj = torch.randn(T, 2 * H * (dk + dv), device=dev).to(BF16)
+    gates = torch.cat([2 * torch.randn(T, H, device=dev), torch.nn.functional.logsigmoid(
+        3 + torch.randn(T, H, device=dev))], 1).contiguous()
+    state = 0.1 * torch.randn(B + 1, H, ops.mlstm_state_size(dk, dv), device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev).flip(0).contiguous()
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    got, err = {}, _err(dev)
+    for chunked in (False, True):
+        s, o = state.clone(), torch.full((T, H * dv), 7.0, device=dev)
+        ops.mlstm_scan(proj, gates, s, qs, slots, o, B, H, dk, dv, dk ** -0.5, err,
+                       max_q=max(lens), chunked=chunked)
+        got[chunked] = (o, s)
+    assert int(err.item()) == 0 and torch.equal(got[True][1][B], state[B])
+    off = {c: [0.0] * 4 for c in got}
+    for b in range(B):
+        a, e, at = int(qs[b]), int(qs[b + 1]), int(slots[b])
+        x = proj[a:e].double()
+        q = x[:, :H * dk].view(-1, H, dk) * dk ** -0.5
+        k = x[:, H * dk:2 * H * dk].view(-1, H, dk)
+        v = x[:, 2 * H * dk:2 * H * dk + H * dv].view(-1, H, dv)
+        s0 = state[at].double()
+        S, n, m = (s0[:, :dk * dv].view(H, dk, dv), s0[:, dk * dv:dk * dv + dk], s0[:, dk * dv + dk])
+        o = torch.empty_like(v)
+        for t in range(e - a):
+            i, f = gates[a + t, :H].double(), gates[a + t, H:].double()
+            m_new = torch.maximum(f + m, i)
+            da, db = torch.exp(f + m - m_new), torch.exp(i - m_new)
+            S = S * da[:, None, None] + (k[t] * db[:, None])[:, :, None] * v[t][:, None, :]
+            n, m = da[:, None] * n + db[:, None] * k[t], m_new
+            den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+            o[t] = (q[t][:, None, :] @ S)[:, 0] / den[:, None]
+        for c, (go, gs) in got.items():
+            g = gs[at].double()
+            for i, (have, want) in enumerate((
+                    (go[a:e].double().view(-1, H, dv), o), (g[:, :dk * dv].reshape(H, dk, dv), S),
+                    (g[:, dk * dv:dk * dv + dk], n), (g[:, dk * dv + dk], m))):
+                off[c][i] = max(off[c][i], float((have - want).norm() / want.norm()))
+    for walk, products in zip(off[False], off[True]):
+        assert products <= 1.5 * walk + 2e-7, off
