@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(LAT_THREADS) latent_attention_kernel(
     const int* __restrict__ tables, int table_stride, __nv_bfloat16* __restrict__ out, int H,
     int W, int rank, int page_size, int num_pages, float scale_log2, float* __restrict__ part_o,
     float* __restrict__ part_ml, int splits, const float* __restrict__ sinks,
-    int* __restrict__ err) {
+    int* __restrict__ err, int n_max) {
   extern __shared__ __align__(16) unsigned char lat_smem[];
   const int pitch = W + 8;
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(lat_smem);       // [32][pitch]
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(LAT_THREADS) latent_attention_kernel(
   const int b = blockIdx.y, row0 = blockIdx.x * LAT_ROWS;
   const int t0 = q_start[b], n_tok = q_start[b + 1] - t0;
   const int rows_total = n_tok * H;
-  if (row0 >= rows_total) return;
+  if (row0 >= rows_total || n_tok > n_max) return;
   const int* table = tables + (size_t)b * table_stride;
   const int p_hi = positions[t0 + min(row0 + LAT_ROWS - 1, rows_total - 1) / H];
   const int n_tiles = p_hi / LAT_KEYS + 1;
@@ -317,11 +317,11 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_o,
                                     const float* __restrict__ part_ml, int splits,
                                     const int* __restrict__ q_start,
                                     __nv_bfloat16* __restrict__ out, int H, int rank,
-                                    const float* __restrict__ sinks) {
+                                    const float* __restrict__ sinks, int n_max) {
   const int r = blockIdx.x, tile = blockIdx.y, b = blockIdx.z;
   const int t0 = q_start[b], rows_total = (q_start[b + 1] - t0) * H;
   const int row = tile * LAT_ROWS + r;
-  if (row >= rows_total) return;
+  if (row >= rows_total || rows_total > n_max * H) return;
   const size_t at = ((size_t)b * gridDim.y + tile) * splits * LAT_ROWS;
   float M = -1e30f;
   for (int x = 0; x < splits; ++x) M = fmaxf(M, part_ml[(at + (size_t)x * LAT_ROWS + r) * 2]);
@@ -350,7 +350,8 @@ BF_EXPORT int bf_latent_attention(const void* q, const void* cache, const int* q
                                   void* out, int B, int max_rows, int H, int W, int rank,
                                   int page_size, int num_pages, float scale, float* part_o,
                                   float* part_ml, int splits, const float* sinks, int* err,
-                                  cudaStream_t stream) {
+                                  int n_max, cudaStream_t stream) {
+  // n_max: requests that bring more tokens are left alone (max_rows counts the others)
   if (B <= 0 || max_rows <= 0) return 0;
   if (W % 16 || rank % 16 || rank <= 0 || rank > 512 || W < rank || W > 640 || !(scale > 0.f))
     return (int)cudaErrorInvalidValue;
@@ -377,7 +378,7 @@ BF_EXPORT int bf_latent_attention(const void* q, const void* cache, const int* q
     latent_attention_kernel<N><<<grid, LAT_THREADS, smem, stream>>>(                            \
         (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, q_start, positions, tables,       \
         table_stride, (__nv_bfloat16*)out, H, W, rank, page_size, num_pages, scale * log2e,     \
-        part_o, part_ml, splits, sinks, err);                                                   \
+        part_o, part_ml, splits, sinks, err, n_max);                                                   \
   }
   if (NP == 2) LAT_GO(2, 0) else if (NP == 4) LAT_GO(4, 1) else LAT_GO(8, 2)
 #undef LAT_GO
@@ -385,7 +386,7 @@ BF_EXPORT int bf_latent_attention(const void* q, const void* cache, const int* q
     const int e = bf_launch_status();
     if (e) return e;
     latent_merge_kernel<<<dim3(LAT_ROWS, tiles, B), 128, 0, stream>>>(
-        part_o, part_ml, splits, q_start, (__nv_bfloat16*)out, H, rank, sinks);
+        part_o, part_ml, splits, q_start, (__nv_bfloat16*)out, H, rank, sinks, n_max);
   }
   return bf_launch_status();
 }

@@ -42,6 +42,14 @@
 // the four warps of a quarter exchange their sums of squares, and the normed head leaves
 // multiplied by its gate.
 //
+// A third instance (LATENT) runs latent attention of prompt portions with keys and values expanded
+// (attention_latent_expand.cu says when): query and key heads of 128 plain + 64 rotated sizes, the
+// rotated key part shared by all heads, values of 128.  Keys and values lie row by row in one
+// buffer [rows, heads x (128 | 128)], the rotated parts in another [rows, 64], a portion's keys
+// from a row that is a multiple of 64 on: no pages, one box per 64 columns.  A K tile is three such
+// blocks and Q three halves, which leaves shared memory for three stages.  The epilogue adds a
+// head's sink to its sums and multiplies by the sigmoid of its gate.
+//
 // Every mbarrier wait is bounded.  A barrier whose waiter could fall two phases behind exists
 // once per parity of the tile number, so that its one-bit phase cannot alias: "P V of tile n
 // done" (waited for only when O must be rescaled), and "P of tile n written" (a softmax
@@ -67,6 +75,8 @@ constexpr int A2_THREADS = 608;  // sixteen softmax warps, the TMA warp, two MMA
 constexpr int A2_TMA_WARP = 16;
 constexpr int A2_MMA_WARP = 17;  // 17 issues for query tile A, 18 for tile B
 constexpr int A2_D = 128;
+constexpr int A2_PLAIN = 0, A2_DIFF = 1, A2_LATENT = 2;   // the instances
+constexpr int A2_ROT = 64;       // LATENT: rotated sizes behind the 128 plain ones
 
 // Barrier among the 256 softmax threads of a group (or THREADS of both) that also ANDs a
 // predicate.
@@ -84,7 +94,7 @@ __device__ __forceinline__ bool group_all(int id, bool ok) {
   return r != 0;
 }
 
-template <bool DIFF>
+template <int MODE>
 __global__ void __launch_bounds__(A2_THREADS, 1)
 prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
                                const __grid_constant__ CUtensorMap map_k,
@@ -97,28 +107,33 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
                                int num_pages, int window, float scale_log2, int splits,
                                float* __restrict__ part_o, float* __restrict__ part_ml,
                                int* __restrict__ err, float cap_pre, float cap_post,
-                               long long out_stride, float out_scale, BfDiffArgs dd) {
+                               long long out_stride, float out_scale, BfDiffArgs dd,
+                               const float* __restrict__ sinks) {
+  constexpr bool DIFF = MODE == A2_DIFF, LATENT = MODE == A2_LATENT;
   constexpr int D = A2_D;
-  constexpr int HALVES = D / 64;
+  constexpr int HALVES = D / 64;                         // blocks of 64 columns of a V tile
+  constexpr int KBLOCKS = LATENT ? HALVES + 1 : HALVES;  // ... of a Q or K tile
+  constexpr int STAGES = LATENT ? 3 : A2_STAGES;
   constexpr int BROWS = DIFF ? A2_BM : 2 * A2_BM;        // query rows of a CTA
   constexpr int TSHIFT = DIFF ? 0 : A2_BM;               // rows from query tile A to tile B
   constexpr int QHALF_BYTES = A2_BM * 128;               // 128 query rows of 128 bytes
   constexpr int KHALF_BYTES = A2_BN * 128;               // 64 key rows of 128 bytes
-  constexpr int Q_BYTES = HALVES * QHALF_BYTES;          // one Q tile
-  constexpr int KV_BYTES = HALVES * KHALF_BYTES;         // one K (or V) tile of 64 keys
+  constexpr int Q_BYTES = KBLOCKS * QHALF_BYTES;         // one Q tile
+  constexpr int K_BYTES = KBLOCKS * KHALF_BYTES;         // one K tile of 64 keys
+  constexpr int V_BYTES = HALVES * KHALF_BYTES;          // one V tile
   constexpr int OH = D / 2;                              // O columns per softmax thread
   extern __shared__ __align__(16) uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* Qs = base;                                    // [2][Q_BYTES]
-  uint8_t* Ks = Qs + 2 * Q_BYTES;                        // [STAGES][KV_BYTES]
-  uint8_t* Vs = Ks + A2_STAGES * KV_BYTES;               // [STAGES][KV_BYTES]
-  float* xm = reinterpret_cast<float*>(Vs + A2_STAGES * KV_BYTES);   // [sums, references][2 groups][128]
+  uint8_t* Ks = Qs + 2 * Q_BYTES;                        // [STAGES][K_BYTES]
+  uint8_t* Vs = Ks + STAGES * K_BYTES;                   // [STAGES][V_BYTES]
+  float* xm = reinterpret_cast<float*>(Vs + STAGES * V_BYTES);   // [sums, references][2 groups][128]
   float* xss = xm + 4 * 128;                             // DIFF: [4 column quarters][128] sums of squares
   uint64_t* bars = reinterpret_cast<uint64_t*>(xss + (DIFF ? 4 * 128 : 0));
   uint64_t* q_full = bars;                     // [1]
   uint64_t* kv_full = bars + 1;                // [STAGES]
-  uint64_t* kv_empty = kv_full + A2_STAGES;    // [STAGES]
-  uint64_t* s_full = kv_empty + A2_STAGES;     // [group][2]: one per S buffer
+  uint64_t* kv_empty = kv_full + STAGES;    // [STAGES]
+  uint64_t* s_full = kv_empty + STAGES;     // [group][2]: one per S buffer
   uint64_t* p_full = s_full + 4;               // [group][2], 8 arrivals (one a warp): P of the tiles of that parity
   uint64_t* o_done = p_full + 4;               // [group][2]: P V of the tiles of that parity
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 4);
@@ -139,7 +154,7 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
   const int g = h / (nh / nkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* table = block_tables + (size_t)seq * table_stride;
-  const int pages = A2_BN / page_size;
+  const int pages = LATENT ? 1 : A2_BN / page_size;
 
   const int p_first = pos0 + qb * BROWS;                                // first row of tile A
   const int p_last_a = min(pos0 + qlen - 1, p_first + A2_BM - 1);
@@ -157,7 +172,7 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < A2_STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(kv_full + s, 1);
       mbar_init(kv_empty + s, active_b ? 2 : 1);         // one arrival per MMA thread
     }
@@ -196,11 +211,34 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-          for (int hh = 0; hh < HALVES; ++hh)
-            tma_load_2d(Qs + t * Q_BYTES + hh * QHALF_BYTES, &map_q, q_full, h * D + hh * 64,
-                        row0 + qb * BROWS + t * A2_BM);
+          for (int hh = 0; hh < KBLOCKS; ++hh)
+            tma_load_2d(Qs + t * Q_BYTES + hh * QHALF_BYTES, &map_q, q_full,
+                        h * (KBLOCKS * 64) + hh * 64, row0 + qb * BROWS + t * A2_BM);
       }
     }
+    if constexpr (LATENT) {
+      // a portion's keys begin at a row that is a multiple of 64 of the expanded buffers, which
+      // are zero up to the next one; block_tables holds that row per portion
+      if (lane == 0) {
+        const int base_row = block_tables[blockIdx.y];
+        for (int n = 0; n < tiles && !*abort; ++n) {
+          const int st = n % STAGES;
+          if (n >= STAGES &&
+              !mbar_wait(kv_empty + st, (uint32_t)(n / STAGES - 1) & 1u, abort))
+            break;
+          const int y = base_row + (kt_first + n) * A2_BN;
+          mbar_expect_tx(kv_full + st, (uint32_t)(K_BYTES + V_BYTES));
+#pragma unroll
+          for (int hh = 0; hh < HALVES; ++hh) {
+            tma_load_2d(Ks + st * K_BYTES + hh * KHALF_BYTES, &map_k, kv_full + st,
+                        h * 2 * D + hh * 64, y);
+            tma_load_2d(Vs + st * V_BYTES + hh * KHALF_BYTES, &map_k, kv_full + st,
+                        h * 2 * D + D + hh * 64, y);
+          }
+          tma_load_2d(Ks + st * K_BYTES + HALVES * KHALF_BYTES, &map_v, kv_full + st, 0, y);
+        }
+      }
+    } else {
     // The warp looks up the pages of several tiles at a time, lane (i, pg) the page pg of the
     // i-th of them: one gather of the block table per 32 / pages tiles, and per tile little
     // more than the wait for its stage and the copies.  (With a lookup, a fence and a dozen
@@ -230,12 +268,12 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
       const bool run = pages > 1 && (in_run & gmask) == gmask;
       const uint32_t tile_bytes = (uint32_t)__popc(live & gmask) * page_size * D * 4;
       for (int i = 0; i < tb && nb + i < tiles; ++i) {
-        const int n = nb + i, st = n % A2_STAGES;
-        if (lane == 0 && n >= A2_STAGES)
-          ok = mbar_wait(kv_empty + st, (uint32_t)(n / A2_STAGES - 1) & 1u, abort);
+        const int n = nb + i, st = n % STAGES;
+        if (lane == 0 && n >= STAGES)
+          ok = mbar_wait(kv_empty + st, (uint32_t)(n / STAGES - 1) & 1u, abort);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
-        uint8_t* vb = Vs + st * KV_BYTES;
+        uint8_t* vb = Vs + st * V_BYTES;
         // V rows of pages that are not fetched must read as zero (the first tile of a
         // window, the last tile of the portion)
         const int t_first = (kt_first + n) * A2_BN;
@@ -262,14 +300,14 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
                 bf_tma_load_4d(vb + hh * KHALF_BYTES, &map_v_run, kv_full + st, hh * 64, 0, g,
                                page0);
               else
-                bf_tma_load_4d(Ks + st * KV_BYTES + hh * KHALF_BYTES, &map_k_run, kv_full + st,
+                bf_tma_load_4d(Ks + st * K_BYTES + hh * KHALF_BYTES, &map_k_run, kv_full + st,
                                hh * 64, 0, g, page0);
             }
           } else if (wanted) {
             const int y = (page * nkv + g) * page_size;
 #pragma unroll
             for (int hh = 0; hh < HALVES; ++hh) {
-              tma_load_2d(Ks + st * KV_BYTES + hh * KHALF_BYTES + my_pg * page_size * 128, &map_k,
+              tma_load_2d(Ks + st * K_BYTES + hh * KHALF_BYTES + my_pg * page_size * 128, &map_k,
                           kv_full + st, hh * 64, y);
               tma_load_2d(vb + hh * KHALF_BYTES + my_pg * page_size * 128, &map_v, kv_full + st,
                           hh * 64, y);
@@ -277,6 +315,7 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
           }
         }
       }
+    }
     }
   } else if (warp >= A2_MMA_WARP) {
     // ----------------------------------------------------------------- MMA issuers
@@ -296,10 +335,10 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
       const uint32_t q_addr = smem_u32(Qs + grp * Q_BYTES);
       auto issue_s = [&](int n) {                        // S of tile n into S buffer n & 1
         const uint32_t k_addr =
-            smem_u32(Ks + (n % A2_STAGES) * KV_BYTES + (DIFF ? grp * KHALF_BYTES : 0));
+            smem_u32(Ks + (n % STAGES) * K_BYTES + (DIFF ? grp * KHALF_BYTES : 0));
         const uint32_t d_addr = tmem_base + (uint32_t)(grp * 128 + (n & 1) * A2_BN);
 #pragma unroll
-        for (int k = 0; k < (DIFF ? 64 : D) / 16; ++k) {
+        for (int k = 0; k < (DIFF ? 64 : KBLOCKS * 64) / 16; ++k) {
           const uint32_t qo = (uint32_t)((k >> 2) * QHALF_BYTES + (k & 3) * 32);
           const uint32_t ko = (uint32_t)((k >> 2) * KHALF_BYTES + (k & 3) * 32);
           umma_bf16(d_addr, umma_desc_k_sw128(q_addr + qo), umma_desc_k_sw128(k_addr + ko),
@@ -313,18 +352,18 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
         issue_s(0);
       }
       for (int n = 0; n < my_tiles && ok; ++n) {
-        const int st = n % A2_STAGES;
+        const int st = n % STAGES;
         if (n + 1 < my_tiles) {
           // the next tile's product runs under this tile's softmax; its S buffer is free
           // since the group signalled P of the tile before this one
-          const int s1 = (n + 1) % A2_STAGES;
-          if (!(ok = mbar_wait(kv_full + s1, (uint32_t)((n + 1) / A2_STAGES) & 1u, abort))) break;
+          const int s1 = (n + 1) % STAGES;
+          if (!(ok = mbar_wait(kv_full + s1, (uint32_t)((n + 1) / STAGES) & 1u, abort))) break;
           tc_fence_after();
           issue_s(n + 1);
         }
         if (!(ok = mbar_wait(p_full + grp * 2 + (n & 1), (uint32_t)(n >> 1) & 1u, abort))) break;
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(Vs + st * KV_BYTES);
+        const uint32_t v_addr = smem_u32(Vs + st * V_BYTES);
         const uint32_t d_addr = tmem_base + (uint32_t)(256 + grp * 128);
         // P lies over the first 32 columns of the tile's S buffer, two keys a column; the
         // next product into that buffer (S of tile n + 2) is issued by this thread after
@@ -343,8 +382,8 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
       // cannot land in an earlier use of the stage)
       if (grp == 0 && active_b)
         for (int n = tiles_a; n < tiles && ok; ++n) {
-          if (!(ok = mbar_wait(kv_full + n % A2_STAGES, (uint32_t)(n / A2_STAGES) & 1u, abort))) break;
-          mbar_arrive(kv_empty + n % A2_STAGES);
+          if (!(ok = mbar_wait(kv_full + n % STAGES, (uint32_t)(n / STAGES) & 1u, abort))) break;
+          mbar_arrive(kv_empty + n % STAGES);
         }
     }
   } else {
@@ -594,7 +633,18 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
         }
       } else if (ok) {
         tc_fence_after();
-        const float inv = out_scale / xl[r];
+        float inv;
+        if constexpr (LATENT) {
+          // (a sink far above the row's scores makes its sum infinite and the result zero)
+          float sum = xl[r];
+          if (sinks) sum += exp2f(fmaf(sinks[h], 1.4426950408889634f, -xr[r]));
+          inv = out_scale / sum;
+          if (dd.gate && valid)
+            inv *= bf_sigmoid_fast(__bfloat162float(
+                ((const __nv_bfloat16*)dd.gate)[(size_t)(row0 + l) * dd.gate_stride + h]));
+        } else {
+          inv = out_scale / xl[r];
+        }
         __nv_bfloat16* dst = out + (size_t)(row0 + l) * out_stride + (size_t)h * D + half * OH;
 #pragma unroll 1
         for (int c0 = 0; c0 < OH; c0 += 32) {
@@ -718,7 +768,7 @@ BF_EXPORT int bf_prefill_attention_umma2_capped(
   if (e) return e;
   // two Q tiles, the stages of K and V, the row sums, barriers
   const size_t smem = 1024 + (size_t)2 * 32768 + (size_t)2 * A2_STAGES * 16384 + 2048 + 256;
-  auto kern = prefill_attention_umma2_kernel<false>;
+  auto kern = prefill_attention_umma2_kernel<A2_PLAIN>;
   static bool configured_on[BF_MAX_DEVICES];
   bool& configured = configured_on[bf_current_device()];
   if (!configured) {
@@ -733,7 +783,7 @@ BF_EXPORT int bf_prefill_attention_umma2_capped(
                                            (__nv_bfloat16*)out, nh, nkv, page_size, num_pages,
                                            window, scale * log2e, splits, part_o, part_ml, err,
                                            cap_pre, cap_post, out_stride, out_scale,
-                                           BfDiffArgs());
+                                           BfDiffArgs(), nullptr);
   if (splits > 1) {
     int st = bf_launch_status();
     if (st) return st;
@@ -791,7 +841,7 @@ BF_EXPORT int bf_diff_attention_prefill_umma(
                                     A2_BN / page_size);
   if (e) return e;
   const size_t smem = 1024 + (size_t)2 * 32768 + (size_t)2 * A2_STAGES * 16384 + 4096 + 256;
-  auto kern = prefill_attention_umma2_kernel<true>;
+  auto kern = prefill_attention_umma2_kernel<A2_DIFF>;
   static bool configured_on[BF_MAX_DEVICES];
   bool& configured = configured_on[bf_current_device()];
   if (!configured) {
@@ -806,12 +856,59 @@ BF_EXPORT int bf_diff_attention_prefill_umma(
   kern<<<grid, A2_THREADS, smem, stream>>>(mq, mk, mv, mkr, mvr, items, block_tables, table_stride,
                                            (__nv_bfloat16*)out, nh, nkv, page_size, num_pages, 0,
                                            scale * 1.4426950408889634f, splits, part_o, part_ml,
-                                           err, 0.f, 0.f, out_stride, 1.f, dd);
+                                           err, 0.f, 0.f, out_stride, 1.f, dd, nullptr);
   if (splits > 1) {
     int st = bf_launch_status();
     if (st) return st;
     return bf_diff_attention_merge_items(part_o, part_ml, items, n_items, max_rows, out, nh, A2_D,
                                          splits, out_stride, dd, stream);
   }
+  return bf_launch_status();
+}
+
+// Latent attention of prompt portions over expanded keys and values.  q: rows `q_stride` elements
+// apart, head h at columns h 192 (128 plain | 64 rotated); kv [kv_rows, nh (128 key | 128 value)]
+// and rot [kv_rows, 64]; kv_base[i]: the row of portion i's first key (a multiple of 64; rows up to
+// the next multiple of 64 behind its last key are finite).  out: rows `out_stride` apart, head h at
+// columns h 128, times the sigmoid of gate[row * gate_stride + h] (null: not); sinks: a logit per
+// head in the softmax's denominator (or null).
+BF_EXPORT int bf_latent_attention_prefill_umma(
+    const void* q, long long q_stride, const void* kv, const void* rot, long long kv_rows,
+    const int* items, int n_items, int max_rows, int total_rows, const int* kv_base, void* out,
+    int nh, float scale, long long out_stride, const void* gate, long long gate_stride,
+    const float* sinks, int* err, cudaStream_t stream) {
+  if (n_items <= 0 || max_rows <= 0) return 0;
+  constexpr int QD = A2_D + A2_ROT;
+  if (nh <= 0 || kv_rows <= 0 || ((uintptr_t)q & 15) || ((uintptr_t)kv & 15) ||
+      ((uintptr_t)rot & 15) || ((uintptr_t)out & 15) || !(scale > 0.f) || (q_stride & 7) ||
+      q_stride < (long long)nh * QD || out_stride < (long long)nh * A2_D || (out_stride & 7) ||
+      !kv_base)
+    return (int)cudaErrorInvalidValue;
+  CUtensorMap mq, mkv, mr;
+  int e = bf_make_tensor_map_bf16_2d(&mq, q, total_rows, (long long)nh * QD, q_stride, A2_BM, 64);
+  if (e) return e;
+  e = bf_make_tensor_map_bf16_2d(&mkv, kv, kv_rows, (long long)nh * 2 * A2_D,
+                                 (long long)nh * 2 * A2_D, A2_BN, 64);
+  if (e) return e;
+  e = bf_make_tensor_map_bf16_2d(&mr, rot, kv_rows, A2_ROT, A2_ROT, A2_BN, 64);
+  if (e) return e;
+  // two Q tiles of three blocks, three stages of K (three blocks) and V (two), row sums, barriers
+  const size_t smem = 1024 + (size_t)2 * 49152 + (size_t)3 * (24576 + 16384) + 2048 + 256;
+  auto kern = prefill_attention_umma2_kernel<A2_LATENT>;
+  static bool configured_on[BF_MAX_DEVICES];
+  bool& configured = configured_on[bf_current_device()];
+  if (!configured) {
+    cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem);
+    if (ce != cudaSuccess) return (int)ce;
+    configured = true;
+  }
+  dim3 grid(nh, n_items, (max_rows + 2 * A2_BM - 1) / (2 * A2_BM));
+  if (grid.y > 65535u || grid.z > 65535u) return (int)cudaErrorInvalidValue;
+  const BfDiffArgs dd = {gate, gate_stride, 0.f, 0.f, 1.f, 0.f, 1};
+  kern<<<grid, A2_THREADS, smem, stream>>>(mq, mkv, mr, mr, mr, items, kv_base, 0,
+                                           (__nv_bfloat16*)out, nh, nh, 1, 1, 0,
+                                           scale * 1.4426950408889634f, 1, nullptr, nullptr, err,
+                                           0.f, 0.f, out_stride, 1.f, dd, sinks);
   return bf_launch_status();
 }

@@ -95,17 +95,18 @@ BF_EXPORT int bf_section_norm(const void* x, long long stride, long long off, in
 // of `proj` or a buffer of its own) and a row of `proj`, from kv_off,
 // [rank numbers that become the latent | dr numbers that become the shared key part].
 // The cache row of a token is [latent (normed, weighted) | key part (rotated)], one "head" of
-// rank + dr numbers.  q_abs [T, H, rank + dr] gets only every head's rotated part, at
-// [rank, rank + dr); the plain part is turned into latent coordinates by a product elsewhere.
-// One block per token.
+// rank + dr numbers.  Every head's rotated part goes to q_out, from column o_off of the head's
+// o_pitch columns on (rows o_stride apart); the plain part is turned into latent coordinates by a
+// product elsewhere.  q_out may be q itself (o_off d, o_pitch d + dr): a thread reads the pair that
+// it writes.  One block per token.
 template <typename A>
 __global__ void latent_encode_kernel(
-    const A* __restrict__ proj, long long stride, const A* __restrict__ q, long long q_stride,
-    long long kv_off,
+    const A* proj, long long stride, const A* q, long long q_stride, long long kv_off,
     const float* __restrict__ norm_w, float eps, const float* __restrict__ inv_freq,
     int rot_half, int interleaved, float rot_mag, const int* __restrict__ positions,
-    const int* __restrict__ slots, A* __restrict__ q_abs, A* __restrict__ cache, int H, int d,
-    int dr, int rank, int page_size, long long num_slots, int* __restrict__ err) {
+    const int* __restrict__ slots, A* q_out, long long o_stride, int o_pitch, int o_off,
+    A* __restrict__ cache, int H, int d, int dr, int rank, int page_size, long long num_slots,
+    int* __restrict__ err) {
   extern __shared__ float sh[];
   float* cs = sh;                   // rot_half cosines, rot_half sines
   float* sn = sh + rot_half;
@@ -151,7 +152,7 @@ __global__ void latent_encode_kernel(
   for (int idx = threadIdx.x; idx < H * rot_half; idx += blockDim.x) {
     const int h = idx / rot_half, m = idx - h * rot_half;
     const A* qr = q + (size_t)t * q_stride + (size_t)h * (d + dr) + d;
-    A* o = q_abs + ((size_t)t * H + h) * W + rank;
+    A* o = q_out + (size_t)t * o_stride + (size_t)h * o_pitch + o_off;
     int a, b;
     me_pair(m, rot_half, interleaved, &a, &b);
     const float u = bf_ld(qr + a), v = bf_ld(qr + b);
@@ -161,7 +162,7 @@ __global__ void latent_encode_kernel(
   const int rest = dr - 2 * rot_half;
   for (int idx = threadIdx.x; idx < H * rest; idx += blockDim.x) {
     const int h = idx / rest, i = 2 * rot_half + idx % rest;
-    bf_st(q_abs + ((size_t)t * H + h) * W + rank + i,
+    bf_st(q_out + (size_t)t * o_stride + (size_t)h * o_pitch + o_off + i,
           bf_ld(q + (size_t)t * q_stride + (size_t)h * (d + dr) + d + i));
   }
 }
@@ -170,8 +171,8 @@ BF_EXPORT int bf_latent_encode(const void* proj, long long stride, const void* q
                                long long q_stride, long long kv_off, const float* norm_w,
                                float eps,
                                const float* inv_freq, int rot_half, int interleaved,
-                               float rot_mag, const int* positions, const int* slots, void* q_abs,
-                               void* cache, int T, int H, int d, int dr, int rank, int page_size,
+                               float rot_mag, const int* positions, const int* slots, void* q_out,
+                               long long o_stride, int o_pitch, int o_off, void* cache, int T, int H, int d, int dr, int rank, int page_size,
                                long long num_slots, int act_dtype, int* err,
                                cudaStream_t stream) {
   if (T <= 0) return 0;
@@ -181,13 +182,14 @@ BF_EXPORT int bf_latent_encode(const void* proj, long long stride, const void* q
   if (act_dtype == BF_DTYPE_F32)
     latent_encode_kernel<float><<<T, threads, smem, stream>>>(
         (const float*)proj, stride, (const float*)q, q_stride, kv_off, norm_w, eps, inv_freq,
-        rot_half, interleaved, rot_mag, positions, slots, (float*)q_abs, (float*)cache, H, d, dr,
+        rot_half, interleaved, rot_mag, positions, slots, (float*)q_out, o_stride, o_pitch, o_off,
+        (float*)cache, H, d, dr,
         rank, page_size, num_slots, err);
   else
     latent_encode_kernel<__nv_bfloat16><<<T, threads, smem, stream>>>(
         (const __nv_bfloat16*)proj, stride, (const __nv_bfloat16*)q, q_stride, kv_off, norm_w,
-        eps, inv_freq, rot_half, interleaved, rot_mag, positions, slots, (__nv_bfloat16*)q_abs,
-        (__nv_bfloat16*)cache, H, d, dr, rank, page_size, num_slots, err);
+        eps, inv_freq, rot_half, interleaved, rot_mag, positions, slots, (__nv_bfloat16*)q_out,
+        o_stride, o_pitch, o_off, (__nv_bfloat16*)cache, H, d, dr, rank, page_size, num_slots, err);
   return bf_launch_status();
 }
 

@@ -933,7 +933,8 @@ def section_norm(x: torch.Tensor, off: int, n: int, weight: torch.Tensor, eps: f
 
 def latent_encode(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Tensor, eps: float,
                   inv_freq: Optional[torch.Tensor], interleaved: bool, rot_magnitude: float,
-                  positions: torch.Tensor, slots: Optional[torch.Tensor], q_abs: torch.Tensor,
+                  positions: torch.Tensor, slots: Optional[torch.Tensor],
+                  q_abs: Optional[torch.Tensor],
                   cache: Optional[torch.Tensor], heads: int, d: int, dr: int, rank: int,
                   err: torch.Tensor, q: Optional[torch.Tensor] = None) -> None:
     """Attention over a cached latent, before the scores: ``proj`` rows hold ``heads`` query
@@ -941,13 +942,16 @@ def latent_encode(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Ten
     them, a buffer of its own of ``proj``'s type) and ``[rank | dr]`` from ``kv_off``.
     The cache row of a token (pages ``[pages, 1, page_size, rank + dr]``, at ``slots``)
     becomes ``[rmsnorm(first rank) * norm_w | rotated dr]``; ``q_abs [T, heads, rank + dr]``
-    gets every head's rotated part at ``[rank, rank + dr)`` and is otherwise left alone."""
+    gets every head's rotated part at ``[rank, rank + dr)`` and is otherwise left alone.
+    ``q_abs`` None: the rotated parts replace the ones they are made of, in ``q``."""
     T = proj.shape[0]
     _want(norm_w, torch.float32, "norm_w")
-    if proj.stride(1) != 1 or not q_abs.is_contiguous() or q_abs.dtype != proj.dtype:
-        raise KernelError("latent_encode: contiguous rows, q_abs contiguous and of proj's type")
-    if tuple(q_abs.shape) != (T, heads, rank + dr) or norm_w.numel() != rank:
-        raise KernelError("latent_encode: q_abs must be [T, heads, rank + dr], norm_w [rank]")
+    if proj.stride(1) != 1 or norm_w.numel() != rank:
+        raise KernelError("latent_encode: contiguous rows, norm_w [rank]")
+    if q_abs is not None and (not q_abs.is_contiguous() or q_abs.dtype != proj.dtype
+                              or tuple(q_abs.shape) != (T, heads, rank + dr)):
+        raise KernelError("latent_encode: q_abs must be contiguous, [T, heads, rank + dr], of "
+                          "proj's type")
     if q is None:
         q = proj[:, q_off:q_off + heads * (d + dr)]
     if q.dtype != proj.dtype or q.stride(1) != 1 or tuple(q.shape) != (T, heads * (d + dr)):
@@ -958,11 +962,13 @@ def latent_encode(proj: torch.Tensor, q_off: int, kv_off: int, norm_w: torch.Ten
         if not cache.is_contiguous() or cache.shape[1] != 1 or cache.shape[3] != rank + dr:
             raise KernelError("latent_encode: pages must be contiguous [pages, 1, size, rank + dr]")
         page_size, num_slots = cache.shape[2], cache.shape[0] * cache.shape[2]
+    q_out, o_stride, o_pitch, o_off = ((q, q.stride(0), d + dr, d) if q_abs is None else
+                                       (q_abs, q_abs.stride(0), rank + dr, rank))
     _run("latent_encode", lib().bf_latent_encode, _ptr(proj), _c_ll(proj.stride(0)), _ptr(q),
          _c_ll(q.stride(0)), _c_ll(kv_off), _ptr(norm_w), _c_float(eps), _ptr(inv_freq), _c_int(rot_half),
          _c_int(1 if interleaved else 0), _c_float(rot_magnitude), _ptr(positions),
-         _ptr(slots if cache is not None else None), _ptr(q_abs), _ptr(cache), _c_int(T),
-         _c_int(heads), _c_int(d), _c_int(dr), _c_int(rank), _c_int(page_size), _c_ll(num_slots),
+         _ptr(slots if cache is not None else None), _ptr(q_out), _c_ll(o_stride),
+         _c_int(o_pitch), _c_int(o_off), _ptr(cache), _c_int(T), _c_int(heads), _c_int(d), _c_int(dr), _c_int(rank), _c_int(page_size), _c_ll(num_slots),
          _c_int(_dtype_code(proj)), _ptr(err), _stream())
 
 
@@ -1509,7 +1515,8 @@ LATENT_ROWS, LATENT_KEYS = 32, 64
 def latent_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tensor,
                      positions: torch.Tensor, tables: torch.Tensor, out: torch.Tensor, B: int,
                      max_tokens: int, H: int, rank: int, scale: float, err: torch.Tensor,
-                     max_ctx: int = 0, sinks: Optional[torch.Tensor] = None) -> None:
+                     max_ctx: int = 0, sinks: Optional[torch.Tensor] = None,
+                     n_max: int = 0) -> None:
     """Causal softmax attention of query rows ``q [T, H, W]`` (already in the latent's
     coordinates) over a cache of one row ``[latent (rank) | shared key part]`` of ``W`` numbers
     per token, whose first ``rank`` numbers are also the value: ``out [T, H, rank]``, on the
@@ -1518,7 +1525,8 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tensor
     longest context in the batch, if the caller knows it: a step with few rows then shares
     each request's key tiles out over several CTAs whose partial results a second kernel
     makes one.  ``sinks`` (float32 ``[H]``): a learned logit per head in the softmax's
-    denominator."""
+    denominator.  ``n_max`` > 0: requests that bring more tokens are left alone (``max_tokens``
+    counts the others)."""
     W = q.shape[-1]
     if sinks is not None:
         _want(sinks, torch.float32, "sinks")
@@ -1547,6 +1555,57 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tensor
          _ptr(positions), _ptr(tables), _c_int(tables.stride(0)), _ptr(out), _c_int(B),
          _c_int(max_rows), _c_int(H), _c_int(W), _c_int(rank), _c_int(cache.shape[2]),
          _c_int(cache.shape[0]), _c_float(scale), _ptr(part_o), _ptr(part_ml), _c_int(splits),
+         _ptr(sinks), _ptr(err), _c_int(n_max if n_max > 0 else 0x7fffffff // H), _stream())
+
+
+def latent_expand_takes(dtype: torch.dtype, d: int, dr: int, dv: int, rank: int) -> bool:
+    """Whether prompt portions of latent attention may run with keys and values expanded: the
+    sizes that ``latent_attention_prefill`` is built for."""
+    return dtype == torch.bfloat16 and (d, dr, dv) == (128, 64, 128) and rank % 8 == 0
+
+
+def latent_gather(cache: torch.Tensor, tables: torch.Tensor, items: torch.Tensor, n_items: int,
+                  rows: int, rank: int, err: torch.Tensor):
+    """The latents and rotated key parts of every prompt portion's whole context out of the pages,
+    row by row: ``(lat [rows, rank], rot [rows, dr], base int32 [n_items])``.  Portion i's keys
+    begin at row ``base[i]``, a multiple of 64; ``rows``: the contexts' sum, each rounded up to 64
+    (what lies between is zero).  ``items`` int32 ``[n_items, 4]`` of (request, first token row,
+    rows, first position)."""
+    if not cache.is_contiguous() or cache.shape[1] != 1 or cache.dtype != torch.bfloat16:
+        raise KernelError("latent_gather: contiguous bfloat16 pages of one head")
+    W = cache.shape[3]
+    lat = torch.empty((rows, rank), dtype=cache.dtype, device=cache.device)
+    rot = torch.empty((rows, W - rank), dtype=cache.dtype, device=cache.device)
+    base = torch.empty((n_items,), dtype=torch.int32, device=cache.device)
+    _run("latent_gather", lib().bf_latent_gather, _ptr(cache), _ptr(tables),
+         _c_int(tables.stride(0)), _ptr(items), _c_int(n_items), _ptr(lat), _ptr(rot), _ptr(base),
+         _c_int(rows), _c_int(rank), _c_int(W - rank), _c_int(cache.shape[2]),
+         _c_int(cache.shape[0]), _ptr(err), _stream())
+    return lat, rot, base
+
+
+def latent_attention_prefill(q: torch.Tensor, kv: torch.Tensor, rot: torch.Tensor,
+                             base: torch.Tensor, items: torch.Tensor, n_items: int, max_rows: int,
+                             out: torch.Tensor, H: int, scale: float, err: torch.Tensor,
+                             gate: Optional[torch.Tensor] = None,
+                             sinks: Optional[torch.Tensor] = None) -> None:
+    """Latent attention of prompt portions over expanded keys and values (bfloat16, tcgen05): ``q
+    [T, H * 192]`` (128 plain | 64 rotated sizes a head; rows may be a column block), ``kv [rows, H
+    * 256]`` (a head's key, then its value, 128 each) and ``rot``, ``base`` from
+    :func:`latent_gather`.  ``out [T, H * 128]`` (a column block is fine): the portions' rows, times
+    ``sigmoid(gate [T, H])`` if there is one; ``sinks`` float32 ``[H]``."""
+    T = q.shape[0]
+    if (q.dtype != torch.bfloat16 or q.stride(1) != 1 or q.shape[1] != H * 192 or q.stride(0) % 8
+            or q.data_ptr() % 16 or not kv.is_contiguous() or kv.shape[1] != H * 256
+            or rot.shape != (kv.shape[0], 64) or not rot.is_contiguous()
+            or out.stride(1) != 1 or out.stride(0) % 8 or out.data_ptr() % 16
+            or (gate is not None and (gate.stride(1) != 1 or gate.dtype != q.dtype))):
+        raise KernelError("latent_attention_prefill: q [T, H 192], kv [rows, H 256], rot [rows, 64], "
+                          "rows on 16-byte boundaries")
+    _run("latent_attention_prefill", lib().bf_latent_attention_prefill_umma, _ptr(q),
+         _c_ll(q.stride(0)), _ptr(kv), _ptr(rot), _c_ll(kv.shape[0]), _ptr(items), _c_int(n_items),
+         _c_int(max_rows), _c_int(T), _ptr(base), _ptr(out), _c_int(H), _c_float(scale),
+         _c_ll(out.stride(0)), _ptr(gate), _c_ll(gate.stride(0) if gate is not None else 0),
          _ptr(sinks), _ptr(err), _stream())
 
 

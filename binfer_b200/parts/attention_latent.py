@@ -13,8 +13,13 @@ token and no values.  Keys and values are never expanded.  Because ``q_h . (W_uk
 (W_uk,h^T q_h) . c``, each query head's plain part is first carried into latent coordinates
 (a product per head against ``W_uk,h^T``), the attention then runs with one shared key head
 of ``rank + dr`` numbers whose first ``rank`` are also the value, and each head's result, a
-mixture of latents, is expanded by ``W_uv,h`` afterwards.  That is one path for prompt
-portions and single tokens alike, so the logits cannot depend on how a prompt was cut.
+mixture of latents, is expanded by ``W_uv,h`` afterwards.  The float32 engine runs every step so,
+and the logits cannot depend on how a prompt was cut.
+
+In bfloat16, prompt portions long enough to pay for it run expanded: the latents of their whole
+context are gathered from the pages, one product against ``[W_uk,h | W_uv,h]`` of all heads makes
+keys and values of them, and a tcgen05 kernel attends with 192 + 128 multiply-adds per score and
+head instead of ``rank + 64 + rank``.  Single tokens in the same step stay in latent coordinates.
 
 With ``q_rank`` the queries go through a latent of their own: the stacked product yields
 ``W_dq h`` in place of the queries, an RMS norm with a weight follows (float arithmetic), and
@@ -39,6 +44,12 @@ from .linear import linear, linear_heads
 # BINFER_B200_LATENT_TENSOR_CORES=0: the one-warp-per-row kernel also in bfloat16 (the float32
 # path), to tell the two apart when something differs
 TENSOR_CORES = os.environ.get("BINFER_B200_LATENT_TENSOR_CORES", "1") != "0"
+
+
+# BINFER_B200_LATENT_EXPAND=0: prompt portions in latent coordinates too
+EXPAND = os.environ.get("BINFER_B200_LATENT_EXPAND", "1") != "0"
+# most bytes of expanded keys and values a step may take
+EXPAND_MAX_BYTES = 768 << 20
 
 
 class LatentAttention(Mixer, StackedOut):
@@ -69,7 +80,9 @@ class LatentAttention(Mixer, StackedOut):
         self.gate_off = self.q_rows + self.kv_size
         self.out_cols = self.H * self.dv
         self.w_proj = self.w_ukT = self.w_uv = self.w_out = self.norm_w = None
-        self.w_uq = self.q_norm_w = self.sinks = None
+        self.w_uq = self.q_norm_w = self.sinks = self.w_ukv = None
+        self.expands = EXPAND and ops.latent_expand_takes(env.dtype, self.d, self.dr, self.dv,
+                                                          self.rank)
 
     # ----------------------------------------------------------------- weights
     def _spec(self, role: str) -> ParamSpec:
@@ -106,6 +119,10 @@ class LatentAttention(Mixer, StackedOut):
         # [dv, rank] expands a mixture of latents into the head's value
         self.w_ukT = g("uk").view(self.H, self.d, self.rank).transpose(1, 2).contiguous()
         self.w_uv = g("uv").view(self.H, self.dv, self.rank).contiguous()
+        if self.expands:       # per head [W_uk,h ; W_uv,h]: rows of keys, then of values
+            both = torch.cat([g("uk").view(self.H, self.d, self.rank), self.w_uv], dim=1)
+            self.w_ukv = both.reshape(-1, self.rank)
+            self.w_uv = both[:, self.d:]         # (the values' rows are kept once)
         self.w_out = g("o")
         if self.spec.sinks:
             self.sinks = g("sink")
@@ -129,31 +146,80 @@ class LatentAttention(Mixer, StackedOut):
             raise ValueError("latent attention keeps a cache of its own")
         g = view.group
         proj = linear(x, self.w_proj)
-        q_abs = torch.empty((T, H, self.kv_size), dtype=x.dtype, device=x.device)
-        pos = self.position
         if self.q_rank:
             c_q = torch.empty((T, self.q_rank), dtype=x.dtype, device=x.device)
             ops.section_norm(proj, 0, self.q_rank, self.q_norm_w, s.norm_eps, c_q)
             q = linear(c_q, self.w_uq)
         else:
             q = proj[:, :self.q_size]
+        rows = self._expanded_rows(q, out, ctx)
+        cache = view.k_cache
+        if not rows or ctx.n_decode:
+            self._in_latent_coordinates(q, proj, out, ctx, view, n_max=1 if rows else 0)
+            cache = None                     # (stored)
+        if rows:
+            # (a step's single tokens went the other way; their rows of q are not read again)
+            self._encode(proj, q, None, cache, ctx, g)
+            lat, rot, base = ops.latent_gather(view.k_cache, ctx.block_tables[g],
+                                               ctx.prefill_items, ctx.n_prefill, rows, self.rank,
+                                               ctx.err)
+            gate = proj[:, self.gate_off:self.gate_off + H] if s.head_gate else None
+            ops.latent_attention_prefill(q, linear(lat, self.w_ukv), rot, base, ctx.prefill_items,
+                                         ctx.n_prefill, ctx.max_prefill_rows, out, H,
+                                         s.softmax_scale, ctx.err, gate=gate, sinks=self.sinks)
+        return True
+
+    def _expanded_rows(self, q: torch.Tensor, out: torch.Tensor, ctx: StepContext) -> int:
+        """Rows of expanded keys and values (contexts of the step's prompt portions, each rounded up
+        to 64), or 0 where the step stays in latent coordinates.  There a pair of a row and a key
+        that it sees costs about 24 ps a head (1,800 rows behind 500 keys, 16 heads: 964 us); the
+        expansion costs 0.22 ns a head and key and 30 us for its launches, and the pairs then next
+        to nothing (the same rows: 60 us, 16 for gathering and expanding)."""
+        if (not self.expands or not ctx.n_prefill or self.spec.softmax_scale <= 0
+                or q.stride(0) % 8 or q.data_ptr() % 16 or out.stride(0) % 8
+                or out.data_ptr() % 16):
+            return 0
+        rows = pairs = 0
+        for n, c in zip(ctx.q_lens, ctx.ctx_lens_host):
+            if n > 1:
+                rows += -(-c // 64) * 64
+                pairs += n * (c - n) + n * (n + 1) // 2
+        if (self.H * (2.4e-11 * pairs - 2.2e-10 * rows) < 3e-5
+                or rows * self.H * 2 * (self.d + self.dv) > EXPAND_MAX_BYTES):
+            return 0
+        return rows
+
+    def _encode(self, proj, q, q_abs, cache, ctx: StepContext, group) -> None:
+        s, pos = self.spec, self.position
         ops.latent_encode(proj, 0, self.q_rows, self.norm_w, s.norm_eps,
                           pos.inv_freq if pos is not None else None,
                           bool(pos is not None and pos.interleaved),
-                          pos.magnitude if pos is not None else 1.0, ctx.positions, ctx.slots[g],
-                          q_abs, view.k_cache, H, self.d, self.dr, self.rank, ctx.err, q=q)
-        q_heads = q.view(T, H, self.d + self.dr)
+                          pos.magnitude if pos is not None else 1.0, ctx.positions,
+                          ctx.slots[group], q_abs, cache, self.H, self.d, self.dr, self.rank,
+                          ctx.err, q=q)
+
+    def _in_latent_coordinates(self, q, proj, out, ctx: StepContext, view: EntryView,
+                               n_max: int) -> None:
+        """The step's rows (``n_max`` > 0: those of requests with at most so many tokens) with the
+        queries carried into latent coordinates; ``q`` is left as it is."""
+        s, T, H, g = self.spec, q.shape[0], self.H, view.group
+        q_abs = torch.empty((T, H, self.kv_size), dtype=q.dtype, device=q.device)
+        self._encode(proj, q, q_abs, view.k_cache, ctx, g)
+        # (unflatten, not view: without a query latent q is a column block of proj)
+        q_heads = q.unflatten(1, (H, self.d + self.dr))
         linear_heads(q_heads[:, :, :self.d], self.w_ukT, q_abs[:, :, :self.rank])
-        o_lat = torch.empty((T, H, self.rank), dtype=x.dtype, device=x.device)
+        o_lat = torch.empty((T, H, self.rank), dtype=q.dtype, device=q.device)
         if (TENSOR_CORES and s.softmax_scale > 0
-                and ops.latent_attention_takes(x.dtype, self.rank, self.dr)):
+                and ops.latent_attention_takes(q.dtype, self.rank, self.dr)):
             # bfloat16: tiles of (token, head) rows against tiles of cache rows, each fetched
             # once as keys and values, on the tensor cores
+            few = ctx.decode_only or n_max == 1
             ops.latent_attention(q_abs, view.k_cache, ctx.q_start, ctx.positions,
                                  ctx.block_tables[g], o_lat, ctx.B,
-                                 1 if ctx.decode_only else ctx.max_q_len, H, self.rank,
-                                 s.softmax_scale, ctx.err, max_ctx=ctx.max_ctx_len,
-                                 sinks=self.sinks)
+                                 1 if few else ctx.max_q_len, H, self.rank,
+                                 s.softmax_scale, ctx.err,
+                                 max_ctx=ctx.max_decode_ctx if n_max == 1 else ctx.max_ctx_len,
+                                 sinks=self.sinks, n_max=n_max)
         else:
             ops.paged_attention_generic(
                 q_abs.view(T, H * self.kv_size), view.k_cache, view.k_cache, ctx.seq_of_token,
@@ -165,13 +231,12 @@ class LatentAttention(Mixer, StackedOut):
             linear_heads(o_lat, self.w_uv, heads)
             if s.head_gate:
                 ops.head_gate_mul(out, proj[:, self.gate_off:self.gate_off + H], H, self.dv)
-            return True
-        own = torch.empty((T, H, self.dv), dtype=x.dtype, device=x.device)
+            return
+        own = torch.empty((T, H, self.dv), dtype=q.dtype, device=q.device)
         linear_heads(o_lat, self.w_uv, own)
         own = own.view(T, H * self.dv)
         ops.head_gate_mul(own, proj[:, self.gate_off:self.gate_off + H], H, self.dv)
         out.copy_(own)
-        return True
 
 
 register_mixer("latent_attention", LatentAttention)

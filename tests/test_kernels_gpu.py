@@ -1186,3 +1186,119 @@ def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
                 off[c][i] = max(off[c][i], float((have - want).norm() / want.norm()))
     for walk, products in zip(off[False], off[True]):
         assert products <= 1.5 * walk + 2e-7, off
+
+
+# ------------------------------------------- latent attention with keys and values expanded
+# portions below, at and above a key tile of 64, a query tile of 128 and a block of 256, from the
+# start and behind cached keys; the rows of two portions and a single token's row in one buffer
+@pytest.mark.parametrize("portions,H,ps,sinks,gate", [
+    ([(2, 0), (64, 63), (257, 130)], 3, 16, True, True), ([(128, 0), (130, 1)], 2, 8, False, False),
+    ([(300, 500)], 1, 64, True, False), ([(65, 0)], 2, 16, False, True)])
+def test_latent_attention_prefill_expanded(cuda_device, portions, H, ps, sinks, gate):
+    from binfer_b200.csrc import ops
+    torch.manual_seed(len(portions) + H)
+    dev, rank, d, dr, dv = cuda_device, 32, 128, 64, 128
+    ctx = [n + p for n, p in portions]
+    T = 1 + sum(n for n, _ in portions)                  # the first row belongs to nobody here
+    width = max(-(-c // ps) for c in ctx)
+    n_pages = 1 + sum(-(-c // ps) for c in ctx)
+    cache = torch.randn(n_pages, 1, ps, rank + dr, device=dev).to(BF16)
+    order = torch.randperm(n_pages - 1) + 1              # pages anywhere in the pool
+    tables = torch.full((len(ctx), width), -1, dtype=torch.int32)
+    items, at, row = [], 0, 1
+    for i, (n, p) in enumerate(portions):
+        k = -(-ctx[i] // ps)
+        tables[i, :k] = order[at:at + k]
+        at += k
+        items.append((i, row, n, p))
+        row += n
+    tables = tables.to(dev)
+    items_d = torch.tensor(items, dtype=torch.int32, device=dev)
+    rows = sum(-(-c // 64) * 64 for c in ctx)
+    err = _err(dev)
+    lat, rot, base = ops.latent_gather(cache, tables, items_d, len(items), rows, rank, err)
+    w = (torch.randn(H * 256, rank, device=dev) * rank ** -0.5).to(BF16)
+    kv = torch.mm(lat, w.t())
+    wide = torch.randn(T, H * 192 + 8, device=dev).to(BF16)
+    q = wide[:, 8:]                                      # a column block
+    g = torch.randn(T, H + 3, device=dev).to(BF16)[:, 3:] if gate else None
+    sk = torch.randn(H, device=dev) * 2 if sinks else None
+    out = torch.full((T, H * 128 + 8), 7.0, device=dev, dtype=BF16)
+    scale = 192 ** -0.5
+    ops.latent_attention_prefill(q, kv, rot, base, items_d, len(items),
+                                 max(n for n, _ in portions), out[:, 8:], H, scale, err, gate=g,
+                                 sinks=sk)
+    assert int(err.item()) == 0
+    assert bool((out[:1] == 7).all()) and bool((out[:, :8] == 7).all())
+    at = 0
+    for i, (n, p) in enumerate(portions):
+        assert int(base[i]) == at
+        flat = cache[tables[i, :-(-ctx[i] // ps)].long(), 0].reshape(-1, rank + dr)[:ctx[i]]
+        assert torch.equal(lat[at:at + ctx[i]], flat[:, :rank])
+        assert torch.equal(rot[at:at + ctx[i]], flat[:, rank:])
+        pad = -(-ctx[i] // 64) * 64
+        assert float(lat[at + ctx[i]:at + pad].abs().sum() + rot[at + ctx[i]:at + pad].abs().sum()) == 0
+        x = kv[at:at + ctx[i]].double().view(-1, H, 2, 128)
+        k = torch.cat([x[:, :, 0], rot[at:at + ctx[i]].double()[:, None].expand(-1, H, -1)], -1)
+        qq = q[items[i][1]:items[i][1] + n].double().view(n, H, 192)
+        s = torch.einsum("qhd,khd->hqk", qq, k) * scale
+        seen = torch.arange(ctx[i], device=dev)[None] <= torch.arange(p, p + n, device=dev)[:, None]
+        s = s.masked_fill(~seen, -math.inf)
+        if sinks:
+            s = torch.cat([s, sk.double().view(H, 1, 1).expand(H, n, 1)], -1)
+        o = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1)[..., :ctx[i]], x[:, :, 1])
+        if gate:
+            o = o * torch.sigmoid(g[items[i][1]:items[i][1] + n].double())[:, :, None]
+        have = out[items[i][1]:items[i][1] + n, 8:].double().view(n, H, 128)
+        # probabilities and results are rounded to bfloat16 (2^-9 each)
+        assert float((have - o).abs().max()) <= 2.0 ** -7 * float(o.abs().max()), i
+        at += pad
+    bad = tables.clone()
+    bad[0, 0] = n_pages
+    ops.latent_gather(cache, bad, items_d, len(items), rows, rank, err)
+    assert int(err.item()) == 4
+    err.zero_()
+
+
+def test_latent_part_expands_portions_beside_single_tokens(cuda_device, monkeypatch):
+    """A step of two portions and two single tokens, expanded and in latent coordinates."""
+    from binfer_b200.config import FolivikConfig
+    from binfer_b200.engine import StepItem, make_env, make_runner, model_from_seed
+    from binfer_b200.parts import attention_latent
+    cfg = FolivikConfig.from_dict({"vocab": 64, "width": 256, "norm": {"eps": 1e-5}, "layers": [
+        {"type": "latent_attention", "mlp": None, "mixer": {
+            "heads": 2, "dim": 128, "rot_dim": 64, "vdim": 128, "kv_rank": 64, "q_rank": 96,
+            "scale": 192 ** -0.5, "rot": {"base": 1e4, "dims": 64}}}]})
+    env = make_env(BF16)
+    model = model_from_seed(cfg, env, seed=3, std=0.06)
+    runner = make_runner(model, env, page_size=16, num_pages=80, max_requests=4)
+    mixer, view = model.blocks[0].mixer, runner.views[0]
+    torch.manual_seed(5)
+    lens = [(40, 150), (0, 70), (30, 1), (5, 1)]
+
+    def one(expand):
+        rule = (lambda self, q, out, ctx: sum(-(-c // 64) * 64 for n, c in zip(
+            ctx.q_lens, ctx.ctx_lens_host) if n > 1)) if expand else (lambda *a: 0)
+        monkeypatch.setattr(attention_latent.LatentAttention, "_expanded_rows", rule)
+        torch.manual_seed(6)
+        ys = []
+        for i, (b, n) in enumerate(lens):
+            runner.add_request(i)
+            if b:
+                x = torch.randn(b, 256, device=cuda_device).to(BF16)
+                runner.reserve([StepItem(i, [0] * b)])
+                ys.append(mixer.forward(x, runner.build_context([StepItem(i, [0] * b)]), view))
+                runner.cache.commit(i, b)
+        items = [StepItem(i, [0] * n) for i, (_, n) in enumerate(lens)]
+        runner.reserve(items)
+        x = torch.randn(sum(n for _, n in lens), 256, device=cuda_device).to(BF16)
+        ys.append(mixer.forward(x, runner.build_context(items), view))
+        for i in range(len(lens)):
+            runner.free_request(i)
+        runner.check_errors()
+        return torch.cat(ys).double()
+
+    plain, expanded = one(False), one(True)
+    # both round what lies between the products to bfloat16, in other places
+    assert float((plain - expanded).norm() / plain.norm()) <= 1.5e-2
+    assert float((plain - expanded).abs().max()) <= 6e-2 * float(plain.abs().max())
