@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(PWM_THREADS) pwm_attention_kernel(
     int has_sink, float sink_log2, float* __restrict__ part_o, float* __restrict__ part_ml,
     int* __restrict__ err, const float* __restrict__ sinks, int keep_first, long long q_stride,
     long long out_stride, float out_scale, float cap_pre, float cap_post,
-    const float* __restrict__ log_slope, const float* __restrict__ log_rate, float inv_scale) {
+    const float* __restrict__ log_slope, const float* __restrict__ log_rate, float inv_scale,
+    int n_max) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pitch_k = dk + 8, pitch_v = dv + 8;
   // two stages of (K tile, V tile); the first K tile's place holds the Q tile to begin with
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(PWM_THREADS) pwm_attention_kernel(
   const int b = blockIdx.z, g = blockIdx.y;
   const int Gh = nh / nkv;
   const int t0 = q_start[b], n_tok = q_start[b + 1] - t0;
+  if (n_tok > n_max) return;
   const int rows_total = n_tok * Gh;
   // SPLIT with scratch for partial results: blockIdx.x is a share of the key tiles (four of
   // them), not a tile of rows; pwm_merge_kernel makes the shares one
@@ -549,12 +551,13 @@ __global__ void pwm_merge_kernel(
     const float* __restrict__ v_inv_freq, int interleaved, __nv_bfloat16* __restrict__ out,
     int nh, int nkv, int dv, int window, int pool, int has_summary, int has_sink,
     float sink_log2, const float* __restrict__ sinks, int keep_first, long long out_stride,
-    float out_scale) {
+    float out_scale, int n_max) {
   __shared__ float wgt[32][16];                   // share x, row r: exp2(m_x - M) / L
   const int g = blockIdx.x, b = blockIdx.y;
   const int Gh = nh / nkv;
   const int t0 = q_start[b], n_tok = q_start[b + 1] - t0;
   const int rows_total = n_tok * Gh;
+  if (n_tok > n_max) return;
   const int p_first = positions[t0];
   const int p_hi = p_first + (rows_total - 1) / Gh;
   const int nb_hi = (window > 0 && pool > 0 && has_summary && p_hi - window + 1 > 0)
@@ -615,7 +618,8 @@ BF_EXPORT int bf_pwm_attention(
     int s_page_size, int s_num_pages, int window, int pool, float scale, int has_sink,
     float sink, float* part_o, float* part_ml, int shares, int* err, const float* sinks,
     int keep_first, long long q_stride, long long out_stride, float out_scale, float softcap,
-    const float* log_slope, const float* log_rate, cudaStream_t stream) {
+    const float* log_slope, const float* log_rate, int n_max, cudaStream_t stream) {
+  // n_max: requests that bring more tokens are left alone (max_tokens counts the others)
   // log_slope, log_rate [nh] (both or neither): b1_h ln(1 + b2_h (p - j)) is taken off the
   // scaled score of the query at p and the key at j (not with pooled blocks)
   // part_o [B, nkv, shares, 16, dv], part_ml [B, nkv, shares, 16, 2] (float, or null): scratch
@@ -654,14 +658,14 @@ BF_EXPORT int bf_pwm_attention(
       s_num_pages, window, pool, scale * log2e, has_sink, sink * log2e, part_o, part_ml, err,
       sinks, keep_first, q_stride, out_stride, out_scale,
       softcap > 0.f ? 2.f * log2e * scale / softcap : 0.f, softcap > 0.f ? softcap / scale : 0.f,
-      log_slope, log_rate, 1.f / scale);
+      log_slope, log_rate, 1.f / scale, n_max);
   if (multi) {
     const int e = bf_launch_status();
     if (e) return e;
     pwm_merge_kernel<<<dim3(nkv, B), 128, 0, stream>>>(
         part_o, part_ml, shares, q_start, positions, (const __nv_bfloat16*)gate, gate_stride,
         v_inv_freq, interleaved, (__nv_bfloat16*)out, nh, nkv, dv, window, pool,
-        ks_cache != nullptr, has_sink, sink * log2e, sinks, keep_first, out_stride, out_scale);
+        ks_cache != nullptr, has_sink, sink * log2e, sinks, keep_first, out_stride, out_scale, n_max);
   }
   return bf_launch_status();
 }

@@ -50,6 +50,10 @@
 // blocks and Q three halves, which leaves shared memory for three stages.  The epilogue adds a
 // head's sink to its sums and multiplies by the sigmoid of its gate.
 //
+// A window may keep a request's first `keep` tokens visible (the tiles that hold them come first,
+// then the window's), and a head may have a sink, a logit that joins its sums in the epilogue or in
+// the merge.  Kept tokens are a fourth instance (KEEP), whose masks the plain one does without.
+//
 // Every mbarrier wait is bounded.  A barrier whose waiter could fall two phases behind exists
 // once per parity of the tile number, so that its one-bit phase cannot alias: "P V of tile n
 // done" (waited for only when O must be rescaled), and "P of tile n written" (a softmax
@@ -75,7 +79,7 @@ constexpr int A2_THREADS = 608;  // sixteen softmax warps, the TMA warp, two MMA
 constexpr int A2_TMA_WARP = 16;
 constexpr int A2_MMA_WARP = 17;  // 17 issues for query tile A, 18 for tile B
 constexpr int A2_D = 128;
-constexpr int A2_PLAIN = 0, A2_DIFF = 1, A2_LATENT = 2;   // the instances
+constexpr int A2_PLAIN = 0, A2_DIFF = 1, A2_LATENT = 2, A2_KEEP = 3;   // the instances
 constexpr int A2_ROT = 64;       // LATENT: rotated sizes behind the 128 plain ones
 
 // Barrier among the 256 softmax threads of a group (or THREADS of both) that also ANDs a
@@ -108,8 +112,8 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
                                float* __restrict__ part_o, float* __restrict__ part_ml,
                                int* __restrict__ err, float cap_pre, float cap_post,
                                long long out_stride, float out_scale, BfDiffArgs dd,
-                               const float* __restrict__ sinks) {
-  constexpr bool DIFF = MODE == A2_DIFF, LATENT = MODE == A2_LATENT;
+                               const float* __restrict__ sinks, int keep) {
+  constexpr bool DIFF = MODE == A2_DIFF, LATENT = MODE == A2_LATENT, KEEP = MODE == A2_KEEP;
   constexpr int D = A2_D;
   constexpr int HALVES = D / 64;                         // blocks of 64 columns of a V tile
   constexpr int KBLOCKS = LATENT ? HALVES + 1 : HALVES;  // ... of a Q or K tile
@@ -161,8 +165,15 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
   const int p_last = active_b ? min(pos0 + qlen - 1, p_first + BROWS - 1) : p_last_a;
   const int j_lo = window > 0 ? max(0, p_first - window + 1) : 0;
   int kt_first = j_lo / A2_BN;
-  int tiles_a = p_last_a / A2_BN - kt_first + 1;
-  int tiles = p_last / A2_BN - kt_first + 1;
+  // key tiles of the tokens that the window keeps, where they lie before the window's first one
+  // (not together with splits)
+  int n_keep = 0;
+  if constexpr (KEEP) n_keep = min(kt_first, (keep + A2_BN - 1) / A2_BN);
+  int tiles_a = p_last_a / A2_BN - kt_first + 1 + n_keep;
+  int tiles = p_last / A2_BN - kt_first + 1 + n_keep;
+  auto tile_key = [&](int n) {                            // the first key of the n-th tile
+    return (KEEP && n < n_keep ? n : kt_first + n - n_keep) * A2_BN;
+  };
   if (splits > 1) {                                       // this CTA's share of the key tiles
     const int b = tiles * split / splits, e = tiles * (split + 1) / splits;
     kt_first += b;
@@ -250,8 +261,9 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
     bool ok = true;
     for (int nb = 0; nb < tiles && ok && !*abort; nb += tb) {
       const int n_mine = nb + my_i;
-      const int jp = (kt_first + n_mine) * A2_BN + my_pg * page_size;
-      const bool wanted = my_i < tb && n_mine < tiles && jp <= p_last && jp + page_size > j_lo;
+      const int jp = tile_key(n_mine) + my_pg * page_size;
+      const bool wanted = my_i < tb && n_mine < tiles && jp <= p_last &&
+                          (jp + page_size > j_lo || (KEEP && jp < keep));
       int page = 0;
       if (wanted) {
         page = table[jp / page_size];
@@ -276,11 +288,12 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
         uint8_t* vb = Vs + st * V_BYTES;
         // V rows of pages that are not fetched must read as zero (the first tile of a
         // window, the last tile of the portion)
-        const int t_first = (kt_first + n) * A2_BN;
+        const int t_first = tile_key(n);
         if (t_first + page_size <= j_lo || t_first + A2_BN - page_size > p_last) {
           for (int pg = 0; pg < pages; ++pg) {
             const int jq = t_first + pg * page_size;
-            if (jq <= p_last && jq + page_size > j_lo) continue;
+            if (jq <= p_last && (jq + page_size > j_lo || (KEEP && jq < keep)))
+              continue;
             for (int c = lane; c < page_size * 8 * HALVES; c += 32) {
               const int hh = c / (page_size * 8), rem = c - hh * page_size * 8;
               *reinterpret_cast<uint4*>(vb + hh * KHALF_BYTES + pg * page_size * 128 + rem * 16) =
@@ -436,7 +449,8 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
             v[i] = __float_as_uint(cap_post - __fdividef(2.f * cap_post, t + 1.f));
           }
         }
-        const int t_lo = (kt_first + n) * A2_BN + 2 * q4;  // key of this thread's first column
+        const int t_lo = tile_key(n) + 2 * q4;             // key of this thread's first column
+        const int kp = KEEP ? keep - t_lo : 0;             // KEEP: columns below it stay visible
         int hi[2], lo[2];          // last and first visible key, counted from t_lo
         bool need_mask[2];
         float tmax[2];
@@ -451,7 +465,7 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
             for (int c = 0; c < 8; ++c)
 #pragma unroll
               for (int i = 0; i < 2; ++i)
-                if (8 * c + i >= lo[e] && 8 * c + i <= hi[e])
+                if ((8 * c + i >= lo[e] || (KEEP && 8 * c + i < kp)) && 8 * c + i <= hi[e])
                   t2[i] = fmaxf(t2[i], __uint_as_float(v[4 * c + 2 * e + i]));
           } else {
 #pragma unroll
@@ -511,8 +525,8 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
                   DIFF ? row_scale[e] : scale_log2, -m_use);
             float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
             if (need_mask[e]) {
-              if (8 * c < lo[e] || 8 * c > hi[e]) e0 = 0.f;
-              if (8 * c + 1 < lo[e] || 8 * c + 1 > hi[e]) e1 = 0.f;
+              if ((8 * c < lo[e] && !(KEEP && 8 * c < kp)) || 8 * c > hi[e]) e0 = 0.f;
+              if ((8 * c + 1 < lo[e] && !(KEEP && 8 * c + 1 < kp)) || 8 * c + 1 > hi[e]) e1 = 0.f;
             }
             add2f(ts0, ts1, e0, e1);
             __nv_bfloat162 p2 = __floats2bfloat162_rn(e0, e1);
@@ -634,16 +648,14 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
       } else if (ok) {
         tc_fence_after();
         float inv;
+        // (a sink far above the row's scores makes its sum infinite and the result zero)
+        float sum = xl[r];
+        if (sinks) sum += exp2f(fmaf(sinks[h], 1.4426950408889634f, -xr[r]));
+        inv = out_scale / sum;
         if constexpr (LATENT) {
-          // (a sink far above the row's scores makes its sum infinite and the result zero)
-          float sum = xl[r];
-          if (sinks) sum += exp2f(fmaf(sinks[h], 1.4426950408889634f, -xr[r]));
-          inv = out_scale / sum;
           if (dd.gate && valid)
             inv *= bf_sigmoid_fast(__bfloat162float(
                 ((const __nv_bfloat16*)dd.gate)[(size_t)(row0 + l) * dd.gate_stride + h]));
-        } else {
-          inv = out_scale / xl[r];
         }
         __nv_bfloat16* dst = out + (size_t)(row0 + l) * out_stride + (size_t)h * D + half * OH;
 #pragma unroll 1
@@ -694,7 +706,8 @@ __global__ void prefill_attention_merge_kernel(const float* __restrict__ part_o,
                                                const float* __restrict__ part_ml,
                                                const int* __restrict__ items,
                                                __nv_bfloat16* __restrict__ out, int nh, int splits,
-                                               long long out_stride, float out_scale) {
+                                               long long out_stride, float out_scale,
+                                               const float* __restrict__ sinks) {
   const int* it = items + 4 * blockIdx.z;
   const int row0 = it[1], qlen = it[2];
   const int r = blockIdx.x * 4 + (threadIdx.x >> 5), h = blockIdx.y, lane = threadIdx.x & 31;
@@ -715,6 +728,7 @@ __global__ void prefill_attention_merge_kernel(const float* __restrict__ part_o,
     acc.z += o.z * w;
     acc.w += o.w * w;
   }
+  if (sinks) L += exp2f(fmaf(sinks[h], 1.4426950408889634f, -M));
   const float inv = L > 0.f ? out_scale / L : 0.f;
   uint2 packed;
   __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&packed);
@@ -733,15 +747,18 @@ __global__ void prefill_attention_merge_kernel(const float* __restrict__ part_o,
 // divide 64; cudaErrorInvalidValue otherwise (nothing launched).  And: a soft cap c > 0 on the
 // scaled scores, s <- c tanh(s / c) (0: none); the result's rows `out_stride` elements apart
 // (a column block of a wider buffer: a multiple of 8, the block 16-byte aligned) and
-// multiplied by `out_scale`.
+// multiplied by `out_scale`; a logit per head in the softmax's denominator (`sinks`, or null); with a
+// window and one split, the first `keep` tokens that stay visible behind it.
 BF_EXPORT int bf_prefill_attention_umma2_capped(
     const void* q, const void* k_cache, const void* v_cache, const int* items, int n_items,
     int max_rows, int total_rows, const int* block_tables, int table_stride, void* out, int nh,
     int nkv, int d, int page_size, int num_pages, int window, float scale, int splits,
     float* part_o, float* part_ml, int* err, float softcap, long long out_stride,
-    float out_scale, cudaStream_t stream) {
+    float out_scale, const float* sinks, int keep, cudaStream_t stream) {
   if (n_items <= 0 || max_rows <= 0) return 0;
   if (splits < 1 || (splits > 1 && (!part_o || !part_ml))) return (int)cudaErrorInvalidValue;
+  if (window <= 0 || keep < 0) keep = 0;
+  if (keep > 0 && splits > 1) return (int)cudaErrorInvalidValue;
   if (d != A2_D || nkv <= 0 || nh % nkv || page_size < 8 || page_size > A2_BN ||
       A2_BN % page_size || ((uintptr_t)q & 15) || ((uintptr_t)k_cache & 15) ||
       ((uintptr_t)v_cache & 15) || ((uintptr_t)out & 15) || !(scale > 0.f) || softcap < 0.f ||
@@ -768,9 +785,10 @@ BF_EXPORT int bf_prefill_attention_umma2_capped(
   if (e) return e;
   // two Q tiles, the stages of K and V, the row sums, barriers
   const size_t smem = 1024 + (size_t)2 * 32768 + (size_t)2 * A2_STAGES * 16384 + 2048 + 256;
-  auto kern = prefill_attention_umma2_kernel<A2_PLAIN>;
-  static bool configured_on[BF_MAX_DEVICES];
-  bool& configured = configured_on[bf_current_device()];
+  auto kern = keep > 0 ? prefill_attention_umma2_kernel<A2_KEEP>
+                       : prefill_attention_umma2_kernel<A2_PLAIN>;
+  static bool configured_on[BF_MAX_DEVICES][2];
+  bool& configured = configured_on[bf_current_device()][keep > 0];
   if (!configured) {
     cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem);
@@ -783,12 +801,12 @@ BF_EXPORT int bf_prefill_attention_umma2_capped(
                                            (__nv_bfloat16*)out, nh, nkv, page_size, num_pages,
                                            window, scale * log2e, splits, part_o, part_ml, err,
                                            cap_pre, cap_post, out_stride, out_scale,
-                                           BfDiffArgs(), nullptr);
+                                           BfDiffArgs(), sinks, keep);
   if (splits > 1) {
     int st = bf_launch_status();
     if (st) return st;
     prefill_attention_merge_kernel<<<dim3((max_rows + 3) / 4, nh, n_items), 128, 0, stream>>>(
-        part_o, part_ml, items, (__nv_bfloat16*)out, nh, splits, out_stride, out_scale);
+        part_o, part_ml, items, (__nv_bfloat16*)out, nh, splits, out_stride, out_scale, sinks);
   }
   return bf_launch_status();
 }
@@ -803,7 +821,8 @@ BF_EXPORT int bf_prefill_attention_umma2(const void* q, const void* k_cache, con
   return bf_prefill_attention_umma2_capped(q, k_cache, v_cache, items, n_items, max_rows,
                                            total_rows, block_tables, table_stride, out, nh, nkv,
                                            d, page_size, num_pages, window, scale, splits, part_o,
-                                           part_ml, err, 0.f, (long long)nh * A2_D, 1.f, stream);
+                                           part_ml, err, 0.f, (long long)nh * A2_D, 1.f, nullptr, 0,
+                                           stream);
 }
 
 // Differential attention of prompt portions: heads of two maps with 64 key columns each (a cached
@@ -856,7 +875,7 @@ BF_EXPORT int bf_diff_attention_prefill_umma(
   kern<<<grid, A2_THREADS, smem, stream>>>(mq, mk, mv, mkr, mvr, items, block_tables, table_stride,
                                            (__nv_bfloat16*)out, nh, nkv, page_size, num_pages, 0,
                                            scale * 1.4426950408889634f, splits, part_o, part_ml,
-                                           err, 0.f, 0.f, out_stride, 1.f, dd, nullptr);
+                                           err, 0.f, 0.f, out_stride, 1.f, dd, nullptr, 0);
   if (splits > 1) {
     int st = bf_launch_status();
     if (st) return st;
@@ -909,6 +928,6 @@ BF_EXPORT int bf_latent_attention_prefill_umma(
   kern<<<grid, A2_THREADS, smem, stream>>>(mq, mkv, mr, mr, mr, items, kv_base, 0,
                                            (__nv_bfloat16*)out, nh, nh, 1, 1, 0,
                                            scale * 1.4426950408889634f, 1, nullptr, nullptr, err,
-                                           0.f, 0.f, out_stride, 1.f, dd, sinks);
+                                           0.f, 0.f, out_stride, 1.f, dd, sinks, 0);
   return bf_launch_status();
 }

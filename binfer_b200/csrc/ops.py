@@ -464,7 +464,8 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                       block_tables: torch.Tensor, out: torch.Tensor, nh: int, nkv: int, d: int,
                       window: Optional[int], scale: float, err: torch.Tensor,
                       variant: str = "auto", max_ctx: int = 0, splits: int = 0,
-                      softcap: float = 0.0, out_scale: float = 1.0) -> None:
+                      softcap: float = 0.0, out_scale: float = 1.0,
+                      sinks: Optional[torch.Tensor] = None, keep_first: int = 0) -> None:
     """Causal flash attention over the pages for prompt portions (bfloat16 only).
     ``items`` int32 [n, 4]: (request index, first token row, rows, first position).
     ``variant``: ``umma2`` (tcgen05 tensor cores, one CTA per SM with two query tiles sharing a
@@ -477,7 +478,9 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     kernel, whose partial results a second kernel merges (``splits`` forces a number).
 
     ``softcap`` c > 0: the scaled scores pass ``c tanh(s / c)``; ``out_scale``: a factor on
-    the result; ``out`` may then also be a column block of a wider buffer.  These three are
+    the result; ``out`` may then also be a column block of a wider buffer; ``sinks`` float32
+    ``[nh]``: a learned logit per head in the softmax's denominator; ``keep_first``: with a
+    window, the request's first that many tokens stay visible behind it.  These five are
     the umma2 variant's alone (``prefill_attention_takes_capped``)."""
     global _launches
     if q.dtype != torch.bfloat16 or d not in DECODE_HEAD_DIMS:
@@ -498,18 +501,25 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     blocks2 = -(-max_rows // 256) * nh * n_items
     use2 = umma2_ok and (variant == "umma2" or (variant == "auto" and (
         blocks2 >= 120 or max_rows > 256 or max_ctx >= 2048)))
-    capped = softcap > 0 or out_scale != 1.0 or not out.is_contiguous()
+    keep_first = int(keep_first) if window else 0
+    capped = (softcap > 0 or out_scale != 1.0 or not out.is_contiguous() or sinks is not None
+              or keep_first > 0)
     fn2, tail2 = lib().bf_prefill_attention_umma2, ()
     if capped:
         if not umma2_ok or variant not in ("auto", "umma2"):
-            raise KernelError("prefill_attention: a soft cap, an output factor or an output in a "
-                              "column block are the umma2 variant's alone")
+            raise KernelError("prefill_attention: a soft cap, an output factor, sinks, kept tokens or "
+                              "an output in a column block are the umma2 variant's alone")
+        if sinks is not None:
+            _want(sinks, torch.float32, "sinks")
+            if sinks.numel() != nh:
+                raise KernelError("prefill_attention: sinks must have one entry per query head")
         if out.stride(1) != 1 or out.stride(0) % 8 or out.data_ptr() % 16 or out.dtype != q.dtype:
             raise KernelError("prefill_attention: out must have contiguous rows a multiple of 8 "
                               "elements apart, 16-byte aligned")
         use2 = True
         fn2 = lib().bf_prefill_attention_umma2_capped
-        tail2 = (_c_float(softcap), _c_ll(out.stride(0)), _c_float(out_scale))
+        tail2 = (_c_float(softcap), _c_ll(out.stride(0)), _c_float(out_scale), _ptr(sinks),
+                 _c_int(keep_first))
     # Few blocks and long contexts: share the keys of each block out (at least 16 key tiles a
     # share, at most 8 shares, no more CTAs than SMs).
     if splits <= 0:
@@ -1439,7 +1449,7 @@ def pwm_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                   err: torch.Tensor, max_ctx: int = 0, sinks: Optional[torch.Tensor] = None,
                   keep_first: int = 0, out_scale: float = 1.0, softcap: float = 0.0,
                   log_slope: Optional[torch.Tensor] = None,
-                  log_rate: Optional[torch.Tensor] = None) -> None:
+                  log_rate: Optional[torch.Tensor] = None, n_max: int = 0) -> None:
     """``apw_attention`` on the tensor cores (bfloat16; sizes: ``pwm_attention_takes``):
     request ``b`` of the batch owns the token rows ``q_start[b] .. q_start[b+1]-1``, at most
     ``max_tokens`` of them.  ``max_ctx``: the longest context in the batch, if the caller
@@ -1451,7 +1461,8 @@ def pwm_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
     buffer; ``out_scale`` multiplies the result.  ``softcap`` c > 0: a scaled score z becomes
     ``c tanh(z / c)``.  ``log_slope`` and ``log_rate`` (float32 ``[nh]`` each, together or not
     at all; not with pooled blocks): ``log_slope_h ln(1 + log_rate_h (p - j))`` is taken off
-    the scaled score of the query at p and the key at j."""
+    the scaled score of the query at p and the key at j.  ``n_max`` > 0: requests that bring more
+    tokens are left alone (``max_tokens`` counts the others)."""
     if (log_slope is None) != (log_rate is None) or (log_slope is not None
                                                      and ks_cache is not None):
         raise KernelError("pwm_attention: log_slope and log_rate go together, without pooled "
@@ -1499,7 +1510,7 @@ def pwm_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
          _c_int(0 if sink is None and sinks is None else 1), _c_float(sink or 0.0),
          _ptr(part_o), _ptr(part_ml), _c_int(shares), _ptr(err), _ptr(sinks), _c_int(keep_first),
          _c_ll(q.stride(0)), _c_ll(out.stride(0)), _c_float(out_scale), _c_float(softcap),
-         _ptr(log_slope), _ptr(log_rate), _stream())
+         _ptr(log_slope), _ptr(log_rate), _c_int(n_max if n_max > 0 else 0x7fffffff), _stream())
 
 
 def latent_attention_takes(dtype: torch.dtype, rank: int, rot: int) -> bool:

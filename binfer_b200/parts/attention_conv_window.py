@@ -216,28 +216,34 @@ class ConvWindowAttention(Mixer, StackedOut):
                                  self.dk, None, s.softmax_scale, ctx.max_ctx_len, ctx.err,
                                  variant="persistent", softcap=s.softcap, out_scale=out_scale)
             return
-        if (DECODE_KERNEL and not biased and not ctx.decode_only and ctx.n_decode == 0 and ctx.n_prefill
-                and ctx.max_prefill_rows >= PREFILL_KERNEL_ROWS and s.window is None
-                and self.sinks is None and s.softmax_scale > 0 and out.stride(0) % 8 == 0
+        rows_left = 0                    # n_max of what runs behind; 0: every request
+        if (DECODE_KERNEL and not biased and not ctx.decode_only and ctx.n_prefill
+                and ctx.max_prefill_rows >= PREFILL_KERNEL_ROWS
+                and s.softmax_scale > 0 and out.stride(0) % 8 == 0
                 and out.data_ptr() % 16 == 0
                 and ops.prefill_attention_takes_capped(q, view.k_cache, self.dk, self.dv)):
-            # bfloat16 steps of prompt portions alone, heads of 128: the engine's tcgen05
-            # prefill kernel, which takes the soft cap and writes into the branch's columns
+            # bfloat16 prompt portions, heads of 128: the engine's tcgen05 prefill kernel, which
+            # takes the soft cap, the window with its kept tokens and the sinks, and writes into
+            # the branch's columns
             ops.prefill_attention(q, view.k_cache, view.v_cache, ctx.prefill_items,
                                   ctx.n_prefill, ctx.max_prefill_rows, ctx.block_tables[g], out,
-                                  self.H, self.G, self.dk, None, s.softmax_scale, ctx.err,
+                                  self.H, self.G, self.dk, s.window, s.softmax_scale, ctx.err,
                                   variant="umma2", max_ctx=ctx.max_ctx_len, softcap=s.softcap,
-                                  out_scale=out_scale)
-            return
+                                  out_scale=out_scale, sinks=self.sinks, keep_first=keep)
+            if not ctx.n_decode:
+                return
+            rows_left = 1                # the step's single tokens
         if (TENSOR_CORES and s.softmax_scale > 0
                 and ops.pwm_attention_takes(proj.dtype, self.H, self.G, self.dk, self.dv)):
             # bfloat16: tiles of (token, head of a group) rows on the tensor cores, prompt
             # portions and single tokens alike (the windowed kernel, without pooled blocks)
             ops.pwm_attention(q, view.k_cache, view.v_cache, None, None, ctx.q_start,
                               ctx.positions, ctx.block_tables[g], None, None, None, False, out,
-                              ctx.B, 1 if ctx.decode_only else ctx.max_q_len, self.H, self.G,
+                              ctx.B, 1 if ctx.decode_only or rows_left else ctx.max_q_len,
+                              self.H, self.G,
                               self.dk, self.dv, s.window, 0, s.softmax_scale, None, ctx.err,
-                              max_ctx=ctx.max_ctx_len, sinks=self.sinks, keep_first=keep,
+                              max_ctx=ctx.max_decode_ctx if rows_left else ctx.max_ctx_len,
+                              sinks=self.sinks, keep_first=keep, n_max=rows_left,
                               out_scale=out_scale, softcap=s.softcap, log_slope=self.bias_slope,
                               log_rate=self.bias_rate)
             return

@@ -179,6 +179,8 @@ class LatentAttention(Mixer, StackedOut):
                 or q.stride(0) % 8 or q.data_ptr() % 16 or out.stride(0) % 8
                 or out.data_ptr() % 16):
             return 0
+        if self.H * 2.4e-11 * q.shape[0] * ctx.max_ctx_len < 3e-5:
+            return 0
         rows = pairs = 0
         for n, c in zip(ctx.q_lens, ctx.ctx_lens_host):
             if n > 1:
@@ -205,8 +207,7 @@ class LatentAttention(Mixer, StackedOut):
         s, T, H, g = self.spec, q.shape[0], self.H, view.group
         q_abs = torch.empty((T, H, self.kv_size), dtype=q.dtype, device=q.device)
         self._encode(proj, q, q_abs, view.k_cache, ctx, g)
-        # (unflatten, not view: without a query latent q is a column block of proj)
-        q_heads = q.unflatten(1, (H, self.d + self.dr))
+        q_heads = q.view(T, H, self.d + self.dr)
         linear_heads(q_heads[:, :, :self.d], self.w_ukT, q_abs[:, :, :self.rank])
         o_lat = torch.empty((T, H, self.rank), dtype=q.dtype, device=q.device)
         if (TENSOR_CORES and s.softmax_scale > 0

@@ -1302,3 +1302,55 @@ def test_latent_part_expands_portions_beside_single_tokens(cuda_device, monkeypa
     # both round what lies between the products to bfloat16, in other places
     assert float((plain - expanded).norm() / plain.norm()) <= 1.5e-2
     assert float((plain - expanded).abs().max()) <= 6e-2 * float(plain.abs().max())
+
+
+# a window of one token, below, at and above a key tile and wider than some portions; kept tokens
+# inside a tile, a whole tile, more than a tile and more than lies before the window; portions with
+# cached keys; sinks alone with the keys shared out
+@pytest.mark.parametrize("nh,nkv,ps,window,keep,sinks,splits", [
+    (4, 2, 16, 64, 4, True, 1), (2, 2, 8, 1, 64, False, 1), (6, 2, 64, 200, 100, True, 1),
+    (2, 1, 16, 90, 0, True, 1), (2, 1, 16, None, 0, True, 3)])
+def test_prefill_attention_kept_tokens_and_sinks(cuda_device, nh, nkv, ps, window, keep, sinks,
+                                                 splits):
+    from binfer_b200.csrc import ops
+    dev, d, gen = cuda_device, 128, torch.Generator().manual_seed(nh + ps + keep)
+    ctxs, qlens = [300, 70, 700, 2, 257], [300, 37, 260, 2, 129]
+    kcs, vcs, tables, qs, refs, items, base, row = [], [], [], [], [], [], 0, 0
+    sk = torch.randn(nh, generator=gen) * 2 if sinks else None
+    for b, (n, ql) in enumerate(zip(ctxs, qlens)):
+        k = torch.randn(n, nkv, d, generator=gen).to(BF16).double()
+        v = torch.randn(n, nkv, d, generator=gen).to(BF16).double()
+        q = torch.randn(ql, nh, d, generator=gen).to(BF16).double()
+        kh, vh = (x.repeat_interleave(nh // nkv, dim=1) for x in (k, v))
+        sc = torch.einsum("qhd,nhd->hqn", q, kh) * d ** -0.5
+        j, p = torch.arange(n)[None, :], (n - ql + torch.arange(ql))[:, None]
+        seen = j <= p
+        if window:
+            seen = seen & ((p - j < window) | (j < keep))
+        sc = sc.masked_fill(~seen[None], float("-inf"))
+        if sinks:
+            sc = torch.cat([sc, sk.double().view(nh, 1, 1).expand(nh, ql, 1)], -1)
+        refs.append(torch.einsum("hqn,nhd->qhd", torch.softmax(sc, dim=-1)[..., :n], vh))
+        kc, vc, ids = _paged(k, v, ps, "cpu", BF16, 70 + b, False)
+        kcs.append(kc)
+        vcs.append(vc)
+        ids = [i + base for i in ids]
+        if window:                       # pages that no query sees have been given back
+            first = max(0, n - ql - window + 1) // ps
+            ids = [i if x < -(-keep // ps) or x >= first else -1 for x, i in enumerate(ids)]
+        tables.append(ids)
+        base += kc.shape[0]
+        qs.append(q)
+        items.append([b, row, ql, n - ql])
+        row += ql
+    bt = torch.full((len(ctxs), max(len(t) for t in tables)), -1, dtype=torch.int32)
+    for b, t in enumerate(tables):
+        bt[b, :len(t)] = torch.tensor(t, dtype=torch.int32)
+    q = torch.cat(qs).reshape(row, nh * d).to(BF16).to(dev)
+    out, err = torch.zeros_like(q), _err(dev)
+    ops.prefill_attention(q, torch.cat(kcs).to(dev), torch.cat(vcs).to(dev),
+                          torch.tensor(items, dtype=torch.int32, device=dev), len(items), max(qlens),
+                          bt.to(dev), out, nh, nkv, d, window, d ** -0.5, err, variant="umma2",
+                          splits=splits, sinks=sk.to(dev) if sinks else None, keep_first=keep)
+    assert int(err.item()) == 0
+    _close(out.cpu(), torch.cat(refs).reshape(row, nh * d), BF16)
