@@ -368,6 +368,31 @@ DECODE_HEAD_DIMS = (32, 64, 96, 128, 256)
 DECODE_SPLIT_KEYS = 128
 
 
+def attention_f32_takes(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                        d: int) -> bool:
+    """Whether :func:`attention_f32` takes these sizes and addresses."""
+    return (q.dtype == torch.float32 and d in (64, 128) and q.is_contiguous()
+            and k_cache.is_contiguous() and v_cache.is_contiguous()
+            and v_cache.shape[3] == k_cache.shape[3] == d
+            and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0)
+
+
+def attention_f32(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                  q_start: torch.Tensor, positions: torch.Tensor, tables: torch.Tensor,
+                  out: torch.Tensor, B: int, max_q: int, nh: int, nkv: int, d: int,
+                  window: Optional[int], scale: float, err: torch.Tensor) -> None:
+    """Causal grouped attention of float32 rows ``q [T, nh * d]`` over the pages, in tiles of rows
+    against tiles of keys; a row's result depends on its own position only.  Request ``b`` owns the
+    token rows ``q_start[b] .. q_start[b+1]-1``, at most ``max_q`` of them."""
+    if (not attention_f32_takes(q, k_cache, v_cache, d) or not out.is_contiguous()
+            or out.dtype != q.dtype or out.data_ptr() % 16):
+        raise KernelError("attention_f32: contiguous float32 on 16-byte boundaries, heads of 64 or 128")
+    _run("attention_f32", lib().bf_attention_f32, _ptr(q), _ptr(k_cache), _ptr(v_cache),
+         _ptr(q_start), _ptr(positions), _ptr(tables), _c_int(tables.stride(0)), _ptr(out),
+         _c_int(B), _c_int(max_q), _c_int(nh), _c_int(nkv), _c_int(d), _c_int(k_cache.shape[2]),
+         _c_int(k_cache.shape[0]), _c_int(window or 0), _c_float(scale), _ptr(err), _stream())
+
+
 def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                      rows: Optional[torch.Tensor], n_rows: int, seq_of_token: torch.Tensor,
                      positions: torch.Tensor, block_tables: torch.Tensor, out: torch.Tensor,

@@ -180,7 +180,8 @@ class GQAAttention(Mixer):
                view: EntryView) -> None:
         """Attention of every token row over its request's pages.
 
-        float32: the generic kernel, whose sums have one fixed order per position.
+        float32: heads of 64 and 128 with plain scores on tiles of rows and keys, the rest on the
+        generic kernel; in both every sum has one fixed order per position.
         bfloat16: rows that bring a single token go to the split-KV decode kernel;
         the rest (and head sizes the tuned kernels do not take) to the generic one.
         """
@@ -188,6 +189,12 @@ class GQAAttention(Mixer):
         tables = ctx.block_tables[view.group]
         fast = (q.dtype == torch.bfloat16 and s.head_dim in ops.DECODE_HEAD_DIMS
                 and s.score is None)
+        if (s.score is None and s.softmax_scale > 0
+                and ops.attention_f32_takes(q, view.k_cache, view.v_cache, s.head_dim)):
+            ops.attention_f32(q, view.k_cache, view.v_cache, ctx.q_start, ctx.positions, tables,
+                              out, ctx.B, 1 if ctx.decode_only else ctx.max_q_len, s.num_heads,
+                              s.num_kv_heads, s.head_dim, s.window, s.softmax_scale, ctx.err)
+            return
         if not fast:
             ops.paged_attention_generic(
                 q, view.k_cache, view.v_cache, ctx.seq_of_token, ctx.positions, tables, out,

@@ -1354,3 +1354,36 @@ def test_prefill_attention_kept_tokens_and_sinks(cuda_device, nh, nkv, ps, windo
                           splits=splits, sinks=sk.to(dev) if sinks else None, keep_first=keep)
     assert int(err.item()) == 0
     _close(out.cpu(), torch.cat(refs).reshape(row, nh * d), BF16)
+
+
+# ----------------------------------------------------------------- float32 attention in tiles
+# rows below, at and above a tile of 64 and of 4, portions from the start and behind cached keys, a
+# window inside, at and above a key tile
+@pytest.mark.parametrize("nh,nkv,d,ps,window", [(4, 2, 128, 16, None), (3, 1, 64, 8, 64),
+                                                (2, 2, 128, 64, 50), (8, 1, 64, 16, 200)])
+def test_attention_f32_tiles(cuda_device, nh, nkv, d, ps, window):
+    from binfer_b200.csrc import ops
+    ctxs, qlens = [70, 200, 129, 300, 64, 1, 193], [70, 37, 5, 130, 64, 1, 1]
+    q, kc, vc, sot, pos, bt, ref = _attention_case(cuda_device, F32, nh, nkv, d, ps, ctxs, qlens,
+                                                   window, False, seed=21)
+    qs = torch.tensor([0] + list(torch.tensor(qlens).cumsum(0)), dtype=torch.int32,
+                      device=cuda_device)
+    out, err = torch.full_like(q, 7.0), _err(cuda_device)
+    ops.attention_f32(q, kc, vc, qs, pos, bt, out, len(ctxs), max(qlens), nh, nkv, d, window,
+                      d ** -0.5, err)
+    assert int(err.item()) == 0
+    _close(out, ref, F32)
+    # a row's bits do not depend on what shares its step: the last rows of every request alone
+    # (tiles of four rows), each with its own table
+    last = qs[1:].long() - 1
+    one = torch.full((len(ctxs), nh * d), 7.0, device=cuda_device)
+    each = torch.arange(len(ctxs) + 1, dtype=torch.int32, device=cuda_device)
+    ops.attention_f32(q[last].contiguous(), kc, vc, each, pos[last].contiguous(), bt, one,
+                      len(ctxs), 1, nh, nkv, d, window, d ** -0.5, err)
+    assert torch.equal(one, out[last])
+    bad = bt.clone()
+    bad[0, 0] = kc.shape[0]
+    ops.attention_f32(q, kc, vc, qs, pos, bad, out, len(ctxs), max(qlens), nh, nkv, d, window,
+                      d ** -0.5, err)
+    assert int(err.item()) == 4
+    err.zero_()
