@@ -19,12 +19,16 @@
 // them there.  bf_conv_state_shift, launched after the encode kernel, moves the step's last
 // rows into the state.
 //
-// One warp per (token, head); heads are counted q heads, then k heads, then v heads.  The
+// One warp per (token, head); heads are counted q heads, then k heads, then v heads.  Keys and values
+// of one size of 16, 32, 64 or 128 with at most four taps: four channels a thread over a run of tokens
+// instead, a head in d / 4 neighbouring lanes, its rotation and its sum of squares by shuffles
+// (conv_encode_run_kernel; 2,118 tokens of 16 + 8 + 8 heads of 128, 3 taps: 32 us, 55 on the other).  The
 // cosines and sines of a token's angles are taken once for all its heads, by a small kernel
 // in front.  All
 // arithmetic is float; only the projection's values and the stored results have the
 // activation type.
 #include "common.cuh"
+#include "conv_taps.cuh"
 
 #define CE_MAX_TAPS 16
 
@@ -186,6 +190,96 @@ __global__ void conv_encode_kernel(
   }
 }
 
+template <typename A, int TAPS>
+__global__ void __launch_bounds__(128) conv_encode_run_kernel(
+    const A* __restrict__ proj, long long stride, const float* __restrict__ conv_w,
+    const float* __restrict__ state, long long state_stride, const int* __restrict__ state_slots,
+    int n_state_slots, const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
+    const float2* __restrict__ rope, int rot_half, const int* __restrict__ slots,
+    A* __restrict__ q_out, long long q_stride, A* __restrict__ k_cache, A* __restrict__ v_cache,
+    int T, int nh, int nkv, int d, int page_size, long long num_slots, int unit_norm, float eps,
+    int run, int* __restrict__ err, const float* __restrict__ pre_factor,
+    const float* __restrict__ pre_weight, const float* __restrict__ head_w,
+    const float* __restrict__ q_head_scale, const float* __restrict__ proj_bias) {
+  // (TAPS 0: no convolution; C / 4 is a multiple of 32, so that warps are whole)
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
+  const int C = (nh + 2 * nkv) * d;
+  if (c >= C) return;
+  const int ta = blockIdx.y * run, tb = min(T, ta + run);
+  const int lanes = d / 4, lane = threadIdx.x & 31, li = lane % lanes, i = li * 4;
+  const int hs = c / d;
+  const int kind = hs < nh ? 0 : hs < nh + nkv ? 1 : 2;
+  const int head = kind == 0 ? hs : kind == 1 ? hs - nh : hs - nh - nkv;
+  const int r4 = rot_half / 4;
+  const bool turn = kind < 2 && li < 2 * r4;
+  const int other = li < 2 * r4 ? lane - li + (li < r4 ? li + r4 : li - r4) : lane;
+  float4 add = make_float4(0.f, 0.f, 0.f, 0.f), pw = add, hw = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (TAPS == 0 && proj_bias)
+    add = make_float4(proj_bias[c], proj_bias[c + 1], proj_bias[c + 2], proj_bias[c + 3]);
+  if (pre_factor && kind < 2)
+    pw = make_float4(pre_weight[c], pre_weight[c + 1], pre_weight[c + 2], pre_weight[c + 3]);
+  if (head_w && kind < 2) {
+    const float* p = head_w + kind * d + i;
+    hw = make_float4(p[0], p[1], p[2], p[3]);
+  }
+  const float q_scale = kind == 0 && q_head_scale ? q_head_scale[head] : 1.f;
+  ConvTaps<(TAPS > 0 ? TAPS : 1)> conv;
+  if (TAPS > 0) conv.weights(conv_w, c);
+  for (int t = ta; t < tb; ++t) {
+    const A* row = proj + (size_t)t * stride;
+    float4 y;
+    if (TAPS > 0) {
+      const ConvPlace at = ct_place(t, seq_of_token, q_start, state_slots, n_state_slots, state,
+                                    state_stride, TAPS, err);
+      if (t == ta || at.local == 0) conv.history(row, stride, c, at.local, at.st, C);
+      y = conv.step(make_float4(0.f, 0.f, 0.f, 0.f), ct_ld4(row + c));
+    } else {
+      y = ct_ld4(row + c);
+      y = make_float4(y.x + add.x, y.y + add.y, y.z + add.z, y.w + add.w);
+    }
+    if (pre_factor && kind < 2) {                // the norm over the whole projection
+      const float f = pre_factor[(size_t)t * 2 + kind];
+      y = make_float4(y.x * (f * pw.x), y.y * (f * pw.y), y.z * (f * pw.z), y.w * (f * pw.w));
+    }
+    if (rot_half > 0) {
+      const float4 o = make_float4(__shfl_sync(0xffffffffu, y.x, other),
+                                   __shfl_sync(0xffffffffu, y.y, other),
+                                   __shfl_sync(0xffffffffu, y.z, other),
+                                   __shfl_sync(0xffffffffu, y.w, other));
+      if (turn) {
+        const float4* cs = reinterpret_cast<const float4*>(
+            rope + (size_t)t * rot_half + (li < r4 ? i : i - rot_half));
+        const float4 a = cs[0], b = cs[1];       // (cos, sin) twice each
+        if (li < r4)
+          y = make_float4(y.x * a.x - o.x * a.y, y.y * a.z - o.y * a.w, y.z * b.x - o.z * b.y,
+                          y.w * b.z - o.w * b.w);
+        else
+          y = make_float4(y.x * a.x + o.x * a.y, y.y * a.z + o.y * a.w, y.z * b.x + o.z * b.y,
+                          y.w * b.z + o.w * b.w);
+      }
+    }
+    float f = 1.f;
+    if (unit_norm) {
+      float ss = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
+      for (int o = 1; o < lanes; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (kind < 2) f = rsqrtf(ss / (float)d + eps);
+    }
+    f *= q_scale;
+    y = make_float4(y.x * hw.x * f, y.y * hw.y * f, y.z * hw.z * f, y.w * hw.w * f);
+    if (kind == 0) {
+      ct_st4(q_out + (size_t)t * q_stride + (size_t)head * d + i, y);
+    } else if (k_cache) {
+      const long long s = slots[t];
+      if (s < 0 || s >= num_slots) {
+        if (li == 0) atomicOr(err, BF_ERR_SLOT);
+      } else {
+        const long long page = s / page_size, off = s - page * page_size;
+        ct_st4((kind == 1 ? k_cache : v_cache) + ((page * nkv + head) * page_size + off) * d + i, y);
+      }
+    }
+  }
+}
+
 BF_EXPORT int bf_conv_encode(
     const void* proj, long long stride, const float* conv_w, int taps, const float* state,
     long long state_stride, const int* state_slots, int n_state_slots, const int* seq_of_token,
@@ -215,6 +309,34 @@ BF_EXPORT int bf_conv_encode(
                     ((uintptr_t)proj % (2 * esz)) == 0 && ((uintptr_t)q_out % (2 * esz)) == 0 &&
                     ((uintptr_t)k_cache % (2 * esz)) == 0 && ((uintptr_t)v_cache % (2 * esz)) == 0 &&
                     ((uintptr_t)state % 8) == 0) ? 1 : 0;
+  // four channels a thread over runs of tokens (the choice does not depend on the tokens' number)
+  const long long C = ((long long)nh + 2 * nkv) * dk;
+  const uintptr_t quad = 4 * esz - 1;
+  if (dk == dv && (dk == 16 || dk == 32 || dk == 64 || dk == 128) && C % 128 == 0 && taps <= 4 &&
+      rot_half % 4 == 0 && stride % 4 == 0 && q_stride % 4 == 0 &&
+      (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & quad) == 0 &&
+      ((uintptr_t)rope_table & 15) == 0 && T <= 65535 * 8) {
+    const int units = (int)(C / 4), run = T > 65535 ? 8 : ct_run(T, units);
+    const dim3 grid((units + 127) / 128, (T + run - 1) / run);
+#define CE_RUN(A, K)                                                                              \
+  conv_encode_run_kernel<A, K><<<grid, 128, 0, stream>>>(                                         \
+      (const A*)proj, stride, conv_w, state, state_stride, state_slots, n_state_slots,            \
+      seq_of_token, q_start, (const float2*)rope_table, rot_half, slots, (A*)q_out, q_stride,     \
+      (A*)k_cache, (A*)v_cache, T, nh, nkv, dk, page_size, num_slots, unit_norm, eps, run, err,   \
+      pre_factor, pre_weight, head_w, q_head_scale, proj_bias)
+#define CE_TAPS(A)                                                                                \
+  {                                                                                               \
+    if (!conv_w) CE_RUN(A, 0);                                                                    \
+    else if (taps == 1) CE_RUN(A, 1);                                                             \
+    else if (taps == 2) CE_RUN(A, 2);                                                             \
+    else if (taps == 3) CE_RUN(A, 3);                                                             \
+    else CE_RUN(A, 4);                                                                            \
+  }
+    if (act_dtype == BF_DTYPE_F32) CE_TAPS(float) else CE_TAPS(__nv_bfloat16)
+#undef CE_TAPS
+#undef CE_RUN
+    return bf_launch_status();
+  }
   const int warps = 4;
   // many tokens: a warp walks four heads of its token (one round of lookups), else one
   const int hpw = (long long)T * (nh + 2 * nkv) >= 16 * 148 * 16 ? 4 : 1;

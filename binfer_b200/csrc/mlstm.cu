@@ -16,13 +16,16 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "norm_out.cuh"
 
 // ----------------------------------------------------------------------------- gates
 // gates[t, r] for r < heads:  cap tanh((w_r . h_t + b_r) / cap)          (log input gate)
 //             for r >= heads: logsigmoid(cap tanh((w_r . h_t + b_r) / cap))  (log forget gate)
-// One warp per (token, gate row); cap <= 0 means no cap.  (A warp that takes eight rows of a
-// token, so as to read the token's input once, measured five times slower at 2,048 tokens and
-// sixteen times slower at 8: too few warps, each a long chain.)
+// cap <= 0 means no cap.  mlstm_gates_kernel: one warp per (token, gate row), any sizes (2,048 tokens
+// of 4,096 x 16 rows: 53 us, the input read sixteen times over; 44 on the other).  mlstm_gates_tile_kernel, widths that
+// are a multiple of 4: a block takes TB tokens and sixteen rows at a time, its eight warps share the
+// width out, a lane multiplies pieces of four of every token with pieces of four of every row, and
+// the lanes' and warps' sums are added in one order.  A token's sums do not depend on the others.
 template <typename A>
 __global__ void mlstm_gates_kernel(const A* __restrict__ h, long long h_stride,
                                    const A* __restrict__ w, const float* __restrict__ bias,
@@ -45,10 +48,88 @@ __global__ void mlstm_gates_kernel(const A* __restrict__ h, long long h_stride,
   }
 }
 
+#define MG_ROWS 16
+template <typename A, int TB>
+__global__ void __launch_bounds__(256) mlstm_gates_tile_kernel(
+    const A* __restrict__ h, long long h_stride, const A* __restrict__ w,
+    const float* __restrict__ bias, float* __restrict__ gates, int T, int width, int heads,
+    float cap) {
+  __shared__ float part[8][TB * MG_ROWS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * TB, r0 = blockIdx.y * MG_ROWS;
+  const int n_gates = 2 * heads;
+  const int rows = min(MG_ROWS, n_gates - r0), nt = min(TB, T - t0);
+  float acc[TB][MG_ROWS];
+#pragma unroll
+  for (int k = 0; k < TB; ++k)
+#pragma unroll
+    for (int r = 0; r < MG_ROWS; ++r) acc[k][r] = 0.f;
+  for (int c = (warp * 32 + lane) * 4; c < width; c += 1024) {
+    float4 x[TB];
+#pragma unroll
+    for (int k = 0; k < TB; ++k)
+      x[k] = k < nt ? ct_ld4(h + (size_t)(t0 + k) * h_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < MG_ROWS; ++r) {
+      if (r < rows) {
+        const float4 p = ct_ld4(w + (size_t)(r0 + r) * width + c);
+#pragma unroll
+        for (int k = 0; k < TB; ++k) {
+          acc[k][r] = fmaf(x[k].x, p.x, acc[k][r]);
+          acc[k][r] = fmaf(x[k].y, p.y, acc[k][r]);
+          acc[k][r] = fmaf(x[k].z, p.z, acc[k][r]);
+          acc[k][r] = fmaf(x[k].w, p.w, acc[k][r]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < TB; ++k)
+#pragma unroll
+    for (int r = 0; r < MG_ROWS; ++r) {
+      const float s = warp_sum(acc[k][r]);
+      if (lane == 0) part[warp][k * MG_ROWS + r] = s;
+    }
+  __syncthreads();
+  const int k = threadIdx.x / MG_ROWS, r = threadIdx.x % MG_ROWS;
+  if (k >= nt || r >= rows) return;
+  float z = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) z += part[i][k * MG_ROWS + r];
+  const int row = r0 + r;
+  z += bias ? bias[row] : 0.f;
+  if (cap > 0.f) z = cap * tanhf(z / cap);
+  if (row >= heads) z = fminf(z, 0.f) - log1pf(expf(-fabsf(z)));
+  gates[(size_t)(t0 + k) * n_gates + row] = z;
+}
+
+template <typename A>
+static void mlstm_gates_tiles(const A* h, long long h_stride, const A* w, const float* bias,
+                              float* gates, int T, int width, int heads, float cap,
+                              cudaStream_t stream) {
+  const int rt = (2 * heads + MG_ROWS - 1) / MG_ROWS;
+  if (T >= 4 * 148)
+    mlstm_gates_tile_kernel<A, 4><<<dim3((T + 3) / 4, rt), 256, 0, stream>>>(
+        h, h_stride, w, bias, gates, T, width, heads, cap);
+  else
+    mlstm_gates_tile_kernel<A, 1><<<dim3(T, rt), 256, 0, stream>>>(h, h_stride, w, bias, gates, T,
+                                                                   width, heads, cap);
+}
+
 BF_EXPORT int bf_mlstm_gates(const void* h, long long h_stride, const void* w, const float* bias,
                              float* gates, int T, int width, int heads, float cap, int act_dtype,
                              cudaStream_t stream) {
   if (T <= 0) return 0;
+  const uintptr_t a = (act_dtype == BF_DTYPE_F32 ? 16 : 8) - 1;
+  if (width % 4 == 0 && h_stride % 4 == 0 && (((uintptr_t)h | (uintptr_t)w) & a) == 0) {
+    if (act_dtype == BF_DTYPE_F32)
+      mlstm_gates_tiles<float>((const float*)h, h_stride, (const float*)w, bias, gates, T, width,
+                               heads, cap, stream);
+    else
+      mlstm_gates_tiles<__nv_bfloat16>((const __nv_bfloat16*)h, h_stride, (const __nv_bfloat16*)w,
+                                       bias, gates, T, width, heads, cap, stream);
+    return bf_launch_status();
+  }
   const long long warps = (long long)T * 2 * heads;
   const int threads = 128;
   const long long blocks = (warps * 32 + threads - 1) / threads;
@@ -497,6 +578,14 @@ BF_EXPORT int bf_mlstm_out(const float* o_raw, const void* proj, long long strid
                            long long g_off, const float* norm_w, void* out, int T, int H, int dv,
                            float eps, int act_dtype, cudaStream_t stream) {
   if (T <= 0) return 0;
+  const long long row = (long long)H * dv;
+  if (act_dtype == BF_DTYPE_F32
+          ? norm_out_vec<float>(o_raw, (const float*)proj, stride, g_off, norm_w, dv, 1,
+                                (float*)out, row, T, H, dv, eps, 1.f, stream)
+          : norm_out_vec<__nv_bfloat16>(o_raw, (const __nv_bfloat16*)proj, stride, g_off, norm_w,
+                                        dv, 1, (__nv_bfloat16*)out, row, T, H, dv, eps, 1.f,
+                                        stream))
+    return bf_launch_status();
   const int threads = 128;
   const long long blocks = ((long long)T * H * 32 + threads - 1) / threads;
   if (act_dtype == BF_DTYPE_F32)

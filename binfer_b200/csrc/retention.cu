@@ -36,6 +36,7 @@
 // retention_out: each head's output divided by its root mean square (no weight), times
 // silu of the gate projection, times out_scale, into a column block of `out`.
 #include "common.cuh"
+#include "norm_out.cuh"
 
 #define RET_CHUNK 16        // tokens whose partial sums a lane holds at a time
 #define RET_STAGE 64        // tokens staged in shared memory at a time (fewer for large heads)
@@ -450,6 +451,13 @@ BF_EXPORT int bf_retention_out(const float* o_raw, const void* proj, long long s
                                int dv, float eps, float out_scale, int act_dtype,
                                cudaStream_t stream) {
   if (T <= 0) return 0;
+  if (act_dtype == BF_DTYPE_F32
+          ? norm_out_vec<float>(o_raw, (const float*)proj, stride, g_off, nullptr, 0, 0,
+                                (float*)out, out_stride, T, H, dv, eps, out_scale, stream)
+          : norm_out_vec<__nv_bfloat16>(o_raw, (const __nv_bfloat16*)proj, stride, g_off, nullptr,
+                                        0, 0, (__nv_bfloat16*)out, out_stride, T, H, dv, eps,
+                                        out_scale, stream))
+    return bf_launch_status();
   const int threads = 128;
   const long long blocks = ((long long)T * H * 32 + threads - 1) / threads;
   if (act_dtype == BF_DTYPE_F32)

@@ -1387,3 +1387,122 @@ def test_attention_f32_tiles(cuda_device, nh, nkv, d, ps, window):
                       d ** -0.5, err)
     assert int(err.item()) == 4
     err.zero_()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("lens", [[1], [3, 1, 9, 2, 17], [1] * 5, [700, 1, 1, 643]])
+def test_convolved_inputs_in_runs(cuda_device, lens, taps, dtype):
+    """The encoders behind a short convolution, on rows of whole pieces of four (a thread takes a run
+    of tokens) and on rows that are not (a warp per token): both against float64.  A sum of at most
+    five products and a root mean square of 32 numbers keep float results within some 10 roundings;
+    bfloat16 outputs are rounded once."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(len(lens) * 8 + taps)
+    dev, T, B = cuda_device, sum(lens), len(lens)
+    H, G, d, nh, nkv = 4, 2, 32, 4, 2
+    C = (2 * G + H) * d                        # the same channels for all three encoders
+    wide = torch.randn(T, C + 2 * H + 4, device=dev).to(dtype)
+    odd = torch.empty(T, wide.shape[1] + 1, dtype=dtype, device=dev)[:, :-1]
+    odd.copy_(wide)
+    w, bias = torch.randn(C, taps, device=dev), torch.randn(C, device=dev)
+    state = torch.randn(B + 1, max(1, (taps - 1) * C), device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev).flip(0).contiguous()
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).int().to(dev)
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    pos = torch.arange(T, dtype=torch.int32, device=dev)
+    A_log, dt_bias, D = (torch.randn(H, device=dev) for _ in range(3))
+    conv = torch.empty(T, C, dtype=torch.float64, device=dev)
+    for b in range(B):
+        a, e = int(qs[b]), int(qs[b + 1])
+        u = torch.cat([state[int(slots[b])].double()[:(taps - 1) * C].view(taps - 1, C),
+                       wide[a:e, :C].double()])
+        conv[a:e] = sum(w[:, j].double() * u[j:j + e - a] for j in range(taps))
+    softplus, silu = torch.nn.functional.softplus, torch.nn.functional.silu
+    err, st = _err(dev), state if taps > 1 else None
+    dt = softplus(wide[:, C:C + H].double() + dt_bias.double())
+    pages, freqs = (T + 15) // 16, 1.0 / 10.0 ** (torch.arange(8, device=dev) / 8.0)
+    for proj in (wide, odd):
+        # the state space layer's
+        qk, decay = torch.empty(T, 2, G, d, device=dev), torch.empty(T, H, device=dev)
+        vf, skip = torch.empty(T, H, d, device=dev), torch.empty(T, H, d, device=dev)
+        ops.mamba2_encode(proj, 0, C, w, bias, taps, st, slots, seq, qs, A_log, dt_bias, D, qk, vf,
+                          skip, decay, H, G, d, d, err)
+        y = silu(conv + bias.double())
+        x = y[:, :H * d].view(T, H, d)
+        _close(vf, x * dt[..., None], F32)
+        _close(skip, x * D.double()[:, None], F32)
+        _close(decay, torch.exp(-A_log.double().exp() * dt), F32)
+        _close(qk[:, 1], y[:, H * d:H * d + G * d].view(T, G, d), F32)
+        _close(qk[:, 0], y[:, H * d + G * d:].view(T, G, d), F32)
+        # the delta rule's
+        qkv, gates = torch.empty(T, C, device=dev), torch.empty(T, 2, H, device=dev)
+        ops.delta_encode(proj, w, taps, st, slots, seq, qs, C + H, C, A_log, dt_bias, qkv, gates, H,
+                         G, d, d, 1e-6, 0.25, err)
+        y = silu(conv)
+        q, k = y[:, :G * d].view(T, G, d), y[:, G * d:2 * G * d].view(T, G, d)
+        unit = lambda z: z * torch.rsqrt((z * z).sum(-1, keepdim=True) + 1e-6)
+        _close(qkv, torch.cat([unit(q).reshape(T, -1) * 0.25, unit(k).reshape(T, -1),
+                               y[:, 2 * G * d:]], 1), F32, scale=4)
+        _close(gates[:, 0], torch.sigmoid(wide[:, C + H:C + 2 * H].double()), F32)
+        _close(gates[:, 1], torch.exp(-A_log.double().exp() * dt), F32)
+        # attention's: heads of 32, 16 of them turned, divided by their root mean square
+        q_out = torch.empty(T, nh * d, dtype=dtype, device=dev)
+        kc = torch.zeros(pages, nkv, 16, d, dtype=dtype, device=dev)
+        vc = torch.zeros_like(kc)
+        ops.conv_encode(proj[:, :C], w, taps, st, slots, seq, qs, freqs, pos, pos, q_out, kc, vc, nh,
+                        nkv, d, d, True, 1e-5, err)
+        y = conv.view(T, nh + 2 * nkv, d).clone()
+        ang = pos.double()[:, None, None] * freqs.double()
+        lo, hi = y[:, :nh + nkv, :8].clone(), y[:, :nh + nkv, 8:16].clone()
+        y[:, :nh + nkv, :8] = lo * ang.cos() - hi * ang.sin()
+        y[:, :nh + nkv, 8:16] = hi * ang.cos() + lo * ang.sin()
+        z = y[:, :nh + nkv]
+        z = z * torch.rsqrt((z * z).mean(-1, keepdim=True) + 1e-5)
+        flat = lambda c: c.transpose(1, 2).reshape(pages * 16, nkv, d)[:T]
+        # (angles up to 1,343 in float: 2^-24 of the angle, beside the roundings)
+        tol = 40 if dtype == F32 else 1
+        _close(q_out.view(T, nh, d), z[:, :nh], dtype, scale=tol)
+        _close(flat(kc), z[:, nh:], dtype, scale=tol)
+        _close(flat(vc), y[:, nh + nkv:], dtype)
+    assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("T,width,heads", [(1, 100, 1), (7, 2052, 8), (593, 1028, 9), (2, 50, 3)])
+def test_mlstm_gates_tiles(cuda_device, T, width, heads, dtype):
+    """Tiles of one and of four tokens, their remainders, and a width for the kernel of any size."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(T + width)
+    h = torch.randn(T, width, device=cuda_device).to(dtype)
+    w = (0.1 * torch.randn(2 * heads, width, device=cuda_device)).to(dtype)
+    bias = torch.randn(2 * heads, device=cuda_device)
+    gates = torch.empty(T, 2 * heads, device=cuda_device)
+    ops.mlstm_gates(h, w, bias, gates, heads, 15.0)
+    z = 15.0 * torch.tanh((h.double() @ w.double().T + bias.double()) / 15.0)
+    z[:, heads:] = torch.nn.functional.logsigmoid(z[:, heads:])
+    _close(gates, z, F32)
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("dv", [128, 256, 512, 1024, 96])
+def test_head_norm_out_in_registers(cuda_device, dv, dtype):
+    """The sizes whose numbers stay in registers and one that does not, rows of odd offsets too."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(dv)
+    T, H, dev = 5, 3, cuda_device
+    o, skip = torch.randn(T, H * dv, device=dev), torch.randn(T, H * dv, device=dev)
+    w = torch.randn(H * dv, device=dev)
+    proj = torch.randn(T, H * dv + 12, device=dev).to(dtype)
+    for off in (8, 7):
+        g = torch.nn.functional.silu(proj[:, off:off + H * dv].double()).view(T, H, dv)
+        sg = torch.sigmoid(proj[:, off:off + H * dv].double()).view(T, H, dv)
+        rms = lambda x: x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+        x, wd = o.double().view(T, H, dv), w.double().view(H, dv)
+        out = torch.empty(T, H * dv, dtype=dtype, device=dev)
+        ops.gate_norm_out(o, skip, proj, off, w, out, H, 1e-5)
+        _close(out.view(T, H, dv), rms((x + skip.double().view(T, H, dv)) * g) * wd, dtype)
+        ops.mlstm_out(o, proj, off, w, out, H, dv, 1e-5)
+        _close(out.view(T, H, dv), rms(x) * wd * sg, dtype)
+        ops.retention_out(o, proj, off, out, H, dv, 1e-5)
+        _close(out.view(T, H, dv), rms(x) * g, dtype)
