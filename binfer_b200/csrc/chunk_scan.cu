@@ -31,6 +31,21 @@
 // reach what the float32 product of sgemm_f32.cu reaches.  They are built like it: 64 x 64 outputs
 // a CTA, 16 terms a step fetched a step ahead, packed multiply-adds of row pairs.
 //
+// The gated delta rule, S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, is the same with u in
+// v's place, and the u of a chunk hang together: with F counted from the chunk's start and S0 the state
+// before it,  (I + L) U = beta (V - e^F K S0),  L_ts = beta_t exp(F_t - F_s) (k_t . k_s) below the
+// diagonal.  So with T = (I + L)^-1:
+//
+//   ds_prep    per chunk and head: L, T (by blocks of 16), W = T (beta e^F K) and Y = T (beta V)
+//   ds_walk    from chunk to chunk: U = Y - W S, S <- exp(F_C) S + K^T (exp(F_C - F) U); leaves U and
+//              the states between chunks.  The only chain: two products a chunk, over (request, head,
+//              32 columns) in parallel
+//   cs_out     as above, on U
+//
+// 1,111 and 694 tokens of 16 heads of 128: 240 us (ds_walk 115, ds_prep 53, cs_out 47, cs_qk 13) against
+// the walk's 366; 2,048 tokens of 32 heads 430 against 730.  Error against 64 bits: o 9.5e-8 (walk
+// 7.3e-8), state 7.6e-8 (7.8e-8).
+//
 // Requests of at most `n_min` tokens have no chunks here (the walk serves them).  The order of sums
 // depends on where a step's portions begin, so the float32 engine, whose results must not depend
 // on the cut, does not use these kernels.
@@ -160,7 +175,7 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
     const float* __restrict__ gates, float* __restrict__ state, long long slot_stride,
     int state_size, const int* __restrict__ q_start, const int* __restrict__ state_slots,
     int n_slots, double* __restrict__ G, double* __restrict__ Hs, float* __restrict__ E,
-    double* __restrict__ g0, int T, int H, int dkdv, int dk, int n_min) {
+    double* __restrict__ g0, int T, int H, int dkdv, int dk, int n_min, int decay_stride) {
   __shared__ double sh[CS_GATE_THREADS / 32];
   const int h = blockIdx.x, b = blockIdx.y;
   const int t0 = q_start[b], n = q_start[b + 1] - t0;
@@ -174,7 +189,7 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
   const double fixed = MLSTM || tok_decay ? 0.0 : cs_log_decay(decays[h]);
   auto log_decay = [&](int t) -> double {
     if (MLSTM) return (double)gates[(size_t)(t0 + t) * 2 * H + H + h];
-    return tok_decay ? cs_log_decay(tok_decay[(size_t)(t0 + t) * H + h]) : fixed;
+    return tok_decay ? cs_log_decay(tok_decay[(size_t)(t0 + t) * decay_stride + h]) : fixed;
   };
   double F = 0.0;
   for (int t = a; t < e; ++t) {
@@ -271,7 +286,7 @@ struct CsIn {
 // grid (chunks, QH, row tiles x column tiles): qkm[chunk][qh][C][C], the tiles at and below the
 // diagonal
 template <typename A>
-__global__ void __launch_bounds__(CS_THREADS) cs_qk_kernel(
+__global__ void __launch_bounds__(CS_THREADS, 4) cs_qk_kernel(
     const A* __restrict__ qk, CsIn p, const int* __restrict__ q_start, float* __restrict__ qkm) {
   __shared__ __align__(16) float As[2][CS_K][CS_P], Bs[2][CS_K][CS_P];
   const int tiles = p.C / CS_T;
@@ -334,7 +349,7 @@ __global__ void __launch_bounds__(CS_THREADS) cs_qk_kernel(
 // grid (chunks, H, row tiles x column tiles).  U[chunk][h]: linear [dv][dk], mLSTM [dk][dv] (each
 // like its state); mLSTM: Un[chunk][h][dk] by the CTAs of the first column tile.
 template <typename A, typename V, bool MLSTM>
-__global__ void __launch_bounds__(CS_THREADS) cs_state_kernel(
+__global__ void __launch_bounds__(CS_THREADS, 4) cs_state_kernel(
     const A* __restrict__ qk, const V* __restrict__ vsrc, CsIn p, const int* __restrict__ q_start,
     const double* __restrict__ G, const double* __restrict__ Hs, float* __restrict__ U,
     float* __restrict__ Un) {
@@ -479,8 +494,9 @@ __global__ void __launch_bounds__(128) cs_prefix_kernel(
 
 // ---------------------------------------------------------------------------------- cs_out
 // grid (chunks, H, row tiles x column tiles of dv)
-template <typename A, typename V, bool MLSTM>
-__global__ void __launch_bounds__(CS_THREADS) cs_out_kernel(
+// KROWS: a chunk's state lies as [dk][dv] (the mLSTM's, and what ds_walk leaves), else [dv][dk]
+template <typename A, typename V, bool MLSTM, bool KROWS>
+__global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
     const A* __restrict__ qk, const V* __restrict__ vsrc, CsIn p, const int* __restrict__ q_start,
     const int* __restrict__ state_slots, int n_slots, const double* __restrict__ G,
     const double* __restrict__ Hs, const double* __restrict__ g0, const float* __restrict__ E,
@@ -534,7 +550,7 @@ __global__ void __launch_bounds__(CS_THREADS) cs_out_kernel(
         const int idx = tid + x * CS_THREADS, r = idx >> 2, kk = k0 + (idx & 3) * 4;
         fa[x] = r0 + r < n && kk < p.dk ? cs_ld4(q + (size_t)(r0 + r) * p.qk_stride + kk)
                                         : cs_zero();
-        if (MLSTM) {                           // S [dk][dv]: rows of terms
+        if (KROWS) {                           // S [dk][dv]: rows of terms
           const int kr = k0 + (idx >> 4), j = c0 + (idx & 15) * 4;
           fb[x] = kr < p.dk && j < p.dv ? cs_ld4(S + (size_t)kr * p.dv + j) : cs_zero();
         } else {                               // S [dv][dk]: rows with the terms side by side
@@ -565,7 +581,7 @@ __global__ void __launch_bounds__(CS_THREADS) cs_out_kernel(
       for (int x = 0; x < 2; ++x) {
         const int idx = tid + x * CS_THREADS;
         cs_put_turned(As[buf], idx, cs_times(fa[x], at_s[idx >> 2]));
-        if (MLSTM) cs_put(Bs[buf], idx, fb[x]);
+        if (KROWS) cs_put(Bs[buf], idx, fb[x]);
         else cs_put_turned(Bs[buf], idx, fb[x]);
       }
     } else {
@@ -633,6 +649,353 @@ __global__ void __launch_bounds__(CS_THREADS) cs_out_kernel(
   }
 }
 
+// ------------------------------------------------------------------- the gated delta rule
+#define DS_C 64            // tokens a chunk
+#define DS_D 128           // most key and value sizes
+#define DS_P (DS_D + 4)
+#define DS_NS 32           // columns of the state a CTA of ds_walk keeps
+#define DS_PREP_THREADS 256
+
+struct DsIn {
+  const float* qkv;        // [T][C]: q (G heads of dk), k, v (H heads of dv)
+  const float* gates;      // [T][2][H]: beta, decay
+  long long stride;        // C
+  int H, G, dk, dv, T, B, n_min;
+};
+
+__device__ __forceinline__ void ds_cp16(float* smem, const float* gmem, bool ok) {
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem),
+               "r"(ok ? 16 : 0));
+}
+
+// grid (chunks, H): W [chunk][H][64][dk], Y [chunk][H][64][dv]
+__global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
+    DsIn p, const int* __restrict__ q_start, const double* __restrict__ F, float* __restrict__ W,
+    float* __restrict__ Y) {
+  extern __shared__ __align__(16) float ds_smem[];
+  float* Ks = ds_smem;                           // [64][DS_P]
+  float* Vs = Ks + DS_C * DS_P;                  // [64][DS_P]
+  float* Ls = Vs + DS_C * DS_P;                  // [64][68]
+  float* Ts = Ls + DS_C * 68;                    // [64][68]
+  float* Rs = Ts + DS_C * 68;                    // [16][52]
+  __shared__ double fs[DS_C];
+  __shared__ float beta[DS_C], grow[DS_C];       // grow: beta e^F
+  const CsChunk c = cs_find(q_start, p.B, DS_C, p.n_min, blockIdx.x, -1);
+  if (c.b < 0) return;
+  const int at = c.index * DS_C, n = min(DS_C, c.n - at);
+  const int h = blockIdx.y, hq = h / (p.H / p.G);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const float* k = p.qkv + (size_t)(c.t0 + at) * p.stride + (size_t)(p.G + hq) * p.dk;
+  const float* v = p.qkv + (size_t)(c.t0 + at) * p.stride + 2 * (size_t)p.G * p.dk + (size_t)h * p.dv;
+  for (int i = tid; i < DS_C * (DS_D / 4); i += DS_PREP_THREADS) {
+    const int r = i / (DS_D / 4), e = i % (DS_D / 4) * 4;
+    const bool ok_k = r < n && e < p.dk, ok_v = r < n && e < p.dv;
+    ds_cp16(Ks + r * DS_P + e, ok_k ? k + (size_t)r * p.stride + e : p.qkv, ok_k);
+    ds_cp16(Vs + r * DS_P + e, ok_v ? v + (size_t)r * p.stride + e : p.qkv, ok_v);
+  }
+  asm volatile("cp.async.commit_group;" ::);
+  const double* f = F + (size_t)h * p.T + c.t0 + at;
+  const double f0 = c.index ? f[-1] : 0.0;
+  if (tid < DS_C) {
+    fs[tid] = tid < n ? f[tid] - f0 : 0.0;
+    beta[tid] = tid < n ? p.gates[(size_t)(c.t0 + at + tid) * 2 * p.H + h] : 0.f;
+    grow[tid] = beta[tid] * expf((float)fs[tid]);
+  }
+  asm volatile("cp.async.wait_group 0;" ::);
+  __syncthreads();
+  // L: thread (tx, ty) has rows 4 ty .. and columns tx + 16 j; even and odd sizes in the two halves
+  {
+    unsigned long long s2[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
+#pragma unroll 2
+    for (int d = 0; d < DS_D; d += 4) {
+      if (d >= p.dk) break;
+      ulonglong2 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        a[i] = *reinterpret_cast<const ulonglong2*>(Ks + (ty * 4 + i) * DS_P + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        b[j] = *reinterpret_cast<const ulonglong2*>(Ks + (tx + 16 * j) * DS_P + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s2[i][j] = cs_fma2(a[i].x, b[j].x, s2[i][j]);
+          s2[i][j] = cs_fma2(a[i].y, b[j].y, s2[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = ty * 4 + i, s = tx + 16 * j;
+        float lo, hi;
+        cs_unpair(s2[i][j], lo, hi);
+        Ls[t * 68 + s] = s < t && t < n ? beta[t] * expf((float)(fs[t] - fs[s])) * (lo + hi) : 0.f;
+      }
+  }
+  __syncthreads();
+  // T = (I + L)^-1 by blocks of 16: the diagonal blocks, a thread a column ...
+  for (int i = tid; i < DS_C * 68; i += DS_PREP_THREADS) Ts[i] = 0.f;
+  __syncthreads();
+  if (tid < DS_C) {
+    const int o = tid & ~15, j = tid & 15;
+    float col[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      float r = t == j ? 1.f : 0.f;
+#pragma unroll
+      for (int s = 0; s < t; ++s) r = fmaf(-Ls[(o + t) * 68 + o + s], col[s], r);
+      col[t] = r;
+      Ts[(o + t) * 68 + o + j] = r;
+    }
+  }
+  __syncthreads();
+  // ... then block row by block row: T_i* = -T_ii (sum_k L_ik T_k*)
+  for (int i = 1; i < 4; ++i) {
+    const int cols = 16 * i;
+    for (int e = tid; e < 16 * cols; e += DS_PREP_THREADS) {
+      const int r = e / cols, j = e % cols;
+      float a0 = 0.f, a1 = 0.f;
+      for (int s = j & ~15; s < cols; s += 2) {
+        a0 = fmaf(Ls[(16 * i + r) * 68 + s], Ts[s * 68 + j], a0);
+        a1 = fmaf(Ls[(16 * i + r) * 68 + s + 1], Ts[(s + 1) * 68 + j], a1);
+      }
+      Rs[r * 52 + j] = a0 + a1;
+    }
+    __syncthreads();
+    for (int e = tid; e < 16 * cols; e += DS_PREP_THREADS) {
+      const int r = e / cols, j = e % cols;
+      float a = 0.f;
+#pragma unroll
+      for (int s = 0; s < 16; ++s) a = fmaf(Ts[(16 * i + r) * 68 + 16 * i + s], Rs[s * 52 + j], a);
+      Ts[(16 * i + r) * 68 + j] = -a;
+    }
+    __syncthreads();
+  }
+  // W = T (beta e^F K), Y = T (beta V): rows 4 ty .., columns 4 tx + 64 j
+#pragma unroll 1
+  for (int what = 0; what < 2; ++what) {
+    const float* B = what ? Vs : Ks;
+    const float* sc = what ? beta : grow;
+    const int width = what ? p.dv : p.dk;
+    unsigned long long acc[4][2][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0ull;
+    for (int s = 0; s < ty * 4 + 4; s += 4) {    // (T is zero above the diagonal)
+      float4 tr[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        tr[i] = *reinterpret_cast<const float4*>(Ts + (ty * 4 + i) * 68 + s);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float fsc = sc[s + x];
+        ulonglong2 b[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          b[j] = *reinterpret_cast<const ulonglong2*>(B + (s + x) * DS_P + 4 * tx + 64 * j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float w = (x == 0 ? tr[i].x : x == 1 ? tr[i].y : x == 2 ? tr[i].z : tr[i].w) * fsc;
+          const unsigned long long w2 = cs_pair(w, w);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            acc[i][j][0] = cs_fma2(w2, b[j].x, acc[i][j][0]);
+            acc[i][j][1] = cs_fma2(w2, b[j].y, acc[i][j][1]);
+          }
+        }
+      }
+    }
+    float* dst = (what ? Y : W) + ((size_t)blockIdx.x * p.H + h) * DS_C * width;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int col = 4 * tx + 64 * j;
+        if (col >= width) continue;
+        float4 r;
+        cs_unpair(acc[i][j][0], r.x, r.y);
+        cs_unpair(acc[i][j][1], r.z, r.w);
+        *reinterpret_cast<float4*>(dst + (size_t)(ty * 4 + i) * width + col) = r;
+      }
+  }
+}
+
+// grid (column slices of 32, H, B): u [T][H][dv], Sc [chunk][H][dk][dv] (the state before each chunk).
+// 128 threads with 4 x 4 outputs of U and 8 x 4 of the state each: what a thread reads from shared
+// memory (at 128 bytes a cycle and SM) is about what its multiply-adds take.  1,111 and 694 tokens of
+// 16 heads of 128: 115 us; 256 threads with half of that 130, and the state's columns in the lanes'
+// registers, W and K read by all lanes alike, 133.
+__global__ void __launch_bounds__(128) ds_walk_kernel(
+    DsIn p, const int* __restrict__ q_start, const int* __restrict__ state_slots, int n_slots,
+    float* __restrict__ state, long long slot_stride, const double* __restrict__ F,
+    const float* __restrict__ W, const float* __restrict__ Y, float* __restrict__ u,
+    float* __restrict__ Sc, int* __restrict__ err) {
+  extern __shared__ __align__(16) float ds_smem[];
+  constexpr int PS = DS_NS + 4;
+  float* Ws = ds_smem;                           // [2][64][DS_P]
+  float* Ks = Ws + 2 * DS_C * DS_P;              // [2][64][DS_P]
+  float* Ss = Ks + 2 * DS_C * DS_P;              // [DS_D][PS]
+  float* Us = Ss + DS_D * PS;                    // [64][PS]: exp(F_C - F_s) u_s
+  const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * DS_NS;
+  const CsChunk c = cs_find(q_start, p.B, DS_C, p.n_min, 0, b);
+  if (c.n <= p.n_min) return;
+  const int slot = state_slots[b];
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;   // 8 x 16
+  if (slot < 0 || slot >= n_slots) {
+    if (tid == 0) atomicOr(err, BF_ERR_SLOT);
+    return;
+  }
+  const int hq = h / (p.H / p.G);
+  float* st = state + (size_t)slot * slot_stride + (size_t)h * p.dv * p.dk;
+  const float* k = p.qkv + (size_t)c.t0 * p.stride + (size_t)(p.G + hq) * p.dk;
+  const double* f = F + (size_t)h * p.T + c.t0;
+  const int chunks = (c.n + DS_C - 1) / DS_C;
+  auto load = [&](int i, int buf) {
+    const int n = min(DS_C, c.n - i * DS_C);
+    const float* w = W + ((size_t)(c.first + i) * p.H + h) * DS_C * p.dk;
+    for (int e = tid; e < DS_C * (DS_D / 4); e += 128) {
+      const int r = e / (DS_D / 4), d = e % (DS_D / 4) * 4;
+      const bool ok = d < p.dk, ok_k = ok && r < n;
+      ds_cp16(Ws + (buf * DS_C + r) * DS_P + d, ok ? w + (size_t)r * p.dk + d : W, ok);
+      ds_cp16(Ks + (buf * DS_C + r) * DS_P + d,
+              ok_k ? k + (size_t)(i * DS_C + r) * p.stride + d : p.qkv, ok_k);
+    }
+    asm volatile("cp.async.commit_group;" ::);
+  };
+  load(0, 0);
+  for (int e = tid; e < DS_D * DS_NS; e += 128) {
+    const int kk = e % DS_D, j = e / DS_D;
+    Ss[kk * PS + j] = kk < p.dk && col0 + j < p.dv ? st[(size_t)(col0 + j) * p.dk + kk] : 0.f;
+  }
+  // this thread's state: rows 8 ty .. 8 ty + 7 (four pairs), columns 4 tx ..; U: rows 4 ty ..
+  const int col = col0 + 4 * tx;
+  double before = 0.0;
+  for (int i = 0; i < chunks; ++i) {
+    const int n = min(DS_C, c.n - i * DS_C);
+    const float* Wt = Ws + (i & 1) * DS_C * DS_P;
+    const float* Kt = Ks + (i & 1) * DS_C * DS_P;
+    const double last = f[i * DS_C + n - 1];
+    asm volatile("cp.async.wait_group 0;" ::);
+    __syncthreads();                             // the chunk and the state are here
+    if (i + 1 < chunks) load(i + 1, (i + 1) & 1);
+    const size_t chunk = (size_t)(c.first + i) * p.H + h;
+    float4 y[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      y[r] = col < p.dv ? *reinterpret_cast<const float4*>(
+                              Y + (chunk * DS_C + ty * 4 + r) * p.dv + col)
+                        : cs_zero();
+    // the state before the chunk, for cs_out
+    if (col < p.dv) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (ty * 8 + r < p.dk)
+          *reinterpret_cast<float4*>(Sc + (chunk * p.dk + ty * 8 + r) * p.dv + col) =
+              *reinterpret_cast<const float4*>(Ss + (ty * 8 + r) * PS + 4 * tx);
+    }
+    // U = Y - W S, in runs of 16 terms
+    unsigned long long tot[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) tot[r][0] = tot[r][1] = 0ull;
+#pragma unroll 1
+    for (int d0 = 0; d0 < p.dk; d0 += 16) {
+      unsigned long long acc[4][2];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0ull;
+#pragma unroll
+      for (int d = d0; d < d0 + 16; d += 4) {
+        float4 w[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          w[r] = *reinterpret_cast<const float4*>(Wt + (ty * 4 + r) * DS_P + d);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(Ss + (d + x) * PS + 4 * tx);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float wv = x == 0 ? w[r].x : x == 1 ? w[r].y : x == 2 ? w[r].z : w[r].w;
+            const unsigned long long w2 = cs_pair(wv, wv);
+            acc[r][0] = cs_fma2(w2, sv.x, acc[r][0]);
+            acc[r][1] = cs_fma2(w2, sv.y, acc[r][1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        tot[r][0] = cs_add2(tot[r][0], acc[r][0]);
+        tot[r][1] = cs_add2(tot[r][1], acc[r][1]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int t = ty * 4 + r;
+      float4 a;
+      cs_unpair(tot[r][0], a.x, a.y);
+      cs_unpair(tot[r][1], a.z, a.w);
+      const float4 uv = make_float4(y[r].x - a.x, y[r].y - a.y, y[r].z - a.z, y[r].w - a.w);
+      const float g = t < n ? expf((float)(last - f[i * DS_C + min(t, n - 1)])) : 0.f;
+      *reinterpret_cast<float4*>(Us + t * PS + 4 * tx) = cs_times(uv, g);
+      if (t < n && col < p.dv)
+        *reinterpret_cast<float4*>(u + ((size_t)(c.t0 + i * DS_C + t) * p.H + h) * p.dv + col) = uv;
+    }
+    __syncthreads();                             // U is whole; the state before it is read
+    // S <- exp(F_C) S + K^T U, in runs of 16 tokens
+    unsigned long long S[4][4];
+    const float g = expf((float)(last - before));
+    before = last;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        S[r][j] = cs_pair(Ss[(ty * 8 + 2 * r) * PS + 4 * tx + j] * g,
+                          Ss[(ty * 8 + 2 * r + 1) * PS + 4 * tx + j] * g);
+#pragma unroll 1
+    for (int s0 = 0; s0 < n; s0 += 16) {         // (rows of Us and Ks from n on are zero)
+      unsigned long long acc[4][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][j] = 0ull;
+#pragma unroll
+      for (int s = s0; s < s0 + 16; ++s) {
+        const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(Kt + s * DS_P + ty * 8);
+        const ulonglong2 k1 = *reinterpret_cast<const ulonglong2*>(Kt + s * DS_P + ty * 8 + 4);
+        const float4 uv = *reinterpret_cast<const float4*>(Us + s * PS + 4 * tx);
+        const unsigned long long a[4] = {k0.x, k0.y, k1.x, k1.y};
+        const unsigned long long w[4] = {cs_pair(uv.x, uv.x), cs_pair(uv.y, uv.y),
+                                         cs_pair(uv.z, uv.z), cs_pair(uv.w, uv.w)};
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[r][j] = cs_fma2(a[r], w[j], acc[r][j]);
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[r][j] = cs_add2(S[r][j], acc[r][j]);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        cs_unpair(S[r][j], Ss[(ty * 8 + 2 * r) * PS + 4 * tx + j],
+                  Ss[(ty * 8 + 2 * r + 1) * PS + 4 * tx + j]);
+  }
+  __syncthreads();
+  for (int e = tid; e < DS_D * DS_NS; e += 128) {
+    const int kk = e % DS_D, j = e / DS_D;
+    if (kk < p.dk && col0 + j < p.dv) st[(size_t)(col0 + j) * p.dk + kk] = Ss[kk * PS + j];
+  }
+}
+
 // -------------------------------------------------------------------------------- launches
 // Scratch (bytes, each part on a 256-byte boundary): G, Hs, g0 | E (mLSTM) | qkm | U | Un (mLSTM).
 struct CsLayout {
@@ -681,7 +1044,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   const int tiles = p.C / CS_T, tk = (p.dk + CS_T - 1) / CS_T, tv = (p.dv + CS_T - 1) / CS_T;
   cs_gates_kernel<MLSTM><<<dim3(p.H, p.B), CS_GATE_THREADS, 0, stream>>>(
       decays, tok_decay, gates, state, slot_stride, state_size, q_start, state_slots, n_slots, G,
-      Hs, E, g0, p.T, p.H, p.dk * p.dv, p.dk, p.n_min);
+      Hs, E, g0, p.T, p.H, p.dk * p.dv, p.dk, p.n_min, p.H);
   cs_qk_kernel<A><<<dim3(l.chunks, p.QH, tiles * tiles), CS_THREADS, 0, stream>>>(qk, p, q_start,
                                                                                  qkm);
   cs_state_kernel<A, V, MLSTM><<<dim3(l.chunks, p.H, tk * tv), CS_THREADS, 0, stream>>>(
@@ -689,7 +1052,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   const int elems = p.dk * p.dv + (MLSTM ? p.dk : 0);
   cs_prefix_kernel<MLSTM><<<dim3((elems + 511) / 512, p.H, p.B), 128, 0, stream>>>(
       state, slot_stride, state_size, state_slots, n_slots, p, q_start, G, g0, U, Un, err);
-  cs_out_kernel<A, V, MLSTM><<<dim3(l.chunks, p.H, tiles * tv), CS_THREADS, 0, stream>>>(
+  cs_out_kernel<A, V, MLSTM, MLSTM><<<dim3(l.chunks, p.H, tiles * tv), CS_THREADS, 0, stream>>>(
       qk, v, p, q_start, state_slots, n_slots, G, Hs, g0, E, qkm, U, Un, o_raw);
   return bf_launch_status();
 }
@@ -734,4 +1097,83 @@ BF_EXPORT int bf_chunk_scan_mlstm(const void* proj, long long stride, const floa
   return cs_launch<__nv_bfloat16, __nv_bfloat16, true>(
       x, x, p, nullptr, nullptr, gates, state, slot_stride, state_size, q_start, state_slots,
       n_slots, o_raw, (char*)scratch, err, stream);
+}
+
+// The gated delta rule.  Scratch: F (G and H are the same array), g0 | qkm | W | Y | u | Sc.
+struct DsLayout {
+  size_t F, g0, qkm, W, Y, u, Sc, total;
+  int chunks;
+};
+static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv) {
+  DsLayout l;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t here = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return here;
+  };
+  l.chunks = T / DS_C + B;
+  l.F = take((size_t)T * H * 8);
+  l.g0 = take((size_t)B * H * 8);
+  l.qkm = take((size_t)l.chunks * G * DS_C * DS_C * 4);
+  l.W = take((size_t)l.chunks * H * DS_C * dk * 4);
+  l.Y = take((size_t)l.chunks * H * DS_C * dv * 4);
+  l.u = take((size_t)T * H * dv * 4);
+  l.Sc = take((size_t)l.chunks * H * dk * dv * 4);
+  l.total = at;
+  return l;
+}
+
+BF_EXPORT long long bf_chunk_scan_delta_scratch(int T, int B, int H, int G, int dk, int dv) {
+  return (long long)ds_layout(T, B, H, G, dk, dv).total;
+}
+
+// qkv, gates, state and o_raw as in bf_delta_scan (keys and values of at most 128, multiples of 4);
+// requests of at most n_min tokens are left alone.
+BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* state,
+                                  long long slot_stride, const int* q_start,
+                                  const int* state_slots, int n_slots, float* o_raw, void* scratch,
+                                  int T, int B, int H, int G, int dk, int dv, int n_min, int* err,
+                                  cudaStream_t stream) {
+  const long long C = 2LL * G * dk + (long long)H * dv;
+  if (T <= 0 || B <= 0 || B > 65535 || H <= 0 || H > 65535 || G <= 0 || H % G || dk <= 0 ||
+      dv <= 0 || dk > DS_D || dv > DS_D || dk % 4 || dv % 4 || !scratch || ((uintptr_t)qkv & 15))
+    return (int)cudaErrorInvalidValue;
+  const DsLayout l = ds_layout(T, B, H, G, dk, dv);
+  char* base = (char*)scratch;
+  double* F = (double*)(base + l.F);
+  double* g0 = (double*)(base + l.g0);
+  float* qkm = (float*)(base + l.qkm);
+  float* W = (float*)(base + l.W);
+  float* Y = (float*)(base + l.Y);
+  float* u = (float*)(base + l.u);
+  float* Sc = (float*)(base + l.Sc);
+  const DsIn d = {qkv, gates, C, H, G, dk, dv, T, B, n_min};
+  // (the decays are the second rows of gates: [T][2][H])
+  const CsIn p = {0, (long long)G * dk, 0, C, (long long)H * dv, H, G, dk, dv, DS_C, T, B, n_min,
+                  1.f};
+  const size_t smem_prep = ((size_t)2 * DS_C * DS_P + 2 * DS_C * 68 + 16 * 52) * sizeof(float);
+  const size_t smem_walk = ((size_t)4 * DS_C * DS_P + (DS_D + DS_C) * (DS_NS + 4)) * sizeof(float);
+  static bool configured[BF_MAX_DEVICES];
+  bool& done = configured[bf_current_device()];
+  if (!done) {
+    cudaError_t e = cudaFuncSetAttribute(
+        ds_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_prep);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(ds_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem_walk);
+    if (e != cudaSuccess) return (int)e;
+    done = true;
+  }
+  cs_gates_kernel<false><<<dim3(H, B), CS_GATE_THREADS, 0, stream>>>(
+      nullptr, gates + H, nullptr, state, slot_stride, dk * dv, q_start, state_slots, n_slots, F, F,
+      nullptr, g0, T, H, dk * dv, dk, n_min, 2 * H);
+  cs_qk_kernel<float><<<dim3(l.chunks, G, 1), CS_THREADS, 0, stream>>>(qkv, p, q_start, qkm);
+  ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, W, Y);
+  ds_walk_kernel<<<dim3((dv + DS_NS - 1) / DS_NS, H, B), 128, smem_walk, stream>>>(
+      d, q_start, state_slots, n_slots, state, slot_stride, F, W, Y, u, Sc, err);
+  cs_out_kernel<float, float, false, true>
+      <<<dim3(l.chunks, H, (dv + CS_T - 1) / CS_T), CS_THREADS, 0, stream>>>(
+          qkv, u, p, q_start, state_slots, n_slots, F, F, g0, nullptr, qkm, Sc, nullptr, o_raw);
+  return bf_launch_status();
 }

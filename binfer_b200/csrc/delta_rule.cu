@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(DR_THREADS) delta_scan_kernel(
     const float* __restrict__ qkv, const float* __restrict__ gates, float* __restrict__ state,
     long long state_stride, const int* __restrict__ q_start, const int* __restrict__ state_slots,
     int n_slots, float* __restrict__ o_raw, int H, int G, int dk, int dv, int stage,
-    int* __restrict__ err) {
+    int* __restrict__ err, int n_max) {
   extern __shared__ __align__(16) float sh[];
   constexpr int R4 = R / 4;
   constexpr int cols = DR_THREADS / KS;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(DR_THREADS) delta_scan_kernel(
   const int cg = tid / KS, part = tid % KS;
   const int col = col0 + cg;
   const int t0 = q_start[b], n = q_start[b + 1] - t0;
-  if (n <= 0) return;
+  if (n <= 0 || n > n_max) return;          // (longer portions: chunk_scan.cu)
   const int slot = state_slots[b];
   if (slot < 0 || slot >= n_slots) {
     if (tid == 0) atomicOr(err, BF_ERR_SLOT);
@@ -229,7 +229,10 @@ __global__ void __launch_bounds__(DR_THREADS) delta_scan_kernel(
 BF_EXPORT int bf_delta_scan(const float* qkv, const float* gates, float* state,
                             long long state_stride, const int* q_start, const int* state_slots,
                             int n_slots, float* o_raw, int T, int B, int max_q, int H, int G,
-                            int dk, int dv, int* err, cudaStream_t stream) {
+                            int dk, int dv, int* err, int n_max, cudaStream_t stream) {
+  // n_max > 0: requests that bring more tokens are left alone
+  if (n_max > 0 && max_q > n_max) max_q = n_max;
+  if (n_max <= 0) n_max = 0x7fffffff;
   if (B <= 0 || T <= 0) return 0;
   if (dk <= 0 || dv <= 0 || dk > 1024 || G <= 0 || H % G) return (int)cudaErrorInvalidValue;
   const int R = dk <= 128 ? 16 : 32;
@@ -250,7 +253,7 @@ BF_EXPORT int bf_delta_scan(const float* qkv, const float* gates, float* state,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);            \
     delta_scan_kernel<RR, KK><<<grid, DR_THREADS, smem, stream>>>(                             \
         qkv, gates, state, state_stride, q_start, state_slots, n_slots, o_raw, H, G, dk, dv,   \
-        stage, err);                                                                           \
+        stage, err, n_max);                                                                           \
   }
   if (R == 16) {
     if (KS == 1) DR_GO(16, 1) else if (KS == 2) DR_GO(16, 2) else if (KS == 4) DR_GO(16, 4)

@@ -755,10 +755,10 @@ def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_hea
     return torch.empty(n, dtype=torch.uint8, device=state.device)
 
 
-def _walk_limit(scratch: Optional[torch.Tensor], B: int) -> int:
+def _walk_limit(scratch: Optional[torch.Tensor], B: int, n_min: int = CHUNK_SCAN_MIN) -> int:
     """For the kernels that walk: the longest portion they take (0: any, -1: none, the step's only
     request has chunks)."""
-    return 0 if scratch is None else -1 if B == 1 else CHUNK_SCAN_MIN
+    return 0 if scratch is None else -1 if B == 1 else n_min
 
 
 def _chunk_scan_linear(name, qk, vf, decays, tok_decay, state, q_start, state_slots, o_raw, scratch,
@@ -1048,15 +1048,19 @@ def delta_encode(proj: torch.Tensor, conv_w: Optional[torch.Tensor], taps: int,
 
 DELTA_MAX_QK_DIM = 1024
 
+# portions of at most so many tokens are walked: the chunks' chain of small kernels takes 82 us for 170
+# tokens of 16 heads of 128 and 98 for 300, the walk 53 and 89; for 1,111 and 694 tokens 253 against 364
+DELTA_CHUNK_MIN = 384
 
 def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
                q_start: torch.Tensor, state_slots: torch.Tensor, o_raw: torch.Tensor, B: int,
                heads: int, qk_heads: int, dk: int, dv: int, err: torch.Tensor,
-               max_q: int = 0) -> None:
+               max_q: int = 0, chunked: bool = False) -> None:
     """The recurrence ``S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q`` over every
     request's tokens of the step, from :func:`delta_encode`'s ``qkv`` and ``gates``.  ``state``
     float32 ``[slots, heads * dv * dk]`` (a column block of the slots' storage); ``o_raw``
-    float32 ``[T, heads dv]``."""
+    float32 ``[T, heads dv]``.  ``chunked``: as for :func:`retention_scan`, from
+    ``DELTA_CHUNK_MIN`` tokens on."""
     T = qkv.shape[0]
     for t, n in ((qkv, "qkv"), (gates, "gates"), (o_raw, "o_raw")):
         _want(t, torch.float32, n)
@@ -1064,9 +1068,28 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
             or state.shape[1] != heads * dk * dv or dk > DELTA_MAX_QK_DIM):
         raise KernelError("delta_scan: state must be float32 [slots, heads * dk * dv]")
     _run("delta_scan", lib().bf_delta_scan, _ptr(qkv), _ptr(gates), _ptr(state),
+    scratch = None
+    if (chunked and (max_q or T) > DELTA_CHUNK_MIN and dk <= 128 and dv <= 128 and dk % 4 == 0
+            and dv % 4 == 0 and B <= 65535 and heads <= 65535 and qkv.is_contiguous()
+            and gates.is_contiguous() and qkv.data_ptr() % 16 == 0):
+        fn = lib().bf_chunk_scan_delta_scratch
+        fn.restype = _c_ll
+        n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv))
+        if n <= CHUNK_SCAN_MAX_BYTES:
+            scratch = torch.empty(n, dtype=torch.uint8, device=state.device)
+    if scratch is not None:
+        _run("delta_scan_chunks", lib().bf_chunk_scan_delta, _ptr(qkv), _ptr(gates), _ptr(state),
+             _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
+             _ptr(o_raw), _ptr(scratch), _c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads),
+             _c_int(dk), _c_int(dv), _c_int(DELTA_CHUNK_MIN), _ptr(err), _stream())
+        global _launches
+        _launches += 4          # five kernels
+        if _walk_limit(scratch, B, DELTA_CHUNK_MIN) < 0:
+            return
          _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
          _ptr(o_raw), _c_int(T), _c_int(B), _c_int(max_q if max_q > 0 else T), _c_int(heads),
-         _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err), _stream())
+         _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err),
+         _c_int(_walk_limit(scratch, B, DELTA_CHUNK_MIN)), _stream())
 
 
 def gated_norm_out(o_raw: torch.Tensor, proj: torch.Tensor, g_off: int,

@@ -1389,6 +1389,58 @@ def test_attention_f32_tiles(cuda_device, nh, nkv, d, ps, window):
     err.zero_()
 
 
+@pytest.mark.parametrize("lens,H,G,dk,dv", [([161, 1, 192, 160, 257], 4, 2, 32, 24),
+                                            ([300], 2, 1, 128, 128), ([193, 3], 3, 3, 68, 100)])
+def test_delta_scan_in_chunks(cuda_device, monkeypatch, lens, H, G, dk, dv):
+    """Against the walking kernel and both against float64: the products are no further off."""
+    from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN", 160)
+    torch.manual_seed(len(lens) + dk)
+    T, B, dev = sum(lens), len(lens), cuda_device
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, dk, device=dev), dim=-1)
+            for _ in range(2))
+    # neighbouring keys alike, so that a chunk's writes hang together
+    k = torch.nn.functional.normalize(k + k.roll(1, 0), dim=-1)
+    v = torch.randn(T, H, dv, device=dev)
+    qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], 1).contiguous()
+    gates = torch.rand(T, 2, H, device=dev)
+    gates[:, 1] = 1 - 0.3 * gates[:, 1] ** 4
+    gates[torch.rand(T, device=dev) < 0.02, 1] = 0.0
+    state = torch.randn(B + 1, H * dk * dv, device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev).flip(0).contiguous()
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    got, err = {}, _err(dev)
+    for chunked in (False, True):
+        s, o = state.clone(), torch.full((T, H * dv), 7.0, device=dev)
+        ops.delta_scan(qkv, gates, s, qs, slots, o, B, H, G, dk, dv, err, max_q=max(lens),
+                       chunked=chunked)
+        got[chunked] = (o, s)
+    assert int(err.item()) == 0 and torch.equal(got[True][1][B], state[B])
+    off = {c: [0.0] * 2 for c in got}
+    for b in range(B):
+        a, e, at = int(qs[b]), int(qs[b + 1]), int(slots[b])
+        qd, kd = (x[a:e].double().repeat_interleave(H // G, 1) for x in (q, k))
+        S = state[at].double().view(H, dv, dk).transpose(1, 2)
+        want = torch.empty(e - a, H, dv, dtype=torch.float64, device=dev)
+        for t in range(e - a):
+            beta, g = gates[a + t].double()
+            S = S * g[:, None, None]
+            u = beta[:, None] * (v[a + t].double() - (kd[t][:, None, :] @ S)[:, 0])
+            S = S + kd[t][:, :, None] * u[:, None, :]
+            want[t] = (qd[t][:, None, :] @ S)[:, 0]
+        for c, (go, gs) in got.items():
+            have = gs[at].double().view(H, dv, dk).transpose(1, 2)
+            for i, (x, y) in enumerate(((go[a:e].double().view(-1, H, dv), want), (have, S))):
+                off[c][i] = max(off[c][i], float((x - y).norm() / y.norm()))
+    for walk, products in zip(off[False], off[True]):
+        assert products <= 1.5 * walk + 2e-7, off
+    bad, keep = slots.clone(), got[True][1].clone()
+    bad[0] = B + 5
+    ops.delta_scan(qkv, gates, keep, qs, bad, o, B, H, G, dk, dv, err, max_q=max(lens), chunked=True)
+    assert int(err.item()) == 2 and torch.equal(keep[int(slots[0])], got[True][1][int(slots[0])])
+    err.zero_()
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("lens", [[1], [3, 1, 9, 2, 17], [1] * 5, [700, 1, 1, 643]])
