@@ -1307,6 +1307,63 @@ def moe_sparse(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor,
 
 
 # ----------------------------------------------------- norm on a sublayer's output
+# bytes up to which moe_grouped's scratch may grow
+MOE_GROUPED_MAX_BYTES = int(os.environ.get("BINFER_B200_MOE_GROUPED_MAX_BYTES", str(1 << 30)))
+
+
+def moe_grouped_takes(tokens: int, width: int, experts: int, ff: int, ff_sh: int,
+                      top: int) -> bool:
+    """Whether :func:`moe_grouped` takes these sizes: rows on 16-byte boundaries, and scratch
+    (the sorted rows, their activations and float results) inside its bound."""
+    rows = 256 * (tokens * top // 256 + experts)
+    scratch = rows * (6 * width + 2 * ff) + tokens * (4 * width + 2 * ff_sh)
+    return (experts <= 64 and width % 8 == 0 and ff % 8 == 0 and ff_sh % 8 == 0
+            and scratch <= MOE_GROUPED_MAX_BYTES)
+
+
+def moe_grouped(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor,
+                top_ids: torch.Tensor, top_w: torch.Tensor, route_w: torch.Tensor,
+                out: torch.Tensor, experts: int, ff: int, ff_sh: int, top: int,
+                shared_gate: bool = False, identity_col: int = -1,
+                expert_act: ExpertAct = SILU_EXPERTS) -> None:
+    """The mixture's output for many tokens in bfloat16, each token through its chosen experts (and
+    the shared one) alone; arguments as in :func:`moe_sparse`."""
+    T, width = h.shape
+    F, n = experts * ff + ff_sh, T * top
+    _want(w_gate_up, torch.bfloat16, "w_gate_up"); _want(out, torch.bfloat16, "out")
+    _want(top_ids, torch.int32, "top_ids"); _want(top_w, torch.float32, "top_w")
+    _want(route_w, torch.float32, "route_w")
+    if (h.dtype != out.dtype or w_down.dtype != out.dtype or h.stride(1) != 1
+            or w_down.stride(1) != 1 or tuple(w_gate_up.shape) != (2 * F, width)
+            or tuple(w_down.shape) != (width, F) or tuple(out.shape) != (T, width) or tuple(top_ids.shape) != (T, top)
+            or tuple(top_w.shape) != (T, top) or route_w.shape[0] != T
+            or route_w.shape[1] < experts + int(shared_gate) + (identity_col >= 0)
+            or identity_col >= route_w.shape[1]):
+        raise KernelError("moe_grouped: stacked weights [2 F, width] and [width, F], out "
+                          "[T, width], choices [T, top], route_w a row per token")
+    if not moe_grouped_takes(T, width, experts, ff, ff_sh, top):
+        raise KernelError("moe_grouped does not take these sizes")
+    if T == 0:
+        return
+    dev, f32 = h.device, torch.float32
+    tiles = n // 256 + experts
+    rows = 256 * tiles
+    ints = torch.empty(n + 1 + tiles, dtype=torch.int32, device=dev)
+    floats = torch.empty(rows * (width + 1) + (T * width if ff_sh else 0), dtype=f32, device=dev)
+    halves = torch.empty(rows * (width + ff) + T * ff_sh, dtype=h.dtype, device=dev)
+    at = lambda t, i: _c_void_p(t.data_ptr() + i * t.element_size())
+    _run("moe_grouped", lib().bf_moe_grouped, _ptr(h), _c_ll(h.stride(0)), _ptr(w_gate_up),
+         _ptr(w_down), _c_ll(w_down.stride(0)), _ptr(top_ids), _ptr(top_w), _ptr(route_w),
+         _c_int(route_w.shape[1]), _c_int(1 if shared_gate else 0), _c_int(identity_col),
+         _c_int(T), _c_int(width), _c_int(experts), _c_int(ff), _c_int(ff_sh), _c_int(top),
+         _c_int(tiles), _ptr(ints), at(floats, floats.numel() - rows), at(ints, n), _ptr(halves),
+         at(halves, rows * width), at(halves, rows * (width + ff)), _ptr(floats),
+         at(floats, rows * width), _ptr(out),
+         *expert_act.args(), _c_int(num_sms(dev)), _ptr(error_word(dev)), _stream())
+    global _launches
+    _launches += 4          # five kernels
+
+
 def rmsnorm_add(resid: torch.Tensor, y: torch.Tensor, weight: torch.Tensor,
                 reading: Optional[torch.Tensor], eps: float,
                 next_weight: Optional[torch.Tensor] = None, next_eps: float = 0.0) -> None:

@@ -25,6 +25,10 @@ count by the sum of its few largest scores, and the chosen scores may stay as th
 ``MoESpec.activation`` "clamped": ``min(g, c) sigmoid(a min(g, c)) (clamp(u, -c, c) + b)`` in silu's
 place, the shared expert with a limit c of its own.
 
+A step of many tokens in bfloat16 computes each token's chosen experts alone (``ops.moe_grouped``):
+the rows are copied expert by expert, the products walk them in tiles, a token's results are
+added in the router's order.  A token's result does not depend on the others there either.
+
 A step of very few tokens in bfloat16 (a request that decodes alone) would read every expert
 for nothing; there the chosen experts' rows alone are read, a warp per output row
 (``ops.moe_sparse``).  The float32 engine keeps the one path, so that its sums have one order.
@@ -48,6 +52,14 @@ from .mlp import FUSE_SWIGLU_FILL
 SPARSE = os.environ.get("BINFER_B200_MOE_SPARSE", "1") != "0"
 # BINFER_B200_FUSE_EXPERTS=0: the experts' gate/up product and their activation as two kernels
 FUSE_EXPERTS = os.environ.get("BINFER_B200_FUSE_EXPERTS", "1") != "0"
+# BINFER_B200_MOE_GROUPED=0: prompts compute every expert for every token
+GROUPED = os.environ.get("BINFER_B200_MOE_GROUPED", "1") != "0"
+# operations that have to be saved by it (every expert for every token against the chosen alone, the
+# shared expert in both; T tokens of width w, E experts of size f: 2.1e11 saved for 2,048 of 2,048, 8 of
+# 1,536: 222 and 144 us; 9.7e10 for 1,024 of those: 129 and 101; 4.9e10 for 2,048 of 1,024, 8 of 704: 94
+# and 81; 1.6e10 for 1,024 of 1,024, 8 of 512: 63 and 71; 2.4e12 for 8,192 of 4,096, 8 of 2,048: 2,780
+# and 1,168)
+GROUPED_MIN_FLOPS = 4e10
 
 
 class MoEFeedForward(FeedForward, StackedOut):
@@ -144,6 +156,16 @@ class MoEFeedForward(FeedForward, StackedOut):
         return (SPARSE and x.dtype == torch.bfloat16 and 2 * x.shape[0] * self.top <= self.E
                 and ops.moe_sparse_takes(self.hidden, self.ff, self.ff_sh, self.top))
 
+    def _grouped(self, x: torch.Tensor) -> bool:
+        """So many tokens that the products left out by the unchosen experts are worth the
+        sorting, the copies and the padding of every expert's rows to whole tiles."""
+        T, pair_from = x.shape[0], pair_token_limit()
+        if not GROUPED or x.dtype != torch.bfloat16 or not pair_from or T < pair_from:
+            return False
+        saved = T * (self.E - self.top) - 128 * self.E          # rows, of one expert each
+        return (6 * saved * self.ff * self.hidden >= GROUPED_MIN_FLOPS
+                and ops.moe_grouped_takes(T, self.hidden, self.E, self.ff, self.ff_sh, self.top))
+
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         route_w, top_ids, top_w = self._route(x)
         if self._sparse(x):
@@ -152,6 +174,12 @@ class MoEFeedForward(FeedForward, StackedOut):
             ops.moe_sparse(x, self.w_gate_up, self.w_out, top_ids, top_w, route_w, out, self.E,
                            self.ff, self.ff_sh, self.top, shared_gate=self.gated_shared,
                            identity_col=self.id_col, expert_act=self.expert_act)
+            return out
+        if self._grouped(x):
+            out = torch.empty((x.shape[0], self.hidden), dtype=x.dtype, device=x.device)
+            ops.moe_grouped(x, self.w_gate_up, self.w_out, top_ids, top_w, route_w, out, self.E,
+                            self.ff, self.ff_sh, self.top, shared_gate=self.gated_shared,
+                            identity_col=self.id_col, expert_act=self.expert_act)
             return out
         act = torch.empty((x.shape[0], self.F), dtype=x.dtype, device=x.device)
         self._activations(x, route_w, act)

@@ -1558,3 +1558,50 @@ def test_head_norm_out_in_registers(cuda_device, dv, dtype):
         _close(out.view(T, H, dv), rms(x) * wd * sg, dtype)
         ops.retention_out(o, proj, off, out, H, dv, 1e-5)
         _close(out.view(T, H, dv), rms(x) * g, dtype)
+
+
+@pytest.mark.parametrize("T,width,E,ff,ff_sh,top,ident,gate,kind", [
+    (1, 64, 1, 8, 0, 1, 0, False, "silu"), (257, 192, 5, 72, 40, 2, 0, True, "clamped"),
+    (700, 128, 3, 128, 0, 2, 4, False, "silu"), (1500, 256, 64, 64, 264, 3, 0, False, "silu"),
+    (300, 136, 8, 32, 8, 8, 2, True, "silu")])
+def test_moe_grouped(cuda_device, T, width, E, ff, ff_sh, top, ident, gate, kind):
+    """Chosen experts alone against float64 from the same bfloat16 numbers.  The activations are
+    rounded to bfloat16 once, their float sums once: 2^-8 of the largest magnitude each at most."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(T + E)
+    dev, F = cuda_device, E * ff + ff_sh
+    h = torch.randn(T, width + 8, device=dev).to(BF16)[:, :width]
+    gu = (torch.randn(2 * F, width, device=dev) * width ** -0.5).to(BF16)
+    down = (torch.randn(width, F, device=dev) * ff ** -0.5).to(BF16)
+    ids = torch.stack([torch.randperm(E + ident)[:top] for _ in range(T)])
+    if E > 4:                                    # an expert that nobody chose, and one for all
+        ids[ids == 1] = 0
+        ids[:, 0] = 2
+    ids = ids.to(dev, torch.int32).contiguous()
+    tw = torch.rand(T, top, device=dev)
+    cols = E + gate + (ident > 0)
+    rw = torch.rand(T, cols, device=dev)
+    act = ops.ExpertAct(kind, 1.0, 0.7, 1.3, 0.5)
+    out, err = torch.full((T, width), 7.0, dtype=BF16, device=dev), ops.error_word(dev)
+    ops.moe_grouped(h, gu, down, ids, tw, rw, out, E, ff, ff_sh, top, shared_gate=gate,
+                    identity_col=cols - 1 if ident else -1, expert_act=act)
+    x, g = h.double(), gu.double()
+
+    def run(lo, n, limit):
+        a, u = x @ g[lo:lo + n].T, x @ g[F + lo:F + lo + n].T
+        if kind == "clamped":
+            a, u = a.clamp(max=limit), u.clamp(-limit, limit) + 0.5
+        z = a * torch.sigmoid((1.3 if kind == "clamped" else 1.0) * a) * u
+        return z, down[:, lo:lo + n].double().T
+    ref = torch.zeros(T, width, dtype=torch.float64, device=dev)
+    for e in range(E):
+        z, d = run(e * ff, ff, 1.0)
+        for j in range(top):
+            ref += torch.where((ids[:, j] == e)[:, None], tw[:, j:j + 1].double() * (z @ d), 0.0)
+    if ff_sh:
+        z, d = run(E * ff, ff_sh, 0.7)
+        ref += (rw[:, E:E + 1].double() if gate else 1.0) * (z @ d)
+    if ident:
+        ref += rw[:, -1:].double() * x
+    assert int(err.item()) == 0
+    _close(out, ref, BF16)
