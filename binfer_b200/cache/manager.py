@@ -264,8 +264,9 @@ class CacheManager:
             want = -(-g.entries_for(new_len) // g.page_size)
             add = max(0, want - len(table))
             first = g.first_needed_page(rc.length)
-            release = sum(1 for p in table[g.kept_pages:first] if p > 0)
-            out.append(add - release)
+            if first > g.kept_pages:
+                add -= sum(1 for p in table[g.kept_pages:first] if p > 0)
+            out.append(add)
         return out
 
     def free_after(self, wants: Sequence[Tuple[Hashable, int]]) -> List[int]:

@@ -57,7 +57,8 @@ def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
 
 
 def _stream() -> _c_void_p:
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (torch.cuda.current_stream() builds an object behind several checks: 3 us of every launch)
+    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _check(code: int, what: str) -> None:
@@ -1047,10 +1048,10 @@ def delta_encode(proj: torch.Tensor, conv_w: Optional[torch.Tensor], taps: int,
 
 
 DELTA_MAX_QK_DIM = 1024
-
 # portions of at most so many tokens are walked: the chunks' chain of small kernels takes 82 us for 170
 # tokens of 16 heads of 128 and 98 for 300, the walk 53 and 89; for 1,111 and 694 tokens 253 against 364
 DELTA_CHUNK_MIN = 384
+
 
 def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
                q_start: torch.Tensor, state_slots: torch.Tensor, o_raw: torch.Tensor, B: int,
@@ -1067,7 +1068,6 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
     if (state.dtype != torch.float32 or state.stride(1) != 1
             or state.shape[1] != heads * dk * dv or dk > DELTA_MAX_QK_DIM):
         raise KernelError("delta_scan: state must be float32 [slots, heads * dk * dv]")
-    _run("delta_scan", lib().bf_delta_scan, _ptr(qkv), _ptr(gates), _ptr(state),
     scratch = None
     if (chunked and (max_q or T) > DELTA_CHUNK_MIN and dk <= 128 and dv <= 128 and dk % 4 == 0
             and dv % 4 == 0 and B <= 65535 and heads <= 65535 and qkv.is_contiguous()
@@ -1086,6 +1086,7 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
         _launches += 4          # five kernels
         if _walk_limit(scratch, B, DELTA_CHUNK_MIN) < 0:
             return
+    _run("delta_scan", lib().bf_delta_scan, _ptr(qkv), _ptr(gates), _ptr(state),
          _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
          _ptr(o_raw), _c_int(T), _c_int(B), _c_int(max_q if max_q > 0 else T), _c_int(heads),
          _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err),
@@ -1306,7 +1307,6 @@ def moe_sparse(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor,
     _launches += 1          # two kernels
 
 
-# ----------------------------------------------------- norm on a sublayer's output
 # bytes up to which moe_grouped's scratch may grow
 MOE_GROUPED_MAX_BYTES = int(os.environ.get("BINFER_B200_MOE_GROUPED_MAX_BYTES", str(1 << 30)))
 
@@ -1364,6 +1364,7 @@ def moe_grouped(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor,
     _launches += 4          # five kernels
 
 
+# ----------------------------------------------------- norm on a sublayer's output
 def rmsnorm_add(resid: torch.Tensor, y: torch.Tensor, weight: torch.Tensor,
                 reading: Optional[torch.Tensor], eps: float,
                 next_weight: Optional[torch.Tensor] = None, next_eps: float = 0.0) -> None:

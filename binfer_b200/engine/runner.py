@@ -150,38 +150,47 @@ class ModelRunner:
         tok, pos, sot = view("token_ids"), view("positions"), view("seq_of_token")
         qs, rows = view("q_start"), view("logit_rows")
         pairs: List[Tuple[int, int]] = []
-        t = r = 0
+        # single tokens are collected and written together: an assignment to one place of an
+        # array costs a tenth of a microsecond, a step of many requests makes hundreds
+        firsts: List[int] = []
+        single: List[int] = []
+        ids: List[int] = []
+        wanted: List[int] = []
+        t = 0
         for b, it in enumerate(items):
             n = q_lens[b]
+            firsts.append(t)
             if n == 1:
+                single.append(b)
                 if it.src_row is not None:
                     pairs.append((t, it.src_row))
-                    tok[t] = 0
+                    ids.append(0)
                 else:
-                    tok[t] = it.tokens[0]
-                pos[t] = starts[b]
-                sot[t] = b
+                    ids.append(it.tokens[0])
             else:
                 tok[t:t + n] = it.tokens
                 pos[t:t + n] = np.arange(starts[b], starts[b] + n, dtype=np.int32)
                 sot[t:t + n] = b
-            qs[b] = t
             if not pad_to:
                 for w in it.want:
                     if not 0 <= w < n:
                         raise ValueError(f"request {it.rid!r}: wanted place {w} is outside "
                                          f"its {n} tokens of this step")
-                    rows[r] = t + w
-                    r += 1
+                    wanted.append(t + w)
             t += n
+        if single:
+            at = [firsts[b] for b in single]
+            tok[at], pos[at], sot[at] = ids, [starts[b] for b in single], single
+        if not pad_to:
+            rows[:] = wanted
         if mixed:
-            view("decode_rows")[:] = [int(qs[b]) for b in dec]
+            view("decode_rows")[:] = [firsts[b] for b in dec]
             items4 = view("prefill_items").reshape(len(pf), 4)
             for i, b in enumerate(pf):
-                items4[i] = (b, int(qs[b]), q_lens[b], starts[b])
-        for b in range(n_real, B):              # padding rows
-            sot[b] = b
-            qs[b] = b
+                items4[i] = (b, firsts[b], q_lens[b], starts[b])
+        qs[:n_real] = firsts
+        if B > n_real:                          # padding rows
+            sot[n_real:B] = qs[n_real:B] = np.arange(n_real, B, dtype=np.int32)
         qs[B] = T
         if pad_to:
             rows[:] = np.arange(B, dtype=np.int32)
@@ -193,6 +202,7 @@ class ModelRunner:
             sl = view(f"slots{gi}")
             tb = view(f"tables{gi}").reshape(B, w)
             t = 0
+            places: List[int] = []              # of the single tokens
             for b, rc in enumerate(rcs):
                 table = rc.table_array(gi)
                 if len(table) > w:
@@ -205,11 +215,13 @@ class ModelRunner:
                     # takes the means; no token has a place of its own in it
                     sl[t:t + n] = -1
                 elif n == 1:
-                    sl[t] = int(table[start // ps]) * ps + start % ps
+                    places.append(rc.tables[gi][start // ps] * ps + start % ps)
                 else:
                     p = np.arange(start, start + n)
                     sl[t:t + n] = table[p // ps] * ps + p % ps
                 t += n
+            if places:
+                sl[at] = places
 
         if pairs:
             view("id_pairs")[:2 * len(pairs)] = np.asarray(pairs, dtype=np.int32).reshape(-1)
