@@ -31,6 +31,27 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// The sums of N values (a power of two) over the warp, for N - 1 shuffles or a few more instead of 5 N:
+// halves of the values change places until a lane has max(1, N / 32) left.  v[i] of lane l is then
+// value i + l N / 32 (N < 32: v[0] is value l N / 32).  Each sum is warp_sum's, bit for bit.
+template <int N>
+__device__ __forceinline__ void warp_sums(float (&v)[N], int lane) {
+  int n = N;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i)
+        if (i < n) {
+          const float keep = lane & o ? v[i + n] : v[i], give = lane & o ? v[i] : v[i + n];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+}
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -22,10 +22,11 @@
 // gates[t, r] for r < heads:  cap tanh((w_r . h_t + b_r) / cap)          (log input gate)
 //             for r >= heads: logsigmoid(cap tanh((w_r . h_t + b_r) / cap))  (log forget gate)
 // cap <= 0 means no cap.  mlstm_gates_kernel: one warp per (token, gate row), any sizes (2,048 tokens
-// of 4,096 x 16 rows: 53 us, the input read sixteen times over; 44 on the other).  mlstm_gates_tile_kernel, widths that
+// of 4,096 x 16 rows: 53 us, the input read sixteen times over; 27 on the other).  mlstm_gates_tile_kernel, widths that
 // are a multiple of 4: a block takes TB tokens and sixteen rows at a time, its eight warps share the
 // width out, a lane multiplies pieces of four of every token with pieces of four of every row, and
-// the lanes' and warps' sums are added in one order.  A token's sums do not depend on the others.
+// the lanes' and warps' sums are added in one order (a branch around each row made sixteen round
+// trips of one: 41 us).  A token's sums do not depend on the others.
 template <typename A>
 __global__ void mlstm_gates_kernel(const A* __restrict__ h, long long h_stride,
                                    const A* __restrict__ w, const float* __restrict__ bias,
@@ -54,42 +55,40 @@ __global__ void __launch_bounds__(256) mlstm_gates_tile_kernel(
     const A* __restrict__ h, long long h_stride, const A* __restrict__ w,
     const float* __restrict__ bias, float* __restrict__ gates, int T, int width, int heads,
     float cap) {
-  __shared__ float part[8][TB * MG_ROWS];
+  static_assert(TB == 1 || TB == 4, "how the lanes hold the sums");
+  __shared__ __align__(16) float part[8][TB * MG_ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = blockIdx.x * TB, r0 = blockIdx.y * MG_ROWS;
   const int n_gates = 2 * heads;
   const int rows = min(MG_ROWS, n_gates - r0), nt = min(TB, T - t0);
-  float acc[TB][MG_ROWS];
+  float acc[TB * MG_ROWS];
 #pragma unroll
-  for (int k = 0; k < TB; ++k)
-#pragma unroll
-    for (int r = 0; r < MG_ROWS; ++r) acc[k][r] = 0.f;
+  for (int i = 0; i < TB * MG_ROWS; ++i) acc[i] = 0.f;
   for (int c = (warp * 32 + lane) * 4; c < width; c += 1024) {
     float4 x[TB];
 #pragma unroll
     for (int k = 0; k < TB; ++k)
       x[k] = k < nt ? ct_ld4(h + (size_t)(t0 + k) * h_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    // (no branch around a row: all sixteen are requested before the first is used; the last row
+    // stands in for those beyond the end, whose sums nobody reads)
 #pragma unroll
     for (int r = 0; r < MG_ROWS; ++r) {
-      if (r < rows) {
-        const float4 p = ct_ld4(w + (size_t)(r0 + r) * width + c);
+      const float4 p = ct_ld4(w + (size_t)min(r0 + r, n_gates - 1) * width + c);
 #pragma unroll
-        for (int k = 0; k < TB; ++k) {
-          acc[k][r] = fmaf(x[k].x, p.x, acc[k][r]);
-          acc[k][r] = fmaf(x[k].y, p.y, acc[k][r]);
-          acc[k][r] = fmaf(x[k].z, p.z, acc[k][r]);
-          acc[k][r] = fmaf(x[k].w, p.w, acc[k][r]);
-        }
+      for (int k = 0; k < TB; ++k) {
+        float& a = acc[k * MG_ROWS + r];
+        a = fmaf(x[k].x, p.x, a);
+        a = fmaf(x[k].y, p.y, a);
+        a = fmaf(x[k].z, p.z, a);
+        a = fmaf(x[k].w, p.w, a);
       }
     }
   }
-#pragma unroll
-  for (int k = 0; k < TB; ++k)
-#pragma unroll
-    for (int r = 0; r < MG_ROWS; ++r) {
-      const float s = warp_sum(acc[k][r]);
-      if (lane == 0) part[warp][k * MG_ROWS + r] = s;
-    }
+  warp_sums(acc, lane);
+  if (TB == 4)
+    *reinterpret_cast<float2*>(&part[warp][2 * lane]) = make_float2(acc[0], acc[1]);
+  else if ((lane & 1) == 0)
+    part[warp][lane >> 1] = acc[0];
   __syncthreads();
   const int k = threadIdx.x / MG_ROWS, r = threadIdx.x % MG_ROWS;
   if (k >= nt || r >= rows) return;

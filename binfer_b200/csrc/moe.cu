@@ -30,10 +30,11 @@
 #include <float.h>
 
 #include "common.cuh"
+#include "conv_taps.cuh"
 #include "gate_act.cuh"
 
 // One block per MR_TOKENS tokens: their rows go to shared memory as float; every warp takes a
-// slice of the width and, row by row of the router, its share of each token's dot product
+// slice of the width and, MR_ROWS rows of the router at a time, its share of each token's dot product
 // (a router row is fetched once for all the block's tokens); the shares are then added in
 // the warps' order, and one warp per token chooses.  A token's sums do not depend on which
 // other tokens share its block.
@@ -60,10 +61,20 @@ __global__ void __launch_bounds__(MR_WARPS * 32) moe_route_kernel(
   float* part = sh + (size_t)MR_TOKENS * wp;       // [MR_WARPS][MR_TOKENS][rows]
   float* zs = part + (size_t)MR_WARPS * MR_TOKENS * rows;   // [MR_TOKENS][rows]
   float* chs = zs + (size_t)MR_TOKENS * rows;      // [MR_TOKENS][rows]: choice scores (mode 1)
-  for (int k = 0; k < nt; ++k) {
-    const A* src = h + (size_t)(t0 + k) * stride;
+  if ((width & 3) == 0 && (stride & 3) == 0 && (((uintptr_t)h) & (4 * sizeof(A) - 1)) == 0) {
+    // pieces of four, all tokens in one round of requests
+    const int w4 = width >> 2;
 #pragma unroll 8
-    for (int c = threadIdx.x; c < width; c += blockDim.x) x[(size_t)k * wp + c] = bf_ld(src + c);
+    for (int i = threadIdx.x; i < nt * w4; i += MR_WARPS * 32) {
+      const int k = i / w4, c = (i - k * w4) * 4;
+      ct_st4(x + (size_t)k * wp + c, ct_ld4(h + (size_t)(t0 + k) * stride + c));
+    }
+  } else {
+    for (int k = 0; k < nt; ++k) {
+      const A* src = h + (size_t)(t0 + k) * stride;
+#pragma unroll 8
+      for (int c = threadIdx.x; c < width; c += blockDim.x) x[(size_t)k * wp + c] = bf_ld(src + c);
+    }
   }
   __syncthreads();
   const bool vec = (width & 3) == 0 && (((uintptr_t)w) & 15) == 0;
@@ -72,7 +83,8 @@ __global__ void __launch_bounds__(MR_WARPS * 32) moe_route_kernel(
   const int per = (units + MR_WARPS - 1) / MR_WARPS;
   const int lo = warp * per, hi = min(units, lo + per);
   // MR_ROWS rows of the router at a time: a token's piece is read from shared memory once for all
-  // of them (2,048 tokens x 9 rows of 2,048: 31 us with one row at a time, 27 so)
+  // of them (2,048 tokens x 9 rows of 2,048: 31 us with one row at a time, 27 so; the tokens staged
+  // in pieces of four in one round of requests and the sums scattered over the lanes: 13)
   for (int e0 = 0; e0 < rows; e0 += MR_ROWS) {
     const float* wr = w + (size_t)e0 * width;
     const int ne = min(MR_ROWS, rows - e0);
@@ -126,13 +138,15 @@ __global__ void __launch_bounds__(MR_WARPS * 32) moe_route_kernel(
             }
         }
     }
+    float sums[16];
+    static_assert(MR_ROWS * MR_TOKENS <= 16, "a row's and token's sum for every other lane");
 #pragma unroll
-    for (int r = 0; r < MR_ROWS; ++r)
-#pragma unroll
-      for (int k = 0; k < MR_TOKENS; ++k) {
-        const float sum = warp_sum(a[r][k]);
-        if (lane == 0 && r < ne) part[((size_t)warp * MR_TOKENS + k) * rows + e0 + r] = sum;
-      }
+    for (int i = 0; i < 16; ++i)
+      sums[i] = i < MR_ROWS * MR_TOKENS ? a[i / MR_TOKENS % MR_ROWS][i % MR_TOKENS] : 0.f;
+    warp_sums(sums, lane);
+    const int r = (lane >> 1) / MR_TOKENS, k = (lane >> 1) % MR_TOKENS;
+    if ((lane & 1) == 0 && r < ne && r < MR_ROWS)
+      part[((size_t)warp * MR_TOKENS + k) * rows + e0 + r] = sums[0];
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nt * rows; i += blockDim.x) {
