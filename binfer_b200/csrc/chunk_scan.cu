@@ -143,8 +143,9 @@ __device__ __forceinline__ CsChunk cs_find(const int* __restrict__ q_start, int 
 #define CS_GATE_THREADS 256
 
 __device__ __forceinline__ double cs_log_decay(float d) {
-  // a decay that underflowed to zero forgets everything: exp(-1e4) is zero in float
-  return d > 0.f ? fmax(log((double)d), -1e4) : -1e4;
+  // a decay that underflowed to zero forgets everything: exp(-1e4) is zero in float.  One below zero
+  // has no logarithm: NaN, like NaN itself (callers leave such decays to the walk)
+  return d > 0.f ? fmax(log((double)d), -1e4) : d == 0.f ? -1e4 : (double)NAN;
 }
 
 // Exclusive scan over the block's threads of `v` by + or min; `seed` comes before the first.

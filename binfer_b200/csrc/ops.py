@@ -787,7 +787,8 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
     ``[T, heads dv]``.  ``max_q``: the most tokens one request brings to the step, if the
     caller knows it (0: not known).  ``silu``: q, k and v pass silu first.  ``chunked``: portions of
     more than ``CHUNK_SCAN_MIN`` tokens may run as products over chunks (``chunk_scan.cu``), whose
-    order of sums depends on where the portion begins."""
+    order of sums depends on where the portion begins and which take no decays below zero (their
+    results are NaN)."""
     _want(decays, torch.float32, "decays"); _want(o_raw, torch.float32, "o_raw")
     if proj.stride(1) != 1 or dk > RETENTION_MAX_QK_DIM:
         raise KernelError(f"retention_scan: contiguous rows and a key size of at most "

@@ -54,6 +54,8 @@ class RetentionMixer(Mixer):
         self.plain_out = (spec.norm_over == "head" and not spec.norm_weight
                           and spec.gate == "silu")
         self.norm_w = None
+        # (the products over chunks take the decays' logarithms)
+        self.chunks = all(d >= 0 for d in spec.decays)
         self.decays = torch.tensor(spec.decays, dtype=torch.float64).to(torch.float32).to(env.device)
         self.names = dict(spec.names)
         self.in_rows, self.out_cols = 2 * self.qk_size + 2 * self.v_size, self.v_size
@@ -99,7 +101,7 @@ class RetentionMixer(Mixer):
                            self.heads, self.dk, self.dv, self.k_scale, ctx.err,
                            max_q=1 if ctx.decode_only else ctx.max_q_len,
                            silu=self.spec.activation == "silu",
-                           chunked=proj.dtype == torch.bfloat16)
+                           chunked=self.chunks and proj.dtype == torch.bfloat16)
         g_off = 2 * self.qk_size + self.v_size
         if self.plain_out:
             ops.retention_out(o_raw, proj, g_off, out, self.heads, self.dv, self.spec.norm_eps,

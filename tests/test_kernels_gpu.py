@@ -1140,6 +1140,55 @@ def test_linear_scan_in_chunks(cuda_device, lens, H, G, dk, dv, decays):
     err.zero_()
 
 
+def test_retention_part_walks_decays_below_zero(cuda_device):
+    """A portion long enough for chunks and the same tokens in two that are walked."""
+    from types import SimpleNamespace
+    from binfer_b200.config import RetentionSpec
+    from binfer_b200.csrc import ops
+    from binfer_b200.engine import make_env
+    from binfer_b200.parts.retention import RetentionMixer
+    dev, T = cuda_device, 2 * ops.CHUNK_SCAN_MIN
+    spec = RetentionSpec(num_heads=2, qk_dim=16, v_dim=128, decays=(-0.9, 0.8), position=None,
+                         norm_eps=1e-5)
+    mixer = RetentionMixer(spec, 64, "", make_env(BF16))
+    torch.manual_seed(3)
+    proj = torch.randn(T, mixer.in_rows, device=dev).to(BF16)
+    got = []
+    for cuts in ([T], [T // 2, T // 2]):
+        view = SimpleNamespace(state=torch.zeros(1, 2 * 16 * 128, device=dev))
+        ys = []
+        for x in proj.split(cuts):
+            n, out = x.shape[0], torch.empty(x.shape[0], mixer.out_cols, dtype=BF16, device=dev)
+            ctx = SimpleNamespace(positions=torch.arange(n, dtype=torch.int32, device=dev),
+                                  q_start=torch.tensor([0, n], dtype=torch.int32, device=dev),
+                                  state_slots=torch.zeros(1, dtype=torch.int32, device=dev), B=1,
+                                  decode_only=False, max_q_len=n, err=_err(dev))
+            mixer.run(x, ctx, view, out, 1.0)
+            ys.append(out)
+        got.append((torch.cat(ys), view.state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert bool(got[0][0].isfinite().all())
+
+
+def test_chunks_pass_nan_decays_on(cuda_device):
+    """A decay that is NaN shows from its token on, in the products over chunks as in the walk."""
+    from binfer_b200.csrc import ops
+    dev, T, H, d, at = cuda_device, 300, 2, 32, 140
+    torch.manual_seed(4)
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev)
+    x = torch.nn.functional.normalize(torch.randn(T, 2, H, d, device=dev), dim=-1)
+    v, decay = torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    decay[at, 1] = float("nan")
+    for chunked in (False, True):
+        out = torch.zeros(T, H * d, device=dev)
+        ops.linear_scan(x, v, decay, torch.zeros(1, H * d * d, device=dev), qs, slots, out, 1, H, H,
+                        d, d, err, max_q=T, chunked=chunked)
+        out = out.view(T, H, d)
+        assert bool(out[:, 0].isfinite().all()) and bool(out[:at, 1].isfinite().all())
+        assert bool(out[at:, 1].isnan().all())
+
+
 @pytest.mark.parametrize("lens,H,dk,dv", [([161, 1, 192, 160, 257], 2, 24, 40),
                                           ([193], 3, 64, 100), ([320, 5], 1, 256, 64)])
 def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
