@@ -262,6 +262,37 @@ __device__ __forceinline__ void cs_mul(const float (&As)[CS_K][CS_P], const floa
     for (int j = 0; j < 4; ++j) total[i][j] = cs_add2(total[i][j], acc[i][j]);
 }
 
+// The same for a step of sixteen tokens whose first is the first of this warp's sixteen rows: row r
+// takes the tokens up to its own.  The others' weights are zero, but what they would multiply may be
+// an infinity, and a token's result must not depend on the ones behind it.
+__device__ __forceinline__ void cs_mul_lower(const float (&As)[CS_K][CS_P],
+                                             const float (&Bs)[CS_K][CS_P], int tx, int ty,
+                                             CsAcc& total) {
+  const int row = (ty & 1) * 8;
+  // (a pair of rows at a time: one step of a CTA's, and registers are scarce)
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll 4
+    for (int kk = 0; kk < CS_K; ++kk) {
+      const unsigned long long a =
+          *reinterpret_cast<const unsigned long long*>(&As[kk][ty * 8 + 2 * i]);
+      const float4 w = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
+      const unsigned long long b[4] = {cs_pair(w.x, w.x), cs_pair(w.y, w.y), cs_pair(w.z, w.z),
+                                       cs_pair(w.w, w.w)};
+      const bool both = kk <= row + 2 * i, second = kk == row + 2 * i + 1;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned long long z = cs_fma2(a, b[j], acc[j]);
+        if (both) acc[j] = z;
+        if (second) acc[j] = (acc[j] & 0xffffffffull) | (z & ~0xffffffffull);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) total[i][j] = cs_add2(total[i][j], acc[j]);
+  }
+}
+
 // A step's pieces of four: `idx` 0..255, two a thread.  Rows with the terms side by side (row
 // idx / 4, terms 4 (idx % 4) ..) are turned on their way into shared memory; rows of terms (term
 // idx / 16, columns 4 (idx % 16) ..) go in as they are.
@@ -610,7 +641,10 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
   int buf = 0;
   for (int k0 = 0; k0 < terms; k0 += CS_K, buf ^= 1) {
     if (k0 + CS_K < terms) fetch(k0 + CS_K);
-    cs_mul(As[buf], Bs[buf], tx, ty, acc);
+    // the tokens before, among and behind this warp's sixteen rows
+    const int ahead = k0 < dk_pad ? -1 : k0 - dk_pad - ((ty & ~1) * 8 + r0);
+    if (ahead < 0) cs_mul(As[buf], Bs[buf], tx, ty, acc);
+    else if (ahead == 0) cs_mul_lower(As[buf], Bs[buf], tx, ty, acc);
     if (MLSTM) {
       // n_t . q_t: the same rows against n and against ones; term tx of the step's sixteen
       const float w = ns[buf][tx];

@@ -1189,6 +1189,41 @@ def test_chunks_pass_nan_decays_on(cuda_device):
         assert bool(out[at:, 1].isnan().all())
 
 
+@pytest.mark.parametrize("kind", ["linear", "mlstm"])
+@pytest.mark.parametrize("at", [64, 140, 255])
+def test_chunks_leave_earlier_tokens_alone(cuda_device, monkeypatch, kind, at):
+    """An infinite value shows from its token on: the bits of the tokens before it stay."""
+    from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN", 160)
+    dev, T, H, d = cuda_device, 300, 2, 32
+    torch.manual_seed(5)
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, outs = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    x = torch.nn.functional.normalize(torch.randn(T, 2, H, d, device=dev), dim=-1)
+    v, decay = torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    for bad in (False, True):
+        if bad:
+            v[at, 1] = float("inf")
+        out = torch.zeros(T, H * d, device=dev)
+        if kind == "linear":
+            ops.linear_scan(x, v, decay, torch.zeros(1, H * d * d, device=dev), qs, slots, out, 1,
+                            H, H, d, d, err, max_q=T, chunked=True)
+        elif kind == "delta":
+            qkv = torch.cat([x.reshape(T, -1), v.reshape(T, -1)], 1).contiguous()
+            gates = torch.stack([1 - decay, decay], 1).contiguous()
+            ops.delta_scan(qkv, gates, torch.zeros(1, H * d * d, device=dev), qs, slots, out, 1, H,
+                           H, d, d, err, max_q=T, chunked=True)
+        else:
+            proj = torch.cat([x.reshape(T, -1), v.reshape(T, -1)], 1).to(BF16)
+            gates = torch.cat([decay, decay.log()], 1).contiguous()
+            ops.mlstm_scan(proj, gates, torch.zeros(1, H, ops.mlstm_state_size(d, d), device=dev),
+                           qs, slots, out, 1, H, d, d, 1.0, err, max_q=T, chunked=True)
+        outs.append(out.view(T, H, d))
+    clean, dirty = outs
+    assert torch.equal(dirty[:, 0], clean[:, 0]) and torch.equal(dirty[:at, 1], clean[:at, 1])
+    assert not bool(dirty[at, 1].isfinite().any())
+
+
 @pytest.mark.parametrize("lens,H,dk,dv", [([161, 1, 192, 160, 257], 2, 24, 40),
                                           ([193], 3, 64, 100), ([320, 5], 1, 256, 64)])
 def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
