@@ -807,8 +807,8 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     for (int e = tid; e < 16 * cols; e += DS_PREP_THREADS) {
       const int r = e / cols, j = e % cols;
       float a = 0.f;
-#pragma unroll
-      for (int s = 0; s < 16; ++s) a = fmaf(Ts[(16 * i + r) * 68 + 16 * i + s], Rs[s * 52 + j], a);
+      // (row s of the block reaches the rows from s on alone, also where it is not finite)
+      for (int s = 0; s <= r; ++s) a = fmaf(Ts[(16 * i + r) * 68 + 16 * i + s], Rs[s * 52 + j], a);
       Ts[(16 * i + r) * 68 + j] = -a;
     }
     __syncthreads();
@@ -824,7 +824,9 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0ull;
-    for (int s = 0; s < ty * 4 + 4; s += 4) {    // (T is zero above the diagonal)
+    // (T is zero above the diagonal, but what stands there may be infinite: a thread's last four terms
+    // are those that its rows have)
+    auto four = [&](int s, bool last) {
       float4 tr[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -838,6 +840,7 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
           b[j] = *reinterpret_cast<const ulonglong2*>(B + (s + x) * DS_P + 4 * tx + 64 * j);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
+          if (last && i < x) continue;
           const float w = (x == 0 ? tr[i].x : x == 1 ? tr[i].y : x == 2 ? tr[i].z : tr[i].w) * fsc;
           const unsigned long long w2 = cs_pair(w, w);
 #pragma unroll
@@ -847,7 +850,9 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
           }
         }
       }
-    }
+    };
+    for (int s = 0; s < ty * 4; s += 4) four(s, false);
+    four(ty * 4, true);
     float* dst = (what ? Y : W) + ((size_t)blockIdx.x * p.H + h) * DS_C * width;
 #pragma unroll
     for (int i = 0; i < 4; ++i)

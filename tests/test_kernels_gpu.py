@@ -1189,7 +1189,7 @@ def test_chunks_pass_nan_decays_on(cuda_device):
         assert bool(out[at:, 1].isnan().all())
 
 
-@pytest.mark.parametrize("kind", ["linear", "mlstm"])
+@pytest.mark.parametrize("kind", ["linear", "mlstm", "delta"])
 @pytest.mark.parametrize("at", [64, 140, 255])
 def test_chunks_leave_earlier_tokens_alone(cuda_device, monkeypatch, kind, at):
     """An infinite value shows from its token on: the bits of the tokens before it stay."""
