@@ -11,11 +11,15 @@
 //
 // Every sum has an order that depends on the row's own position alone: a tile that a row does not see
 // multiplies its sums by one and adds zeros.  So a row's result does not depend on how a prompt was
-// cut, on BM, or on what else is in the batch.
+// cut, on BM, or on what else is in the batch.  A value that is not finite would make such a zero NaN:
+// tiles of which a row sees a part only are looked through for one, and if there is, they are added
+// key by key, each row its own.
 //
 // What bounds it: the FP32 pipes and, for them, shared-memory reads (one 16-byte read per eight
 // multiply-adds).  The kernel for any size has one warp per (token, head), whose lanes share a key's
 // sizes and meet in five shuffles per key: 333 tokens of 16 heads of 128 took 557 us there, 58 here.
+#include <float.h>
+
 #include "common.cuh"
 #include "mma_utils.cuh"
 
@@ -106,7 +110,7 @@ __global__ void __launch_bounds__(BM / TM * 16) attention_f32_kernel(
   for (int i = 0; i < TM; ++i) {
     const int row = row0 + ty * TM + i;
     pos[i] = row < rows ? positions[t0 + row / Gh] : -1;
-    m[i] = -INFINITY;
+    m[i] = -FLT_MAX;      // (not -inf: a score may be that, and counts as none)
     l[i] = 0.f;
 #pragma unroll
     for (int j = 0; j < CJ; ++j) o[i][j][0] = o[i][j][1] = 0ull;
@@ -176,7 +180,40 @@ __global__ void __launch_bounds__(BM / TM * 16) attention_f32_kernel(
         o[i][j][1] = af_mul2(o[i][j][1], c2);
       }
     }
+    // keys that are here and that some row does not see: behind the first row's position, before the
+    // last row's window
+    bool odd = false;
+    if (p_lo < p_hi && ((tile + 1) * AF_KEYS - 1 > p_lo ||
+                        (window > 0 && tile * AF_KEYS < p_hi - window + 1))) {
+      for (int i = tid; i < AF_KEYS * CHUNKS; i += THREADS) {
+        const float4 x = *reinterpret_cast<const float4*>(Vt + i / CHUNKS * P + i % CHUNKS * 4);
+        // (a number times zero is zero if it is finite, and only then)
+        odd |= !(x.x * 0.f + x.y * 0.f + x.z * 0.f + x.w * 0.f == 0.f);
+      }
+      odd = __syncthreads_or(odd);
+    }
     __syncwarp();                               // a row's probabilities come from its own half warp
+    if (odd) {
+      for (int e = 0; e < AF_KEYS; ++e) {
+        const int key = tile * AF_KEYS + e;
+        ulonglong2 v[CJ];
+#pragma unroll
+        for (int j = 0; j < CJ; ++j)
+          v[j] = *reinterpret_cast<const ulonglong2*>(Vt + e * P + 4 * tx + 64 * j);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+          if (key > pos[i] || (window > 0 && key < pos[i] - window + 1)) continue;
+          const float w = Ps[(ty * TM + i) * PP + e];
+          const unsigned long long w2 = af_pair(w, w);
+#pragma unroll
+          for (int j = 0; j < CJ; ++j) {
+            o[i][j][0] = af_fma2(w2, v[j].x, o[i][j][0]);
+            o[i][j][1] = af_fma2(w2, v[j].y, o[i][j][1]);
+          }
+        }
+      }
+      continue;
+    }
 #pragma unroll 4
     for (int e = 0; e < AF_KEYS; e += 4) {
       float4 p[TM];

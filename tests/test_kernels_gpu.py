@@ -1473,6 +1473,41 @@ def test_attention_f32_tiles(cuda_device, nh, nkv, d, ps, window):
     err.zero_()
 
 
+@pytest.mark.parametrize("window", [None, 70])
+def test_attention_f32_keys_that_a_row_does_not_see(cuda_device, window):
+    """Values that are not finite reach the rows that see them alone; scores of -inf count as none.
+    A portion's rows against the same rows alone, and against the kernel for any size."""
+    from binfer_b200.csrc import ops
+    n, at, d, dev = 200, 130, 64, cuda_device
+    q, kc, vc, sot, pos, bt, ref = _attention_case(dev, F32, 2, 1, d, 16, [n], [n], window, False,
+                                                   seed=22)
+    def put(cache, key, x):
+        cache[int(bt[0, key // 16]), 0, key % 16] = x
+    put(vc, at, float("inf"))
+    if window:
+        put(vc, 3, float("nan"))
+    q, err = q.abs(), _err(dev)
+    for key in range(64):                # q . k overflows
+        put(kc, key, -3e38)
+    qs = torch.tensor([0, n], dtype=torch.int32, device=dev)
+    out, want = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
+    ops.attention_f32(q, kc, vc, qs, pos, bt, out, 1, n, 2, 1, d, window, d ** -0.5, err)
+    ops.paged_attention_generic(q, kc, vc, sot, pos, bt, want, 2, 1, d, window, d ** -0.5, err)
+    fin = want.isfinite()
+    assert torch.equal(fin, out.isfinite())
+    # from the first key with a score on, or where the window has left the NaN behind
+    assert bool(fin[73 if window else 64:at].all()) and not bool(fin[at:].any())
+    assert not bool(fin[:64].any())
+    one, each = torch.full_like(q[:1], 7.0), qs.new_tensor([0, 1])
+    for t in (63, 64, 128, 129, 130, 199):
+        ops.attention_f32(q[t:t + 1].contiguous(), kc, vc, each, pos[t:t + 1].contiguous(), bt, one,
+                          1, 1, 2, 1, d, window, d ** -0.5, err)
+        assert torch.equal(one[0].isfinite(), out[t].isfinite())
+        assert torch.equal(one[0][one[0].isfinite()], out[t][out[t].isfinite()])
+    assert int(err.item()) == 0
+    _close(out[fin].cpu(), want[fin].cpu(), F32)
+
+
 @pytest.mark.parametrize("lens,H,G,dk,dv", [([161, 1, 192, 160, 257], 4, 2, 32, 24),
                                             ([300], 2, 1, 128, 128), ([193, 3], 3, 3, 68, 100)])
 def test_delta_scan_in_chunks(cuda_device, monkeypatch, lens, H, G, dk, dv):
