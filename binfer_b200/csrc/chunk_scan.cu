@@ -1097,11 +1097,12 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   return bf_launch_status();
 }
 
-static bool cs_sizes_ok(const CsIn& p, const void* state, long long slot_stride) {
+static bool cs_sizes_ok(const CsIn& p, const void* state, long long slot_stride,
+                        const void* o_raw) {
   return p.T > 0 && p.B > 0 && p.B <= 65535 && p.H > 0 && p.H <= 65535 && p.QH > 0 &&
          p.H % p.QH == 0 && p.dk > 0 && p.dv > 0 && p.dk % 4 == 0 && p.dv % 4 == 0 && p.C > 0 &&
          p.C % CS_T == 0 && p.qk_stride % 4 == 0 && p.v_stride % 4 == 0 && slot_stride % 4 == 0 &&
-         ((uintptr_t)state & 15) == 0;
+         (((uintptr_t)state | (uintptr_t)o_raw) & 15) == 0;
 }
 
 // qk [T][2][QH][dk] (q, then k), vf [T][H][dv], float; a decay per head or per (token, head).
@@ -1114,7 +1115,8 @@ BF_EXPORT int bf_chunk_scan_linear(const float* qk, const float* vf, const float
                                    cudaStream_t stream) {
   CsIn p = {0, (long long)QH * dk, 0, 2LL * QH * dk, (long long)H * dv, H, QH, dk, dv, C, T, B,
             n_min, 1.f};
-  if (!cs_sizes_ok(p, state, slot_stride) || (!decays && !tok_decay) || !scratch)
+  if (!cs_sizes_ok(p, state, slot_stride, o_raw) || (!decays && !tok_decay) || !scratch ||
+      (((uintptr_t)qk | (uintptr_t)vf) & 15))
     return (int)cudaErrorInvalidValue;
   return cs_launch<float, float, false>(qk, vf, p, decays, tok_decay, nullptr, state, slot_stride,
                                         dk * dv, q_start, state_slots, n_slots, o_raw,
@@ -1130,7 +1132,7 @@ BF_EXPORT int bf_chunk_scan_mlstm(const void* proj, long long stride, const floa
                                   cudaStream_t stream) {
   CsIn p = {0, (long long)H * dk, 2LL * H * dk, stride, stride, H, H, dk, dv, C, T, B, n_min,
             q_scale};
-  if (!cs_sizes_ok(p, state, slot_stride) || state_size % 4 || !gates || !scratch ||
+  if (!cs_sizes_ok(p, state, slot_stride, o_raw) || state_size % 4 || !gates || !scratch ||
       ((uintptr_t)proj & 7))
     return (int)cudaErrorInvalidValue;
   const __nv_bfloat16* x = (const __nv_bfloat16*)proj;
@@ -1177,7 +1179,8 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
                                   cudaStream_t stream) {
   const long long C = 2LL * G * dk + (long long)H * dv;
   if (T <= 0 || B <= 0 || B > 65535 || H <= 0 || H > 65535 || G <= 0 || H % G || dk <= 0 ||
-      dv <= 0 || dk > DS_D || dv > DS_D || dk % 4 || dv % 4 || !scratch || ((uintptr_t)qkv & 15))
+      dv <= 0 || dk > DS_D || dv > DS_D || dk % 4 || dv % 4 || !scratch ||
+      (((uintptr_t)qkv | (uintptr_t)o_raw) & 15))
     return (int)cudaErrorInvalidValue;
   const DsLayout l = ds_layout(T, B, H, G, dk, dv);
   char* base = (char*)scratch;

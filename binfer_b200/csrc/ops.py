@@ -741,11 +741,13 @@ CHUNK_SCAN_MAX_BYTES = 768 << 20
 
 
 def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_heads: int, dk: int,
-                   dv: int, state: torch.Tensor, mlstm: int) -> Optional[torch.Tensor]:
+                   dv: int, state: torch.Tensor, mlstm: int,
+                   *buffers: torch.Tensor) -> Optional[torch.Tensor]:
     """Scratch for the products over chunks, or None where a step's recurrence is walked: single
-    tokens and short portions, and sizes or addresses that are no whole 16-byte pieces."""
+    tokens and short portions, and sizes or addresses (of the state and of ``buffers``, float)
+    that are no whole 16-byte pieces."""
     if (not chunked or max_q <= CHUNK_SCAN_MIN or dk % 4 or dv % 4 or state.stride(0) % 4
-            or state.data_ptr() % 16 or B > 65535 or heads > 65535):
+            or any(t.data_ptr() % 16 for t in (state, *buffers)) or B > 65535 or heads > 65535):
         return None
     fn = lib().bf_chunk_scan_scratch
     fn.restype = _c_ll
@@ -805,7 +807,8 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
     # two kernels
     qk = torch.empty((T, 2, heads, dk), dtype=torch.float32, device=proj.device)
     vf = torch.empty((T, heads, dv), dtype=torch.float32, device=proj.device)
-    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, heads, dk, dv, state, 0)
+    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, heads, dk, dv, state, 0,
+                             o_raw)
     _run("retention_scan", lib().bf_retention_scan, _ptr(proj), _c_ll(proj.stride(0)),
          _c_ll(q_off), _c_ll(k_off), _c_ll(v_off), _ptr(decays), _ptr(inv_freq), _c_int(rot_half),
          _ptr(positions), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
@@ -842,7 +845,8 @@ def linear_scan(qk: torch.Tensor, vf: torch.Tensor, tok_decay: torch.Tensor, sta
     if (state.dtype != torch.float32 or state.stride(1) != 1
             or state.shape[1] != heads * dk * dv):
         raise KernelError("linear_scan: state must be float32 [slots, heads * dk * dv]")
-    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, qk_heads, dk, dv, state, 0)
+    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, qk_heads, dk, dv, state, 0,
+                             qk, vf, o_raw)
     if scratch is not None:
         _chunk_scan_linear("linear_scan", qk, vf, None, tok_decay, state, q_start, state_slots,
                            o_raw, scratch, B, heads, qk_heads, dk, dv, err)
@@ -1072,7 +1076,7 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
     scratch = None
     if (chunked and (max_q or T) > DELTA_CHUNK_MIN and dk <= 128 and dv <= 128 and dk % 4 == 0
             and dv % 4 == 0 and B <= 65535 and heads <= 65535 and qkv.is_contiguous()
-            and gates.is_contiguous() and qkv.data_ptr() % 16 == 0):
+            and gates.is_contiguous() and qkv.data_ptr() % 16 == 0 and o_raw.data_ptr() % 16 == 0):
         fn = lib().bf_chunk_scan_delta_scratch
         fn.restype = _c_ll
         n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv))
@@ -1440,7 +1444,7 @@ def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
     T = proj.shape[0]
     takes = (chunked and proj.dtype == torch.bfloat16 and proj.stride(0) % 4 == 0
              and proj.data_ptr() % 8 == 0 and state.stride(1) == state.shape[2])
-    scratch = _chunk_scratch(takes, max_q or T, T, B, heads, heads, dk, dv, state, 1)
+    scratch = _chunk_scratch(takes, max_q or T, T, B, heads, heads, dk, dv, state, 1, o_raw)
     if scratch is not None:
         _run("mlstm_scan_chunks", lib().bf_chunk_scan_mlstm, _ptr(proj), _c_ll(proj.stride(0)),
              _ptr(gates), _ptr(state), _c_ll(state.stride(0)), _c_int(state.shape[2]),
