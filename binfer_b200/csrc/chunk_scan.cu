@@ -1042,7 +1042,13 @@ struct CsLayout {
   size_t G, Hs, g0, E, qkm, U, Un, total;
   int chunks;
 };
-static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, int mlstm) {
+// The most chunks of C tokens that a step's portions of more than n_min tokens can have.
+static int cs_most_chunks(int T, int B, int C, int n_min) {
+  const int long_ones = T / (n_min + 1);
+  return T / C + (B < long_ones ? B : long_ones);
+}
+static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, int mlstm,
+                          int n_min) {
   CsLayout l;
   size_t at = 0;
   auto take = [&](size_t bytes) {
@@ -1050,7 +1056,7 @@ static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, in
     at += (bytes + 255) & ~(size_t)255;
     return here;
   };
-  l.chunks = T / C + B;                // the most that portions of T tokens in all can have
+  l.chunks = cs_most_chunks(T, B, C, n_min);
   l.G = take((size_t)T * H * 8);
   l.Hs = take((size_t)T * H * 8);
   l.g0 = take((size_t)B * H * 8);
@@ -1063,8 +1069,8 @@ static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, in
 }
 
 BF_EXPORT long long bf_chunk_scan_scratch(int T, int B, int H, int QH, int dk, int dv, int C,
-                                          int mlstm) {
-  return (long long)cs_layout(T, B, H, QH, dk, dv, C, mlstm).total;
+                                          int mlstm, int n_min) {
+  return (long long)cs_layout(T, B, H, QH, dk, dv, C, mlstm, n_min).total;
 }
 
 template <typename A, typename V, bool MLSTM>
@@ -1073,7 +1079,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
                      long long slot_stride, int state_size, const int* q_start,
                      const int* state_slots, int n_slots, float* o_raw, char* scratch, int* err,
                      cudaStream_t stream) {
-  const CsLayout l = cs_layout(p.T, p.B, p.H, p.QH, p.dk, p.dv, p.C, MLSTM);
+  const CsLayout l = cs_layout(p.T, p.B, p.H, p.QH, p.dk, p.dv, p.C, MLSTM, p.n_min);
   double* G = (double*)(scratch + l.G);
   double* Hs = (double*)(scratch + l.Hs);
   double* g0 = (double*)(scratch + l.g0);
@@ -1100,7 +1106,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
 static bool cs_sizes_ok(const CsIn& p, const void* state, long long slot_stride,
                         const void* o_raw) {
   return p.T > 0 && p.B > 0 && p.B <= 65535 && p.H > 0 && p.H <= 65535 && p.QH > 0 &&
-         p.H % p.QH == 0 && p.dk > 0 && p.dv > 0 && p.dk % 4 == 0 && p.dv % 4 == 0 && p.C > 0 &&
+         p.n_min >= 0 && p.H % p.QH == 0 && p.dk > 0 && p.dv > 0 && p.dk % 4 == 0 && p.dv % 4 == 0 && p.C > 0 &&
          p.C % CS_T == 0 && p.qk_stride % 4 == 0 && p.v_stride % 4 == 0 && slot_stride % 4 == 0 &&
          (((uintptr_t)state | (uintptr_t)o_raw) & 15) == 0;
 }
@@ -1146,7 +1152,7 @@ struct DsLayout {
   size_t F, g0, qkm, W, Y, u, Sc, total;
   int chunks;
 };
-static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv) {
+static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min) {
   DsLayout l;
   size_t at = 0;
   auto take = [&](size_t bytes) {
@@ -1154,7 +1160,7 @@ static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv) {
     at += (bytes + 255) & ~(size_t)255;
     return here;
   };
-  l.chunks = T / DS_C + B;
+  l.chunks = cs_most_chunks(T, B, DS_C, n_min);
   l.F = take((size_t)T * H * 8);
   l.g0 = take((size_t)B * H * 8);
   l.qkm = take((size_t)l.chunks * G * DS_C * DS_C * 4);
@@ -1166,8 +1172,9 @@ static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv) {
   return l;
 }
 
-BF_EXPORT long long bf_chunk_scan_delta_scratch(int T, int B, int H, int G, int dk, int dv) {
-  return (long long)ds_layout(T, B, H, G, dk, dv).total;
+BF_EXPORT long long bf_chunk_scan_delta_scratch(int T, int B, int H, int G, int dk, int dv,
+                                                int n_min) {
+  return (long long)ds_layout(T, B, H, G, dk, dv, n_min).total;
 }
 
 // qkv, gates, state and o_raw as in bf_delta_scan (keys and values of at most 128, multiples of 4);
@@ -1179,10 +1186,10 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
                                   cudaStream_t stream) {
   const long long C = 2LL * G * dk + (long long)H * dv;
   if (T <= 0 || B <= 0 || B > 65535 || H <= 0 || H > 65535 || G <= 0 || H % G || dk <= 0 ||
-      dv <= 0 || dk > DS_D || dv > DS_D || dk % 4 || dv % 4 || !scratch ||
+      n_min < 0 || dv <= 0 || dk > DS_D || dv > DS_D || dk % 4 || dv % 4 || !scratch ||
       (((uintptr_t)qkv | (uintptr_t)o_raw) & 15))
     return (int)cudaErrorInvalidValue;
-  const DsLayout l = ds_layout(T, B, H, G, dk, dv);
+  const DsLayout l = ds_layout(T, B, H, G, dk, dv, n_min);
   char* base = (char*)scratch;
   double* F = (double*)(base + l.F);
   double* g0 = (double*)(base + l.g0);

@@ -752,7 +752,7 @@ def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_hea
     fn = lib().bf_chunk_scan_scratch
     fn.restype = _c_ll
     n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
-           _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm))
+           _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm), _c_int(CHUNK_SCAN_MIN))
     if n > CHUNK_SCAN_MAX_BYTES:
         return None
     return torch.empty(n, dtype=torch.uint8, device=state.device)
@@ -1079,7 +1079,8 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
             and gates.is_contiguous() and qkv.data_ptr() % 16 == 0 and o_raw.data_ptr() % 16 == 0):
         fn = lib().bf_chunk_scan_delta_scratch
         fn.restype = _c_ll
-        n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv))
+        n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
+               _c_int(DELTA_CHUNK_MIN))
         if n <= CHUNK_SCAN_MAX_BYTES:
             scratch = torch.empty(n, dtype=torch.uint8, device=state.device)
     if scratch is not None:

@@ -1224,6 +1224,32 @@ def test_chunks_leave_earlier_tokens_alone(cuda_device, monkeypatch, kind, at):
     assert not bool(dirty[at, 1].isfinite().any())
 
 
+@pytest.mark.parametrize("kind", ["linear", "delta"])
+def test_chunks_beside_many_single_tokens(cuda_device, kind):
+    """A long portion has its chunks whatever else decodes in the step, and the same bits."""
+    from binfer_b200.csrc import ops
+    dev, n, singles, H, d = cuda_device, 400, 200, 64, 128
+    torch.manual_seed(6)
+    T, B, err, outs = n + singles, 1 + singles, _err(dev), []
+    x = torch.nn.functional.normalize(torch.randn(T, 2, H, d, device=dev), dim=-1)
+    v, decay = torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    for t, b in ((T, B), (n, 1)):
+        qs = torch.tensor([0] + list(range(n, t + 1)), dtype=torch.int32, device=dev)
+        slots = torch.arange(b, dtype=torch.int32, device=dev)
+        state, out = torch.zeros(b, H * d * d, device=dev), torch.empty(t, H * d, device=dev)
+        before = ops.launches()
+        if kind == "linear":
+            ops.linear_scan(x[:t], v[:t], decay[:t], state, qs, slots, out, b, H, H, d, d, err,
+                            max_q=n, chunked=True)
+        else:
+            qkv = torch.cat([x[:t].reshape(t, -1), v[:t].reshape(t, -1)], 1).contiguous()
+            ops.delta_scan(qkv, torch.stack([1 - decay, decay], 1)[:t].contiguous(), state, qs,
+                           slots, out, b, H, H, d, d, err, max_q=n, chunked=True)
+        assert ops.launches() - before == 5 + (b > 1)    # (the walk serves the single tokens)
+        outs.append((out[:n], state[0]))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("lens,H,dk,dv", [([161, 1, 192, 160, 257], 2, 24, 40),
                                           ([193], 3, 64, 100), ([320, 5], 1, 256, 64)])
 def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
