@@ -752,15 +752,20 @@ def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_hea
     fn = lib().bf_chunk_scan_scratch
     fn.restype = _c_ll
     n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
-           _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm), _c_int(CHUNK_SCAN_MIN))
+           _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)))
     if n > CHUNK_SCAN_MAX_BYTES:
         return None
     return torch.empty(n, dtype=torch.uint8, device=state.device)
 
 
-def _walk_limit(scratch: Optional[torch.Tensor], B: int, n_min: int = CHUNK_SCAN_MIN) -> int:
-    """For the kernels that walk: the longest portion they take (0: any, -1: none, the step's only
-    request has chunks)."""
+def _chunk_limit(B: int, n_min: int) -> int:
+    """For the kernels over chunks: the longest portion that is left to the walk (0: none, the step's
+    only request has chunks however many of its ``T`` rows are its own)."""
+    return 0 if B == 1 else n_min
+
+
+def _walk_limit(scratch: Optional[torch.Tensor], B: int, n_min: int) -> int:
+    """For the kernels that walk: the longest portion they take (0: any, -1: none)."""
     return 0 if scratch is None else -1 if B == 1 else n_min
 
 
@@ -770,7 +775,7 @@ def _chunk_scan_linear(name, qk, vf, decays, tok_decay, state, q_start, state_sl
          _ptr(tok_decay), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
          _c_int(state.shape[0]), _ptr(o_raw), _ptr(scratch), _c_int(vf.shape[0]), _c_int(B),
          _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv), _c_int(CHUNK_SCAN_TOKENS),
-         _c_int(CHUNK_SCAN_MIN), _ptr(err), _stream())
+         _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _ptr(err), _stream())
     global _launches
     _launches += 4          # five kernels
 
@@ -814,7 +819,7 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
          _ptr(positions), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
          _c_int(state.shape[0]), _ptr(o_raw), _ptr(qk), _ptr(vf), _c_int(T), _c_int(B),
          _c_int(max_q if max_q > 0 else T), _c_int(heads), _c_int(dk), _c_int(dv), _c_float(k_scale), _c_int(_dtype_code(proj)), _ptr(err),
-         _c_int(1 if silu else 0), _c_int(_walk_limit(scratch, B)), _stream())
+         _c_int(1 if silu else 0), _c_int(_walk_limit(scratch, B, CHUNK_SCAN_MIN)), _stream())
     global _launches
     _launches += 1          # two kernels: the rotation and the scan
     if scratch is not None:
@@ -850,12 +855,12 @@ def linear_scan(qk: torch.Tensor, vf: torch.Tensor, tok_decay: torch.Tensor, sta
     if scratch is not None:
         _chunk_scan_linear("linear_scan", qk, vf, None, tok_decay, state, q_start, state_slots,
                            o_raw, scratch, B, heads, qk_heads, dk, dv, err)
-        if _walk_limit(scratch, B) < 0:
+        if _walk_limit(scratch, B, CHUNK_SCAN_MIN) < 0:
             return
     _run("linear_scan", lib().bf_linear_scan, _ptr(qk), _ptr(vf), _ptr(tok_decay), _ptr(state),
          _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
          _ptr(o_raw), _c_int(T), _c_int(B), _c_int(max_q if max_q > 0 else T), _c_int(heads),
-         _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err), _c_int(_walk_limit(scratch, B)),
+         _c_int(qk_heads), _c_int(dk), _c_int(dv), _ptr(err), _c_int(_walk_limit(scratch, B, CHUNK_SCAN_MIN)),
          _stream())
 
 
@@ -1080,14 +1085,14 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
         fn = lib().bf_chunk_scan_delta_scratch
         fn.restype = _c_ll
         n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
-               _c_int(DELTA_CHUNK_MIN))
+               _c_int(_chunk_limit(B, DELTA_CHUNK_MIN)))
         if n <= CHUNK_SCAN_MAX_BYTES:
             scratch = torch.empty(n, dtype=torch.uint8, device=state.device)
     if scratch is not None:
         _run("delta_scan_chunks", lib().bf_chunk_scan_delta, _ptr(qkv), _ptr(gates), _ptr(state),
              _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
              _ptr(o_raw), _ptr(scratch), _c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads),
-             _c_int(dk), _c_int(dv), _c_int(DELTA_CHUNK_MIN), _ptr(err), _stream())
+             _c_int(dk), _c_int(dv), _c_int(_chunk_limit(B, DELTA_CHUNK_MIN)), _ptr(err), _stream())
         global _launches
         _launches += 4          # five kernels
         if _walk_limit(scratch, B, DELTA_CHUNK_MIN) < 0:
@@ -1451,17 +1456,17 @@ def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
              _ptr(gates), _ptr(state), _c_ll(state.stride(0)), _c_int(state.shape[2]),
              _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]), _ptr(o_raw),
              _ptr(scratch), _c_int(T), _c_int(B), _c_int(heads), _c_int(dk), _c_int(dv),
-             _c_float(q_scale), _c_int(CHUNK_SCAN_TOKENS), _c_int(CHUNK_SCAN_MIN), _ptr(err),
-             _stream())
+             _c_float(q_scale), _c_int(CHUNK_SCAN_TOKENS),
+             _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _ptr(err), _stream())
         global _launches
         _launches += 4          # five kernels
-        if _walk_limit(scratch, B) < 0:
+        if _walk_limit(scratch, B, CHUNK_SCAN_MIN) < 0:
             return
     _run("mlstm_scan", lib().bf_mlstm_scan, _ptr(proj), _c_ll(proj.stride(0)), _ptr(gates),
          _ptr(state), _c_ll(state.stride(0)), _c_int(state.shape[2]), _ptr(q_start),
          _ptr(state_slots), _c_int(state.shape[0]), _ptr(o_raw), _c_int(B), _c_int(heads),
          _c_int(dk), _c_int(dv), _c_float(q_scale), _c_int(_dtype_code(proj)), _ptr(err),
-         _c_int(_walk_limit(scratch, B)), _stream())
+         _c_int(_walk_limit(scratch, B, CHUNK_SCAN_MIN)), _stream())
 
 
 def mlstm_out(o_raw: torch.Tensor, proj: torch.Tensor, g_off: int, norm_w: torch.Tensor,

@@ -1224,6 +1224,40 @@ def test_chunks_leave_earlier_tokens_alone(cuda_device, monkeypatch, kind, at):
     assert not bool(dirty[at, 1].isfinite().any())
 
 
+@pytest.mark.parametrize("kind", ["linear", "delta", "mlstm", "retention"])
+@pytest.mark.parametrize("own", [1, 70, 300])
+def test_chunks_take_a_short_request_in_a_long_buffer(cuda_device, monkeypatch, kind, own):
+    """One request that owns the first rows of a buffer long enough for chunks, nothing said about
+    the longest portion: its rows are computed, the others left alone."""
+    from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN", 160)
+    dev, T, H, d = cuda_device, 300, 2, 32
+    torch.manual_seed(8)
+    qs = torch.tensor([0, own], dtype=torch.int32, device=dev)
+    slots, err, outs = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    x = torch.nn.functional.normalize(torch.randn(T, 2, H, d, device=dev), dim=-1)
+    v, decay = torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    flat = torch.cat([x.reshape(T, -1), v.reshape(T, -1)], 1).contiguous()
+    for chunked in (False, True):
+        out, state = torch.full((T, H * d), 7.0, device=dev), torch.zeros(1, H * d * d, device=dev)
+        if kind == "linear":
+            ops.linear_scan(x, v, decay, state, qs, slots, out, 1, H, H, d, d, err, chunked=chunked)
+        elif kind == "delta":
+            ops.delta_scan(flat, torch.stack([1 - decay, decay], 1).contiguous(), state, qs, slots,
+                           out, 1, H, H, d, d, err, chunked=chunked)
+        elif kind == "retention":
+            ops.retention_scan(flat, 0, H * d, 2 * H * d, decay[0].contiguous(), None,
+                               torch.arange(T, dtype=torch.int32, device=dev), state, qs, slots, out,
+                               1, H, d, d, 1.0, err, chunked=chunked)
+        else:
+            state = torch.zeros(1, H, ops.mlstm_state_size(d, d), device=dev)
+            ops.mlstm_scan(flat.to(BF16), torch.cat([decay, decay.log()], 1).contiguous(), state, qs,
+                           slots, out, 1, H, d, d, 1.0, err, chunked=chunked)
+        assert bool((out[own:] == 7.0).all())
+        outs.append(torch.cat([out[:own].flatten(), state.flatten()]))
+    _close(outs[1], outs[0], F32, scale=4)           # (sums of up to 300 terms, in other orders)
+
+
 @pytest.mark.parametrize("kind", ["linear", "delta"])
 def test_chunks_beside_many_single_tokens(cuda_device, kind):
     """A long portion has its chunks whatever else decodes in the step, and the same bits."""
