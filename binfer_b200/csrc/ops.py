@@ -480,8 +480,7 @@ def decode_attention_takes_capped(q: torch.Tensor, k_cache: torch.Tensor, nh: in
             and n_rows <= 512 and q.is_contiguous() and q.data_ptr() % 16 == 0)
 
 
-# scratch for the shares of split prefill attention, per device (grown as needed, up to a limit)
-_prefill_split_scratch = {}
+# most scratch for the shares of split prefill attention
 _PREFILL_SPLIT_BYTES = 256 << 20
 
 
@@ -556,18 +555,15 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         T = q.shape[0]
         need = T * nh * splits
         if need * d * 4 <= _PREFILL_SPLIT_BYTES:
-            key = q.device.index
-            buf = _prefill_split_scratch.get(key)
-            if buf is None or buf[0].numel() < need * d:
-                buf = _prefill_split_scratch[key] = (
-                    torch.empty(need * d, dtype=torch.float32, device=q.device),
-                    torch.empty(need * 2, dtype=torch.float32, device=q.device))
+            # (a call's own, from its stream's pool: runners on several streams share nothing)
+            part_o = torch.empty(need * d, dtype=torch.float32, device=q.device)
+            part_ml = torch.empty(need * 2, dtype=torch.float32, device=q.device)
             _run("prefill_attention_umma2", fn2,
                  _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(items), _c_int(n_items),
                  _c_int(max_rows), _c_int(T), _ptr(block_tables),
                  _c_int(block_tables.stride(0)), _ptr(out), _c_int(nh), _c_int(nkv), _c_int(d),
                  _c_int(page_size), _c_int(k_cache.shape[0]), _c_int(window or 0),
-                 _c_float(scale), _c_int(splits), _ptr(buf[0]), _ptr(buf[1]), _ptr(err),
+                 _c_float(scale), _c_int(splits), _ptr(part_o), _ptr(part_ml), _ptr(err),
                  *tail2, _stream())
             _launches += 1          # two kernels: the shares and their merge
             return

@@ -1500,6 +1500,36 @@ def test_prefill_attention_kept_tokens_and_sinks(cuda_device, nh, nkv, ps, windo
     _close(out.cpu(), torch.cat(refs).reshape(row, nh * d), BF16)
 
 
+def test_split_prefill_on_two_streams_shares_no_scratch(cuda_device, monkeypatch):
+    """The partial results of two calls on two streams lie in memory of their own."""
+    from binfer_b200.csrc import ops
+    nh, d, n, rows = 2, 128, 3000, 64
+    q, kc, vc, sot, pos, bt, ref = _attention_case(cuda_device, BF16, nh, 1, d, 16, [n], [rows],
+                                                   None, False, seed=31)
+    items = torch.tensor([[0, 0, rows, n - rows]], dtype=torch.int32, device=cuda_device)
+    real, spans = ops._run, []
+
+    def spy(name, fn, *args):
+        o, ml, splits = args[18].value, args[19].value, args[17].value
+        size = rows * nh * splits * 4
+        spans.extend([(o, o + size * d), (ml, ml + 2 * size)])
+        real(name, fn, *args)
+    monkeypatch.setattr(ops, "_run", spy)
+    outs, err = [], _err(cuda_device)
+    for _ in range(2):
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            outs.append(torch.zeros_like(q))
+            ops.prefill_attention(q, kc, vc, items, 1, rows, bt, outs[-1], nh, 1, d, None, d ** -0.5,
+                                  err, variant="umma2", max_ctx=n)
+    torch.cuda.synchronize()
+    spans.sort()
+    assert len(spans) == 4 and all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
+    for out in outs:
+        _close(out, ref, BF16)
+
+
 # ----------------------------------------------------------------- float32 attention in tiles
 # rows below, at and above a tile of 64 and of 4, portions from the start and behind cached keys, a
 # window inside, at and above a key tile
