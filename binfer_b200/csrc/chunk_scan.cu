@@ -189,7 +189,11 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
   double* hs = Hs + (size_t)h * T + t0;
   const double fixed = MLSTM || tok_decay ? 0.0 : cs_log_decay(decays[h]);
   auto log_decay = [&](int t) -> double {
-    if (MLSTM) return (double)gates[(size_t)(t0 + t) * 2 * H + H + h];
+    if (MLSTM) {
+      // (-inf, a gate that is shut: exp(-1e5) is zero, and the sums behind it stay numbers)
+      const double f = (double)gates[(size_t)(t0 + t) * 2 * H + H + h];
+      return f < -1e5 ? -1e5 : f;
+    }
     return tok_decay ? cs_log_decay(tok_decay[(size_t)(t0 + t) * decay_stride + h]) : fixed;
   };
   double F = 0.0;

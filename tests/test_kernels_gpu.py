@@ -1224,6 +1224,30 @@ def test_chunks_leave_earlier_tokens_alone(cuda_device, monkeypatch, kind, at):
     assert not bool(dirty[at, 1].isfinite().any())
 
 
+def test_mlstm_chunks_take_shut_gates(cuda_device):
+    """A log forget gate of -inf forgets what came before, a log input gate of -inf keeps its token
+    out: the chunks give numbers there, the walk's."""
+    from binfer_b200.csrc import ops
+    dev, T, H, d = cuda_device, 300, 2, 32
+    torch.manual_seed(9)
+    proj = torch.randn(T, 4 * H * d, device=dev).to(BF16)
+    gates = torch.cat([torch.randn(T, H, device=dev),
+                       torch.nn.functional.logsigmoid(2 + torch.randn(T, H, device=dev))], 1).contiguous()
+    gates[[64, 100, 101, 299], H] = float("-inf")
+    gates[[70, 128], 1] = float("-inf")
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, outs = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    for chunked in (False, True):
+        out, state = torch.empty(T, H * d, device=dev), torch.zeros(
+            1, H, ops.mlstm_state_size(d, d), device=dev)
+        ops.mlstm_scan(proj, gates, state, qs, slots, out, 1, H, d, d, d ** -0.5, err, max_q=T,
+                       chunked=chunked)
+        outs.append(torch.cat([out.flatten(), state.flatten()]))
+    assert bool(outs[0].isfinite().all())
+    # as close as two orders of sums behind a quotient are (its denominator may be small)
+    assert float((outs[1] - outs[0]).norm() / outs[0].norm()) <= 2e-5
+
+
 @pytest.mark.parametrize("kind", ["linear", "delta", "mlstm", "retention"])
 @pytest.mark.parametrize("own", [1, 70, 300])
 def test_chunks_take_a_short_request_in_a_long_buffer(cuda_device, monkeypatch, kind, own):
