@@ -185,16 +185,22 @@ template <int BM, int BN, int BK, int TM, int TN>
 static void sgemm_go(const float* A, const float* W, float* C, int M, int N, int K, long long lda,
                      long long ldw, long long ldc, int batch, long long batch_a,
                      long long batch_w, long long batch_c, cudaStream_t stream) {
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-  constexpr int threads = (BM / TM) * (BN / TN);
+  constexpr int threads = (BM / TM) * (BN / TN), most = 65535 * BM;   // (rows of a launch)
   const bool vec = ((K | lda | ldw | batch_a | batch_w) & 3) == 0 &&
                    (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-  if (vec)
-    sgemm_nt_kernel<BM, BN, BK, TM, TN, true><<<grid, threads, 0, stream>>>(
-        A, W, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);
-  else
-    sgemm_nt_kernel<BM, BN, BK, TM, TN, false><<<grid, threads, 0, stream>>>(
-        A, W, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);
+  for (int m0 = 0; m0 < M; m0 += most) {
+    const int m = M - m0 < most ? M - m0 : most;
+    const dim3 grid((N + BN - 1) / BN, (m + BM - 1) / BM, batch);
+    const float* a = A + m0 * lda;
+    float* c = C + m0 * ldc;
+    if (vec)
+      sgemm_nt_kernel<BM, BN, BK, TM, TN, true><<<grid, threads, 0, stream>>>(
+          a, W, c, m, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);
+    else
+      sgemm_nt_kernel<BM, BN, BK, TM, TN, false><<<grid, threads, 0, stream>>>(
+          a, W, c, m, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);
+    if (M - m0 <= most) break;
+  }
 }
 
 static int sgemm_nt_launch(const float* A, const float* W, float* C, int M, int N, int K,

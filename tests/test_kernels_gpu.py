@@ -115,6 +115,16 @@ def test_sgemm_tiles_and_alignments_agree(cuda_device, M, N, K):
     assert torch.equal(one[0], out[M - 1])
 
 
+def test_sgemm_more_rows_than_a_grid_has_tiles(cuda_device):
+    from binfer_b200.csrc import ops
+    M = 64 * 65535 + 70
+    a, w = torch.randn(M, 4, device=cuda_device), torch.randn(3, 4, device=cuda_device)
+    out = torch.full((M, 3), 7.0, device=cuda_device)
+    ops.sgemm_nt(a, w, out)
+    bound = 5 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)     # four products, their sums
+    assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
+
+
 # ------------------------------------------------------- q/k norm, rotation, cache write
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("nh,nkv,d,rot,norm", [(3, 1, 16, 16, True), (4, 2, 48, 24, True),
