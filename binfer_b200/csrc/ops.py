@@ -56,9 +56,15 @@ def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
     return _c_void_p(t.data_ptr())
 
 
+# torch.cuda.current_stream() builds an object behind several checks: 3 us of every launch.  (The name
+# is not part of torch's public interface: where it is missing, the public one serves.)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> _c_void_p:
-    # (torch.cuda.current_stream() builds an object behind several checks: 3 us of every launch)
-    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    if _raw_stream is None:
+        return _c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _c_void_p(_raw_stream(torch.cuda.current_device()))
 
 
 def _check(code: int, what: str) -> None:

@@ -22,6 +22,16 @@ def _err(dev):
     return torch.zeros(1, dtype=torch.int32, device=dev)
 
 
+def test_launches_go_to_the_current_stream(cuda_device, monkeypatch):
+    from binfer_b200.csrc import ops
+    for _ in range(2):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            assert ops._stream().value == s.cuda_stream
+        assert (ops._stream().value or 0) == torch.cuda.current_stream().cuda_stream
+        monkeypatch.setattr(ops, "_raw_stream", None)      # a torch without the private name
+
+
 # ------------------------------------------------------------------ elementwise
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_embed_gather(cuda_device, dtype):
