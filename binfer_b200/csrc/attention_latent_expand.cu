@@ -8,8 +8,9 @@
 // rows pays for it, a single token does not.  1,800 rows behind 500 cached keys, 16 heads: 964 us in
 // latent coordinates (mma.sync, 91 TFLOP/s); 4.6 us for this kernel, 11 for the product and 60 for
 // the attention (tcgen05; 432 TFLOP/s of the 26 GFLOP that are left), and the two products that
-// carry queries into latent coordinates and results out of them fall away.  The layer: 1,061 ->
-// 143 us.
+// carry queries into latent coordinates and results out of them fall away (for the single tokens of a
+// mixed step they stay: for their rows alone where they come first, as the scheduler puts them, else
+// for all rows).  The layer: 1,061 -> 143 us.
 #include "common.cuh"
 
 // A warp per row.  Portion i's keys (items[i]: request, first token row, rows, first position) take

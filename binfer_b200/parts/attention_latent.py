@@ -153,13 +153,19 @@ class LatentAttention(Mixer, StackedOut):
         else:
             q = proj[:, :self.q_size]
         rows = self._expanded_rows(q, out, ctx)
-        cache = view.k_cache
-        if not rows or ctx.n_decode:
-            self._in_latent_coordinates(q, proj, out, ctx, view, n_max=1 if rows else 0)
-            cache = None                     # (stored)
+        cache, lead = view.k_cache, 0
+        if not rows:
+            self._in_latent_coordinates(q, proj, out, ctx, view, T)
+        elif ctx.n_decode:
+            # single tokens in front of the portions, as the scheduler puts them, are a step of
+            # their own; elsewhere all rows go through the products and the attention takes theirs
+            lead = next(b for b, n in enumerate(ctx.q_lens) if n != 1)
+            lead = lead if lead == ctx.n_decode else 0
+            self._in_latent_coordinates(q, proj, out, ctx, view, lead or T, n_max=1)
+            if not lead:
+                cache = None                     # (stored)
         if rows:
-            # (a step's single tokens went the other way; their rows of q are not read again)
-            self._encode(proj, q, None, cache, ctx, g)
+            self._encode(proj, q, None, cache, ctx, g, lead, T)
             lat, rot, base = ops.latent_gather(view.k_cache, ctx.block_tables[g],
                                                ctx.prefill_items, ctx.n_prefill, rows, self.rank,
                                                ctx.err)
@@ -191,32 +197,39 @@ class LatentAttention(Mixer, StackedOut):
             return 0
         return rows
 
-    def _encode(self, proj, q, q_abs, cache, ctx: StepContext, group) -> None:
+    def _encode(self, proj, q, q_abs, cache, ctx: StepContext, group, first: int,
+                last: int) -> None:
+        """Rows ``first .. last - 1`` of the step; ``q_abs`` (None: in place) begins with the first."""
         s, pos = self.spec, self.position
-        ops.latent_encode(proj, 0, self.q_rows, self.norm_w, s.norm_eps,
+        ops.latent_encode(proj[first:last], 0, self.q_rows, self.norm_w, s.norm_eps,
                           pos.inv_freq if pos is not None else None,
                           bool(pos is not None and pos.interleaved),
-                          pos.magnitude if pos is not None else 1.0, ctx.positions,
-                          ctx.slots[group], q_abs, cache, self.H, self.d, self.dr, self.rank,
-                          ctx.err, q=q)
+                          pos.magnitude if pos is not None else 1.0, ctx.positions[first:last],
+                          ctx.slots[group][first:last], q_abs, cache, self.H, self.d, self.dr,
+                          self.rank, ctx.err, q=q[first:last])
 
-    def _in_latent_coordinates(self, q, proj, out, ctx: StepContext, view: EntryView,
-                               n_max: int) -> None:
-        """The step's rows (``n_max`` > 0: those of requests with at most so many tokens) with the
-        queries carried into latent coordinates; ``q`` is left as it is."""
-        s, T, H, g = self.spec, q.shape[0], self.H, view.group
+    def _in_latent_coordinates(self, q, proj, out, ctx: StepContext, view: EntryView, T: int,
+                               n_max: int = 0) -> None:
+        """The step's first ``T`` rows (``n_max`` > 0: those of requests with at most so many tokens;
+        what ``out`` holds for the others says nothing) with the queries carried into latent
+        coordinates; ``q`` is left as it is."""
+        s, H, g = self.spec, self.H, view.group
+        B = T if T < q.shape[0] else ctx.B       # (fewer rows than the step's: single tokens)
+        q, proj, out = q[:T], proj[:T], out[:T]
         q_abs = torch.empty((T, H, self.kv_size), dtype=q.dtype, device=q.device)
-        self._encode(proj, q, q_abs, view.k_cache, ctx, g)
+        self._encode(proj, q, q_abs, view.k_cache, ctx, g, 0, T)
         q_heads = q.view(T, H, self.d + self.dr)
         linear_heads(q_heads[:, :, :self.d], self.w_ukT, q_abs[:, :, :self.rank])
-        o_lat = torch.empty((T, H, self.rank), dtype=q.dtype, device=q.device)
+        # (rows that the attention leaves alone go through the product behind it as zeros)
+        o_lat = (torch.zeros if n_max and B < T else torch.empty)(
+            (T, H, self.rank), dtype=q.dtype, device=q.device)
         if (TENSOR_CORES and s.softmax_scale > 0
                 and ops.latent_attention_takes(q.dtype, self.rank, self.dr)):
             # bfloat16: tiles of (token, head) rows against tiles of cache rows, each fetched
             # once as keys and values, on the tensor cores
             few = ctx.decode_only or n_max == 1
             ops.latent_attention(q_abs, view.k_cache, ctx.q_start, ctx.positions,
-                                 ctx.block_tables[g], o_lat, ctx.B,
+                                 ctx.block_tables[g], o_lat, B,
                                  1 if few else ctx.max_q_len, H, self.rank,
                                  s.softmax_scale, ctx.err,
                                  max_ctx=ctx.max_decode_ctx if n_max == 1 else ctx.max_ctx_len,

@@ -1492,6 +1492,70 @@ def test_latent_part_expands_portions_beside_single_tokens(cuda_device, monkeypa
     assert float((plain - expanded).abs().max()) <= 6e-2 * float(plain.abs().max())
 
 
+@pytest.mark.parametrize("order", ["single tokens first", "portions first", "a short portion"])
+def test_latent_part_chooses_and_splits_a_mixed_step(cuda_device, monkeypatch, order):
+    """The part's own rule on a step of single tokens and a portion: a long portion is expanded and
+    the single tokens in front of it are the only rows in latent coordinates, a short one is not."""
+    from binfer_b200.config import FolivikConfig
+    from binfer_b200.csrc import ops
+    from binfer_b200.engine import StepItem, make_env, make_runner, model_from_seed
+    H = 2
+    cfg = FolivikConfig.from_dict({"vocab": 64, "width": 256, "norm": {"eps": 1e-5}, "layers": [
+        {"type": "latent_attention", "mlp": None, "mixer": {
+            "heads": H, "dim": 128, "rot_dim": 64, "vdim": 128, "kv_rank": 64, "q_rank": 96,
+            "scale": 192 ** -0.5, "rot": {"base": 1e4, "dims": 64}}}]})
+    env = make_env(BF16)
+    model = model_from_seed(cfg, env, seed=3, std=0.06)
+    runner = make_runner(model, env, page_size=16, num_pages=120, max_requests=4)
+    mixer, view = model.blocks[0].mixer, runner.views[0]
+    long = 200 if order == "a short portion" else 1200
+    lens = [(30, 1), (5, 1), (0, long)]
+    if order == "portions first":
+        lens = lens[::-1]
+    calls = {"gather": 0, "rows": []}
+    gather, attend = ops.latent_gather, ops.latent_attention
+
+    def spy_gather(*a, **k):
+        calls["gather"] += 1
+        return gather(*a, **k)
+
+    def spy_attend(q, *a, **k):
+        calls["rows"].append(q.shape[0])
+        return attend(q, *a, **k)
+    monkeypatch.setattr(ops, "latent_gather", spy_gather)
+    monkeypatch.setattr(ops, "latent_attention", spy_attend)
+
+    def one(expands):
+        mixer.expands = expands
+        torch.manual_seed(6)
+        for i, (b, n) in enumerate(lens):
+            runner.add_request(i)
+            if b:
+                x = torch.randn(b, 256, device=cuda_device).to(BF16)
+                runner.reserve([StepItem(i, [0] * b)])
+                mixer.forward(x, runner.build_context([StepItem(i, [0] * b)]), view)
+                runner.cache.commit(i, b)
+        items = [StepItem(i, [0] * n) for i, (_, n) in enumerate(lens)]
+        runner.reserve(items)
+        x = torch.randn(sum(n for _, n in lens), 256, device=cuda_device).to(BF16)
+        calls["gather"], calls["rows"] = 0, []
+        y = mixer.forward(x, runner.build_context(items), view)
+        for i in range(len(lens)):
+            runner.free_request(i)
+        runner.check_errors()
+        return y.double(), calls["gather"], calls["rows"]
+
+    plain, gathers, rows = one(False)
+    assert gathers == 0 and rows == [long + 2]
+    expanded, gathers, rows = one(True)
+    if order == "a short portion":
+        assert gathers == 0 and rows == [long + 2]
+    else:
+        assert gathers == 1 and rows == [2 if order == "single tokens first" else long + 2]
+    assert float((plain - expanded).norm() / plain.norm()) <= 1.5e-2
+    assert float((plain - expanded).abs().max()) <= 6e-2 * float(plain.abs().max())
+
+
 # a window of one token, below, at and above a key tile and wider than some portions; kept tokens
 # inside a tile, a whole tile, more than a tile and more than lies before the window; portions with
 # cached keys; sinks alone with the keys shared out
