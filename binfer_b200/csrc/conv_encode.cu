@@ -22,7 +22,8 @@
 // One warp per (token, head); heads are counted q heads, then k heads, then v heads.  Keys and values
 // of one size of 16, 32, 64 or 128 with at most four taps: four channels a thread over a run of tokens
 // instead, a head in d / 4 neighbouring lanes, its rotation and its sum of squares by shuffles
-// (conv_encode_run_kernel; 2,118 tokens of 16 + 8 + 8 heads of 128, 3 taps: 32 us, 55 on the other).  The
+// (conv_encode_run_kernel; 2,048 tokens of 16 + 8 + 8 heads of 128, 3 taps: 26 us, 51 on the other; 256
+// tokens 8 and 11).  The
 // cosines and sines of a token's angles are taken once for all its heads, by a small kernel
 // in front.  All
 // arithmetic is float; only the projection's values and the stored results have the
@@ -313,6 +314,7 @@ BF_EXPORT int bf_conv_encode(
   const long long C = ((long long)nh + 2 * nkv) * dk;
   const uintptr_t quad = 4 * esz - 1;
   if (dk == dv && (dk == 16 || dk == 32 || dk == 64 || dk == 128) && C % 128 == 0 && taps <= 4 &&
+      ct_aligned(conv_w, state, state_stride) &&
       rot_half % 4 == 0 && stride % 4 == 0 && q_stride % 4 == 0 &&
       (((uintptr_t)proj | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & quad) == 0 &&
       ((uintptr_t)rope_table & 15) == 0 && T <= 65535 * 8) {

@@ -30,6 +30,11 @@ __device__ __forceinline__ float4 ct_silu4(float4 y) {
   return make_float4(ct_silu(y.x), ct_silu(y.y), ct_silu(y.z), ct_silu(y.w));
 }
 
+// Whether weights and states can be read so (channels in fours).
+static inline bool ct_aligned(const float* conv_w, const float* state, long long state_stride) {
+  return ((((uintptr_t)conv_w | (uintptr_t)state) & 15) | (state_stride & 3)) == 0;
+}
+
 // Tokens of a run, for `units` threads of four channels a token: runs share fetches, but a step of
 // few tokens needs its threads.
 static inline int ct_run(long long T, long long units) {
@@ -42,10 +47,19 @@ struct ConvTaps {
   float4 h[TAPS > 1 ? TAPS - 1 : 1];         // the values before the current one, oldest first
 
   __device__ __forceinline__ void weights(const float* __restrict__ conv_w, int c) {
-    const float* p = conv_w + (size_t)c * TAPS;
+    // four channels' taps side by side, in 16-byte pieces
+    float v[4 * TAPS];
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) {
+      const float4 x = ct_ld4(conv_w + (size_t)c * TAPS + 4 * j);
+      v[4 * j] = x.x;
+      v[4 * j + 1] = x.y;
+      v[4 * j + 2] = x.z;
+      v[4 * j + 3] = x.w;
+    }
 #pragma unroll
     for (int j = 0; j < TAPS; ++j)
-      w[j] = make_float4(p[j], p[TAPS + j], p[2 * TAPS + j], p[3 * TAPS + j]);
+      w[j] = make_float4(v[j], v[TAPS + j], v[2 * TAPS + j], v[3 * TAPS + j]);
   }
   // the values before the request's token `local` of this step, whose row is `row`
   template <typename A>
@@ -57,8 +71,7 @@ struct ConvTaps {
       if (local >= back) {
         h[j] = ct_ld4(row - (size_t)back * stride + c);
       } else {
-        const float* s = st + (size_t)(TAPS - 1 + local - back) * C + c;
-        h[j] = make_float4(s[0], s[1], s[2], s[3]);
+        h[j] = ct_ld4(st + (size_t)(TAPS - 1 + local - back) * C + c);
       }
     }
   }

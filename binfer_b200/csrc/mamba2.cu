@@ -85,8 +85,9 @@ __global__ void mamba2_encode_kernel(
 }
 
 // The same, four channels a thread over a run of tokens (conv_taps.cuh), for heads and groups that
-// are a multiple of four wide.  2,008 tokens of 4,096 + 2 x 1,024 channels, 4 taps: 45 us
-// (bfloat16 in, float out), 112 with a warp per token.
+// are a multiple of four wide.  2,048 tokens of 4,096 + 2 x 1,024 channels, 4 taps: 40 us
+// (bfloat16 in, float out), 112 with a warp per token; 256 tokens 10 and 16 (19 with the weights read
+// number by number, a line of their own each).
 template <typename A, int TAPS>
 __global__ void __launch_bounds__(128) mamba2_encode_run_kernel(
     const A* __restrict__ proj, long long stride, long long xbc_off, long long dt_off,
@@ -140,7 +141,7 @@ static bool mamba2_encode_run(const A* proj, long long stride, long long xbc_off
                               const float* A_log, const float* dt_bias, const float* D, float* qk,
                               float* vf, float* skip, float* decay, int T, int H, int G, int N,
                               int P, int* err, cudaStream_t stream) {
-  if (taps < 1 || taps > 4 || P % 4 || N % 4 || stride % 4 || xbc_off % 4 ||
+  if (taps < 1 || taps > 4 || !ct_aligned(conv_w, state, state_stride) || P % 4 || N % 4 || stride % 4 || xbc_off % 4 ||
       ((uintptr_t)proj & (4 * sizeof(A) - 1)) ||
       (((uintptr_t)qk | (uintptr_t)vf | (uintptr_t)skip) & 15))
     return false;

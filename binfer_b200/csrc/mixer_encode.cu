@@ -268,8 +268,8 @@ __global__ void delta_encode_kernel(
 
 // The same, four channels a thread over a run of tokens (conv_taps.cuh): keys and values of one size
 // of 16, 32, 64 or 128, a head in d / 4 neighbouring lanes.  Behind the channels H threads take the
-// gates.  1,805 tokens of 16 + 16 heads of 128, 4 taps: 42 us, 62 with a
-// warp per (token, head).
+// gates.  2,048 tokens of 8 + 8 + 16 heads of 128, 4 taps: 22 us, 65 with a
+// warp per (token, head); 256 tokens 7 and 11.
 template <typename A, int TAPS>
 __global__ void __launch_bounds__(128) delta_encode_run_kernel(
     const A* __restrict__ proj, long long stride, const float* __restrict__ conv_w,
@@ -322,7 +322,7 @@ static bool delta_encode_run(const A* proj, long long stride, const float* conv_
                              int dk, int dv, float unit_eps, float q_scale, int* err,
                              cudaStream_t stream) {
   const long long C = (2LL * G + H) * dk;
-  if (taps < 1 || taps > 4 || dk != dv || (dk != 16 && dk != 32 && dk != 64 && dk != 128) ||
+  if (taps < 1 || taps > 4 || !ct_aligned(conv_w, state, state_stride) || dk != dv || (dk != 16 && dk != 32 && dk != 64 && dk != 128) ||
       C % 128 || stride % 4 || ((uintptr_t)proj & (4 * sizeof(A) - 1)) || ((uintptr_t)qkv & 15))
     return false;
   const int units = (int)(C / 4) + H, run = ct_run(T, units);
