@@ -164,6 +164,7 @@ class MoEFeedForward(FeedForward, StackedOut):
             return False
         saved = T * (self.E - self.top) - 128 * self.E          # rows, of one expert each
         return (6 * saved * self.ff * self.hidden >= GROUPED_MIN_FLOPS
+                and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
                 and ops.moe_grouped_takes(T, self.hidden, self.E, self.ff, self.ff_sh, self.top))
 
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:

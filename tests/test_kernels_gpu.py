@@ -1922,3 +1922,37 @@ def test_moe_grouped(cuda_device, T, width, E, ff, ff_sh, top, ident, gate, kind
         ref += rw[:, -1:].double() * x
     assert int(err.item()) == 0
     _close(out, ref, BF16)
+
+
+@pytest.mark.parametrize("identity,shared,gate", [(2, 64, True), (0, 0, False)])
+def test_moe_part_takes_the_chosen_experts_alone(cuda_device, monkeypatch, identity, shared, gate):
+    """The part's own rule and what it hands over, against every expert for every token; a column
+    block that the grouped kernels cannot read stays there."""
+    from binfer_b200.config import MoESpec
+    from binfer_b200.csrc import ops
+    from binfer_b200.engine import make_env
+    from binfer_b200.parts import moe
+    dev, T, width, E = cuda_device, 1100, 256, 8
+    spec = MoESpec(num_experts=E, top=2, expert_size=64, shared_size=shared, shared_gate=gate,
+                   identity=identity, scoring="softmax_all" if identity else "softmax_top")
+    part = moe.MoEFeedForward(spec, width, "", make_env(BF16))
+    torch.manual_seed(12)
+    part.load(lambda s: (torch.randn(s.shape, device=dev) * s.shape[-1] ** -0.5).to(
+        F32 if s.role == "vector" else BF16))
+    wide = torch.randn(T, width + 8, device=dev).to(BF16)
+    x, calls, grouped = wide[:, :width].contiguous(), [], ops.moe_grouped
+    monkeypatch.setattr(ops, "moe_grouped", lambda *a, **k: (calls.append(1), grouped(*a, **k)))
+    every = part.forward(x, None).double()                   # (far fewer operations than the rule's)
+    assert not calls
+    monkeypatch.setattr(moe, "GROUPED_MIN_FLOPS", 1)
+    chosen = part.forward(x, None).double()
+    assert len(calls) == 1
+    # activations rounded to bfloat16 and results rounded once on either side
+    assert float((chosen - every).norm() / every.norm()) <= 1e-2
+    assert float((chosen - every).abs().max()) <= 2.0 ** -6 * float(every.abs().max())
+    wide[:, 1:1 + width] = x
+    apart = part.forward(wide[:, 1:1 + width], None).double()
+    assert len(calls) == 1 and float((apart - every).norm() / every.norm()) <= 1e-2
+    monkeypatch.setattr(moe, "GROUPED", False)
+    part.forward(x, None)
+    assert len(calls) == 1
