@@ -9,22 +9,26 @@
 // H_s) (linear: i = m = 0 and G = H = F), token s reaches token t with the weight exp(G_t - H_s)
 // <= 1 and the state before a chunk whose last earlier token is c with exp(G_t - G_c); for the
 // mLSTM m_t = F_t - G_t.  F, G and H are double, so a difference of two of them is good to a
-// float's last bit; every product below is float (FP32 multiply-adds, no tensor-core mode), every
-// sum of one order.  Per chunk of `C` tokens and head:
+// float's last bit; its exponential is a float and what is left of it (cs_exp), the products of q and k
+// (and of k and k) inside a chunk are summed in double and rounded once, every other product is float
+// (FP32 multiply-adds, no tensor-core mode), every sum of one order.  Per chunk of `C` tokens and head:
 //
-//   cs_gates   F, G, H of every token; one block per (head, request)
-//   cs_qk      Q K^T of a chunk, once per q/k head (several heads may share them)
+//   cs_gates   F, G, H of every token, its weight behind its chunk; one block per (head, request)
+//   cs_qk      Q K^T of a chunk, once per q/k head (several heads may share them), in double
 //   cs_state   U = sum_s exp(G_last - H_s) k_s v_s^T: what the chunk adds to the state
 //   cs_prefix  from chunk to chunk: S <- exp(G_last - G_c) S + U; U's place takes the state before
 //              the chunk; the request's slot takes the last one
 //   cs_out     o = [exp(G_t - G_c) q_t | exp(G_t - H_s) (q_t . k_s)] [S ; V]: one product with dk +
 //              C terms, the weights applied as its operands are stored into shared memory
 //
-// Measured (GPU time of the kernels / of the walk): 2,000 tokens, 64 heads of 128 x 64 over 8
-// q/k heads: 220 / 459 us (cs_out 96, cs_state 76, cs_prefix 23, cs_qk 14, cs_gates 11); 2,048 tokens
-// of 8 heads of 128 x 256: 127 / 289; mLSTM, 8 heads of 256 x 512: 394 / 979 (168, 138, 54, 22, 12).
-// Error against 64 bits, decays of 0.98 to 1: o 1.4e-7 (walk 1.9e-7), state 1.1e-7 (1.8e-7); mLSTM: o
-// 5e-6 (2e-5), state 0.9e-7 (4.0e-7).
+// GPU time at 2,048 tokens (the walk at 2,000): 64 heads of 128 x 64 over 8 q/k heads 211 us (459; cs_out
+// 100, cs_state 62, cs_prefix 26, cs_qk 14, cs_gates 9); 8 heads of 128 x 256 126 (289); mLSTM, 8 heads of
+// 256 x 512, 394 (979; 172, 123, 55, 32, 11).  With expf, float products of q and k and the states' sums
+// in runs of 16 these were 204, 119 and 381 us, and further from 64 bits than the walk where decays are
+// fast.  Relative errors against 64 bits over 777 tokens, walk / chunks: decays of 0.98 to 1: o 1.9e-7 /
+// 1.4e-7, state 1.8e-7 / 1.3e-7; spread over 0 to 1: o 8.3e-8 / 5.0e-8, state 4.0e-8 / 4.2e-8 (half a unit
+// in the last place is up to 6.0e-8); mLSTM, gates that forget in a few tokens and in twenty: o 4.8e-7 /
+// 2.3e-7 and 1.3e-5 / 1.2e-6, state 2.9e-8 / 3.7e-8 and 2.3e-7 / 1.0e-7.
 //
 // Why: the walk has heads x dk x dv independent elements and a chain of multiply-adds from token to
 // token, so it left the FP32 pipes at 15 to 20 % (see those files); the products have no chain and
@@ -36,15 +40,20 @@
 // before it,  (I + L) U = beta (V - e^F K S0),  L_ts = beta_t exp(F_t - F_s) (k_t . k_s) below the
 // diagonal.  So with T = (I + L)^-1:
 //
+//   cs_qk      K K^T as well
 //   ds_prep    per chunk and head: L, T (by blocks of 16), W = T (beta e^F K) and Y = T (beta V)
 //   ds_walk    from chunk to chunk: U = Y - W S, S <- exp(F_C) S + K^T (exp(F_C - F) U); leaves U and
 //              the states between chunks.  The only chain: two products a chunk, over (request, head,
 //              32 columns) in parallel
 //   cs_out     as above, on U
 //
-// 1,111 and 694 tokens of 16 heads of 128: 240 us (ds_walk 115, ds_prep 53, cs_out 47, cs_qk 13) against
-// the walk's 366; 2,048 tokens of 32 heads 430 against 730.  Error against 64 bits: o 9.5e-8 (walk
-// 7.3e-8), state 7.6e-8 (7.8e-8).
+// 2,048 tokens of 16 heads of 128: 342 us (ds_walk 186, cs_out 55, ds_prep 49, cs_qk 42); 1,000 tokens 168
+// against the walk's 277, three portions of 1,000 381 against 431.  Errors against 64 bits, walk / chunks:
+// keys at random, decays of 0.98 to 1: o 2.3e-7 / 1.6e-7, state 2.3e-7 / 1.8e-7; keys of a cosine of 0.9
+// 2.6e-7 / 2.6e-7 and 2.5e-7 / 2.5e-7; fast decays o 1.1e-7 / 7.8e-8, state 6.2e-8 / 7.1e-8.  (What the walk
+// has and a chunk's inverse has not is that a token's u answers to the rounding of the one before it:
+// where queries, too, lie along what all keys share, a cosine of 0.9 on both sides and slow decays, the
+// outputs are 3e-7 from 64 bits and the walk's 0.8e-7.)
 //
 // Requests of at most `n_min` tokens have no chunks here (the walk serves them).  The order of sums
 // depends on where a step's portions begin, so the float32 engine, whose results must not depend
@@ -89,6 +98,36 @@ __device__ __forceinline__ float4 cs_ld4(const __nv_bfloat16* p) {
 __device__ __forceinline__ float4 cs_zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ float4 cs_times(float4 v, float f) {
   return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+}
+
+// v (hi + lo), rounded once
+__device__ __forceinline__ float cs_times(float v, float2 w) { return fmaf(v, w.x, v * w.y); }
+__device__ __forceinline__ float4 cs_times(float4 v, float2 w) {
+  return make_float4(cs_times(v.x, w), cs_times(v.y, w), cs_times(v.z, w), cs_times(v.w, w));
+}
+
+// e^x as a float and what is left of it, good to some 2^-28: x = n ln 2 + r in double, the power series
+// of e^r to the seventh power (|r| <= ln 2 / 2: the eighth is below 2^-27) on top of 1 + r, whose
+// rounding is kept.  (The weights of tokens hang together in every result: with expf, up to two units
+// off in the last place, an output of keys and queries alike was four times as far from 64 bits as
+// the walk's.)
+__device__ __forceinline__ float2 cs_exp(double x) {
+  if (!(x > -104.0)) return make_float2(x != x ? NAN : 0.f, 0.f);
+  if (x > 89.0) return make_float2(INFINITY, 0.f);
+  const int n = __double2int_rn(x * 1.4426950408889634);
+  const double r = fma((double)n, -0.69314718055994531, x);
+  const float rh = (float)r, rl = (float)(r - (double)rh);
+  float q = fmaf(rh, 1.f / 5040.f, 1.f / 720.f);
+  q = fmaf(rh, q, 1.f / 120.f);
+  q = fmaf(rh, q, 1.f / 24.f);
+  q = fmaf(rh, q, 1.f / 6.f);
+  q = fmaf(rh, q, 0.5f);
+  const float s = 1.f + rh, rest = fmaf(rh * rh, q, (rh - (s - 1.f)) + rl);
+  const float hi = s + rest, lo = rest - (hi - s);
+  // (two factors: n may lie below the smallest normal exponent)
+  const int n1 = n >> 1;
+  const float f1 = __int_as_float((n1 + 127) << 23), f2 = __int_as_float((n - n1 + 127) << 23);
+  return make_float2(hi * f1 * f2, lo * f1 * f2);
 }
 
 // ------------------------------------------------------------------------ which chunk is it
@@ -140,7 +179,7 @@ __device__ __forceinline__ CsChunk cs_find(const int* __restrict__ q_start, int 
 }
 
 // ------------------------------------------------------------------------------- cs_gates
-#define CS_GATE_THREADS 256
+#define CS_GATE_THREADS 512
 
 __device__ __forceinline__ double cs_log_decay(float d) {
   // a decay that underflowed to zero forgets everything: exp(-1e4) is zero in float.  One below zero
@@ -175,8 +214,9 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
     const float* __restrict__ decays, const float* __restrict__ tok_decay,
     const float* __restrict__ gates, float* __restrict__ state, long long slot_stride,
     int state_size, const int* __restrict__ q_start, const int* __restrict__ state_slots,
-    int n_slots, double* __restrict__ G, double* __restrict__ Hs, float* __restrict__ E,
-    double* __restrict__ g0, int T, int H, int dkdv, int dk, int n_min, int decay_stride) {
+    int n_slots, double* G, double* Hs, float* __restrict__ E,
+    double* __restrict__ g0, float2* __restrict__ Wl, int C, int T, int H, int dkdv, int dk, int n_min,
+    int decay_stride) {
   __shared__ double sh[CS_GATE_THREADS / 32];
   const int h = blockIdx.x, b = blockIdx.y;
   const int t0 = q_start[b], n = q_start[b + 1] - t0;
@@ -196,6 +236,16 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
     }
     return tok_decay ? cs_log_decay(tok_decay[(size_t)(t0 + t) * decay_stride + h]) : fixed;
   };
+  // Wl [H][T]: a token's weight in the state behind its chunk, as a float and what
+  // is left, so that a weighted value is rounded once.  (Where decays are fast the state is
+  // made up of the last few tokens and the walk rounds little: its state is 4.0e-8 from 64 bits, the
+  // chunks' was 4.6e-8 with expf and is 4.2e-8.)
+  auto chunk_weights = [&]() {
+    __syncthreads();                               // all of g and hs are there
+    float2* wl = Wl + (size_t)h * T + t0;
+    for (int t = threadIdx.x; t < n; t += CS_GATE_THREADS)
+      wl[t] = cs_exp(g[min(n, (t / C + 1) * C) - 1] - hs[t]);
+  };
   double F = 0.0;
   for (int t = a; t < e; ++t) {
     F += log_decay(t);
@@ -209,6 +259,7 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
       g[t] = x;
     }
     if (threadIdx.x == 0) g0[(size_t)b * H + h] = 0.0;
+    chunk_weights();
     return;
   }
   double low = 1e300;
@@ -227,6 +278,7 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
     if (t == n - 1) *m_at = (float)(x - run);
   }
   if (threadIdx.x == 0) g0[(size_t)b * H + h] = -m0;
+  chunk_weights();
 }
 
 // ---------------------------------------------------------------------- the products' tiles
@@ -297,6 +349,26 @@ __device__ __forceinline__ void cs_mul_lower(const float (&As)[CS_K][CS_P],
   }
 }
 
+// One chain of multiply-adds from step to step, for the states: their sums are rounded as often as the
+// walk's there, and a chunk's 64 terms are few.
+__device__ __forceinline__ void cs_mul_chain(const float (&As)[CS_K][CS_P],
+                                             const float (&Bs)[CS_K][CS_P], int tx, int ty,
+                                             CsAcc& acc) {
+#pragma unroll
+  for (int kk = 0; kk < CS_K; ++kk) {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(&As[kk][ty * 8]);
+    const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(&As[kk][ty * 8 + 4]);
+    const float4 w = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
+    const unsigned long long a[4] = {a0.x, a0.y, a1.x, a1.y};
+    const unsigned long long b[4] = {cs_pair(w.x, w.x), cs_pair(w.y, w.y), cs_pair(w.z, w.z),
+                                     cs_pair(w.w, w.w)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = cs_fma2(a[i], b[j], acc[i][j]);
+  }
+}
+
 // A step's pieces of four: `idx` 0..255, two a thread.  Rows with the terms side by side (row
 // idx / 4, terms 4 (idx % 4) ..) are turned on their way into shared memory; rows of terms (term
 // idx / 16, columns 4 (idx % 16) ..) go in as they are.
@@ -319,12 +391,30 @@ struct CsIn {
 };
 
 // ---------------------------------------------------------------------------------- cs_qk
-// grid (chunks, QH, row tiles x column tiles): qkm[chunk][qh][C][C], the tiles at and below the
-// diagonal
-template <typename A>
-__global__ void __launch_bounds__(CS_THREADS, 4) cs_qk_kernel(
-    const A* __restrict__ qk, CsIn p, const int* __restrict__ q_start, float* __restrict__ qkm) {
-  __shared__ __align__(16) float As[2][CS_K][CS_P], Bs[2][CS_K][CS_P];
+// grid (chunks, QH, row tiles x column tiles): qkm[chunk][qh][C][C] = q_scale Q K^T up to the diagonal
+// of every block of 16, and (KK, chunks of one tile) kkm = K K^T.  In double, on the tensor cores
+// (mma.sync m8n8k4): a weight inside the chunk is one of these numbers times an exponential, and the
+// sums of up to 64 of them behind it show an error that is one of |q| |k|, however small q . k is
+// itself.  In float, in runs of 16, outputs were 1.2 to 1.7 times as far from 64 bits as the walk's (fast
+// decays; the delta rule's keys alike), at 12 us instead of 14 (2,048 tokens, 8 q/k heads of 128) and 21
+// instead of 42 (16 heads, K K^T too, which ds_prep then computed itself in another 5).  Warp w takes 16
+// rows; with K's rows behind Q's the blocks run the other way, so that every scheduler has the same
+// share of the triangle.
+#define CS_QS 32            // sizes a stage
+#define CS_QP (CS_QS + 4)   // pitch: eight rows of four neighbouring sizes on different banks
+
+__device__ __forceinline__ void cs_dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+template <typename A, bool KK>
+__global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
+    const A* __restrict__ qk, CsIn p, const int* __restrict__ q_start, float* __restrict__ qkm,
+    float* __restrict__ kkm) {
+  constexpr int THREADS = KK ? 256 : 128, PIECES = 128 * (CS_QS / 4) / THREADS;
+  __shared__ __align__(16) double rows_s[128][CS_QP];      // 64 rows of q, 64 of k
   const int tiles = p.C / CS_T;
   const int rt = blockIdx.z / tiles, ct = blockIdx.z % tiles;
   if (ct > rt) return;
@@ -333,52 +423,63 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_qk_kernel(
   const int at = c.index * p.C;                  // the chunk's first token inside the request
   const int n = min(p.C, c.n - at);
   if (rt * CS_T >= n) return;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hq = blockIdx.y;
   const A* q = qk + (size_t)(c.t0 + at) * p.qk_stride + p.q_off + (size_t)hq * p.dk;
   const A* k = qk + (size_t)(c.t0 + at) * p.qk_stride + p.k_off + (size_t)hq * p.dk;
-  CsAcc acc;
-  cs_clear(acc);
-  float4 fa[2], fb[2];
+  const int block = warp >= 4 ? 7 - warp : !KK && (blockIdx.x & 1) ? 3 - warp : warp;
+  const int row0 = (warp >= 4 ? 64 : 0) + block * 16;
+  const int cols = ct < rt ? 8 : 2 * (block + 1);          // blocks of eight columns
+  double acc[2][8][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  float4 f[PIECES];
   auto fetch = [&](int k0) {
 #pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      const int idx = tid + x * CS_THREADS, r = idx >> 2, kk = k0 + (idx & 3) * 4;
-      const int ra = rt * CS_T + r, rb = ct * CS_T + r;
-      fa[x] = ra < n && kk < p.dk ? cs_ld4(q + (size_t)ra * p.qk_stride + kk) : cs_zero();
-      fb[x] = rb < n && kk < p.dk ? cs_ld4(k + (size_t)rb * p.qk_stride + kk) : cs_zero();
-    }
-  };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      cs_put_turned(As[buf], tid + x * CS_THREADS, fa[x]);
-      cs_put_turned(Bs[buf], tid + x * CS_THREADS, fb[x]);
+    for (int x = 0; x < PIECES; ++x) {
+      const int idx = tid + x * THREADS, r = idx / (CS_QS / 4), kk = k0 + idx % (CS_QS / 4) * 4;
+      const int row = (r < 64 ? rt : ct) * CS_T + (r & 63);
+      f[x] = row < n && kk < p.dk ? cs_ld4((r < 64 ? q : k) + (size_t)row * p.qk_stride + kk)
+                                  : cs_zero();
     }
   };
   fetch(0);
-  store(0);
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = 0; k0 < p.dk; k0 += CS_K, buf ^= 1) {
-    if (k0 + CS_K < p.dk) fetch(k0 + CS_K);
-    cs_mul(As[buf], Bs[buf], tx, ty, acc);
-    if (k0 + CS_K < p.dk) store(buf ^ 1);
+  for (int k0 = 0; k0 < p.dk; k0 += CS_QS) {
+#pragma unroll
+    for (int x = 0; x < PIECES; ++x) {
+      const int idx = tid + x * THREADS;
+      double2* d = reinterpret_cast<double2*>(&rows_s[idx / (CS_QS / 4)][idx % (CS_QS / 4) * 4]);
+      d[0] = make_double2(f[x].x, f[x].y);
+      d[1] = make_double2(f[x].z, f[x].w);
+    }
+    __syncthreads();
+    if (k0 + CS_QS < p.dk) fetch(k0 + CS_QS);
+#pragma unroll 2
+    for (int kk = 0; kk < CS_QS; kk += 4) {
+      const double a0 = rows_s[row0 + (lane >> 2)][kk + (lane & 3)];
+      const double a1 = rows_s[row0 + 8 + (lane >> 2)][kk + (lane & 3)];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < cols) {
+          const double b = rows_s[64 + 8 * j + (lane >> 2)][kk + (lane & 3)];
+          cs_dmma(acc[0][j], a0, b);
+          cs_dmma(acc[1][j], a1, b);
+        }
+    }
     __syncthreads();
   }
-  float* dst = qkm + ((size_t)blockIdx.x * p.QH + hq) * p.C * p.C;
+  const double scale = warp >= 4 ? 1.0 : (double)p.q_scale;
+  float* dst = (warp >= 4 ? kkm : qkm) + ((size_t)blockIdx.x * p.QH + hq) * p.C * p.C;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float lo[4], hi[4];
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) cs_unpair(acc[i][j], lo[j], hi[j]);
-    const int r = rt * CS_T + ty * 8 + 2 * i, col = ct * CS_T + tx * 4;
-    const float f = p.q_scale;
-    *reinterpret_cast<float4*>(dst + (size_t)r * p.C + col) =
-        make_float4(lo[0] * f, lo[1] * f, lo[2] * f, lo[3] * f);
-    *reinterpret_cast<float4*>(dst + (size_t)(r + 1) * p.C + col) =
-        make_float4(hi[0] * f, hi[1] * f, hi[2] * f, hi[3] * f);
-  }
+    for (int j = 0; j < 8; ++j)
+      if (j < cols)
+        *reinterpret_cast<float2*>(
+            dst + (size_t)(rt * CS_T + block * 16 + 8 * i + (lane >> 2)) * p.C + ct * CS_T + 8 * j +
+            (lane & 3) * 2) = make_float2((float)(acc[i][j][0] * scale), (float)(acc[i][j][1] * scale));
 }
 
 // ------------------------------------------------------------------------------- cs_state
@@ -387,8 +488,7 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_qk_kernel(
 template <typename A, typename V, bool MLSTM>
 __global__ void __launch_bounds__(CS_THREADS, 4) cs_state_kernel(
     const A* __restrict__ qk, const V* __restrict__ vsrc, CsIn p, const int* __restrict__ q_start,
-    const double* __restrict__ G, const double* __restrict__ Hs, float* __restrict__ U,
-    float* __restrict__ Un) {
+    const float2* __restrict__ Wl, float* __restrict__ U, float* __restrict__ Un) {
   __shared__ __align__(16) float As[2][CS_K][CS_P], Bs[2][CS_K][CS_P];
   __shared__ float ws[2][CS_K];
   const int rows = MLSTM ? p.dk : p.dv, cols = MLSTM ? p.dv : p.dk;
@@ -402,21 +502,20 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_state_kernel(
   const int h = blockIdx.y, hq = h / (p.H / p.QH);
   const A* k = qk + (size_t)(c.t0 + at) * p.qk_stride + p.k_off + (size_t)hq * p.dk;
   const V* v = vsrc + (size_t)(c.t0 + at) * p.v_stride + p.v_off + (size_t)h * p.dv;
-  const double* hs = Hs + (size_t)h * p.T + c.t0 + at;
-  const double g_last = G[(size_t)h * p.T + c.t0 + at + n - 1];
+  const float2* wl = Wl + (size_t)h * p.T + c.t0 + at;
   CsAcc acc;
   cs_clear(acc);
   float nacc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) nacc[i] = 0.f;
   float4 fk[2], fv[2];
-  float fw[2];
+  float2 fw[2];
   auto fetch = [&](int s0) {
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
       const int idx = tid + x * CS_THREADS, s = s0 + (idx >> 4), d = (idx & 15) * 4;
       const int dkk = (MLSTM ? r0 : c0) + d, dvv = (MLSTM ? c0 : r0) + d;
-      fw[x] = s < n ? expf((float)(g_last - hs[s])) : 0.f;
+      fw[x] = s < n ? wl[s] : make_float2(0.f, 0.f);
       fk[x] = s < n && dkk < p.dk ? cs_ld4(k + (size_t)s * p.qk_stride + dkk) : cs_zero();
       fv[x] = s < n && dvv < p.dv ? cs_ld4(v + (size_t)s * p.v_stride + dvv) : cs_zero();
     }
@@ -427,7 +526,7 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_state_kernel(
       const int idx = tid + x * CS_THREADS;
       cs_put(MLSTM ? As[buf] : Bs[buf], idx, fk[x]);
       cs_put(MLSTM ? Bs[buf] : As[buf], idx, cs_times(fv[x], fw[x]));
-      if (MLSTM && (idx & 15) == 0) ws[buf][idx >> 4] = fw[x];
+      if (MLSTM && (idx & 15) == 0) ws[buf][idx >> 4] = fw[x].x;
     }
   };
   fetch(0);
@@ -436,7 +535,7 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_state_kernel(
   int buf = 0;
   for (int s0 = 0; s0 < n; s0 += CS_K, buf ^= 1) {
     if (s0 + CS_K < n) fetch(s0 + CS_K);
-    cs_mul(As[buf], Bs[buf], tx, ty, acc);
+    cs_mul_chain(As[buf], Bs[buf], tx, ty, acc);
     if (MLSTM && c0 == 0) {
       // n's share: term tx of the step's sixteen, for this thread's eight rows
       const float w = ws[buf][tx];
@@ -518,10 +617,10 @@ __global__ void __launch_bounds__(128) cs_prefix_kernel(
           next[j] = *reinterpret_cast<const float4*>(u + (size_t)(i + CS_AHEAD) * step);
         *reinterpret_cast<float4*>(u + (size_t)i * step) = S;
         const double last = g[min(c.n, (i + 1) * p.C) - 1];
-        const float d = expf((float)(last - before));
+        const float2 d = cs_exp(last - before);
         before = last;
-        S = make_float4(fmaf(d, S.x, add.x), fmaf(d, S.y, add.y), fmaf(d, S.z, add.z),
-                        fmaf(d, S.w, add.w));
+        S = make_float4(fmaf(d.x, S.x, fmaf(d.y, S.x, add.x)), fmaf(d.x, S.y, fmaf(d.y, S.y, add.y)),
+                        fmaf(d.x, S.z, fmaf(d.y, S.z, add.z)), fmaf(d.x, S.w, fmaf(d.y, S.w, add.w)));
       }
     }
   }
@@ -540,7 +639,9 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
     float* __restrict__ o_raw) {
   __shared__ __align__(16) float As[2][CS_K][CS_P], Bs[2][CS_K][CS_P];
   __shared__ double gt[CS_T];
-  __shared__ float at_s[CS_T], ns[2][CS_K];
+  __shared__ float2 at_s[CS_T];
+  __shared__ float ns[2][CS_K];
+  __shared__ int odd[2];        // the step whose values in this buffer are not all finite
   const int cts = (p.dv + CS_T - 1) / CS_T;
   const int rt = blockIdx.z / cts, c0 = (blockIdx.z % cts) * CS_T;
   const CsChunk c = cs_find(q_start, p.B, p.C, p.n_min, blockIdx.x, -1);
@@ -564,8 +665,17 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
   if (tid < CS_T) {
     const double x = r0 + tid < n ? g[r0 + tid] : 0.0;
     gt[tid] = x;
-    at_s[tid] = r0 + tid < n ? expf((float)(x - before)) * p.q_scale : 0.f;
+    float2 w = make_float2(0.f, 0.f);
+    if (r0 + tid < n) {
+      w = cs_exp(x - before);
+      // (times q_scale: its products' roundings are part of what is left)
+      const float f = w.x * p.q_scale;
+      w = make_float2(f, fmaf(w.x, p.q_scale, -f) + w.y * p.q_scale);
+      if (!(fabsf(f) < INFINITY)) w.y = 0.f;
+    }
+    at_s[tid] = w;
   }
+  if (tid < 2) odd[tid] = -1;
   __syncthreads();
   CsAcc acc;
   cs_clear(acc);
@@ -628,11 +738,15 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
         // row r0 + r sees the chunk's tokens up to itself
         const double gr = gt[r];
         const int last = r0 + r < n ? r0 + r : -1;
-        float4 w;
-        w.x = s <= last ? fa[x].x * expf((float)(gr - fh[0])) : 0.f;
-        w.y = s + 1 <= last ? fa[x].y * expf((float)(gr - fh[1])) : 0.f;
-        w.z = s + 2 <= last ? fa[x].z * expf((float)(gr - fh[2])) : 0.f;
-        w.w = s + 3 <= last ? fa[x].w * expf((float)(gr - fh[3])) : 0.f;
+        float4 w = cs_zero();
+        if (s <= last) {
+          w.x = cs_times(fa[x].x, cs_exp(gr - fh[0]));
+          if (s + 1 <= last) w.y = cs_times(fa[x].y, cs_exp(gr - fh[1]));
+          if (s + 2 <= last) w.z = cs_times(fa[x].z, cs_exp(gr - fh[2]));
+          if (s + 3 <= last) w.w = cs_times(fa[x].w, cs_exp(gr - fh[3]));
+        }
+        // (a number times zero is zero if it is finite, and only then)
+        if (!(fb[x].x * 0.f + fb[x].y * 0.f + fb[x].z * 0.f + fb[x].w * 0.f == 0.f)) odd[buf] = k0;
         cs_put_turned(As[buf], idx, w);
         cs_put(Bs[buf], idx, fb[x]);
       }
@@ -648,6 +762,7 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
     // the tokens before, among and behind this warp's sixteen rows
     const int ahead = k0 < dk_pad ? -1 : k0 - dk_pad - ((ty & ~1) * 8 + r0);
     if (ahead < 0) cs_mul(As[buf], Bs[buf], tx, ty, acc);
+    else if (ahead == 0 && odd[buf] != k0) cs_mul(As[buf], Bs[buf], tx, ty, acc);
     else if (ahead == 0) cs_mul_lower(As[buf], Bs[buf], tx, ty, acc);
     if (MLSTM) {
       // n_t . q_t: the same rows against n and against ones; term tx of the step's sixteen
@@ -710,8 +825,8 @@ __device__ __forceinline__ void ds_cp16(float* smem, const float* gmem, bool ok)
 
 // grid (chunks, H): W [chunk][H][64][dk], Y [chunk][H][64][dv]
 __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
-    DsIn p, const int* __restrict__ q_start, const double* __restrict__ F, float* __restrict__ W,
-    float* __restrict__ Y) {
+    DsIn p, const int* __restrict__ q_start, const double* __restrict__ F,
+    const float* __restrict__ KKm, float* __restrict__ W, float* __restrict__ Y) {
   extern __shared__ __align__(16) float ds_smem[];
   float* Ks = ds_smem;                           // [64][DS_P]
   float* Vs = Ks + DS_C * DS_P;                  // [64][DS_P]
@@ -739,44 +854,27 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
   if (tid < DS_C) {
     fs[tid] = tid < n ? f[tid] - f0 : 0.0;
     beta[tid] = tid < n ? p.gates[(size_t)(c.t0 + at + tid) * 2 * p.H + h] : 0.f;
-    grow[tid] = beta[tid] * expf((float)fs[tid]);
+    grow[tid] = cs_times(beta[tid], cs_exp(fs[tid]));
   }
   asm volatile("cp.async.wait_group 0;" ::);
   __syncthreads();
-  // L: thread (tx, ty) has rows 4 ty .. and columns tx + 16 j; even and odd sizes in the two halves
-  {
-    unsigned long long s2[4][4];
+  // L: rows 4 ty .., columns 4 tx .., rounded once (keys alike make it hang on every bit)
+  const float* kk = KKm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 4; ++i) {
+    const int t = ty * 4 + i;
+    const float4 x = *reinterpret_cast<const float4*>(kk + t * DS_C + 4 * tx);
+    const float xs[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
-#pragma unroll 2
-    for (int d = 0; d < DS_D; d += 4) {
-      if (d >= p.dk) break;
-      ulonglong2 a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        a[i] = *reinterpret_cast<const ulonglong2*>(Ks + (ty * 4 + i) * DS_P + d);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        b[j] = *reinterpret_cast<const ulonglong2*>(Ks + (tx + 16 * j) * DS_P + d);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          s2[i][j] = cs_fma2(a[i].x, b[j].x, s2[i][j]);
-          s2[i][j] = cs_fma2(a[i].y, b[j].y, s2[i][j]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int t = ty * 4 + i, s = tx + 16 * j;
-        float lo, hi;
-        cs_unpair(s2[i][j], lo, hi);
-        Ls[t * 68 + s] = s < t && t < n ? beta[t] * expf((float)(fs[t] - fs[s])) * (lo + hi) : 0.f;
+    for (int j = 0; j < 4; ++j) {
+      const int s = 4 * tx + j;
+      float l = 0.f;
+      if (s < t && t < n) {
+        const float2 w = cs_exp(fs[t] - fs[s]);
+        l = (float)((double)beta[t] * ((double)w.x + (double)w.y) * (double)xs[j]);
       }
+      Ls[t * 68 + s] = l;
+    }
   }
   __syncthreads();
   // T = (I + L)^-1 by blocks of 16: the diagonal blocks, a thread a column ...
@@ -880,7 +978,8 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
 __global__ void __launch_bounds__(128) ds_walk_kernel(
     DsIn p, const int* __restrict__ q_start, const int* __restrict__ state_slots, int n_slots,
     float* __restrict__ state, long long slot_stride, const double* __restrict__ F,
-    const float* __restrict__ W, const float* __restrict__ Y, float* __restrict__ u,
+    const float2* __restrict__ Wl, const float* __restrict__ W, const float* __restrict__ Y,
+    float* __restrict__ u,
     float* __restrict__ Sc, int* __restrict__ err) {
   extern __shared__ __align__(16) float ds_smem[];
   constexpr int PS = DS_NS + 4;
@@ -901,6 +1000,7 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
   float* st = state + (size_t)slot * slot_stride + (size_t)h * p.dv * p.dk;
   const float* k = p.qkv + (size_t)c.t0 * p.stride + (size_t)(p.G + hq) * p.dk;
   const double* f = F + (size_t)h * p.T + c.t0;
+  const float2* wl = Wl + (size_t)h * p.T + c.t0;
   const int chunks = (c.n + DS_C - 1) / DS_C;
   auto load = [&](int i, int buf) {
     const int n = min(DS_C, c.n - i * DS_C);
@@ -985,29 +1085,24 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
       cs_unpair(tot[r][0], a.x, a.y);
       cs_unpair(tot[r][1], a.z, a.w);
       const float4 uv = make_float4(y[r].x - a.x, y[r].y - a.y, y[r].z - a.z, y[r].w - a.w);
-      const float g = t < n ? expf((float)(last - f[i * DS_C + min(t, n - 1)])) : 0.f;
+      const float2 g = t < n ? wl[i * DS_C + t] : make_float2(0.f, 0.f);
       *reinterpret_cast<float4*>(Us + t * PS + 4 * tx) = cs_times(uv, g);
       if (t < n && col < p.dv)
         *reinterpret_cast<float4*>(u + ((size_t)(c.t0 + i * DS_C + t) * p.H + h) * p.dv + col) = uv;
     }
     __syncthreads();                             // U is whole; the state before it is read
-    // S <- exp(F_C) S + K^T U, in runs of 16 tokens
+    // S <- exp(F_C) S + K^T U, one chain (rounded as often as the walk's)
     unsigned long long S[4][4];
-    const float g = expf((float)(last - before));
+    const float2 g = cs_exp(last - before);
     before = last;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        S[r][j] = cs_pair(Ss[(ty * 8 + 2 * r) * PS + 4 * tx + j] * g,
-                          Ss[(ty * 8 + 2 * r + 1) * PS + 4 * tx + j] * g);
+        S[r][j] = cs_pair(cs_times(Ss[(ty * 8 + 2 * r) * PS + 4 * tx + j], g),
+                          cs_times(Ss[(ty * 8 + 2 * r + 1) * PS + 4 * tx + j], g));
 #pragma unroll 1
     for (int s0 = 0; s0 < n; s0 += 16) {         // (rows of Us and Ks from n on are zero)
-      unsigned long long acc[4][4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[r][j] = 0ull;
 #pragma unroll
       for (int s = s0; s < s0 + 16; ++s) {
         const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(Kt + s * DS_P + ty * 8);
@@ -1019,12 +1114,8 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[r][j] = cs_fma2(a[r], w[j], acc[r][j]);
+          for (int j = 0; j < 4; ++j) S[r][j] = cs_fma2(a[r], w[j], S[r][j]);
       }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) S[r][j] = cs_add2(S[r][j], acc[r][j]);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
@@ -1041,9 +1132,10 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
 }
 
 // -------------------------------------------------------------------------------- launches
-// Scratch (bytes, each part on a 256-byte boundary): G, Hs, g0 | E (mLSTM) | qkm | U | Un (mLSTM).
+// Scratch (bytes, each part on a 256-byte boundary): G, Hs, g0, Wl | E (mLSTM) | qkm | U | Un
+// (mLSTM).
 struct CsLayout {
-  size_t G, Hs, g0, E, qkm, U, Un, total;
+  size_t G, Hs, g0, Wl, E, qkm, U, Un, total;
   int chunks;
 };
 // The most chunks of C tokens that a step's portions of more than n_min tokens can have.
@@ -1064,6 +1156,7 @@ static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, in
   l.G = take((size_t)T * H * 8);
   l.Hs = take((size_t)T * H * 8);
   l.g0 = take((size_t)B * H * 8);
+  l.Wl = take((size_t)T * H * 8);
   l.E = take(mlstm ? (size_t)T * H * 4 : 0);
   l.qkm = take((size_t)l.chunks * QH * C * C * 4);
   l.U = take((size_t)l.chunks * H * dk * dv * 4);
@@ -1087,6 +1180,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   double* G = (double*)(scratch + l.G);
   double* Hs = (double*)(scratch + l.Hs);
   double* g0 = (double*)(scratch + l.g0);
+  float2* Wl = (float2*)(scratch + l.Wl);
   float* E = (float*)(scratch + l.E);
   float* qkm = (float*)(scratch + l.qkm);
   float* U = (float*)(scratch + l.U);
@@ -1094,11 +1188,11 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   const int tiles = p.C / CS_T, tk = (p.dk + CS_T - 1) / CS_T, tv = (p.dv + CS_T - 1) / CS_T;
   cs_gates_kernel<MLSTM><<<dim3(p.H, p.B), CS_GATE_THREADS, 0, stream>>>(
       decays, tok_decay, gates, state, slot_stride, state_size, q_start, state_slots, n_slots, G,
-      Hs, E, g0, p.T, p.H, p.dk * p.dv, p.dk, p.n_min, p.H);
-  cs_qk_kernel<A><<<dim3(l.chunks, p.QH, tiles * tiles), CS_THREADS, 0, stream>>>(qk, p, q_start,
-                                                                                 qkm);
+      Hs, E, g0, Wl, p.C, p.T, p.H, p.dk * p.dv, p.dk, p.n_min, p.H);
+  cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles), 128, 0, stream>>>(qk, p, q_start,
+                                                                                 qkm, nullptr);
   cs_state_kernel<A, V, MLSTM><<<dim3(l.chunks, p.H, tk * tv), CS_THREADS, 0, stream>>>(
-      qk, v, p, q_start, G, Hs, U, Un);
+      qk, v, p, q_start, Wl, U, Un);
   const int elems = p.dk * p.dv + (MLSTM ? p.dk : 0);
   cs_prefix_kernel<MLSTM><<<dim3((elems + 511) / 512, p.H, p.B), 128, 0, stream>>>(
       state, slot_stride, state_size, state_slots, n_slots, p, q_start, G, g0, U, Un, err);
@@ -1151,9 +1245,10 @@ BF_EXPORT int bf_chunk_scan_mlstm(const void* proj, long long stride, const floa
       n_slots, o_raw, (char*)scratch, err, stream);
 }
 
-// The gated delta rule.  Scratch: F (G and H are the same array), g0 | qkm | W | Y | u | Sc.
+// The gated delta rule.  Scratch: F (G and H are the same array), g0, Wl | qkm | kkm | W | Y |
+// u | Sc.
 struct DsLayout {
-  size_t F, g0, qkm, W, Y, u, Sc, total;
+  size_t F, g0, Wl, qkm, kkm, W, Y, u, Sc, total;
   int chunks;
 };
 static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min) {
@@ -1167,7 +1262,9 @@ static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min)
   l.chunks = cs_most_chunks(T, B, DS_C, n_min);
   l.F = take((size_t)T * H * 8);
   l.g0 = take((size_t)B * H * 8);
+  l.Wl = take((size_t)T * H * 8);
   l.qkm = take((size_t)l.chunks * G * DS_C * DS_C * 4);
+  l.kkm = take((size_t)l.chunks * G * DS_C * DS_C * 4);
   l.W = take((size_t)l.chunks * H * DS_C * dk * 4);
   l.Y = take((size_t)l.chunks * H * DS_C * dv * 4);
   l.u = take((size_t)T * H * dv * 4);
@@ -1197,7 +1294,9 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
   char* base = (char*)scratch;
   double* F = (double*)(base + l.F);
   double* g0 = (double*)(base + l.g0);
+  float2* Wl = (float2*)(base + l.Wl);
   float* qkm = (float*)(base + l.qkm);
+  float* kkm = (float*)(base + l.kkm);
   float* W = (float*)(base + l.W);
   float* Y = (float*)(base + l.Y);
   float* u = (float*)(base + l.u);
@@ -1221,11 +1320,12 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
   }
   cs_gates_kernel<false><<<dim3(H, B), CS_GATE_THREADS, 0, stream>>>(
       nullptr, gates + H, nullptr, state, slot_stride, dk * dv, q_start, state_slots, n_slots, F, F,
-      nullptr, g0, T, H, dk * dv, dk, n_min, 2 * H);
-  cs_qk_kernel<float><<<dim3(l.chunks, G, 1), CS_THREADS, 0, stream>>>(qkv, p, q_start, qkm);
-  ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, W, Y);
+      nullptr, g0, Wl, DS_C, T, H, dk * dv, dk, n_min, 2 * H);
+  cs_qk_kernel<float, true><<<dim3(l.chunks, G, 1), 256, 0, stream>>>(qkv, p, q_start, qkm, kkm);
+  ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, kkm, W,
+                                                                            Y);
   ds_walk_kernel<<<dim3((dv + DS_NS - 1) / DS_NS, H, B), 128, smem_walk, stream>>>(
-      d, q_start, state_slots, n_slots, state, slot_stride, F, W, Y, u, Sc, err);
+      d, q_start, state_slots, n_slots, state, slot_stride, F, Wl, W, Y, u, Sc, err);
   cs_out_kernel<float, float, false, true>
       <<<dim3(l.chunks, H, (dv + CS_T - 1) / CS_T), CS_THREADS, 0, stream>>>(
           qkv, u, p, q_start, state_slots, n_slots, F, F, g0, nullptr, qkm, Sc, nullptr, o_raw);

@@ -1758,6 +1758,54 @@ def test_delta_scan_in_chunks(cuda_device, monkeypatch, lens, H, G, dk, dv):
     err.zero_()
 
 
+# keys at random, alike by a half and nearly the same; decays that forget in a few tokens and slow ones
+@pytest.mark.parametrize("alike", [0.0, 0.5, 0.9])
+@pytest.mark.parametrize("decays", ["fast", "slow"])
+@pytest.mark.parametrize("kind", ["linear", "delta"])
+def test_chunks_are_as_close_to_64_bits_as_the_walk(cuda_device, kind, decays, alike):
+    """Relative errors over 777 tokens of 16 heads: a million numbers and more, so that what is left
+    to chance is far below the tenth that is allowed."""
+    from binfer_b200.csrc import ops
+    T, H, d, dev = 777, 16, 128, cuda_device
+    torch.manual_seed(13)
+    norm = lambda x: torch.nn.functional.normalize(x, dim=-1)
+    base = norm(torch.randn(H, d, device=dev))
+    q = norm(torch.randn(T, H, d, device=dev))
+    k = alike ** 0.5 * base + (1 - alike) ** 0.5 * norm(torch.randn(T, H, d, device=dev))
+    v, g = torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    if decays == "slow":
+        g = 1 - 0.02 * g
+    beta = torch.sigmoid(torch.randn(T, H, device=dev))
+    s0 = 0.1 * torch.randn(1, H * d * d, device=dev)
+    S, want = s0.double().view(H, d, d).transpose(1, 2), torch.empty(T, H, d, dtype=torch.float64,
+                                                                       device=dev)
+    qd, kd, vd, gd, bd = (x.double() for x in (q, k, v, g, beta))
+    for t in range(T):
+        S = S * gd[t][:, None, None]
+        u = vd[t]
+        if kind == "delta":
+            u = bd[t][:, None] * (u - (kd[t][:, None] @ S)[:, 0])
+        S = S + kd[t][:, :, None] * u[:, None]
+        want[t] = (qd[t][:, None] @ S)[:, 0]
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, off = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    for chunked in (False, True):
+        s, o = s0.clone(), torch.empty(T, H * d, device=dev)
+        if kind == "linear":
+            ops.linear_scan(torch.stack([q, k], 1).contiguous(), v, g, s, qs, slots, o, 1, H, H, d, d,
+                            err, max_q=T, chunked=chunked)
+        else:
+            ops.delta_scan(torch.cat([x.reshape(T, -1) for x in (q, k, v)], 1).contiguous(),
+                           torch.stack([beta, g], 1).contiguous(), s, qs, slots, o, 1, H, H, d, d,
+                           err, max_q=T, chunked=chunked)
+        have = s.double().view(H, d, d).transpose(1, 2)
+        off.append([float((x - y).norm() / y.norm()) for x, y in ((o.double().view(T, H, d), want),
+                                                                    (have, S))])
+    # (or half a unit in the last place, which one rounding of the result is)
+    for walk, products in zip(*off):
+        assert products <= max(1.1 * walk, 2.0 ** -24), off
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("lens", [[1], [3, 1, 9, 2, 17], [1] * 5, [700, 1, 1, 643]])
