@@ -56,14 +56,14 @@ __global__ void __launch_bounds__(BM / TM * 16) attention_f32_kernel(
     const float* __restrict__ v_cache, const int* __restrict__ q_start,
     const int* __restrict__ positions, const int* __restrict__ tables, int table_stride,
     float* __restrict__ out, int nh, int nkv, int page_size, int num_pages, int window,
-    float scale_log2, int* __restrict__ err) {
+    float scale_log2, int* __restrict__ err, int bufs) {
   constexpr int THREADS = BM / TM * 16, P = D + 4, PP = AF_KEYS + 4, CJ = D / 64;
   constexpr int CHUNKS = D / 4;                 // 16-byte pieces of a row
   extern __shared__ __align__(16) float af_smem[];
   float* Qs = af_smem;                          // [BM][P]
-  float* Ks = Qs + BM * P;                      // [2][64][P]
-  float* Vs = Ks + 2 * AF_KEYS * P;             // [2][64][P]
-  float* Ps = Vs + 2 * AF_KEYS * P;             // [BM][PP]
+  float* Ks = Qs + BM * P;                      // [bufs][64][P]
+  float* Vs = Ks + bufs * AF_KEYS * P;          // [bufs][64][P]
+  float* Ps = Vs + bufs * AF_KEYS * P;          // [BM][PP]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int g = blockIdx.y, b = blockIdx.z, Gh = nh / nkv;
   const int t0 = q_start[b], n_tok = q_start[b + 1] - t0;
@@ -116,10 +116,14 @@ __global__ void __launch_bounds__(BM / TM * 16) attention_f32_kernel(
     for (int j = 0; j < CJ; ++j) o[i][j][0] = o[i][j][1] = 0ull;
   }
   for (int tile = tile_a; tile < tile_b; ++tile) {
-    const int buf = (tile - tile_a) & 1;
+    if (bufs == 1 && tile > tile_a) {           // (a context longer than the caller said)
+      __syncthreads();
+      load(tile, 0);
+    }
+    const int buf = bufs == 1 ? 0 : (tile - tile_a) & 1;
     cp_async_wait<0>();
     __syncthreads();                            // the tile is here; the other buffer is used up
-    if (tile + 1 < tile_b) load(tile + 1, buf ^ 1);
+    if (bufs == 2 && tile + 1 < tile_b) load(tile + 1, buf ^ 1);
     const float* Kt = Ks + buf * AF_KEYS * P;
     const float* Vt = Vs + buf * AF_KEYS * P;
     unsigned long long s2[TM][4];
@@ -260,44 +264,51 @@ template <int D, int BM, int TM>
 static int af_launch(const float* q, const float* k, const float* v, const int* q_start,
                      const int* positions, const int* tables, int table_stride, float* out, int B,
                      int max_q, int nh, int nkv, int page_size, int num_pages, int window,
-                     float scale, int* err, cudaStream_t stream) {
-  const size_t smem = ((size_t)BM * (D + 4) + (size_t)4 * AF_KEYS * (D + 4) +
-                       (size_t)BM * (AF_KEYS + 4)) * sizeof(float);
+                     float scale, int bufs, int* err, cudaStream_t stream) {
+  const auto bytes = [](int n) {
+    return ((size_t)BM * (D + 4) + (size_t)2 * n * AF_KEYS * (D + 4) +
+            (size_t)BM * (AF_KEYS + 4)) * sizeof(float);
+  };
+  const size_t smem = bytes(bufs);
   auto kern = attention_f32_kernel<D, BM, TM>;
   static bool configured[BF_MAX_DEVICES];
   bool& done = configured[bf_current_device()];
   if (!done) {
     const cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(2));
     if (e != cudaSuccess) return (int)e;
     done = true;
   }
   const long long rows = (long long)max_q * (nh / nkv);
   kern<<<dim3((unsigned)((rows + BM - 1) / BM), nkv, B), BM / TM * 16, smem, stream>>>(
       q, k, v, q_start, positions, tables, table_stride, out, nh, nkv, page_size, num_pages, window,
-      scale * 1.4426950408889634f, err);
+      scale * 1.4426950408889634f, err, bufs);
   return bf_launch_status();
 }
 
 // q and out [T, nh, d] contiguous; request b's token rows q_start[b] .. q_start[b + 1] - 1, at most
-// max_q of them, its pages in tables[b]; window 0: every earlier key.
+// max_q of them, its pages in tables[b]; window 0: every earlier key; max_ctx: the longest context, or
+// 0 (contexts of one tile need one buffer for K and V, and three CTAs of four rows fit an SM instead of
+// one: 48 single tokens of 8 kv heads of 128 behind 0 and 15 keys 17 and 20 us -> 8.4 and 9.8; the kernel
+// for any size 7.9 and 18.5).
 BF_EXPORT int bf_attention_f32(const float* q, const float* k_cache, const float* v_cache,
                                const int* q_start, const int* positions, const int* tables,
                                int table_stride, float* out, int B, int max_q, int nh, int nkv,
                                int d, int page_size, int num_pages, int window, float scale,
-                               int* err, cudaStream_t stream) {
+                               int max_ctx, int* err, cudaStream_t stream) {
   if (B <= 0 || max_q <= 0) return 0;
   if (nkv <= 0 || nh % nkv || nkv > 65535 || B > 65535 || (d != 64 && d != 128) || !(scale > 0.f) ||
       (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15))
     return (int)cudaErrorInvalidValue;
-  // few rows (single tokens): tiles of four, each with as many threads a row, so that the chain from
-  // key tile to key tile is short
+  // few rows from every request of the step (single tokens alone): tiles of four, each with as many
+  // threads a row, so that the chain from key tile to key tile is short
+  const int bufs = max_ctx > 0 && max_ctx <= AF_KEYS ? 1 : 2;
   const bool few = (long long)max_q * (nh / nkv) <= 16;
 #define AF_GO(D)                                                                                \
   (few ? af_launch<D, 4, 1>(q, k_cache, v_cache, q_start, positions, tables, table_stride, out, \
-                            B, max_q, nh, nkv, page_size, num_pages, window, scale, err, stream) \
+                            B, max_q, nh, nkv, page_size, num_pages, window, scale, bufs, err, stream) \
        : af_launch<D, 64, 4>(q, k_cache, v_cache, q_start, positions, tables, table_stride, out, \
-                             B, max_q, nh, nkv, page_size, num_pages, window, scale, err, stream))
+                             B, max_q, nh, nkv, page_size, num_pages, window, scale, bufs, err, stream))
   return d == 64 ? AF_GO(64) : AF_GO(128);
 #undef AF_GO
 }

@@ -387,17 +387,20 @@ def attention_f32_takes(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.T
 def attention_f32(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                   q_start: torch.Tensor, positions: torch.Tensor, tables: torch.Tensor,
                   out: torch.Tensor, B: int, max_q: int, nh: int, nkv: int, d: int,
-                  window: Optional[int], scale: float, err: torch.Tensor) -> None:
+                  window: Optional[int], scale: float, err: torch.Tensor,
+                  max_ctx: int = 0) -> None:
     """Causal grouped attention of float32 rows ``q [T, nh * d]`` over the pages, in tiles of rows
     against tiles of keys; a row's result depends on its own position only.  Request ``b`` owns the
-    token rows ``q_start[b] .. q_start[b+1]-1``, at most ``max_q`` of them."""
+    token rows ``q_start[b] .. q_start[b+1]-1``, at most ``max_q`` of them.  ``max_ctx``: the longest
+    context, if the caller knows it (short ones take less shared memory)."""
     if (not attention_f32_takes(q, k_cache, v_cache, d) or not out.is_contiguous()
             or out.dtype != q.dtype or out.data_ptr() % 16):
         raise KernelError("attention_f32: contiguous float32 on 16-byte boundaries, heads of 64 or 128")
     _run("attention_f32", lib().bf_attention_f32, _ptr(q), _ptr(k_cache), _ptr(v_cache),
          _ptr(q_start), _ptr(positions), _ptr(tables), _c_int(tables.stride(0)), _ptr(out),
          _c_int(B), _c_int(max_q), _c_int(nh), _c_int(nkv), _c_int(d), _c_int(k_cache.shape[2]),
-         _c_int(k_cache.shape[0]), _c_int(window or 0), _c_float(scale), _ptr(err), _stream())
+         _c_int(k_cache.shape[0]), _c_int(window or 0), _c_float(scale), _c_int(max_ctx), _ptr(err),
+         _stream())
 
 
 def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,

@@ -193,7 +193,8 @@ class GQAAttention(Mixer):
                 and ops.attention_f32_takes(q, view.k_cache, view.v_cache, s.head_dim)):
             ops.attention_f32(q, view.k_cache, view.v_cache, ctx.q_start, ctx.positions, tables,
                               out, ctx.B, 1 if ctx.decode_only else ctx.max_q_len, s.num_heads,
-                              s.num_kv_heads, s.head_dim, s.window, s.softmax_scale, ctx.err)
+                              s.num_kv_heads, s.head_dim, s.window, s.softmax_scale, ctx.err,
+                              max_ctx=ctx.max_ctx_len)
             return
         if not fast:
             ops.paged_attention_generic(

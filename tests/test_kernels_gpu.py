@@ -1663,6 +1663,10 @@ def test_attention_f32_tiles(cuda_device, nh, nkv, d, ps, window):
     ops.attention_f32(q[last].contiguous(), kc, vc, each, pos[last].contiguous(), bt, one,
                       len(ctxs), 1, nh, nkv, d, window, d ** -0.5, err)
     assert torch.equal(one, out[last])
+    # nor on the buffers that a context of one tile does without (a hint that is too small included)
+    ops.attention_f32(q, kc, vc, qs, pos, bt, again := torch.full_like(q, 7.0), len(ctxs), max(qlens),
+                      nh, nkv, d, window, d ** -0.5, err, max_ctx=64)
+    assert torch.equal(again, out)
     bad = bt.clone()
     bad[0, 0] = kc.shape[0]
     ops.attention_f32(q, kc, vc, qs, pos, bad, out, len(ctxs), max(qlens), nh, nkv, d, window,
