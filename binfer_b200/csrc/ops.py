@@ -732,17 +732,31 @@ def conv_state_shift(proj: torch.Tensor, state: torch.Tensor, state_slots: torch
 # ------------------------------------------------------------------------- retention
 RETENTION_MAX_QK_DIM = 1024
 
-# Portions of at most this many tokens are walked token by token also where the products over
-# chunks may run: their five kernels take 40 to 55 us whatever the portion, the walk 0.14 to 0.5 us a
-# token.  One portion, walk / products: 64 heads of 128 x 64: 39 / 51 us at 130 tokens, 76 / 65 at
-# 300, 459 / 226 at 2,000; mLSTM, 8 heads of 256 x 512: 40 / 83 at 64, 150 / 107 at 300, 982 / 396 at
-# 2,048.
+# Portions of at most this many tokens are walked token by token whatever runs beside them.  (For the
+# matrix memory that is the line: 8 heads of 256 x 512, walk / products over chunks in us: one portion of
+# 161 tokens 82 / 79, two 108 / 111, three 213 / 129; 4 heads of 128 x 256 67 / 45, 67 / 48, 67 / 52.)
 CHUNK_SCAN_MIN = 160
-# tokens a chunk (of 64 / 128: 226 / 228 us and 396 / 390 for the two above; 64 takes half the
-# products inside a chunk, 128 half the states between them)
+# tokens a chunk (64 or 128 measured alike, 2,000 tokens of 64 heads of 128 x 64 and 2,048 of the matrix
+# memory's 8 heads of 256 x 512; 64 takes half the products inside a chunk, 128 half the states between
+# them)
 CHUNK_SCAN_TOKENS = 64
 # most scratch that a step's chunks may take; a step that needs more is walked
 CHUNK_SCAN_MAX_BYTES = 768 << 20
+
+
+def chunk_scan_pays(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bool:
+    """Whether a step's linear scan is the faster one in chunks: ``tokens`` of all requests, of which
+    the longest brings ``max_q``.  The walk is a chain over the longest portion until the portions'
+    states fill the chip; the chunks' kernels take 35 to 60 us and then grow with the tokens.  Walk /
+    chunks in us at 161, 200 and 300 tokens, equal portions: 8 heads of 128 x 256, one portion 28 / 39,
+    33 / 39, 46 / 46, two 41 / 48, 49 / 49, 72 / 58; 64 heads of 128 x 64, one 42 / 46, 51 / 50, 72 / 56, two
+    64 / 65, 76 / 70, 111 / 88.  Heads of 64 x 64 and less fill half of a tile's terms: 32 of them, one portion
+    of 260 tokens 36 / 36, six of 400 98 / 101.  (``tokens / max_q`` stands for the number of portions: single
+    tokens beside them hardly count.)"""
+    if dk * dv < 8192:
+        return max_q > 448
+    elements = tokens * heads * dk * dv / max(1, max_q)
+    return max_q > (304 if elements < 450_000 else 200 if elements < 1_000_000 else CHUNK_SCAN_MIN)
 
 
 def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_heads: int, dk: int,
@@ -1063,9 +1077,21 @@ def delta_encode(proj: torch.Tensor, conv_w: Optional[torch.Tensor], taps: int,
 
 
 DELTA_MAX_QK_DIM = 1024
-# portions of at most so many tokens are walked: the chunks' chain of small kernels takes 82 us for 170
-# tokens of 16 heads of 128 and 98 for 300, the walk 53 and 89; for 1,111 and 694 tokens 253 against 364
+# portions of at most so many tokens are walked whatever runs beside them
 DELTA_CHUNK_MIN = 384
+
+
+def delta_chunks_pay(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bool:
+    """Whether a step's gated delta rule is the faster one in chunks (arguments as for
+    :func:`chunk_scan_pays`), whose chain has a block per portion, head and 32 columns, one an SM (148) and
+    built for keys of 128.  Walk / chunks in us, 16 heads of 128, portions of 400 and 500 tokens: one
+    113 / 97, 140 / 103, two 144 / 116, 180 / 124, three (192 blocks, a second round of 44) 174 / 200, 217 / 218,
+    six 342 / 308, 428 / 342.  16 heads of 64: one 96 / 77, 119 / 82, three 96 / 110, 119 / 117, six (the walk has
+    a quarter of the work) 123 / 189, 153 / 212 and 303 / 385 at 1,000."""
+    blocks = tokens * heads * -(-dv // 32) / max(1, max_q)
+    if dk * dv < 14_000:
+        return blocks <= 148 and max_q > (DELTA_CHUNK_MIN if blocks <= 74 else 520)
+    return max_q > (520 if 148 < blocks <= 220 else DELTA_CHUNK_MIN)
 
 
 def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,

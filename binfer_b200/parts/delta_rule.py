@@ -111,7 +111,8 @@ class GatedDeltaRule(Mixer):
         ops.delta_scan(qkv, gates, memory, ctx.q_start, ctx.state_slots, o_raw, ctx.B, self.H,
                        self.G, self.dk, self.dv, ctx.err,
                        max_q=1 if ctx.decode_only else ctx.max_q_len,
-                       chunked=x.dtype == torch.bfloat16)
+                       chunked=x.dtype == torch.bfloat16 and
+                       ops.delta_chunks_pay(T, ctx.max_q_len, self.H, self.dk, self.dv))
         out = torch.empty((T, self.v_size), dtype=x.dtype, device=x.device)
         ops.gated_norm_out(o_raw, proj, self.g_off, self.norm_w, out, self.H, self.dv,
                            s.norm_eps, over_all=False, gate="silu")

@@ -124,7 +124,8 @@ class Mamba2(Mixer):
         ops.linear_scan(qk, vf, decay, memory, ctx.q_start, ctx.state_slots, o_raw, ctx.B, self.H,
                         self.G, self.N, self.P, ctx.err,
                         max_q=1 if ctx.decode_only else ctx.max_q_len,
-                        chunked=x.dtype == torch.bfloat16)
+                        chunked=x.dtype == torch.bfloat16 and
+                        ops.chunk_scan_pays(T, ctx.max_q_len, self.H, self.N, self.P))
         out = torch.empty((T, self.inner), dtype=x.dtype, device=dev)
         ops.gate_norm_out(o_raw, skip, proj, 0, self.norm_w, out, s.norm_groups, s.norm_eps)
         return linear(out, self.w_o)

@@ -101,7 +101,8 @@ class RetentionMixer(Mixer):
                            self.heads, self.dk, self.dv, self.k_scale, ctx.err,
                            max_q=1 if ctx.decode_only else ctx.max_q_len,
                            silu=self.spec.activation == "silu",
-                           chunked=self.chunks and proj.dtype == torch.bfloat16)
+                           chunked=self.chunks and proj.dtype == torch.bfloat16 and
+                           ops.chunk_scan_pays(T, ctx.max_q_len, self.heads, self.dk, self.dv))
         g_off = 2 * self.qk_size + self.v_size
         if self.plain_out:
             ops.retention_out(o_raw, proj, g_off, out, self.heads, self.dv, self.spec.norm_eps,

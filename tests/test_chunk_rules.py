@@ -1,6 +1,7 @@
 """Which recurrences run as products over chunks: the rule alone, without a GPU."""
 import math
 
+import pytest
 import torch
 
 BF16 = torch.bfloat16
@@ -70,3 +71,41 @@ def test_scans_off_16_byte_boundaries_are_walked(monkeypatch):
             seen.clear()
             call(off)
             assert seen and not any(n.endswith("_chunks") for n in seen), (call, off)
+
+
+# us on a B200: (heads, dk, dv, portions, tokens of each): (walk, products over chunks)
+LINEAR_US = {
+    (64, 128, 64, 1, 161): (42, 46), (64, 128, 64, 1, 200): (51, 50), (64, 128, 64, 1, 260): (64, 55),
+    (64, 128, 64, 1, 1000): (232, 112), (64, 128, 64, 2, 161): (64, 65), (64, 128, 64, 2, 200): (76, 70),
+    (64, 128, 64, 3, 161): (98, 74), (64, 128, 64, 12, 161): (310, 236), (8, 128, 256, 1, 161): (28, 39),
+    (8, 128, 256, 1, 260): (41, 45), (8, 128, 256, 1, 350): (53, 46), (8, 128, 256, 2, 161): (41, 48),
+    (8, 128, 256, 2, 220): (54, 49), (8, 128, 256, 3, 161): (52, 55), (8, 128, 256, 3, 220): (66, 60),
+    (8, 128, 256, 6, 161): (98, 78), (8, 128, 256, 24, 161): (308, 238), (32, 64, 64, 1, 200): (28, 32),
+    (32, 64, 64, 1, 500): (64, 38), (32, 64, 64, 2, 300): (40, 44), (32, 64, 64, 2, 500): (64, 50),
+    (32, 64, 64, 6, 300): (75, 80), (32, 64, 64, 6, 400): (98, 101), (32, 64, 64, 6, 500): (122, 114),
+    (32, 64, 64, 12, 260): (124, 133), (32, 64, 64, 12, 500): (237, 203), (32, 64, 64, 24, 240): (198, 203),
+    (128, 128, 64, 1, 161): (65, 59), (128, 128, 64, 6, 161): (310, 230), (16, 128, 128, 1, 220): (35, 40),
+    (16, 128, 128, 1, 350): (53, 47), (16, 128, 128, 2, 180): (46, 49), (16, 128, 128, 6, 180): (106, 78)}
+DELTA_US = {
+    (16, 128, 128, 1, 260): (74, 86), (16, 128, 128, 1, 400): (113, 97), (16, 128, 128, 2, 400): (144, 116),
+    (16, 128, 128, 3, 400): (174, 200), (16, 128, 128, 3, 500): (217, 218), (16, 128, 128, 3, 700): (302, 275),
+    (16, 128, 128, 6, 400): (342, 308), (16, 128, 128, 12, 400): (581, 566), (32, 128, 128, 1, 400): (144, 114),
+    (32, 128, 128, 2, 400): (212, 216), (32, 128, 128, 2, 500): (265, 234), (32, 128, 128, 6, 500): (728, 646),
+    (8, 128, 128, 3, 400): (144, 109), (8, 128, 128, 6, 400): (174, 200), (8, 128, 128, 6, 700): (302, 275),
+    (16, 64, 64, 1, 400): (96, 77), (16, 64, 64, 2, 400): (96, 87), (16, 64, 64, 3, 400): (96, 110),
+    (16, 64, 64, 3, 700): (165, 144), (16, 64, 64, 6, 700): (213, 279), (16, 64, 64, 6, 1000): (303, 385),
+    (16, 64, 64, 12, 700): (270, 468), (16, 64, 64, 24, 350): (267, 509)}
+
+
+@pytest.mark.parametrize("kind", ["linear", "delta"])
+def test_the_rules_take_the_faster_way(kind):
+    """At every measured point: within 8 % of the faster one, which is what runs of one side differ by
+    and the points between which a line lies are apart."""
+    from binfer_b200.csrc import ops
+    rule, table = ((ops.chunk_scan_pays, LINEAR_US) if kind == "linear" else
+                   (ops.delta_chunks_pay, DELTA_US))
+    for (heads, dk, dv, portions, n), (walk, chunks) in table.items():
+        pays = rule(portions * n, n, heads, dk, dv)
+        assert (chunks if pays else walk) <= 1.08 * min(walk, chunks), (heads, dk, dv, portions, n)
+        # single tokens beside the portions change little
+        assert rule(portions * n + n // 50, n, heads, dk, dv) == pays

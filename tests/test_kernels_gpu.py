@@ -1160,13 +1160,14 @@ def test_linear_scan_in_chunks(cuda_device, lens, H, G, dk, dv, decays):
     err.zero_()
 
 
-def test_retention_part_walks_decays_below_zero(cuda_device):
+def test_retention_part_walks_decays_below_zero(cuda_device, monkeypatch):
     """A portion long enough for chunks and the same tokens in two that are walked."""
     from types import SimpleNamespace
     from binfer_b200.config import RetentionSpec
     from binfer_b200.csrc import ops
     from binfer_b200.engine import make_env
     from binfer_b200.parts.retention import RetentionMixer
+    monkeypatch.setattr(ops, "chunk_scan_pays", lambda *a: True)
     dev, T = cuda_device, 2 * ops.CHUNK_SCAN_MIN
     spec = RetentionSpec(num_heads=2, qk_dim=16, v_dim=128, decays=(-0.9, 0.8), position=None,
                          norm_eps=1e-5)
