@@ -361,9 +361,10 @@ def scan(a):
     token and head, q and k shared by groups of heads: the state space layer's), ``delta``
     (the gated delta rule) or ``retention`` (a fixed decay per head), --heads heads with
     --kv-heads heads of q and k, keys (the state's first size) of --state and values of
-    --head-dim.  Arithmetic is counted as the recurrence's own multiply-adds (state update and
-    read-out: 5 flops a state element and token, the delta rule 9) against the nominal float
-    rate of the FMA pipes; there is no measured peak for it."""
+    --head-dim; ``--chunked``: in chunks, as the bfloat16 engine runs long prompt portions.
+    Arithmetic is counted as the recurrence's own multiply-adds (state update and read-out: 5
+    flops a state element and token, the delta rule 9) against the nominal float rate of the FMA
+    pipes; there is no measured peak for it."""
     dev = torch.device("cuda:0")
     B, n, H, G, N, P = a.batch, a.tokens, a.heads, a.kv_heads, a.state, a.head_dim
     T = B * n
@@ -379,23 +380,26 @@ def scan(a):
             vf = torch.randn(T, H, P, device=dev)
             dec = torch.rand(T, H, device=dev) * 0.2 + 0.8
             sets.append(lambda qk=qk, vf=vf, dec=dec: ops.linear_scan(
-                qk, vf, dec, state, q_start, slots, o, B, H, G, N, P, err, max_q=n))
+                qk, vf, dec, state, q_start, slots, o, B, H, G, N, P, err, max_q=n,
+                chunked=a.chunked))
         elif a.kind == "delta":
             qkv = torch.randn(T, 2 * G * N + H * P, device=dev) * 0.1
             gates = torch.rand(T, 2, H, device=dev) * 0.2 + 0.8
             sets.append(lambda qkv=qkv, gates=gates: ops.delta_scan(
-                qkv, gates, state, q_start, slots, o, B, H, G, N, P, err, max_q=n))
+                qkv, gates, state, q_start, slots, o, B, H, G, N, P, err, max_q=n,
+                chunked=a.chunked))
         else:
             proj = (torch.randn(T, H * (2 * N + P), device=dev) * 0.1).to(BF16)
             dec = torch.rand(H, device=dev) * 0.2 + 0.8
             pos = torch.arange(n, device=dev, dtype=torch.int32).repeat(B)
             sets.append(lambda proj=proj, dec=dec, pos=pos: ops.retention_scan(
                 proj, 0, H * N, 2 * H * N, dec, None, pos, state, q_start, slots, o, B, H, N, P,
-                1.0, err, max_q=n))
+                1.0, err, max_q=n, chunked=a.chunked))
     us = timed(sets, a.iters, a.warmup)
     flops = (9.0 if a.kind == "delta" else 5.0) * T * H * N * P
-    out = {"kernel": a.kind + "_scan", "us": round(us, 2), "tokens": n, "requests": B, "heads": H,
-           "qk_heads": G, "keys": N, "values": P, "TFLOP/s": round(flops / us / 1e6, 2),
+    out = {"kernel": a.kind + "_scan" + ("_chunks" if a.chunked else ""), "us": round(us, 2),
+           "tokens": n, "requests": B, "heads": H, "qk_heads": G, "keys": N, "values": P,
+           "TFLOP/s": round(flops / us / 1e6, 2),
            "frac_of_nominal_fp32": round(flops / us / 1e6 / FP32_TFLOPS_NOMINAL, 3)}
     print(json.dumps(out), flush=True)
     assert int(err.item()) == 0
@@ -492,6 +496,7 @@ def main(argv=None):
     ap.add_argument("--hidden", type=int, default=4096)
     ap.add_argument("--kind", default="linear", choices=["linear", "delta", "retention"],
                     help="scan: which recurrence")
+    ap.add_argument("--chunked", action="store_true", help="scan: long portions in chunks")
     ap.add_argument("--state", type=int, default=128, help="scan: size of a key (the state's rows)")
     ap.add_argument("--layers", type=int, default=6, help="step_timeline: layers of the model")
     ap.add_argument("--intermediate", type=int, default=12288)

@@ -201,12 +201,14 @@ class LatentAttention(Mixer, StackedOut):
                 last: int) -> None:
         """Rows ``first .. last - 1`` of the step; ``q_abs`` (None: in place) begins with the first."""
         s, pos = self.spec, self.position
-        ops.latent_encode(proj[first:last], 0, self.q_rows, self.norm_w, s.norm_eps,
+        positions, slots = ctx.positions, ctx.slots[group]
+        if last - first < ctx.T:                 # (a view of each costs the host a microsecond)
+            proj, q, positions, slots = (x[first:last] for x in (proj, q, positions, slots))
+        ops.latent_encode(proj, 0, self.q_rows, self.norm_w, s.norm_eps,
                           pos.inv_freq if pos is not None else None,
                           bool(pos is not None and pos.interleaved),
-                          pos.magnitude if pos is not None else 1.0, ctx.positions[first:last],
-                          ctx.slots[group][first:last], q_abs, cache, self.H, self.d, self.dr,
-                          self.rank, ctx.err, q=q[first:last])
+                          pos.magnitude if pos is not None else 1.0, positions, slots, q_abs, cache,
+                          self.H, self.d, self.dr, self.rank, ctx.err, q=q)
 
     def _in_latent_coordinates(self, q, proj, out, ctx: StepContext, view: EntryView, T: int,
                                n_max: int = 0) -> None:
@@ -214,10 +216,11 @@ class LatentAttention(Mixer, StackedOut):
         what ``out`` holds for the others says nothing) with the queries carried into latent
         coordinates; ``q`` is left as it is."""
         s, H, g = self.spec, self.H, view.group
-        B = T if T < q.shape[0] else ctx.B       # (fewer rows than the step's: single tokens)
-        q, proj, out = q[:T], proj[:T], out[:T]
+        B = ctx.B
         q_abs = torch.empty((T, H, self.kv_size), dtype=q.dtype, device=q.device)
         self._encode(proj, q, q_abs, view.k_cache, ctx, g, 0, T)
+        if T < q.shape[0]:                       # fewer rows than the step's: single tokens
+            B, q, proj, out = T, q[:T], proj[:T], out[:T]
         q_heads = q.view(T, H, self.d + self.dr)
         linear_heads(q_heads[:, :, :self.d], self.w_ukT, q_abs[:, :, :self.rank])
         # (rows that the attention leaves alone go through the product behind it as zeros)
