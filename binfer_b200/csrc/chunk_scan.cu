@@ -21,11 +21,12 @@
 //   cs_out     o = [exp(G_t - G_c) q_t | exp(G_t - H_s) (q_t . k_s)] [S ; V]: one product with dk +
 //              C terms, the weights applied as its operands are stored into shared memory
 //
-// GPU time at 2,048 tokens (the walk at 2,000): 64 heads of 128 x 64 over 8 q/k heads 211 us (459; cs_out
-// 100, cs_state 62, cs_prefix 26, cs_qk 14, cs_gates 9); 8 heads of 128 x 256 126 (289); mLSTM, 8 heads of
-// 256 x 512, 394 (979; 172, 123, 55, 32, 11).  With expf, float products of q and k and the states' sums
-// in runs of 16 these were 204, 119 and 381 us, and further from 64 bits than the walk where decays are
-// fast.  Relative errors against 64 bits over 777 tokens, walk / chunks: decays of 0.98 to 1: o 1.9e-7 /
+// GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads 208 / 467 us (cs_out 99,
+// cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8); 8 heads of 128 x 256 124 / 270; mLSTM, 8 heads of 256 x
+// 512, 392 / 979 (171, 123, 55, 32, 11).  What bounds them: cs_state and cs_out shared-memory reads (the
+// pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
+// expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
+// further from 64 bits than the walk where decays are fast.  Relative errors against 64 bits over 777 tokens, walk / chunks: decays of 0.98 to 1: o 1.9e-7 /
 // 1.4e-7, state 1.8e-7 / 1.3e-7; spread over 0 to 1: o 8.3e-8 / 5.0e-8, state 4.0e-8 / 4.2e-8 (half a unit
 // in the last place is up to 6.0e-8); mLSTM, gates that forget in a few tokens and in twenty: o 4.8e-7 /
 // 2.3e-7 and 1.3e-5 / 1.2e-6, state 2.9e-8 / 3.7e-8 and 2.3e-7 / 1.0e-7.
@@ -47,8 +48,8 @@
 //              32 columns) in parallel
 //   cs_out     as above, on U
 //
-// 2,048 tokens of 16 heads of 128: 342 us (ds_walk 186, cs_out 55, ds_prep 49, cs_qk 42); 1,000 tokens 168
-// against the walk's 277, three portions of 1,000 381 against 431.  Errors against 64 bits, walk / chunks:
+// 2,048 tokens of 16 heads of 128: 341 us (ds_walk 187, cs_out 54, ds_prep 48, cs_qk 42) against the walk's
+// 563; 1,000 tokens 168 and 277, three portions of 1,000 381 and 431.  Errors against 64 bits, walk / chunks:
 // keys at random, decays of 0.98 to 1: o 2.3e-7 / 1.6e-7, state 2.3e-7 / 1.8e-7; keys of a cosine of 0.9
 // 2.6e-7 / 2.6e-7 and 2.5e-7 / 2.5e-7; fast decays o 1.1e-7 / 7.8e-8, state 6.2e-8 / 7.1e-8.  (What the walk
 // has and a chunk's inverse has not is that a token's u answers to the rounding of the one before it:
@@ -106,23 +107,25 @@ __device__ __forceinline__ float4 cs_times(float4 v, float2 w) {
   return make_float4(cs_times(v.x, w), cs_times(v.y, w), cs_times(v.z, w), cs_times(v.w, w));
 }
 
-// e^x as a float and what is left of it, good to some 2^-28: x = n ln 2 + r in double, the power series
-// of e^r to the seventh power (|r| <= ln 2 / 2: the eighth is below 2^-27) on top of 1 + r, whose
-// rounding is kept.  (The weights of tokens hang together in every result: with expf, up to two units
+// e^x as a float and what is left of it, good to some 2^-26: x = n ln 2 + r in double (n by adding what
+// leaves no place for a fraction), the power series of e^r to the seventh power (|r| <= ln 2 / 2: the
+// eighth is below 2^-27) on top of 1 + r, whose rounding is kept.  One conversion: those and the double
+// operations are what it costs.  (The weights of tokens hang together in every result: with expf, up to two units
 // off in the last place, an output of keys and queries alike was four times as far from 64 bits as
 // the walk's.)
 __device__ __forceinline__ float2 cs_exp(double x) {
   if (!(x > -104.0)) return make_float2(x != x ? NAN : 0.f, 0.f);
   if (x > 89.0) return make_float2(INFINITY, 0.f);
-  const int n = __double2int_rn(x * 1.4426950408889634);
-  const double r = fma((double)n, -0.69314718055994531, x);
-  const float rh = (float)r, rl = (float)(r - (double)rh);
+  const double whole = 6755399441055744.0;            // 1.5 2^52
+  const double t = fma(x, 1.4426950408889634, whole);
+  const int n = __double2loint(t);
+  const float rh = (float)fma(t - whole, -0.69314718055994531, x);
   float q = fmaf(rh, 1.f / 5040.f, 1.f / 720.f);
   q = fmaf(rh, q, 1.f / 120.f);
   q = fmaf(rh, q, 1.f / 24.f);
   q = fmaf(rh, q, 1.f / 6.f);
   q = fmaf(rh, q, 0.5f);
-  const float s = 1.f + rh, rest = fmaf(rh * rh, q, (rh - (s - 1.f)) + rl);
+  const float s = 1.f + rh, rest = fmaf(rh * rh, q, rh - (s - 1.f));
   const float hi = s + rest, lo = rest - (hi - s);
   // (two factors: n may lie below the smallest normal exponent)
   const int n1 = n >> 1;
