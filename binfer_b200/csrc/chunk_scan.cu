@@ -26,10 +26,12 @@
 // 512, 392 / 979 (171, 123, 55, 32, 11).  What bounds them: cs_state and cs_out shared-memory reads (the
 // pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
 // expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
-// further from 64 bits than the walk where decays are fast.  Relative errors against 64 bits over 777 tokens, walk / chunks: decays of 0.98 to 1: o 1.9e-7 /
-// 1.4e-7, state 1.8e-7 / 1.3e-7; spread over 0 to 1: o 8.3e-8 / 5.0e-8, state 4.0e-8 / 4.2e-8 (half a unit
-// in the last place is up to 6.0e-8); mLSTM, gates that forget in a few tokens and in twenty: o 4.8e-7 /
-// 2.3e-7 and 1.3e-5 / 1.2e-6, state 2.9e-8 / 3.7e-8 and 2.3e-7 / 1.0e-7.
+// further from 64 bits than the walk where decays are fast.
+//
+// Relative errors against 64 bits over 777 tokens, walk / chunks: decays of 0.98 to 1: o 1.9e-7 / 1.4e-7,
+// state 1.8e-7 / 1.3e-7; spread over 0 to 1: o 8.3e-8 / 5.0e-8, state 4.0e-8 / 4.2e-8 (half a unit in the
+// last place is up to 6.0e-8); mLSTM, gates that forget in a few tokens and in twenty: o 4.8e-7 / 2.3e-7 and
+// 1.3e-5 / 1.2e-6, state 2.9e-8 / 3.7e-8 and 2.3e-7 / 1.0e-7.
 //
 // Why: the walk has heads x dk x dv independent elements and a chain of multiply-adds from token to
 // token, so it left the FP32 pipes at 15 to 20 % (see those files); the products have no chain and
