@@ -1906,6 +1906,39 @@ def test_mlstm_gates_tiles(cuda_device, T, width, heads, dtype):
     _close(gates, z, F32)
 
 
+@pytest.mark.parametrize("what", ["weights", "state", "rows of states"])
+def test_convolutions_off_a_boundary(cuda_device, what):
+    """Weights, states or the way from state to state off 16-byte pieces: read as before."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(7)
+    dev, T, H, G, d, taps = cuda_device, 5, 4, 2, 32, 4
+    C = (H + 2 * G) * d
+    proj = torch.randn(T, C + H, device=dev).to(BF16)
+    w, bias = torch.randn(C, taps, device=dev), torch.randn(C, device=dev)
+    state = torch.randn(2, (taps - 1) * C, device=dev)
+    A_log, dt_bias, D = (torch.randn(H, device=dev) for _ in range(3))
+    slots, qs = torch.tensor([1], dtype=torch.int32, device=dev), torch.tensor([0, T], dtype=torch.int32,
+                                                                               device=dev)
+    seq, err, got = torch.zeros(T, dtype=torch.int32, device=dev), _err(dev), []
+
+    def off(x):
+        y = torch.empty(x.numel() + 1, device=dev)[1:].view_as(x)
+        return y.copy_(x)
+    wide = torch.empty(2, state.shape[1] + 1, device=dev)
+    for case in ("aligned", what):
+        a = off(w) if case == "weights" else w
+        b = off(state) if case == "state" else state
+        if case == "rows of states":
+            b = wide[:, :-1].copy_(state)
+        qk, decay = torch.empty(T, 2, G, d, device=dev), torch.empty(T, H, device=dev)
+        vf, skip = torch.empty(T, H, d, device=dev), torch.empty(T, H, d, device=dev)
+        ops.mamba2_encode(proj, 0, C, a, bias, taps, b, slots, seq, qs, A_log, dt_bias, D, qk, vf,
+                          skip, decay, H, G, d, d, err)
+        got.append(torch.cat([x.flatten() for x in (qk, vf, skip, decay)]))
+    assert int(err.item()) == 0
+    _close(got[1], got[0], F32)
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("dv", [128, 256, 512, 1024, 96])
 def test_head_norm_out_in_registers(cuda_device, dv, dtype):
