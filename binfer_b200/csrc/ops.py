@@ -827,6 +827,8 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
     if 2 * rot_half > dk:
         raise KernelError("retention_scan: more rotated sizes than a head has")
     T = proj.shape[0]
+    if positions is None or positions.numel() < T:        # (read for every row, turned or not)
+        raise KernelError("retention_scan: positions must have one number per row")
     # the turned q and k and the values of every token in float: written by the first of the
     # two kernels
     qk = torch.empty((T, 2, heads, dk), dtype=torch.float32, device=proj.device)

@@ -50,7 +50,8 @@ def test_scans_off_16_byte_boundaries_are_walked(monkeypatch):
                         err, max_q=T, chunked=True)
 
     def retention(off):
-        ops.retention_scan(torch.zeros(T, 3 * H * d), 0, H * d, 2 * H * d, buf(H), None, slots,
+        ops.retention_scan(torch.zeros(T, 3 * H * d), 0, H * d, 2 * H * d, buf(H), None,
+                           torch.arange(T, dtype=torch.int32),
                            buf(1, H * d * d), qs, slots, buf(T, H * d, off=off == 2), 1, H, d, d, 1.0,
                            err, max_q=T, chunked=True)
 
@@ -109,3 +110,14 @@ def test_the_rules_take_the_faster_way(kind):
         assert (chunks if pays else walk) <= 1.08 * min(walk, chunks), (heads, dk, dv, portions, n)
         # single tokens beside the portions change little
         assert rule(portions * n + n // 50, n, heads, dk, dv) == pays
+
+
+@pytest.mark.parametrize("positions", [None, torch.zeros(3, dtype=torch.int32)])
+def test_retention_wants_a_position_per_row(monkeypatch, positions):
+    from binfer_b200.csrc import ops
+    seen = fake_library(monkeypatch, ops)
+    one = torch.zeros(1, dtype=torch.int32)
+    with pytest.raises(ops.KernelError, match="positions"):
+        ops.retention_scan(torch.zeros(4, 24), 0, 8, 16, torch.zeros(1), None, positions,
+                           torch.zeros(1, 64), one, one, torch.zeros(4, 8), 1, 1, 8, 8, 1.0, one)
+    assert not seen
