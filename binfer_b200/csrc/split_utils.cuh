@@ -1,0 +1,82 @@
+// Floats as sums of bfloat16 terms, for products of 32-bit operands on the tensor cores.
+//
+// A float has 24 significant bits, a bfloat16 eight and the same range of exponents: the nearest
+// bfloat16, the nearest one to what is left and what is left then are three bfloat16 numbers whose
+// sum is the float.  A product of two floats is then nine products of terms, each exact in float; the
+// three smallest (below 2^-26 of the product together) are left out.
+#pragma once
+#include "common.cuh"
+#include "umma_utils.cuh"
+
+namespace {
+
+// (a, b) -> the terms of a in the low halves, those of b in the high halves: hi, mid, lo.
+__device__ __forceinline__ uint32_t split_pack(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+__device__ __forceinline__ void sub2f(float& x, float& y, float a, float b, uint32_t terms) {
+  asm("{\n\t.reg .b64 u, v;\n\t"
+      "mov.b64 u, {%2, %3};\n\t"
+      "mov.b64 v, {%4, %5};\n\t"
+      "sub.rn.f32x2 u, u, v;\n\t"
+      "mov.b64 {%0, %1}, u;\n\t}"
+      : "=f"(x), "=f"(y)
+      : "f"(a), "f"(b), "f"(__uint_as_float(terms << 16)), "f"(__uint_as_float(terms & 0xffff0000u)));
+}
+// left: gets what is left behind the first terms added up, which is finite exactly where both
+// floats have terms.
+__device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo,
+                                       float2& left) {
+  float x, y;
+  hi = split_pack(a, b);
+  sub2f(x, y, a, b, hi);
+  add2f(left.x, left.y, x, y);
+  mid = split_pack(x, y);
+  sub2f(x, y, x, y, mid);
+  lo = split_pack(x, y);
+}
+
+// tcgen05.mma by one lane of a converged warp.  All lanes compute the operands, so that these stay in
+// uniform registers: issued from a branch of one lane, each product first moves its six
+// operands there, at some 55 cycles a product.
+__device__ __forceinline__ void umma_bf16_warp(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc,
+                                               uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_u32(bar))
+      : "memory");
+}
+
+// Infinities, NaN and the floats above the largest bfloat16 have no such terms (inf - inf).
+__device__ __forceinline__ bool have_terms(const float4& v) {
+  const uint32_t top = max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
+                           max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
+  return top < 0x7f7f8000u;
+}
+
+// K-major operand tile in rows of 64 bytes (32 bfloat16) with the 64-byte swizzle: 8-row groups
+// 512 bytes apart.  A row's 16-byte piece p lies at piece p ^ (row / 2 % 4).
+__device__ __forceinline__ uint64_t umma_desc_k_sw64(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;                            // leading byte offset (unused here)
+  d |= (uint64_t)(512 >> 4) << 32;                   // stride byte offset: 8 rows
+  d |= (uint64_t)1 << 46;                            // descriptor version of sm_100
+  d |= (uint64_t)4 << 61;                            // SWIZZLE_64B
+  return d;
+}
+
+}  // namespace

@@ -1,6 +1,6 @@
 """The dense matrix product ``y = x W^T`` with weights as stored (``[out, in]`` row-major).
 
-float32 engine: the engine's own FP32-FMA kernel (no reduced-precision matrix mode).
+float32 engine: the engine's own kernels of 32-bit precision (no reduced-precision matrix mode).
 bfloat16 engine: the engine's tcgen05/TMEM/TMA kernel (``csrc/gemm_tcgen05.cu``) or
 cuBLAS through ``torch.mm`` with float accumulation, the library call the reference
 makes for every dense product (cuda/kernels/gemm.cu:244-267: ``cublasGemmEx``, bf16
@@ -213,7 +213,7 @@ def linear_add_tanh(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor,
 def linear_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """``out[:, h] = x[:, h] @ w[h]^T`` for every head h: ``x [T, H, K]`` and ``out [T, H, N]``
     may be strided views of wider rows (innermost stride 1), ``w [H, N, K]`` contiguous.
-    float32: the engine's own FP32-FMA kernel, one launch for all heads; bfloat16: the
+    float32: the engine's own kernels, one launch for all heads; bfloat16: the
     library's strided batched product with float accumulation."""
     if x.dtype == torch.float32:
         ops.sgemm_nt_batched(x, w, out)

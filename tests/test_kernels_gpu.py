@@ -135,6 +135,71 @@ def test_sgemm_more_rows_than_a_grid_has_tiles(cuda_device):
     assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
 
 
+# 512 terms and more: three bfloat16 terms an operand.  Rows about the tiles (16, 112, 176), features
+# about 128 and about the numbers of tiles that share K among 4, 2 and 1 CTAs; K about steps of 32
+# and runs of 8 steps.
+@pytest.mark.parametrize("M,N,K", [(1, 127, 512), (16, 129, 516), (17, 2304, 800), (112, 2305, 2048),
+                                   (113, 64, 1027), (177, 9472, 640), (353, 9473, 544), (300, 8, 6145)])
+def test_sgemm_of_terms(cuda_device, M, N, K):
+    from binfer_b200.csrc import ops
+    a = torch.randn(M, K, device=cuda_device)
+    w = torch.randn(N, K, device=cuda_device)
+    a[:, 1] *= 1e-30                                  # (terms far below the others)
+    out = torch.full((M, N + 3), 7.0, device=cuda_device)[:, :N]
+    ops.sgemm_nt(a, w, out)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # twelve products of terms a step, each sum cut off behind 24 bits (2^-23), then rounded sums
+    # in runs of eight steps, of the runs, of four CTAs; terms left out below 2^-26
+    bound = (12 * 2 + 8 + K / 256 + 4 + 1) * 2.0 ** -24 * size
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    assert float((out.double() - ref).norm() / ref.norm()) < 1.6e-7      # (measured 1.1e-7)
+    off = torch.randn(M, K + 1, device=cuda_device)
+    off[:, 1:] = a
+    other = torch.full((M, N), 7.0, device=cuda_device)
+    ops.sgemm_nt(off[:, 1:], w, other)
+    assert torch.equal(out, other)
+    one = torch.full((1, N), 7.0, device=cuda_device)
+    ops.sgemm_nt(a[M - 1:], w, one)
+    assert torch.equal(one[0], out[M - 1])
+    heads = torch.full((M, 2, N), 7.0, device=cuda_device)
+    ops.sgemm_nt_batched(torch.stack([w[:1].expand(M, K), a], 1), torch.stack([w, w]), heads)
+    assert torch.equal(heads[:, 1], out)
+    assert int(ops.error_word(cuda_device).item()) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512)])
+def test_sgemm_of_terms_with_infinities(cuda_device, M, N, K):
+    """Infinities, NaN and floats that no bfloat16 reaches give what multiply-adds give, and stay in
+    their rows and columns."""
+    from binfer_b200.csrc import ops
+    a, w = torch.randn(M, K, device=cuda_device), torch.randn(N, K, device=cuda_device)
+    clean = torch.empty(M, N, device=cuda_device)
+    ops.sgemm_nt(a, w, clean)
+    a[1, 5], a[2, 7], a[3, 9] = float("inf"), float("nan"), 3.4e38
+    w[9, 2], w[11, 0], w[12, 5] = -float("inf"), float("nan"), 0.0
+    w[:, 9] *= 1e-3
+    a[:, 9][a[:, 9].abs() < 1e30] = 0.0
+    want = (a.double() @ w.double().T).float()
+    out = torch.empty(M, N, device=cuda_device)
+    ops.sgemm_nt(a, w, out)
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    fin = want.isfinite()
+    # (rows of multiply-adds: one sequential sum)
+    bound = K * 2.0 ** -24 * (torch.nan_to_num(a, 0, 0, 0).double().abs()
+                              @ torch.nan_to_num(w, 0, 0, 0).double().abs().T)
+    assert bool(((out.double() - want.double()).abs() <= bound)[fin].all())
+    a[:, 9], w[:, 9] = 0.0, 0.0
+    for t in (a, w):
+        t[~t.isfinite().all(-1)] = 1.0
+    again = torch.empty(M, N, device=cuda_device)
+    ops.sgemm_nt(a, w, again)
+    rows = torch.ones(M, dtype=torch.bool, device=cuda_device)
+    rows[1:4] = False
+    cols = torch.ones(N, dtype=torch.bool, device=cuda_device)
+    cols[[9, 11]] = False
+    assert torch.equal(out[rows][:, cols], again[rows][:, cols])
+
+
 # ------------------------------------------------------- q/k norm, rotation, cache write
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("nh,nkv,d,rot,norm", [(3, 1, 16, 16, True), (4, 2, 48, 24, True),
