@@ -21,9 +21,12 @@
 //   cs_out     o = [exp(G_t - G_c) q_t | exp(G_t - H_s) (q_t . k_s)] [S ; V]: one product with dk +
 //              C terms, the weights applied as its operands are stored into shared memory
 //
+// The mLSTM with keys in whole steps of 64 and values in whole tiles of 128 runs its products on the tensor
+// cores (mlstm_tensor.cuh: the last three kernels become two).
+//
 // GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads 208 / 467 us (cs_out 99,
 // cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8); 8 heads of 128 x 256 124 / 270; mLSTM, 8 heads of 256 x
-// 512, 392 / 979 (171, 123, 55, 32, 11).  What bounds them: cs_state and cs_out shared-memory reads (the
+// 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 208).  What bounds them: cs_state and cs_out shared-memory reads (the
 // pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
 // expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
 // further from 64 bits than the walk where decays are fast.
@@ -808,6 +811,8 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
   }
 }
 
+#include "mlstm_tensor.cuh"
+
 // ------------------------------------------------------------------- the gated delta rule
 #define DS_C 64            // tokens a chunk
 #define DS_D 128           // most key and value sizes
@@ -1196,6 +1201,11 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
       Hs, E, g0, Wl, p.C, p.T, p.H, p.dk * p.dv, p.dk, p.n_min, p.H);
   cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles), 128, 0, stream>>>(qk, p, q_start,
                                                                                  qkm, nullptr);
+  if constexpr (MLSTM) {
+    if (mt_takes(p, qk) && (long long)l.chunks * p.H * (p.dv / MT_M) < 0x7fffffff)
+      return mt_launch(qk, p, l.chunks, q_start, state, slot_stride, state_size, state_slots, n_slots, G, Hs, g0,
+                       Wl, E, qkm, U, Un, o_raw, err, stream);
+  }
   cs_state_kernel<A, V, MLSTM><<<dim3(l.chunks, p.H, tk * tv), CS_THREADS, 0, stream>>>(
       qk, v, p, q_start, Wl, U, Un);
   const int elems = p.dk * p.dv + (MLSTM ? p.dk : 0);

@@ -1442,6 +1442,70 @@ def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
         assert products <= 1.5 * walk + 2e-7, off
 
 
+# keys in whole steps of 64 and values in whole tiles of 128: the products on the tensor cores.  One chunk
+# and its edges, chunks behind the 32 whose decays are at hand, one to three tiles of either, requests that
+# are walked between them
+@pytest.mark.parametrize("lens,H,dk,dv", [([161, 1, 192, 160, 257], 2, 64, 128), ([2177], 1, 64, 128),
+                                          ([193, 320], 3, 128, 384), ([170, 3, 449], 2, 192, 256)])
+def test_mlstm_chunks_on_tensor_cores(cuda_device, monkeypatch, lens, H, dk, dv):
+    from binfer_b200.csrc import ops
+    test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv)
+    # rows off the 16-byte boundaries take the multiply-adds: the same but for the order of sums
+    dev, T, B = cuda_device, sum(lens), len(lens)
+    wide = torch.randn(T, 2 * H * (dk + dv) + 4, device=dev).to(BF16)
+    gates = torch.cat([torch.randn(T, H, device=dev), -torch.rand(T, H, device=dev)], 1).contiguous()
+    slots, err = torch.arange(B, dtype=torch.int32, device=dev), _err(dev)
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    got = []
+    for proj in (wide[:, 4:].contiguous(), wide[:, 4:]):
+        s = torch.zeros(B, H, ops.mlstm_state_size(dk, dv), device=dev)
+        o = torch.zeros(T, H * dv, device=dev)
+        ops.mlstm_scan(proj, gates, s, qs, slots, o, B, H, dk, dv, dk ** -0.5, err, max_q=max(lens),
+                       chunked=True)
+        got.append((o, s))
+    assert int(err.item()) == 0
+    # (a request's outputs are quotients whose denominators may nearly vanish)
+    assert float((got[0][0] - got[1][0]).norm() / got[1][0].norm()) < 2e-5
+    assert float((got[0][1] - got[1][1]).norm() / got[1][1].norm()) < 1e-6
+    bad = slots.clone()
+    bad[0] = -1
+    keep = got[0][1].clone()
+    ops.mlstm_scan(wide[:, 4:].contiguous(), gates, keep, qs, bad, got[0][0], B, H, dk, dv, 1.0, err,
+                   max_q=max(lens), chunked=True)
+    assert int(err.item()) == 2 and torch.equal(keep[0], got[0][1][0])
+    err.zero_()
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v"])
+@pytest.mark.parametrize("at", [64, 140, 255])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_mlstm_chunks_on_tensor_cores_keep_infinities_apart(cuda_device, what, at, bad):
+    """What is not a number shows where the multiply-adds show it, and nowhere else changes a bit of the
+    tokens before it and of the other head."""
+    from binfer_b200.csrc import ops
+    dev, T, H, dk, dv = cuda_device, 300, 2, 128, 256
+    torch.manual_seed(6)
+    proj = torch.randn(T, 2 * H * (dk + dv), device=dev).to(BF16)
+    gates = torch.cat([torch.randn(T, H, device=dev), -torch.rand(T, H, device=dev)], 1).contiguous()
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, got = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    column = {"q": dk + 5, "k": H * dk + dk + 5, "v": 2 * H * dk + dv + 130}[what]     # of head 1
+    for spoil, walk in ((False, False), (True, False), (True, True)):
+        x = proj.clone()
+        if spoil:
+            x[at, column] = bad
+        s = torch.zeros(1, H, ops.mlstm_state_size(dk, dv), device=dev)
+        o = torch.zeros(T, H * dv, device=dev)
+        ops.mlstm_scan(x, gates, s, qs, slots, o, 1, H, dk, dv, dk ** -0.5, err, max_q=T, chunked=not walk)
+        got.append((o.view(T, H, dv), s[0]))
+    (clean, cs), (out, os), (want, ws) = got
+    assert torch.equal(out[:, 0], clean[:, 0]) and torch.equal(os[0], cs[0])
+    assert torch.equal(out[:at, 1], clean[:at, 1])
+    assert torch.equal(out.isfinite(), want.isfinite()) and torch.equal(os.isfinite(), ws.isfinite())
+    if what == "v":                                # (the other values' sizes)
+        assert torch.equal(out[:, 1, :130], clean[:, 1, :130]) and torch.equal(out[:, 1, 131:], clean[:, 1, 131:])
+
+
 # ------------------------------------------- latent attention with keys and values expanded
 # portions below, at and above a key tile of 64, a query tile of 128 and a block of 256, from the
 # start and behind cached keys; the rows of two portions and a single token's row in one buffer
