@@ -220,7 +220,7 @@ prefill_attention_umma_kernel(const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp == AU_MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
       // S: a = Q (K-major), b = K tile (K-major), N = 64 keys
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) |
                                ((uint32_t)(AU_BN >> 3) << 17) | ((uint32_t)(AU_BM >> 4) << 24);
@@ -240,7 +240,7 @@ prefill_attention_umma_kernel(const __grid_constant__ CUtensorMap map_q,
         umma_commit(s_full + (n & 1));
       };
       const int tiles = kt_last - kt_first + 1;
-      bool ok = mbar_wait(q_full, 0, abort) && mbar_wait(kv_full, 0, abort);
+      bool ok = mbar_wait_warp(q_full, 0, abort) && mbar_wait_warp(kv_full, 0, abort);
       if (ok) {
         tc_fence_after();
         issue_s(0);
@@ -250,11 +250,11 @@ prefill_attention_umma_kernel(const __grid_constant__ CUtensorMap map_q,
         if (n + 1 < tiles) {
           // S of the next tile runs under the softmax of this one; its buffer is free since
           // the softmax threads signalled P of the tile before this one
-          if (!(ok = mbar_wait(kv_full + ((n + 1) & 1), ((n + 1) >> 1) & 1, abort))) break;
+          if (!(ok = mbar_wait_warp(kv_full + ((n + 1) & 1), ((n + 1) >> 1) & 1, abort))) break;
           tc_fence_after();
           issue_s(n + 1);
         }
-        if (!(ok = mbar_wait(p_full + (n & 1), (uint32_t)(n >> 1) & 1u, abort))) break;
+        if (!(ok = mbar_wait_warp(p_full + (n & 1), (uint32_t)(n >> 1) & 1u, abort))) break;
         tc_fence_after();
         const uint32_t p_addr = smem_u32(P_OVER_K ? Ks + buf * KV_BYTES : Psep);
         const uint32_t v_addr = smem_u32(Vs + buf * KV_BYTES);

@@ -338,7 +338,7 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
     // tensor memory; they share the K and V tiles, which are released when both have arrived.
     const int grp = warp - A2_MMA_WARP;
     const int my_tiles = grp == 0 ? tiles_a : (active_b ? tiles : 0);
-    if (lane == 0) {
+    {
       // S: a = Q (K-major), b = K tile (K-major), N = 64 keys
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) |
                                ((uint32_t)(A2_BN >> 3) << 17) | ((uint32_t)(A2_BM >> 4) << 24);
@@ -359,7 +359,7 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         umma_commit(s_full + grp * 2 + (n & 1));
       };
-      bool ok = my_tiles == 0 || (mbar_wait(q_full, 0, abort) && mbar_wait(kv_full, 0, abort));
+      bool ok = my_tiles == 0 || (mbar_wait_warp(q_full, 0, abort) && mbar_wait_warp(kv_full, 0, abort));
       if (ok && my_tiles > 0) {
         tc_fence_after();
         issue_s(0);
@@ -370,11 +370,11 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
           // the next tile's product runs under this tile's softmax; its S buffer is free
           // since the group signalled P of the tile before this one
           const int s1 = (n + 1) % STAGES;
-          if (!(ok = mbar_wait(kv_full + s1, (uint32_t)((n + 1) / STAGES) & 1u, abort))) break;
+          if (!(ok = mbar_wait_warp(kv_full + s1, (uint32_t)((n + 1) / STAGES) & 1u, abort))) break;
           tc_fence_after();
           issue_s(n + 1);
         }
-        if (!(ok = mbar_wait(p_full + grp * 2 + (n & 1), (uint32_t)(n >> 1) & 1u, abort))) break;
+        if (!(ok = mbar_wait_warp(p_full + grp * 2 + (n & 1), (uint32_t)(n >> 1) & 1u, abort))) break;
         tc_fence_after();
         const uint32_t v_addr = smem_u32(Vs + st * V_BYTES);
         const uint32_t d_addr = tmem_base + (uint32_t)(256 + grp * 128);
@@ -395,8 +395,8 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
       // cannot land in an earlier use of the stage)
       if (grp == 0 && active_b)
         for (int n = tiles_a; n < tiles && ok; ++n) {
-          if (!(ok = mbar_wait(kv_full + n % STAGES, (uint32_t)(n / STAGES) & 1u, abort))) break;
-          mbar_arrive(kv_empty + n % STAGES);
+          if (!(ok = mbar_wait_warp(kv_full + n % STAGES, (uint32_t)(n / STAGES) & 1u, abort))) break;
+          if (lane == 0) mbar_arrive(kv_empty + n % STAGES);
         }
     }
   } else {

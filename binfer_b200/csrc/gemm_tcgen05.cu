@@ -131,19 +131,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       // c = float, a = b = bf16, both K-major, N = bn, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                              ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(p.mma_rows >> 4) << 24);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
-      for (int u = blockIdx.x; u < units && !*abort; u += gridDim.x) {
-        if (!mbar_wait(acc_empty + acc, acc_phase ^ 1, abort)) break;
+      for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        if (!mbar_wait_warp(acc_empty + acc, acc_phase ^ 1, abort)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
         bool ok = true;
         for (int kc = 0; kc < kc_total; ++kc) {
-          if (!mbar_wait(full + stage, phase, abort)) {
+          if (!mbar_wait_warp(full + stage, phase, abort)) {
             ok = false;
             break;
           }
@@ -238,7 +238,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
         }
       }
     }
-    if (warp == 1 && lane == 0) {
+    if (warp == 1) {
       umma_commit(drain);                      // products still in flight
       const long long t0 = clock64();
       while (!mbar_try_wait(drain, 0) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {

@@ -305,7 +305,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_x,
     // with few K steps, an "unspecified launch failure" (or a wait that gave up) once in a
     // thousand launches with a hundred of them.
     const int who = warp == 1 ? 0 : 1;
-    if (lane == 0 && who < p.issuers && kc1 - kc0 > who) {
+    if (who < p.issuers && kc1 - kc0 > who) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                              ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(p.mma_rows >> 4) << 24);
       const uint32_t acc = tmem_base + (uint32_t)(who * p.acc_stride);
@@ -313,7 +313,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_x,
       for (int n = 0; n < kc1 - kc0; ++n) {
         const int stage = n % STAGES;
         if (p.issuers == 2 && (stage & 1) != who) continue;
-        if (!mbar_wait(full + stage, (uint32_t)(n / STAGES) & 1u, abort)) {
+        if (!mbar_wait_warp(full + stage, (uint32_t)(n / STAGES) & 1u, abort)) {
           ok = false;
           break;
         }

@@ -215,19 +215,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       // c = float, a = b = bf16, both K-major, N = bn, M = 256 over the pair
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                              ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(PM >> 4) << 24);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
-      for (int u = pair; u < units && !*abort; u += pairs) {
-        if (!mbar_wait(acc_empty + acc, acc_phase ^ 1, abort)) break;
+      for (int u = pair; u < units; u += pairs) {
+        if (!mbar_wait_warp(acc_empty + acc, acc_phase ^ 1, abort)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * 256);
         bool ok = true;
         for (int kc = 0; kc < kc_total; ++kc) {
-          if (!mbar_wait(full + stage, phase, abort)) {
+          if (!mbar_wait_warp(full + stage, phase, abort)) {
             ok = false;
             break;
           }
@@ -396,7 +396,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x,
         }
       }
     }
-    if (warp == 1 && lane == 0 && rank == 0) {
+    if (warp == 1 && rank == 0) {
       pair_commit_own(drain);                  // products still in flight
       const long long t0 = clock64();
       while (!mbar_try_wait(drain, 0) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {

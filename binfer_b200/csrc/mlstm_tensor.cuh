@@ -147,11 +147,11 @@ __device__ __forceinline__ void mt_products(uint32_t d, uint32_t a, uint32_t b) 
   for (int t = 2; t > 0; --t)                    // (one side has one term) the smallest first
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      umma_bf16_warp(d + 2 * MT_C, da + (uint64_t)(((TA > 1 ? t : 0) * MT_TILE + k * ka) >> 4),
+      umma_bf16(d + 2 * MT_C, da + (uint64_t)(((TA > 1 ? t : 0) * MT_TILE + k * ka) >> 4),
                      db + (uint64_t)(((TB > 1 ? t : 0) * MT_TOK + k * kb) >> 4), idesc, t < 2 || k > 0);
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    umma_bf16_warp(d + (k >> 1) * MT_C, da + (uint64_t)(k * ka >> 4), db + (uint64_t)(k * kb >> 4), idesc, k & 1);
+    umma_bf16(d + (k >> 1) * MT_C, da + (uint64_t)(k * ka >> 4), db + (uint64_t)(k * kb >> 4), idesc, k & 1);
 }
 
 struct MtShared {
@@ -187,7 +187,7 @@ __device__ __forceinline__ void mt_end(MtShared& s, uint32_t tmem, int* err) {
   if (*(volatile int*)&s.abort) {                        // (a wait gave up)
     if (threadIdx.x == 0) atomicOr(err, BF_ERR_WAIT);
     if (threadIdx.x >> 5 == MT_MMA) {                    // products still in flight
-      umma_commit_warp(&s.drain);
+      umma_commit(&s.drain);
       const long long t0 = clock64();
       while (!mbar_try_wait(&s.drain, 0) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
       }
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_state_kernel(
       tc_fence_after();
       const uint32_t at = smem_u32(tiles) + (uint32_t)((i & 1) * MT_STATE_STAGE);
       mt_products<3, 1, true>(tmem + (uint32_t)((i & 1) * 3 * MT_C), at, at + 3 * MT_TILE);
-      umma_commit_warp(sh.done + (i & 1));
+      umma_commit(sh.done + (i & 1));
     }
     mt_end(sh, tmem, err);
     return;
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
         const uint32_t d = tmem + (uint32_t)((i & 1) * 3 * MT_C);
         if (step < steps) mt_products<3, 1, false>(d, tm, tm + 3 * MT_TILE);
         else mt_products<1, 3, false>(d, tm, tm + 3 * MT_TILE);
-        umma_commit_warp(sh.done + (i & 1));
+        umma_commit(sh.done + (i & 1));
         if (step == 0) more = next();            // (read by the others behind a later step's barrier)
       }
     }

@@ -466,10 +466,10 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
       for (int t = 0; t < 6; ++t)
 #pragma unroll
         for (int k = 0; k < SP_K / 16; ++k)
-          umma_bf16_warp(d, wd + (uint64_t)(TW[t] * (W_BYTES >> 4) + 2 * k),
+          umma_bf16(d, wd + (uint64_t)(TW[t] * (W_BYTES >> 4) + 2 * k),
                     ad + (uint64_t)(TA[t] * (A_BYTES >> 4) + 2 * k), idesc, t > 0 || k > 0);
-      umma_commit_warp(empty + stage);
-      umma_commit_warp(acc_full + acc);
+      umma_commit(empty + stage);
+      umma_commit(acc_full + acc);
       if (++stage == p.stages) {
         stage = 0;
         phase ^= 1;
@@ -488,7 +488,7 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
   const bool sums = warp >= SP_FETCH && warp < SP_FETCH + SP_SUM;
   if (*abort) {                            // products still in flight (bounded), then leave
     if (tid == 0) atomicOr(p.err, BF_ERR_WAIT);
-    if (warp == SP_MMA && lane == 0) {
+    if (warp == SP_MMA) {
       umma_commit(drain);
       const long long t0 = clock64();
       while (!mbar_try_wait(drain, 0) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {

@@ -38,28 +38,6 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
   lo = split_pack(x, y);
 }
 
-// tcgen05.mma by one lane of a converged warp.  All lanes compute the operands, so that these stay in
-// uniform registers: issued from a branch of one lane, each product first moves its six
-// operands there, at some 55 cycles a product.
-__device__ __forceinline__ void umma_bf16_warp(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc,
-                                               uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
-          smem_u32(bar))
-      : "memory");
-}
-
 // Infinities, NaN and the floats above the largest bfloat16 have no such terms (inf - inf).
 __device__ __forceinline__ bool have_terms(const float4& v) {
   const uint32_t top = max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
