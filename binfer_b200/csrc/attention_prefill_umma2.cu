@@ -451,32 +451,46 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         const int t_lo = tile_key(n) + 2 * q4;             // key of this thread's first column
         const int kp = KEEP ? keep - t_lo : 0;             // KEEP: columns below it stay visible
-        int hi[2], lo[2];          // last and first visible key, counted from t_lo
-        bool need_mask[2];
-        float tmax[2];
+        // A row that does not see the whole tile: what it does not see counts as minus infinity.  (Both
+        // rows then go through one straight piece of code, and their chains fill each other's waits.)
+        bool need_mask = false;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          hi[e] = validr[e] ? prr[e] - t_lo : -1;
-          lo[e] = jlr[e] - t_lo;
-          need_mask[e] = !validr[e] || t_lo + 63 > prr[e] || t_lo - 6 < jlr[e];
-          float t2[2] = {-INFINITY, -INFINITY};
-          if (need_mask[e]) {
+        for (int e = 0; e < 2; ++e)
+          need_mask |= !validr[e] || t_lo + 63 > prr[e] || t_lo - 6 < jlr[e];
+        if (need_mask) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            // last and first visible key, counted from t_lo
+            const int hi = validr[e] ? prr[e] - t_lo : -1, lo = jlr[e] - t_lo;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
 #pragma unroll
               for (int i = 0; i < 2; ++i)
-                if ((8 * c + i >= lo[e] || (KEEP && 8 * c + i < kp)) && 8 * c + i <= hi[e])
-                  t2[i] = fmaxf(t2[i], __uint_as_float(v[4 * c + 2 * e + i]));
-          } else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-              t2[c & 1] = max3f(t2[c & 1], __uint_as_float(v[4 * c + 2 * e]),
-                                __uint_as_float(v[4 * c + 2 * e + 1]));
+                if ((8 * c + i < lo && !(KEEP && 8 * c + i < kp)) || 8 * c + i > hi)
+                  v[4 * c + 2 * e + i] = 0xff800000u;
           }
-          float t = fmaxf(t2[0], t2[1]);
-          t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, 1));
-          t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, 2));
-          tmax[e] = t * (DIFF ? row_scale[e] : scale_log2);   // the scale is positive
+        }
+        float tmax[2];
+        {
+          float t2[2][2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              t2[e][j] = fmaxf(__uint_as_float(v[4 * j + 2 * e]), __uint_as_float(v[4 * j + 2 * e + 1]));
+#pragma unroll
+          for (int c = 2; c < 8; ++c)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              t2[e][c & 1] = max3f(t2[e][c & 1], __uint_as_float(v[4 * c + 2 * e]),
+                                   __uint_as_float(v[4 * c + 2 * e + 1]));
+          float t0 = fmaxf(t2[0][0], t2[0][1]), t1 = fmaxf(t2[1][0], t2[1][1]);
+          const float u0 = __shfl_xor_sync(0xffffffffu, t0, 1), u1 = __shfl_xor_sync(0xffffffffu, t1, 1);
+          t0 = fmaxf(t0, u0);
+          t1 = fmaxf(t1, u1);
+          const float w0 = __shfl_xor_sync(0xffffffffu, t0, 2), w1 = __shfl_xor_sync(0xffffffffu, t1, 2);
+          tmax[0] = fmaxf(t0, w0) * (DIFF ? row_scale[0] : scale_log2);   // the scale is positive
+          tmax[1] = fmaxf(t1, w1) * (DIFF ? row_scale[1] : scale_log2);
         }
         float factor[2] = {1.f, 1.f};
         bool rescale = false;
@@ -513,27 +527,26 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
           }
         }
         uint32_t packed[16];       // packed[2c + e]: row e, keys 8c + 2 q4, + 1 = P column 4c + q4
+        float m_use[2], ts[2][2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          lsum[e] *= factor[e];
-          const float m_use = m_ref[e] == -INFINITY ? 0.f : m_ref[e];
-          float ts0 = 0.f, ts1 = 0.f;
+          m_use[e] = m_ref[e] == -INFINITY ? 0.f : m_ref[e];
+          ts[e][0] = ts[e][1] = 0.f;
+        }
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
             float x0, x1;
             fma2f(x0, x1, __uint_as_float(v[4 * c + 2 * e]), __uint_as_float(v[4 * c + 2 * e + 1]),
-                  DIFF ? row_scale[e] : scale_log2, -m_use);
-            float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
-            if (need_mask[e]) {
-              if ((8 * c < lo[e] && !(KEEP && 8 * c < kp)) || 8 * c > hi[e]) e0 = 0.f;
-              if ((8 * c + 1 < lo[e] && !(KEEP && 8 * c + 1 < kp)) || 8 * c + 1 > hi[e]) e1 = 0.f;
-            }
-            add2f(ts0, ts1, e0, e1);
-            __nv_bfloat162 p2 = __floats2bfloat162_rn(e0, e1);
-            packed[2 * c + e] = *reinterpret_cast<uint32_t*>(&p2);
+                  DIFF ? row_scale[e] : scale_log2, -m_use[e]);
+            const float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
+            add2f(ts[e][0], ts[e][1], e0, e1);
+            const __nv_bfloat162 p2 = __floats2bfloat162_rn(e0, e1);
+            packed[2 * c + e] = *reinterpret_cast<const uint32_t*>(&p2);
           }
-          lsum[e] += ts0 + ts1;
-        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) lsum[e] = lsum[e] * factor[e] + (ts[e][0] + ts[e][1]);
         // P over the first 32 columns of S, in this warp's 16 lanes: scores it has read
         tmem_st_frag32(my_s + (uint32_t)((n & 1) * A2_BN), packed);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
