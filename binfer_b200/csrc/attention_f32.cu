@@ -17,7 +17,9 @@
 //
 // What bounds it: the FP32 pipes and, for them, shared-memory reads (one 16-byte read per eight
 // multiply-adds).  The kernel for any size has one warp per (token, head), whose lanes share a key's
-// sizes and meet in five shuffles per key: 333 tokens of 16 heads of 128 took 557 us there, 58 here.
+// sizes and meet in five shuffles per key: 333 tokens of 16 heads of 128 took 557 us there, 38 here (one
+// token behind 499: 324 and 34).  With a page lookup for every 16-byte piece instead of every row these were
+// 60 and 72.
 #include <float.h>
 
 #include "common.cuh"
@@ -67,7 +69,8 @@ __global__ void __launch_bounds__(BM / TM * 16) attention_f32_kernel(
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int g = blockIdx.y, b = blockIdx.z, Gh = nh / nkv;
   const int t0 = q_start[b], n_tok = q_start[b + 1] - t0;
-  const int rows = n_tok * Gh, row0 = blockIdx.x * BM;
+  // (the last rows see the most keys and start first)
+  const int rows = n_tok * Gh, row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * BM;
   if (row0 >= rows) return;
   const int* table = tables + (size_t)b * table_stride;
   const int p_lo = positions[t0 + row0 / Gh];
@@ -75,22 +78,28 @@ __global__ void __launch_bounds__(BM / TM * 16) attention_f32_kernel(
   const int j_lo = window > 0 ? max(0, p_lo - window + 1) : 0;
   const int tile_a = j_lo / AF_KEYS, tile_b = p_hi / AF_KEYS + 1;
 
+  // A warp takes OWN rows of the tile: its lanes look one row each up in the table (a lookup and a division
+  // per 16-byte piece took longer than the tile's products), then whole rows are copied.
+  constexpr int OWN = AF_KEYS / (THREADS / 32), AT_ONCE = 32 / CHUNKS;
+  static_assert(THREADS % 32 == 0 && OWN >= AT_ONCE && OWN <= 32, "rows of a warp");
+  const int lane = tid & 31, own0 = tid / 32 * OWN;
   auto load = [&](int tile, int buf) {
-    for (int i = tid; i < AF_KEYS * CHUNKS; i += THREADS) {
-      const int r = i / CHUNKS, c = i - r * CHUNKS, e = tile * AF_KEYS + r;
-      bool ok = e >= j_lo && e <= p_hi;
-      size_t at = 0;
-      if (ok) {
-        const int lp = e / page_size, page = table[lp];
-        if (page < 0 || page >= num_pages) {
-          if (c == 0) atomicOr(err, BF_ERR_PAGE);
-          ok = false;
-        } else {
-          at = (((size_t)page * nkv + g) * page_size + (e - lp * page_size)) * D + c * 4;
-        }
-      }
-      af_cp16(Ks + (buf * AF_KEYS + r) * P + c * 4, k_cache + at, ok);
-      af_cp16(Vs + (buf * AF_KEYS + r) * P + c * 4, v_cache + at, ok);
+    const int e = tile * AF_KEYS + own0 + lane;
+    long long at = -1;
+    if (lane < OWN && e >= j_lo && e <= p_hi) {
+      const int lp = e / page_size, page = table[lp];
+      if (page < 0 || page >= num_pages) atomicOr(err, BF_ERR_PAGE);
+      else at = (((long long)page * nkv + g) * page_size + (e - lp * page_size)) * D;
+    }
+    const int c = lane % CHUNKS * 4;
+#pragma unroll
+    for (int i = 0; i < OWN; i += AT_ONCE) {
+      const int r = i + lane / CHUNKS;
+      const long long from = __shfl_sync(0xffffffffu, at, r);
+      const bool ok = from >= 0;
+      const size_t off = ok ? (size_t)(from + c) : 0;
+      af_cp16(Ks + (buf * AF_KEYS + own0 + r) * P + c, k_cache + off, ok);
+      af_cp16(Vs + (buf * AF_KEYS + own0 + r) * P + c, v_cache + off, ok);
     }
     cp_async_commit();
   };
@@ -289,8 +298,8 @@ static int af_launch(const float* q, const float* k, const float* v, const int* 
 // q and out [T, nh, d] contiguous; request b's token rows q_start[b] .. q_start[b + 1] - 1, at most
 // max_q of them, its pages in tables[b]; window 0: every earlier key; max_ctx: the longest context, or
 // 0 (contexts of one tile need one buffer for K and V, and three CTAs of four rows fit an SM instead of
-// one: 48 single tokens of 8 kv heads of 128 behind 0 and 15 keys 17 and 20 us -> 8.4 and 9.8; the kernel
-// for any size 7.9 and 18.5).
+// one: 48 single tokens of 8 kv heads of 128 behind 0 and 15 keys 17 and 20 us -> 8.4 and 9.8, then with the
+// rows' lookups 7.6 and 7.7; the kernel for any size 7.9 and 18.5).
 BF_EXPORT int bf_attention_f32(const float* q, const float* k_cache, const float* v_cache,
                                const int* q_start, const int* positions, const int* tables,
                                int table_stride, float* out, int B, int max_q, int nh, int nkv,
@@ -303,10 +312,18 @@ BF_EXPORT int bf_attention_f32(const float* q, const float* k_cache, const float
   // few rows from every request of the step (single tokens alone): tiles of four, each with as many
   // threads a row, so that the chain from key tile to key tile is short
   const int bufs = max_ctx > 0 && max_ctx <= AF_KEYS ? 1 : 2;
-  const bool few = (long long)max_q * (nh / nkv) <= 16;
+  const long long rows = (long long)max_q * (nh / nkv);
+  const bool few = rows <= 16;
+  // tiles of 64 rows, or of 32 where those would leave SMs idle: a key tile of half the rows takes half
+  // the time, and the CTA of the last rows, which walks them all, is what a short portion waits for (333
+  // tokens of 16 heads, 8 kv heads of 128: 60 -> 38 us with the rows' lookups; threads of two rows
+  // instead of four 45)
+  const bool small = (rows + 63) / 64 * nkv * B < 148;
 #define AF_GO(D)                                                                                \
   (few ? af_launch<D, 4, 1>(q, k_cache, v_cache, q_start, positions, tables, table_stride, out, \
                             B, max_q, nh, nkv, page_size, num_pages, window, scale, bufs, err, stream) \
+   : small ? af_launch<D, 32, 4>(q, k_cache, v_cache, q_start, positions, tables, table_stride, out, B, max_q, \
+                                 nh, nkv, page_size, num_pages, window, scale, bufs, err, stream) \
        : af_launch<D, 64, 4>(q, k_cache, v_cache, q_start, positions, tables, table_stride, out, \
                              B, max_q, nh, nkv, page_size, num_pages, window, scale, bufs, err, stream))
   return d == 64 ? AF_GO(64) : AF_GO(128);

@@ -1805,6 +1805,30 @@ def test_attention_f32_tiles(cuda_device, nh, nkv, d, ps, window):
     err.zero_()
 
 
+# heads of 64 (two rows of a tile at a time) and of 128
+@pytest.mark.parametrize("nh,nkv,d,window", [(8, 4, 128, None), (16, 8, 64, 70)])
+def test_attention_f32_tiles_of_32_and_64_rows(cuda_device, nh, nkv, d, window):
+    """Enough requests for an SM each take tiles of 64 rows, one request tiles of 32: the same bits."""
+    from binfer_b200.csrc import ops
+    ctxs = [33 + 17 * i for i in range(20)]
+    qlens = [min(c, 40) for c in ctxs]
+    q, kc, vc, sot, pos, bt, ref = _attention_case(cuda_device, F32, nh, nkv, d, 16, ctxs, qlens,
+                                                   window, False, seed=22)
+    ends = [0] + list(torch.tensor(qlens).cumsum(0))
+    qs = torch.tensor(ends, dtype=torch.int32, device=cuda_device)
+    out, err = torch.full_like(q, 7.0), _err(cuda_device)
+    ops.attention_f32(q, kc, vc, qs, pos, bt, out, 20, 40, nh, nkv, d, window, d ** -0.5, err)
+    assert int(err.item()) == 0
+    _close(out, ref, F32)
+    for b in (0, 7, 19):
+        a, e = int(ends[b]), int(ends[b + 1])
+        alone = torch.full((e - a, nh * d), 7.0, device=cuda_device)
+        ops.attention_f32(q[a:e].contiguous(), kc, vc, torch.tensor([0, e - a], dtype=torch.int32,
+                          device=cuda_device), pos[a:e].contiguous(), bt[b:b + 1].contiguous(), alone,
+                          1, e - a, nh, nkv, d, window, d ** -0.5, err)
+        assert torch.equal(alone, out[a:e])
+
+
 @pytest.mark.parametrize("window", [None, 70])
 def test_attention_f32_keys_that_a_row_does_not_see(cuda_device, window):
     """Values that are not finite reach the rows that see them alone; scores of -inf count as none.
