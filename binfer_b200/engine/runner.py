@@ -261,12 +261,10 @@ class ModelRunner:
     def reserve(self, items: Sequence[StepItem]) -> None:
         """Pages for every item, or :class:`OutOfPages` with nothing changed."""
         wants = [(it.rid, self.cache.get(it.rid).length + len(it.tokens)) for it in items]
-        if not self.cache.can_reserve(wants):
+        if not self.cache.reserve_all(wants):
             raise OutOfPages(
                 f"not enough free pages for this step (free per group: "
                 f"{self.cache.num_free_pages()})")
-        for rid, new_len in wants:
-            self.cache.reserve(rid, new_len)
 
     def step(self, items: Sequence[StepItem], device_ids: Optional[torch.Tensor] = None,
              bucket: Optional[int] = None) -> torch.Tensor:
@@ -285,16 +283,17 @@ class ModelRunner:
                 raise ValueError(f"request {it.rid!r} appears twice in one step")
             seen.add(it.rid)
         self.reserve(items)
-        for it in items:
-            self.cache.zero_fresh_state(self.cache.get(it.rid))
-        new_lens = [self.cache.get(it.rid).length + len(it.tokens) for it in items]
+        rcs = [self.cache.get(it.rid) for it in items]
+        for rc in rcs:
+            if rc.fresh:
+                self.cache.zero_fresh_state(rc)
+        new_lens = [rc.length + len(it.tokens) for rc, it in zip(rcs, items)]
         if self._can_replay(items, new_lens):
             logits = self._graph_step(items, device_ids, bucket)
         else:
             ctx = self.build_context(items, device_ids=device_ids)
             logits = self.model.forward(ctx, self.views)
-        for it, new_len in zip(items, new_lens):
-            self.cache.commit(it.rid, new_len)
+        self.cache.commit_all(rcs, new_lens)
         self.steps += 1
         return logits
 
