@@ -48,6 +48,37 @@ def test_groups_by_geometry_and_window():
     assert len(same.groups) == 1 and same.entry_location == [(0, 0), (0, 1), None]
 
 
+@pytest.mark.parametrize("window", [None, 8])
+def test_a_step_reserved_and_kept_at_once_is_its_requests_one_by_one(window):
+    """Pages, lengths and refusals of ``reserve_all`` / ``commit_all`` against ``can_reserve``,
+    ``reserve`` and ``commit``, until the pages run out."""
+    one, all_ = _mgr(pages=16, window=window), _mgr(pages=16, window=window)
+    rng, refused = random.Random(5), 0
+    rids = ["a", "b", "c"]
+    for m in (one, all_):
+        for r in rids:
+            m.add_request(r)
+    for _ in range(40):
+        wants = [(r, one.get(r).length + rng.choice([0, 1, 1, 3, 9])) for r in rng.sample(rids, 2)]
+        fits = one.can_reserve(wants)
+        assert all_.reserve_all(wants) == fits
+        if fits:
+            for r, n in wants:
+                one.reserve(r, n)
+                one.commit(r, n)
+            all_.commit_all([all_.get(r) for r, _ in wants], [n for _, n in wants])
+        refused += not fits
+        for r in rids:
+            assert one.get(r).tables == all_.get(r).tables
+            assert one.get(r).length == all_.get(r).length
+        assert one.num_free_pages() == all_.num_free_pages()
+    assert refused or window
+    grown = one.get("a").length
+    for m in (one, all_):
+        with pytest.raises(ValueError, match="cannot shrink"):
+            m.reserve_all([("a", grown - 1)])
+
+
 def test_reserve_is_all_or_nothing():
     m = _mgr(pages=4, page_size=4)
     m.add_request("a")
