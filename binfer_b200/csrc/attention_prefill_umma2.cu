@@ -13,7 +13,7 @@
 //               per (page, 64 columns) of K and of V, or one per 64 columns where the tile's
 //               pages follow one another in the pool; four key tiles in flight; the block
 //               table is read for 32 / (pages per tile) tiles at a time;
-//   warps 17,18 one thread each issues the tcgen05.mma of one query tile: per key tile
+//   warps 17,18 each issue the tcgen05.mma of one query tile (one elected lane): per key tile
 //               S = Q K^T (into one of two S buffers of its own in tensor memory, so the
 //               product of tile n+1 runs under the softmax of tile n), then O += P V with P
 //               as the operand FROM TENSOR MEMORY, once the probabilities lie there.  All 512
@@ -332,10 +332,10 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp >= A2_MMA_WARP) {
     // ----------------------------------------------------------------- MMA issuers
-    // One thread per query tile: issuing a tcgen05.mma costs the issuing thread about a
-    // hundred cycles whatever its size, and with one thread for both tiles that, not the
-    // tensor pipe (a quarter busy), set the pace.  The two threads' products touch disjoint
-    // tensor memory; they share the K and V tiles, which are released when both have arrived.
+    // One warp per query tile, converged, one elected lane issuing: out of a branch of one lane a
+    // tcgen05.mma cost 55 to 100 cycles whatever its size (operands moved into uniform registers
+    // one lane at a time).  The two warps' products touch disjoint tensor memory; they share the
+    // K and V tiles, which are released when both have arrived.
     const int grp = warp - A2_MMA_WARP;
     const int my_tiles = grp == 0 ? tiles_a : (active_b ? tiles : 0);
     {

@@ -16,7 +16,7 @@
 //   warps 0-7    take 32 terms of K of the features apart and store the terms as swizzled tiles
 //                into a ring of stages;
 //   warps 8-23   take each finished sum out of tensor memory and add;
-//   warp 24      one thread issues the products; the warp owns the tensor memory;
+//   warp 24      issues the products (one elected lane); the warp owns the tensor memory;
 //   warp 25      one thread copies the token rows' terms, which a kernel of its own has laid out
 //                as the tiles lie in shared memory (up to 16 rows: warps 0-7 do those too);
 //   warp 26      one thread fetches the features' floats (TMA) into a ring of its own.  (Rows off
@@ -28,7 +28,7 @@
 // Rows with an infinity or a NaN have no terms; their outputs are computed one by one with
 // multiply-adds in the epilogue.
 //
-// What bounds it: the thread that issues the products and the shared-memory reads of their
+// What bounds it: the warp that issues the products and the shared-memory reads of their
 // operands (a step of 32 terms in 0.74 us for 112 token rows, 0.85 for 176; the products alone 0.36
 // and 0.56), and waves of tiles that do not fill the chip.  In us against plain multiply-adds:
 //   rows x outputs x terms       1      333             2,048
