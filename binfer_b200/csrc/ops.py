@@ -1975,8 +1975,10 @@ def _sgemm_split(a, w, out, M, N, K, batch, lda, ldw, ldc, batch_a, batch_w, bat
         _launches += n > 0           # two kernels: the rows' terms and the product
 
 
-def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true 32-bit arithmetic."""
+def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
+             multiply_adds: bool = False) -> None:
+    """out[M, N] = a[M, K] @ w[N, K]^T in 32-bit precision.  ``multiply_adds``: FP32 multiply-adds
+    (``sgemm_f32.cu``) whatever K, not the tensor cores from ``SGEMM_SPLIT_MIN_K`` terms on."""
     for t, n in ((a, "a"), (w, "w"), (out, "out")):
         if t.dtype != torch.float32 or t.stride(-1) != 1:
             raise KernelError(f"sgemm_nt: {n} must be float32 with contiguous rows")
@@ -1985,15 +1987,16 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     if w.shape[1] != K or out.shape != (M, N):
         raise KernelError(f"sgemm_nt: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> "
                           f"{tuple(out.shape)} do not agree")
-    if K >= SGEMM_SPLIT_MIN_K:
+    if K >= SGEMM_SPLIT_MIN_K and not multiply_adds:
         return _sgemm_split(a, w, out, M, N, K, 1, a.stride(0), w.stride(0), out.stride(0), 0, 0, 0)
     _run("sgemm_nt", lib().bf_sgemm_nt, _ptr(a), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K),
                              _c_ll(a.stride(0)), _c_ll(w.stride(0)), _c_ll(out.stride(0)),
                              _stream())
 
 
-def sgemm_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[:, b] = a[:, b] @ w[b]^T for every b, in true 32-bit arithmetic: ``a [M, B, K]`` and
+def sgemm_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
+                     multiply_adds: bool = False) -> None:
+    """out[:, b] = a[:, b] @ w[b]^T for every b, as :func:`sgemm_nt`: ``a [M, B, K]`` and
     ``out [M, B, N]`` may be strided views (innermost stride 1), ``w [B, N, K]``."""
     for t, n in ((a, "a"), (w, "w"), (out, "out")):
         if t.dtype != torch.float32 or t.stride(-1) != 1 or t.dim() != 3:
@@ -2002,7 +2005,7 @@ def sgemm_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> Non
     N = w.shape[1]
     if w.shape != (Bn, N, K) or out.shape != (M, Bn, N):
         raise KernelError("sgemm_nt_batched: shapes do not agree")
-    if K >= SGEMM_SPLIT_MIN_K and 0 < Bn <= 65535:
+    if K >= SGEMM_SPLIT_MIN_K and 0 < Bn <= 65535 and not multiply_adds:
         return _sgemm_split(a, w, out, M, N, K, Bn, a.stride(0), w.stride(1), out.stride(0),
                             a.stride(1), w.stride(0), out.stride(1))
     _run("sgemm_nt_batched", lib().bf_sgemm_nt_batched, _ptr(a), _ptr(w), _ptr(out), _c_int(M),

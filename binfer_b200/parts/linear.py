@@ -1,6 +1,10 @@
 """The dense matrix product ``y = x W^T`` with weights as stored (``[out, in]`` row-major).
 
-float32 engine: the engine's own kernels of 32-bit precision (no reduced-precision matrix mode).
+float32 engine: the engine's own kernels of 32-bit precision (no reduced-precision matrix mode):
+from 512 terms on ``csrc/sgemm_split.cu``, which runs on the tensor cores, below that FP32
+multiply-adds (``csrc/sgemm_f32.cu``).  A float32 engine that checks the tensor-core paths should
+share nothing with them: inside ``float32_multiply_adds()`` (for the calling thread), or with
+``BINFER_B200_F32_MULTIPLY_ADDS=1``, every product is multiply-adds.
 bfloat16 engine: the engine's tcgen05/TMEM/TMA kernel (``csrc/gemm_tcgen05.cu``) or
 cuBLAS through ``torch.mm`` with float accumulation, the library call the reference
 makes for every dense product (cuda/kernels/gemm.cu:244-267: ``cublasGemmEx``, bf16
@@ -16,6 +20,8 @@ it and has its first weight tiles under way when that kernel ends.
 """
 from __future__ import annotations
 
+import contextlib
+import contextvars
 from typing import Optional
 
 import os
@@ -25,6 +31,19 @@ import torch
 from ..csrc import ops
 
 _POLICY = os.environ.get("BINFER_B200_GEMM", "auto")
+_MULTIPLY_ADDS = contextvars.ContextVar(
+    "float32_multiply_adds", default=os.environ.get("BINFER_B200_F32_MULTIPLY_ADDS", "0") != "0")
+
+
+@contextlib.contextmanager
+def float32_multiply_adds(on: bool = True):
+    """Every float32 product that this thread launches inside runs as FP32 multiply-adds.  (A
+    captured decode step replays the products that it was captured with.)"""
+    token = _MULTIPLY_ADDS.set(on)
+    try:
+        yield
+    finally:
+        _MULTIPLY_ADDS.reset(token)
 
 
 def set_gemm_policy(policy: str) -> None:
@@ -128,7 +147,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     if x.dtype == torch.float32:
         if out is None:
             out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-        ops.sgemm_nt(x, w, out)
+        ops.sgemm_nt(x, w, out, _MULTIPLY_ADDS.get())
         return out
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise TypeError(f"linear: unsupported dtypes {x.dtype} x {w.dtype}")
@@ -216,7 +235,7 @@ def linear_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.T
     float32: the engine's own kernels, one launch for all heads; bfloat16: the
     library's strided batched product with float accumulation."""
     if x.dtype == torch.float32:
-        ops.sgemm_nt_batched(x, w, out)
+        ops.sgemm_nt_batched(x, w, out, _MULTIPLY_ADDS.get())
         return out
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise TypeError(f"linear_heads: unsupported dtypes {x.dtype} x {w.dtype}")

@@ -186,6 +186,35 @@ def test_replay_at_qwen3_8b_layer_sizes(shape, dtype, regime, page_size):
         assert not missing, f"{regime}: kernels that did not run: {sorted(missing)}"
 
 
+def test_float32_by_multiply_adds_at_qwen3_8b_layer_sizes(shape):
+    """The float32 engine with its products on FP32 multiply-adds alone, which share nothing with
+    the tensor cores, against the plain implementation and against its products of terms: both
+    within the bounds, the products of terms no further off."""
+    from binfer_b200.csrc import ops
+    from binfer_b200.parts.linear import float32_multiply_adds
+    reqs = _requests()
+    ref = shape.plain(reqs)
+    steps = _trace("portions", reqs)
+    got, names = [], []
+    for on in (False, True):
+        runner = shape.runner(torch.float32, 64, H.peak_pages(steps, 64))
+        seen = _Names()
+        ops.set_profiler(seen)
+        try:
+            with float32_multiply_adds(on):
+                got.append(H.run_trace(runner, steps))
+        finally:
+            ops.set_profiler(None)
+        names.append(seen.names)
+        _compare(got[-1], ref, torch.float32, f"8B sizes/multiply-adds {on}", None)
+    assert "sgemm_split" in names[0] and "sgemm_nt" not in names[0]
+    assert "sgemm_nt" in names[1] and "sgemm_split" not in names[1]
+    keys = [(rid, p) for rid, rows in ref.items() for p in rows]
+    want = torch.stack([ref[rid][p] for rid, p in keys])
+    terms, adds = (H.rel_rms(torch.stack([g[k].cpu() for k in keys]), want) for g in got)
+    assert terms <= 1.1 * adds, (terms, adds)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
 def test_six_requests_decode_together_from_the_bucket_of_eight(shape, dtype):
     """Six requests, prefilled one after the other, then sixteen steps in which all of them
