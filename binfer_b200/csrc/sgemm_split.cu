@@ -25,8 +25,10 @@
 // K alone) then share a tile along K and their sums are added in ascending order through
 // distributed shared memory.
 //
-// Rows with an infinity or a NaN have no terms; their outputs are computed one by one with
-// multiply-adds in the epilogue.
+// Infinities, NaN and floats above the largest bfloat16 have no terms: one of theirs is a NaN, and so is
+// every sum that they reach.  A product beyond float's range shows as an infinity or, where a
+// smaller product of terms overflows with a sign of its own, as a NaN.  So every output whose sum is
+// not finite is computed with multiply-adds in the epilogue, one by one.
 //
 // What bounds it: the warp that issues the products and the shared-memory reads of their
 // operands (a step of 32 terms in 0.74 us for 112 token rows, 0.85 for 176; the products alone 0.36
@@ -57,13 +59,12 @@ constexpr int SP_MAX_FLOATS = 6;                               // such stages
 constexpr int SP_MAX_STAGES = 8;
 constexpr int SP_RUN = 8;                // sums of a run
 constexpr int SP_FEW = 16;               // token rows up to which the product takes them apart itself
-constexpr int SP_HEAD = 1024;            // barriers and flags, in front of the ring
+constexpr int SP_HEAD = 1024;            // barriers, in front of the ring
 
 struct SplitParams {
   const float *A, *W;
   float* C;
   const uint8_t* terms;                  // of A: [batch][step][term][rows][32], rows of 64 bytes
-  const uint8_t* odd;                    // [batch][rows]: the row has an element without terms
   long long rows;                        // token rows of a step, whole tiles
   int M, N, K, parts;                    // parts: CTAs that share a tile along K
   int stages, floats;                    // stages of terms; of the features' floats
@@ -103,11 +104,6 @@ __device__ __forceinline__ float4 sp_ld4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint32_t sp_ld_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
 }
 __device__ __forceinline__ void sp_take(uint32_t taddr, float (&t)[16]) {
@@ -163,7 +159,8 @@ __device__ __forceinline__ void sp_store_columns(uint32_t taddr, const float* t)
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// The plain sum, for rows that the terms do not stand for.  (Once NaN, always NaN.)
+// The plain sum, where that of the terms does not stand for it.  (Once NaN, always NaN.)
+__device__ __forceinline__ bool sp_finite(float v) { return fabsf(v) < INFINITY; }
 __device__ __noinline__ float sp_plain(const float* a, const float* w, int K) {
   float s = 0.f;
   for (int k = 0; k < K && s == s; ++k) s = fmaf(a[k], w[k], s);
@@ -174,45 +171,36 @@ __device__ __noinline__ float sp_plain(const float* a, const float* w, int K) {
 template <bool VEC>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, int M, int K,
                                                          long long lda, long long batch_a,
-                                                         uint8_t* __restrict__ terms,
-                                                         uint8_t* __restrict__ odd, long long rows) {
+                                                         uint8_t* __restrict__ terms, long long rows) {
   bf_pdl_trigger();
   const int row = blockIdx.x * 2 + (threadIdx.x >> 7), at = threadIdx.x & 127;
   const int steps = (K + SP_K - 1) / SP_K;
   const float* src = A + blockIdx.z * batch_a + (size_t)min(row, M - 1) * lda;
   uint8_t* dst = terms + (size_t)blockIdx.z * steps * 3 * rows * 64 + (size_t)row * 64 +
                  ((((at & 7) >> 1) ^ ((row >> 1) & 3)) << 4) + ((at & 1) << 3);
-  float2 left = make_float2(0.f, 0.f);
-  if (row < M) {
+  if (row >= M) return;
 #pragma unroll 4
-    for (int k = 4 * at; k < steps * SP_K; k += 512) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (VEC) {
-        if (k < K) v = *reinterpret_cast<const float4*>(src + k);
-      } else {
-        if (k < K) v.x = src[k];
-        if (k + 1 < K) v.y = src[k + 1];
-        if (k + 2 < K) v.z = src[k + 2];
-        if (k + 3 < K) v.w = src[k + 3];
-      }
-      uint2 hi, mid, lo;
-      split3(v.x, v.y, hi.x, mid.x, lo.x, left);
-      split3(v.z, v.w, hi.y, mid.y, lo.y, left);
-      uint8_t* to = dst + (size_t)(k / SP_K) * 3 * rows * 64;
-      *reinterpret_cast<uint2*>(to) = hi;
-      *reinterpret_cast<uint2*>(to + rows * 64) = mid;
-      *reinterpret_cast<uint2*>(to + 2 * rows * 64) = lo;
+  for (int k = 4 * at; k < steps * SP_K; k += 512) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC) {
+      if (k < K) v = *reinterpret_cast<const float4*>(src + k);
+    } else {
+      if (k < K) v.x = src[k];
+      if (k + 1 < K) v.y = src[k + 1];
+      if (k + 2 < K) v.z = src[k + 2];
+      if (k + 3 < K) v.w = src[k + 3];
     }
+    uint2 hi, mid, lo;
+    split3(v.x, v.y, hi.x, mid.x, lo.x);
+    split3(v.z, v.w, hi.y, mid.y, lo.y);
+    uint8_t* to = dst + (size_t)(k / SP_K) * 3 * rows * 64;
+    *reinterpret_cast<uint2*>(to) = hi;
+    *reinterpret_cast<uint2*>(to + rows * 64) = mid;
+    *reinterpret_cast<uint2*>(to + 2 * rows * 64) = lo;
   }
-  __shared__ int bad[2];
-  if (threadIdx.x < 2) bad[threadIdx.x] = 0;
-  __syncthreads();
-  if (!(fabsf(left.x + left.y) < INFINITY)) bad[threadIdx.x >> 7] = 1;
-  __syncthreads();
-  if (at == 0 && row < M) odd[blockIdx.z * rows + row] = (uint8_t)bad[threadIdx.x >> 7];
 }
 
-// PRE: A's terms and flags come laid out.
+// PRE: A's terms come laid out.
 template <int NT, bool VEC, bool PRE>
 __global__ void __launch_bounds__(SP_THREADS, 1)
 sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams p) {
@@ -236,8 +224,6 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
   uint64_t* drain = w_empty + SP_MAX_FLOATS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint32_t* odd = tmem_slot + 2;                            // some row is not finite
-  uint8_t* odd_row = reinterpret_cast<uint8_t*>(tmem_slot + 4);   // [128 features][NT tokens]
   uint8_t* tiles = base + SP_HEAD;
   uint8_t* floats = tiles + (size_t)p.stages * STAGE;
 
@@ -265,10 +251,8 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
     }
     mbar_init(drain, 1);
     *abort = 0;
-    *odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int i = tid; i < SP_F + NT; i += SP_THREADS) odd_row[i] = 0;
   if (warp == SP_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
@@ -301,10 +285,10 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
       return v;
     };
     const int spot = row * 64 + (((piece >> 1) ^ ((row >> 1) & 3)) << 4) + ((piece & 1) << 3);
-    auto put = [&](uint8_t* at, int bytes, const float4& v, float2& left) {
+    auto put = [&](uint8_t* at, int bytes, const float4& v) {
       uint2 hi, mid, lo;
-      split3(v.x, v.y, hi.x, mid.x, lo.x, left);
-      split3(v.z, v.w, hi.y, mid.y, lo.y, left);
+      split3(v.x, v.y, hi.x, mid.x, lo.x);
+      split3(v.z, v.w, hi.y, mid.y, lo.y);
       *reinterpret_cast<uint2*>(at) = hi;
       *reinterpret_cast<uint2*>(at + bytes) = mid;
       *reinterpret_cast<uint2*>(at + 2 * bytes) = lo;
@@ -331,24 +315,12 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
       const bool ok = mbar_wait(empty + stage, phase ^ 1, abort);
       if (!__all_sync(0xffffffffu, ok)) break;
       uint8_t* at = tiles + (size_t)stage * STAGE + spot;
-      // (one test a step, so that the pieces' instructions can mix)
-      float2 left = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) put(at + j * 2048, W_BYTES, wf[j], left);
+      for (int j = 0; j < 4; ++j) put(at + j * 2048, W_BYTES, wf[j]);
 #pragma unroll
       for (int j = 0; j < PA; ++j)
         if (NT % 32 == 0 || j + 1 < PA || row < NT % 32)
-          put(at + 3 * W_BYTES + j * 2048, A_BYTES, af[j], left);
-      if (!(fabsf(left.x + left.y) < INFINITY)) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (!have_terms(wf[j])) odd_row[row + 32 * j] = 1;
-#pragma unroll
-        for (int j = 0; j < PA; ++j)
-          if ((NT % 32 == 0 || j + 1 < PA || row < NT % 32) && !have_terms(af[j]))
-            odd_row[SP_F + row + 32 * j] = 1;
-        *odd = 1;
-      }
+          put(at + 3 * W_BYTES + j * 2048, A_BYTES, af[j]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
@@ -425,12 +397,6 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
         }
       }
     }
-    __syncwarp();
-    for (int t = lane; t < NT && m0 + t < p.M; t += 32)
-      if (p.odd[blockIdx.z * p.rows + m0 + t]) {
-        odd_row[SP_F + t] = 1;
-        *odd = 1;
-      }
   } else if (VEC && warp == SP_TMA) {
     // ------------------------------------------------------------------ features' floats
     if (lane == 0) {
@@ -510,13 +476,12 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
   if (parts == 1) {
     const int f = f0 + quarter * 32 + lane;
     if (sums && f < p.N) {
-      const bool f_odd = *odd && odd_row[f - f0];
 #pragma unroll
       for (int i = 0; i < MINE; ++i) {
         const int t = group * MINE + i;
         if (m0 + t < p.M) {
           float v = total[i];
-          if (f_odd || (*odd && odd_row[SP_F + t]))
+          if (!sp_finite(v))
             v = sp_plain(A + (size_t)(m0 + t) * p.lda, W + (size_t)f * p.ldw, p.K);
           C[(size_t)(m0 + t) * p.ldc + f] = v;
         }
@@ -530,9 +495,7 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
       for (int i = 0; i < MINE; ++i) mine[(group * MINE + i) * SP_F + quarter * 32 + lane] = total[i];
     }
     sp_cluster_sync();
-    const uint32_t mine_at = smem_u32(mine), odd_at = smem_u32(odd);
-    bool any_odd = false;
-    for (int r = 0; r < parts; ++r) any_odd |= sp_ld_u32(sp_map(odd_at, r)) != 0;
+    const uint32_t mine_at = smem_u32(mine);
     const int f = f0 + 4 * lane;
     const bool vec = f + 4 <= p.N && (p.ldc & 3) == 0 && ((uintptr_t)C & 15) == 0;
     if (warp < SP_FETCH + SP_SUM) {
@@ -546,20 +509,12 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
           v.z += u.z;
           v.w += u.w;
         }
-        if (any_odd) {
+        if (!(sp_finite(v.x) && sp_finite(v.y) && sp_finite(v.z) && sp_finite(v.w))) {
           float* e[4] = {&v.x, &v.y, &v.z, &v.w};
-          const uint32_t flags = smem_u32(odd_row);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t bad = 0;
-            for (int r = 0; r < parts; ++r) {
-              const uint32_t word = sp_ld_u32(sp_map(flags + 4 * lane, r));
-              const uint32_t tok = sp_ld_u32(sp_map(flags + SP_F + (t & ~3), r));
-              bad |= (word >> (8 * j)) & 255u | (tok >> (8 * (t & 3))) & 255u;
-            }
-            if (bad && f + j < p.N)
+          for (int j = 0; j < 4; ++j)
+            if (!sp_finite(*e[j]) && f + j < p.N)
               *e[j] = sp_plain(A + (size_t)(m0 + t) * p.lda, W + (size_t)(f + j) * p.ldw, p.K);
-          }
         }
         float* dst = C + (size_t)(m0 + t) * p.ldc + f;
         if (vec) {
@@ -607,11 +562,9 @@ int sp_launch(const CUtensorMap& map, SplitParams p, int batch, uint8_t* scratch
   const int tiles = (p.M + NT - 1) / NT;
   if (PRE) {
     p.rows = (long long)tiles * NT;
-    const int steps = (p.K + SP_K - 1) / SP_K;
     p.terms = scratch;
-    p.odd = scratch + (size_t)batch * steps * 3 * p.rows * 64;
     split_rows_kernel<VEC><<<dim3((p.M + 1) / 2, 1, batch), 256, 0, stream>>>(
-        p.A, p.M, p.K, p.lda, p.batch_a, scratch, const_cast<uint8_t*>(p.odd), p.rows);
+        p.A, p.M, p.K, p.lda, p.batch_a, scratch, p.rows);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((p.N + SP_F - 1) / SP_F * p.parts), tiles, batch);
@@ -646,7 +599,7 @@ BF_EXPORT long long bf_sgemm_split_scratch(int M, int N, int K, int batch, int n
   if (M <= SP_FEW) return 0;
   if (!nt) nt = sp_tile(M, N, batch);
   const long long rows = (long long)((M + nt - 1) / nt) * nt, steps = (K + SP_K - 1) / SP_K;
-  return batch * (steps * 3 * rows * 64 + rows);
+  return batch * steps * 3 * rows * 64;
 }
 
 // C[M, N] = A[M, K] * W[N, K]^T, `batch` of them (bf_sgemm_nt_batched's strides).  nt: token rows of
@@ -660,7 +613,7 @@ BF_EXPORT int bf_sgemm_split(const float* A, const float* W, float* C, int M, in
   if (K <= 0 || batch > 65535 || (M + nt - 1) / nt > 65535 || ((uintptr_t)scratch & 15) ||
       (nt > SP_FEW && !scratch))
     return (int)cudaErrorInvalidValue;
-  SplitParams p = {A, W, C, nullptr, nullptr, 0, M, N, K, K < 512 ? 1 : sp_parts(N), 0, 0, lda, ldw, ldc,
+  SplitParams p = {A, W, C, nullptr, 0, M, N, K, K < 512 ? 1 : sp_parts(N), 0, 0, lda, ldw, ldc,
                    batch_a, batch_w, batch_c, err};
   CUtensorMap map = {};
   bool vec = ((K | lda | ldw | batch_a | batch_w) & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 &&

@@ -25,8 +25,16 @@ __device__ __forceinline__ void sub2f(float& x, float& y, float a, float b, uint
       : "=f"(x), "=f"(y)
       : "f"(a), "f"(b), "f"(__uint_as_float(terms << 16)), "f"(__uint_as_float(terms & 0xffff0000u)));
 }
+__device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  float x, y;
+  hi = split_pack(a, b);
+  sub2f(x, y, a, b, hi);
+  mid = split_pack(x, y);
+  sub2f(x, y, x, y, mid);
+  lo = split_pack(x, y);
+}
 // left: gets what is left behind the first terms added up, which is finite exactly where both
-// floats have terms.
+// floats have terms.  (Infinities, NaN and the floats above the largest bfloat16 have none: inf - inf.)
 __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo,
                                        float2& left) {
   float x, y;
@@ -36,13 +44,6 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
   mid = split_pack(x, y);
   sub2f(x, y, x, y, mid);
   lo = split_pack(x, y);
-}
-
-// Infinities, NaN and the floats above the largest bfloat16 have no such terms (inf - inf).
-__device__ __forceinline__ bool have_terms(const float4& v) {
-  const uint32_t top = max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
-                           max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
-  return top < 0x7f7f8000u;
 }
 
 // K-major operand tile in rows of 64 bytes (32 bfloat16) with the 64-byte swizzle: 8-row groups

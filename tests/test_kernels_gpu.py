@@ -135,6 +135,13 @@ def test_sgemm_more_rows_than_a_grid_has_tiles(cuda_device):
     assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
 
 
+def _multiply_adds(a, w):
+    from binfer_b200.csrc import ops
+    out = torch.empty(a.shape[0], w.shape[0], device=a.device)
+    ops.sgemm_nt(a, w, out, multiply_adds=True)
+    return out
+
+
 # 512 terms and more: three bfloat16 terms an operand.  Rows about the tiles (16, 112, 176), features
 # about 128 and about the numbers of tiles that share K among 4, 2 and 1 CTAs; K about steps of 32
 # and runs of 8 steps.
@@ -165,6 +172,30 @@ def test_sgemm_of_terms(cuda_device, M, N, K):
     ops.sgemm_nt_batched(torch.stack([w[:1].expand(M, K), a], 1), torch.stack([w, w]), heads)
     assert torch.equal(heads[:, 1], out)
     assert int(ops.error_word(cuda_device).item()) == 0
+
+
+# tiles of 16, 176 and 112 rows, features shared by clusters of 4 and 2 CTAs and not
+@pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512), (224, 4200, 512)])
+def test_sgemm_of_terms_with_products_that_overflow(cuda_device, M, N, K):
+    """Finite operands whose products or sums leave float's range give the infinities and NaN of the
+    multiply-adds; a smaller product of terms must not overflow with a sign of its own."""
+    from binfer_b200.csrc import ops
+    a, w = torch.randn(M, K, device=cuda_device), torch.randn(N, K, device=cuda_device)
+    a[3, 7], w[5, 7], w[N - 1, 7] = 1.7e25, 1.3e20, -1.1e20
+    a[2, 11], a[2, 12], w[8, 11], w[8, 12] = 1.7e25, -1.9e25, 1.1e20, 1.3e20
+    a[M - 1], w[9] = 1e23 * torch.rand(K, device=cuda_device), 1e23 * torch.rand(K, device=cuda_device)
+    a[1, 20], w[17, 20], a[1, 21], w[17, 21] = 1.5e19, 1.9e19, -1.4e19, 1.9e19     # (the sum is finite)
+    out, want = torch.empty(M, N, device=cuda_device), _multiply_adds(a, w)
+    ops.sgemm_nt(a, w, out)
+    assert want[3, 5] == float("inf") and want[3, N - 1] == -float("inf") and not want[2, 8].isfinite()
+    assert want[M - 1, 9] == float("inf") and want[1, 17].isfinite()
+    assert torch.equal(out.isnan(), want.isnan())
+    odd = ~want.isfinite() & ~want.isnan()
+    assert torch.equal(out[odd], want[odd]) and bool(out[want.isfinite()].isfinite().all())
+    size = a.double().abs() @ w.double().abs().T
+    ref = a.double() @ w.double().T
+    fin = want.isfinite()
+    assert bool(((out.double() - ref).abs() <= 100 * 2.0 ** -24 * size)[fin].all())
 
 
 @pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512)])
