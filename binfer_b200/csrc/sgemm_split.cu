@@ -159,12 +159,18 @@ __device__ __forceinline__ void sp_store_columns(uint32_t taddr, const float* t)
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// The plain sum, where that of the terms does not stand for it.  (Once NaN, always NaN.)
+// The plain sum, where that of the terms does not stand for it: in the order of sgemm_f32.cu, ascending
+// runs of 64 terms.  (Once NaN, always NaN.)
 __device__ __forceinline__ bool sp_finite(float v) { return fabsf(v) < INFINITY; }
 __device__ __noinline__ float sp_plain(const float* a, const float* w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K && s == s; ++k) s = fmaf(a[k], w[k], s);
-  return s;
+  float total = 0.f;
+  for (int k0 = 0; k0 < K && total == total; k0 += 64) {
+    float s = 0.f;
+#pragma unroll 8
+    for (int k = k0; k < min(K, k0 + 64); ++k) s = fmaf(a[k], w[k], s);
+    total += s;
+  }
+  return total;
 }
 
 // The terms of A, laid out for the product.  A block takes two rows, four warps to a row.

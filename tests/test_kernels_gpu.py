@@ -198,6 +198,18 @@ def test_sgemm_of_terms_with_products_that_overflow(cuda_device, M, N, K):
     assert bool(((out.double() - ref).abs() <= 100 * 2.0 ** -24 * size)[fin].all())
 
 
+@pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 6145)])
+def test_sgemm_of_terms_where_no_terms_are(cuda_device, M, N, K):
+    """Rows without terms get the multiply-adds' sums, in their order: the same bits."""
+    from binfer_b200.csrc import ops
+    a, w = torch.randn(M, K, device=cuda_device), torch.randn(N, K, device=cuda_device)
+    a[3, 9], w[:, 9], w[8, 5], a[:, 5] = 3.4e38, 0.0, -3.4e38, 0.0
+    out, want = torch.empty(M, N, device=cuda_device), _multiply_adds(a, w)
+    ops.sgemm_nt(a, w, out)
+    assert bool(want.isfinite().all())
+    assert torch.equal(out[3], want[3]) and torch.equal(out[:, 8], want[:, 8])
+
+
 @pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512)])
 def test_sgemm_of_terms_with_infinities(cuda_device, M, N, K):
     """Infinities, NaN and floats that no bfloat16 reaches give what multiply-adds give, and stay in
