@@ -2,14 +2,31 @@
 //
 // A float has 24 significant bits, a bfloat16 eight and the same range of exponents: the nearest
 // bfloat16, the nearest one to what is left and what is left then are three bfloat16 numbers whose
-// sum is the float.  A product of two floats is then nine products of terms, each exact in float; the
-// three smallest (below 2^-26 of the product together) are left out.
+// sum is the float, as long as its last bit is no smaller than bfloat16's smallest (2^-133).  Floats of less
+// than 2^-110 have smaller ones (of 1e-36 the terms keep some 14 bits); multiplied by 2^24 first, every
+// float up to 2^104 is the sum of its terms, and these are normal numbers.
+//
+// A product of two floats is then nine products of terms, each exact in float; the three smallest
+// (together up to 2^-24 of the product) are left out.  Taking floats apart into bfloat16 terms for
+// matrix hardware: Henry, Tang, Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For
+// Higher-Precision Computations", ARITH 2019.
 #pragma once
 #include "common.cuh"
 #include "umma_utils.cuh"
 
 namespace {
 
+constexpr float SPLIT_UP = 16777216.f, SPLIT_DOWN = 1.f / 16777216.f;      // 2^24
+
+__device__ __forceinline__ void split_up(float& a, float& b) {
+  asm("{\n\t.reg .b64 u, v;\n\t"
+      "mov.b64 u, {%0, %1};\n\t"
+      "mov.b64 v, {%2, %2};\n\t"
+      "mul.rn.f32x2 u, u, v;\n\t"
+      "mov.b64 {%0, %1}, u;\n\t}"
+      : "+f"(a), "+f"(b)
+      : "f"(SPLIT_UP));
+}
 // (a, b) -> the terms of a in the low halves, those of b in the high halves: hi, mid, lo.
 __device__ __forceinline__ uint32_t split_pack(float a, float b) {
   uint32_t r;

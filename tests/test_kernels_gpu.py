@@ -156,7 +156,7 @@ def test_sgemm_of_terms(cuda_device, M, N, K):
     ops.sgemm_nt(a, w, out)
     ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
     # twelve products of terms a step, each sum cut off behind 24 bits (2^-23), then rounded sums
-    # in runs of eight steps, of the runs, of four CTAs; terms left out below 2^-26
+    # in runs of eight steps, of the runs, of four CTAs; products of terms left out, up to 2^-24
     bound = (12 * 2 + 8 + K / 256 + 4 + 1) * 2.0 ** -24 * size
     assert bool(((out.double() - ref).abs() <= bound).all())
     assert float((out.double() - ref).norm() / ref.norm()) < 1.6e-7      # (measured 1.1e-7)
@@ -208,6 +208,31 @@ def test_sgemm_of_terms_where_no_terms_are(cuda_device, M, N, K):
     ops.sgemm_nt(a, w, out)
     assert bool(want.isfinite().all())
     assert torch.equal(out[3], want[3]) and torch.equal(out[:, 8], want[:, 8])
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512), (224, 4200, 800)])
+def test_sgemm_of_terms_holds_floats_of_every_size(cuda_device, M, N, K):
+    """Operands down to the smallest float keep all their bits, against large ones and among them;
+    sums as large as float holds are there."""
+    from binfer_b200.csrc import ops
+    dev = cuda_device
+    a, w = torch.randn(M, K, device=dev), torch.randn(N, K, device=dev)
+    a *= 10.0 ** torch.tensor([0, -36, -38, -40, 6], device=dev)[torch.arange(M, device=dev) % 5][:, None]
+    w *= 10.0 ** torch.tensor([30, 0, -36, 20], device=dev)[torch.arange(N, device=dev) % 4][:, None]
+    a[0, 1::2] *= 1e-37                                      # in one row
+    w[0, ::2] *= 1e-35
+    out, want = torch.empty(M, N, device=dev), _multiply_adds(a, w)
+    ops.sgemm_nt(a, w, out)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # (test_sgemm_of_terms' bound; each rounded result is off by half the smallest float at most)
+    bound = (12 * 2 + 8 + K / 256 + 4 + 1) * 2.0 ** -24 * size + 2.0 ** -150
+    assert bool(out.isfinite().all()) and bool(((out.double() - ref).abs() <= bound).all())
+    for i in range(5):
+        for j in range(4):
+            r = ref[i::5, j::4]
+            if float(r.abs().max()) > 1e-30:                 # (results that float itself holds)
+                off = [float((x.double()[i::5, j::4] - r).norm() / r.norm()) for x in (out, want)]
+                assert off[0] <= max(off[1], 1.6e-7), (i, j, off)
 
 
 @pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512)])
