@@ -1955,7 +1955,22 @@ def diff_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
 # outputs: with 512 terms faster at every size (1.0 to 3.6 times; 13.9 against 8.1 us for one row
 # and 1,024 outputs), with 256 slower for few rows or outputs (7.6 against 9.0 us).
 SGEMM_SPLIT_MIN_K = 512
-SGEMM_SPLIT_MAX_BYTES = 256 << 20     # scratch of a call; more rows go in several
+SGEMM_SPLIT_MAX_BYTES = 256 << 20     # scratch of a call; more rows or products go in several
+
+
+def _sgemm_split_calls(M: int, K: int, batch: int):
+    """``(first product, products, first row, rows)`` of the calls that a product takes: as few as keep
+    the rows' terms (six bytes an element, in whole tiles of 112 or 176 rows) within
+    ``SGEMM_SPLIT_MAX_BYTES``, or a tile a call where one takes more."""
+    def padded(m):
+        return max(-(-m // 112) * 112, -(-m // 176) * 176)
+    if M <= 16:                                              # (these rows need no scratch)
+        return [(0, batch, 0, M)]
+    most = SGEMM_SPLIT_MAX_BYTES // (192 * -(-K // 32))      # rows of a call
+    rows = M if padded(M) <= most else max(most // 1232 * 1232, 112)     # (1,232: whole tiles of both)
+    products = max(1, min(batch, most // padded(rows)))
+    return [(b, min(products, batch - b), m, min(rows, M - m))
+            for b in range(0, batch, products) for m in range(0, M, rows)]
 
 
 def _sgemm_split(a, w, out, M, N, K, batch, lda, ldw, ldc, batch_a, batch_w, batch_c) -> None:
@@ -1963,14 +1978,12 @@ def _sgemm_split(a, w, out, M, N, K, batch, lda, ldw, ldc, batch_a, batch_w, bat
     fn = lib().bf_sgemm_split_scratch
     fn.restype = _c_ll
     err = error_word(a.device)
-    # (rows of a call: their terms take six bytes an element)
-    most = max(4096, SGEMM_SPLIT_MAX_BYTES // (6 * K * batch))
-    for m0 in range(0, M, most):
-        m = min(most, M - m0)
-        n = fn(_c_int(m), _c_int(N), _c_int(K), _c_int(batch), _c_int(0))
+    for b, nb, m0, m in _sgemm_split_calls(M, K, batch):
+        x, v, y = (a[m0:], w, out[m0:]) if a.dim() == 2 else (a[m0:, b:], w[b:], out[m0:, b:])
+        n = fn(_c_int(m), _c_int(N), _c_int(K), _c_int(nb), _c_int(0))
         scratch = torch.empty(n, dtype=torch.uint8, device=a.device) if n else None
-        _run("sgemm_split", lib().bf_sgemm_split, _ptr(a[m0:]), _ptr(w), _ptr(out[m0:]), _c_int(m),
-             _c_int(N), _c_int(K), _c_ll(lda), _c_ll(ldw), _c_ll(ldc), _c_int(batch), _c_ll(batch_a),
+        _run("sgemm_split", lib().bf_sgemm_split, _ptr(x), _ptr(v), _ptr(y), _c_int(m),
+             _c_int(N), _c_int(K), _c_ll(lda), _c_ll(ldw), _c_ll(ldc), _c_int(nb), _c_ll(batch_a),
              _c_ll(batch_w), _c_ll(batch_c), _c_int(0), _ptr(scratch), _ptr(err), _stream())
         _launches += n > 0           # two kernels: the rows' terms and the product
 

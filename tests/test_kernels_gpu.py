@@ -174,6 +174,27 @@ def test_sgemm_of_terms(cuda_device, M, N, K):
     assert int(ops.error_word(cuda_device).item()) == 0
 
 
+@pytest.mark.parametrize("M,N,K,batch", [(1241, 130, 1024, 1), (300, 40, 600, 5), (40, 8, 2048, 7)])
+def test_sgemm_of_terms_in_several_calls(cuda_device, monkeypatch, M, N, K, batch):
+    """A product whose rows' terms pass the limit, cut by rows and by products: the same bits."""
+    from binfer_b200.csrc import ops
+    a = torch.randn(M, batch, K + 4, device=cuda_device)[:, :, :K]
+    w = torch.randn(batch, N, K, device=cuda_device)
+    outs = []
+    for limit in (1 << 30, 6 * K * 1232, 6 * K * 300):
+        monkeypatch.setattr(ops, "SGEMM_SPLIT_MAX_BYTES", limit)
+        outs.append(torch.full((M, batch, N), 7.0, device=cuda_device))
+        before = ops.launches()
+        if batch == 1:
+            ops.sgemm_nt(a[:, 0], w[0], outs[-1][:, 0])
+        else:
+            ops.sgemm_nt_batched(a, w, outs[-1])
+        calls = ops._sgemm_split_calls(M, K, batch)
+        assert ops.launches() - before == sum(1 + (m > 16) for _, _, _, m in calls)
+    assert len(calls) > 1
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 # tiles of 16, 176 and 112 rows, features shared by clusters of 4 and 2 CTAs and not
 @pytest.mark.parametrize("M,N,K", [(5, 300, 700), (40, 3000, 513), (200, 9500, 512), (224, 4200, 512)])
 def test_sgemm_of_terms_with_products_that_overflow(cuda_device, M, N, K):
