@@ -108,12 +108,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  int stage = 0;                               // (copying thread, issuing warp) their next stage of the ring
+  uint32_t phase = 0;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
       for (int u = blockIdx.x; u < units && !*abort; u += gridDim.x) {
         const int tt = u % p.tiles_t, tf = u / p.tiles_t;
         for (int kc = 0; kc < kc_total; ++kc) {
@@ -135,8 +135,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
       // c = float, a = b = bf16, both K-major, N = bn, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                              ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(p.mma_rows >> 4) << 24);
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      int acc = 0;
+      uint32_t acc_phase = 0;
       for (int u = blockIdx.x; u < units; u += gridDim.x) {
         if (!mbar_wait_warp(acc_empty + acc, acc_phase ^ 1, abort)) break;
         tc_fence_after();
@@ -230,13 +230,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x,
   if (*abort) {
     if (threadIdx.x == 0) atomicOr(p.err, BF_ERR_WAIT);
     if (warp == 0 && lane == 0) {
-      // copies that were issued but never consumed: give each stage's barrier a bounded chance
-      for (int s = 0; s < STAGES; ++s) {
-        const long long t0 = clock64();
-        while (!mbar_try_wait(full + s, 0) && !mbar_try_wait(full + s, 1) &&
-               clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
-        }
-      }
+      mbar_drain(full, STAGES, stage, phase);  // copies that were issued but never consumed
     }
     if (warp == 1) {
       umma_commit(drain);                      // products still in flight

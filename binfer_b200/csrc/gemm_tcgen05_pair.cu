@@ -169,6 +169,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x,
   pair_sync();                               // the peer's barriers exist before anything lands
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  int next = 0;                                // (copying thread) the stage behind its last fill
+  uint32_t next_phase = 0;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -204,6 +206,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x,
           }
         }
       }
+      next = stage;
+      next_phase = phase;
       // every arrival that the leader's commits send to this CTA's barriers lands before it ends
       for (int s = 0; s < STAGES && ok && !*abort; ++s) {
         ok = mbar_wait(empty + stage, phase ^ 1, abort);
@@ -388,13 +392,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x,
                    : "memory");
     }
     if (warp == 0 && lane == 0 && rank == 0) {
-      // copies that were issued but never consumed: give each stage's barrier a bounded chance
-      for (int s = 0; s < STAGES; ++s) {
-        const long long t0 = clock64();
-        while (!mbar_try_wait(full + s, 0) && !mbar_try_wait(full + s, 1) &&
-               clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
-        }
-      }
+      mbar_drain(full, STAGES, next, next_phase);  // copies that were issued but never consumed
     }
     if (warp == 1 && rank == 0) {
       pair_commit_own(drain);                  // products still in flight

@@ -275,6 +275,8 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   float total[MINE];                       // (summing warps) the columns' sums over K
+  int next = 0;                            // (copying threads) the stage that they would fill next,
+  uint32_t next_phase = 0;                 // and its phase
 
   if (warp < SP_FETCH) {
     // ----------------------------------------------------------------- take apart, store
@@ -394,34 +396,30 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
     bf_pdl_wait();                         // (the kernel that laid them out)
     const uint8_t* src = p.terms + ((size_t)blockIdx.z * steps * 3 * p.rows + m0) * 64;
     if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
       for (int s = s0; s < s1; ++s) {
-        if (!mbar_wait(empty + stage, phase ^ 1, abort)) break;
-        uint8_t* to = tiles + (size_t)stage * STAGE + 3 * W_BYTES;
-        mbar_expect_tx(full + stage, 3 * A_BYTES);
+        if (!mbar_wait(empty + next, next_phase ^ 1, abort)) break;
+        uint8_t* to = tiles + (size_t)next * STAGE + 3 * W_BYTES;
+        mbar_expect_tx(full + next, 3 * A_BYTES);
 #pragma unroll
         for (int t = 0; t < 3; ++t)
-          bf_bulk_load(to + t * A_BYTES, src + ((size_t)s * 3 + t) * p.rows * 64, A_BYTES, full + stage);
-        if (++stage == p.stages) {
-          stage = 0;
-          phase ^= 1;
+          bf_bulk_load(to + t * A_BYTES, src + ((size_t)s * 3 + t) * p.rows * 64, A_BYTES, full + next);
+        if (++next == p.stages) {
+          next = 0;
+          next_phase ^= 1;
         }
       }
     }
   } else if (VEC && warp == SP_TMA) {
     // ------------------------------------------------------------------ features' floats
     if (lane == 0) {
-      int slot = 0;
-      uint32_t phase = 0;
       for (int s = s0; s < s1; ++s) {
-        if (!mbar_wait(w_empty + slot, phase ^ 1, abort)) break;
-        mbar_expect_tx(w_full + slot, SP_FLOATS);
-        sp_tma_load_3d(floats + (size_t)slot * SP_FLOATS, &map_w, w_full + slot, s * SP_K, f0,
+        if (!mbar_wait(w_empty + next, next_phase ^ 1, abort)) break;
+        mbar_expect_tx(w_full + next, SP_FLOATS);
+        sp_tma_load_3d(floats + (size_t)next * SP_FLOATS, &map_w, w_full + next, s * SP_K, f0,
                        blockIdx.z);
-        if (++slot == p.floats) {
-          slot = 0;
-          phase ^= 1;
+        if (++next == p.floats) {
+          next = 0;
+          next_phase ^= 1;
         }
       }
     }
@@ -472,15 +470,9 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
       while (!mbar_try_wait(drain, 0) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
       }
     }
-    if ((warp == SP_COPY && PRE || warp == SP_TMA && VEC) && lane == 0) {
-      uint64_t* bar = warp == SP_COPY ? full : w_full;    // copies that nobody waited for
-      for (int s = 0; s < (warp == SP_COPY ? p.stages : p.floats); ++s) {
-        const long long t0 = clock64();
-        while (!mbar_try_wait(bar + s, 0) && !mbar_try_wait(bar + s, 1) &&
-               clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
-        }
-      }
-    }
+    // copies that nobody waited for
+    if (PRE && warp == SP_COPY && lane == 0) mbar_drain(full, p.stages, next, next_phase);
+    if (VEC && warp == SP_TMA && lane == 0) mbar_drain(w_full, p.floats, next, next_phase);
     __syncwarp();
     __syncthreads();
   }

@@ -5,6 +5,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "ring_drain.cuh"
+
 namespace {
 
 
@@ -49,6 +51,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
   }
   return true;
+}
+// After a wait that gave up, by the thread that asked for a ring's copies: until the last fill of every
+// stage has landed (ring_drain.cuh), each with a limit.
+__device__ __forceinline__ void mbar_drain(uint64_t* bars, int stages, int stage, uint32_t phase) {
+  ring_drain(stages, stage, phase, [&](int s, unsigned parity) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bars + s, parity) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
+    }
+  });
 }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
                                             int x, int y) {
