@@ -207,7 +207,8 @@ __device__ __forceinline__ void mt_stored() {
   tc_fence_before();
   __syncthreads();
 }
-// Step `i`'s products are complete.  (When a wait gives up the kernel goes on, without waits, to its end.)
+// Step `i`'s products are complete.  (When a wait gives up the kernel goes on, without waits and without
+// further copies into shared memory, to its end.)
 __device__ __forceinline__ void mt_done(MtShared& s, int i) {
   mbar_wait(s.done + (i & 1), (i >> 1) & 1, &s.abort);
   __syncwarp();
@@ -534,23 +535,29 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
   auto raw = [&](int x) { return *reinterpret_cast<const uint4*>(mine + x * 16 * MT_WORK); };
 
   MtUnit c = {};                                 // the tile whose operands are fetched
+  OnePlace copies;                               // (of thread 0)
+  auto gave_up = [&]() { return *(volatile int*)&sh.abort != 0; };
   // (all have read the step before; rows beyond the last repeat it: q's results are not stored, values'
   // weights are zero)
   auto fetch = [&](int step) {
     const size_t head = (size_t)c.chunk * p.H + c.h;
     if (step < steps) {
       if (tid == 0) {
-        mbar_expect_tx(&sh.got, MT_C * MT_M * 4 + MT_C * 4);
-        bf_bulk_load(n_s, Un + head * p.dk + step * MT_C, MT_C * 4, &sh.got);
-        bf_bulk_load(block, U + head * p.dk * p.dv + (size_t)c.m0 * p.dk + step * MT_C * MT_M, MT_C * MT_M * 4,
-                     &sh.got);
+        copies.fill(gave_up(), [&]() {
+          mbar_expect_tx(&sh.got, MT_C * MT_M * 4 + MT_C * 4);
+          bf_bulk_load(n_s, Un + head * p.dk + step * MT_C, MT_C * 4, &sh.got);
+          bf_bulk_load(block, U + head * p.dk * p.dv + (size_t)c.m0 * p.dk + step * MT_C * MT_M,
+                       MT_C * MT_M * 4, &sh.got);
+        });
       }
       mt_fetch(mine, proj + (size_t)(c.t0 + min(tr, c.n - 1)) * p.qk_stride + p.q_off + (size_t)c.h * p.dk +
                          step * MT_C + 8 * tq);
     } else {
       if (tid == 0) {
-        mbar_expect_tx(&sh.got, MT_C * MT_C * 4);
-        bf_bulk_load(block, qkm + head * MT_C * MT_C, MT_C * MT_C * 4, &sh.got);
+        copies.fill(gave_up(), [&]() {
+          mbar_expect_tx(&sh.got, MT_C * MT_C * 4);
+          bf_bulk_load(block, qkm + head * MT_C * MT_C, MT_C * MT_C * 4, &sh.got);
+        });
       }
       const mt_bf16* v = proj + (size_t)c.t0 * p.v_stride + p.v_off + (size_t)c.h * p.dv + c.m0 + 8 * mq;
       mt_fetch(mine, v + (size_t)min(mr, c.n - 1) * p.v_stride);
@@ -755,6 +762,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
     tab ^= 1;
   }
   if (i) finish(table[tab ^ 1], steps, i - 1);
+  if (tid == 0 && gave_up())                     // (a copy that this thread did not see land)
+    copies.drain([&](int, unsigned parity) { mbar_drain_one(&sh.got, parity); });
   mt_end(sh, tmem, err);
 }
 

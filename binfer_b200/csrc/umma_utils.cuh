@@ -54,12 +54,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 }
 // After a wait that gave up, by the thread that asked for a ring's copies: until the last fill of every
 // stage has landed (ring_drain.cuh), each with a limit.
+__device__ __forceinline__ void mbar_drain_one(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
+  }
+}
 __device__ __forceinline__ void mbar_drain(uint64_t* bars, int stages, int stage, uint32_t phase) {
-  ring_drain(stages, stage, phase, [&](int s, unsigned parity) {
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bars + s, parity) && clock64() - t0 < WAIT_LIMIT_CYCLES / 16) {
-    }
-  });
+  ring_drain(stages, stage, phase, [&](int s, unsigned parity) { mbar_drain_one(bars + s, parity); });
 }
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
                                             int x, int y) {

@@ -10,8 +10,30 @@ PROGRAM = r"""
 #include "ring_drain.cuh"
 // a barrier's completed phases; a wait for a parity passes unless the phase at work has it
 struct Bar { int done = 0; bool passes(unsigned parity) const { return (done & 1) != (int)parity; } };
+// one place, `steps` fills of it, the copy of step `slow` (if any) landing only behind the end: whether an
+// arrival met an open phase (the barrier takes one a phase) or the end did not wait for that copy
+static bool one_place(int steps, int slow, bool heeds) {
+  OnePlace copies; Bar bar;
+  int flying = 0, bad = 0; bool gave_up = false;
+  for (int i = 0; i < steps; ++i) {
+    copies.fill(heeds && gave_up, [&] { bad += flying; ++flying; });
+    if (flying && i != slow && !gave_up) { --flying; ++bar.done; }
+    if (!bar.passes(i & 1)) gave_up = true;                          // the wait runs out
+  }
+  copies.drain([&](int s, unsigned parity) {
+    bad += s != 0 || bar.passes(parity) == (flying > 0);
+    if (flying) { --flying; ++bar.done; }
+    bad += !bar.passes(parity);
+  });
+  return bad || flying;
+}
 int main() {
   int cases = 0;
+  for (int steps = 0; steps < 9; ++steps)
+    for (int slow = 0; slow <= steps; ++slow) {
+      if (one_place(steps, slow, true)) { std::printf("one place %d %d\\n", steps, slow); return 1; }
+      if (one_place(steps, slow, false) != (slow + 1 < steps)) return 1;       // (the model sees it)
+    }
   for (int stages = 1; stages <= 8; ++stages)
     for (int fills = 0; fills <= 3 * stages + 1; ++fills)
       for (unsigned flying = 0; flying < 1u << (fills < stages ? fills : stages); ++flying) {
