@@ -15,7 +15,9 @@
 // A product of a float and a bfloat16 number is three products of terms.  The tensor core's sums cut
 // where arithmetic rounds, so the leading terms' products are summed 32 at a time, apart from the
 // smaller terms', and the sums are added in rounded float.  Operands that have no terms (infinities,
-// NaN) are zero in the products, and the results that they reach are computed by multiply-adds.
+// NaN) are zero in the products, and the results that they reach are computed by multiply-adds; so are
+// sums that are not finite (where finite operands' product leaves float's range, that of a smaller term may
+// overflow with a sign of its own).
 //
 // 2,048 tokens, 8 heads of 256 x 512: mt_state 72 us (cs_state and cs_prefix 177), mt_out 92 (cs_out 168).
 // What bounds them: mt_state the issue slots (a chunk's keys and values to take apart, its sums, its states
@@ -381,17 +383,33 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_state_kernel(
       to[(2 * j + 1) * MT_M] = e;
     }
     mt_done(sh, i);
+    unsigned long long zero = 0ull;              // (NaN where some sum is not finite)
 #pragma unroll
     for (int j0 = 0; j0 < 8; j0 += 4) {
       unsigned long long u[4];
       mt_take(at + (uint32_t)((i & 1) * 3 * MT_C + 2 * j0), u);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) S[j0 + j] = cs_fma2(dx2, S[j0 + j], cs_fma2(dy2, S[j0 + j], u[j]));
+      for (int j = 0; j < 4; ++j) {
+        S[j0 + j] = cs_fma2(dx2, S[j0 + j], cs_fma2(dy2, S[j0 + j], u[j]));
+        zero = cs_fma2(u[j], 0ull, zero);
+      }
     }
-    if (odd) {
+    float z0, z1;
+    cs_unpair(zero, z0, z1);
+    const bool lost = z0 + z1 != 0.f;
+    if (odd || lost) {
 #pragma unroll 1
       for (int j = 0; j < 16; ++j) {
-        if (odd_v[i % 3][v_own] != i && odd_k[i % 3][group * 16 + j] != i) continue;
+        float now = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          float a, x;
+          cs_unpair(S[k], a, x);
+          now = 2 * k == j ? a : 2 * k + 1 == j ? x : now;
+        }
+        if (odd_v[i % 3][v_own] != i && odd_k[i % 3][group * 16 + j] != i &&
+            !(lost && !(fabsf(now) < INFINITY)))
+          continue;
         const int e = min(c.n, (i + 1) * MT_C);
         float y = 0.f;                           // the chunk's share by multiply-adds
 #pragma unroll 1
@@ -634,7 +652,17 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
     }
     MtEight w = weighted(tb);
     // n_t . q_t: the state's share with the token's weight, and the row's sum
-    den = cs_times(den, tb.at[tr]) +
+    den = cs_times(den, tb.at[tr]);
+    if (!(fabsf(den) < INFINITY) && tr < c.n) {  // (the weight on q: it may keep the products finite)
+      const mt_bf16* q = proj + (size_t)(c.t0 + tr) * p.qk_stride + p.q_off + (size_t)c.h * p.dk + 8 * tq;
+      const float* n = Un + ((size_t)c.chunk * p.H + c.h) * p.dk + 8 * tq;
+      den = 0.f;
+#pragma unroll 1
+      for (int k = 0; k < p.dk; k += MT_C)
+#pragma unroll 1
+        for (int j = k; j < k + 8; ++j) den = fmaf(cs_times(bf_ld(q + j), tb.at[tr]), n[j], den);
+    }
+    den +=
           (((w.v[0] + w.v[1]) + (w.v[2] + w.v[3])) + ((w.v[4] + w.v[5]) + (w.v[6] + w.v[7])));
     mt_put(tt, MT_TOK, w, left);
     if (mt_bad(left)) {
@@ -670,29 +698,42 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
     const size_t row = (size_t)p.H * p.dv;
     float* dst = o_raw + (size_t)(x.t0 + group * 16) * row + (size_t)x.h * p.dv + x.m0 + m;
     const int n = x.n - group * 16;
+    unsigned lost = 0;                           // tokens whose sum is not finite
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float a, b;
       cs_unpair(sum[j], a, b);
+      lost |= (fabsf(a) < INFINITY ? 0u : 1u << 2 * j) | (fabsf(b) < INFINITY ? 0u : 2u << 2 * j);
       if (2 * j < n) dst[0] = a / tb.den[group * 16 + 2 * j];
       if (2 * j + 1 < n) dst[row] = b / tb.den[group * 16 + 2 * j + 1];
       dst += 2 * row;
     }
-    if (!tb.odd) return;
+    if (!tb.odd && !lost) return;
+    // (in cs_out's order: runs of sixteen, the weight on q)
 #pragma unroll 1
     for (int t = group * 16; t < min(group * 16 + 16, x.n); ++t) {
-      if (!tb.odd_t[t] && tb.odd_m[m] > t) continue;
+      if (!tb.odd_t[t] && tb.odd_m[m] > t && !(lost >> (t & 15) & 1)) continue;
       const mt_bf16* q = proj + (size_t)(x.t0 + t) * p.qk_stride + p.q_off + (size_t)x.h * p.dk;
       const mt_bf16* v = proj + (size_t)x.t0 * p.v_stride + p.v_off + (size_t)x.h * p.dv + x.m0 + m;
       const float* P = qkm + (((size_t)x.chunk * p.H + x.h) * MT_C + t) * MT_C;
       const float* S = U + ((size_t)x.chunk * p.H + x.h) * p.dk * p.dv + (size_t)x.m0 * p.dk + m;
       float o = 0.f;
 #pragma unroll 1
-      for (int k = 0; k < p.dk; ++k) o = fmaf(bf_ld(q + k), S[(size_t)k * MT_M], o);
-      o = cs_times(o, tb.at[t]);
+      for (int k0 = 0; k0 < p.dk; k0 += 16) {
+        float run = 0.f;
 #pragma unroll 1
-      for (int y = 0; y <= t; ++y)
-        o = fmaf(cs_times(P[y], cs_exp(tb.g[t] - tb.h[y])), bf_ld(v + (size_t)y * p.v_stride), o);
+        for (int k = k0; k < k0 + 16; ++k)
+          run = fmaf(cs_times(bf_ld(q + k), tb.at[t]), S[(size_t)k * MT_M], run);
+        o += run;
+      }
+#pragma unroll 1
+      for (int y0 = 0; y0 <= t; y0 += 16) {
+        float run = 0.f;
+#pragma unroll 1
+        for (int y = y0; y <= min(t, y0 + 15); ++y)
+          run = fmaf(cs_times(P[y], cs_exp(tb.g[t] - tb.h[y])), bf_ld(v + (size_t)y * p.v_stride), run);
+        o += run;
+      }
       o_raw[(size_t)(x.t0 + t) * row + (size_t)x.h * p.dv + x.m0 + m] = o / tb.den[t];
     }
   };

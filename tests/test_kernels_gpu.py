@@ -1595,6 +1595,43 @@ def test_mlstm_chunks_on_tensor_cores_keep_infinities_apart(cuda_device, what, a
         assert torch.equal(out[:, 1, :130], clean[:, 1, :130]) and torch.equal(out[:, 1, 131:], clean[:, 1, 131:])
 
 
+@pytest.mark.parametrize("at", [64, 140, 255])
+@pytest.mark.parametrize("what", ["state", "q.k", "output", "faded"])
+def test_mlstm_chunks_on_tensor_cores_with_products_that_overflow(cuda_device, at, what):
+    """Finite operands whose products leave float's range: the infinities and NaN of the multiply-adds."""
+    from binfer_b200.csrc import ops
+    dev, T, H, dk, dv = cuda_device, 300, 2, 128, 256
+    torch.manual_seed(6)
+    wide = torch.randn(T, 2 * H * (dk + dv) + 4, device=dev).to(BF16)
+    x = wide[:, 4:]
+    q, k, v = x[:, dk:2 * dk], x[:, H * dk + dk:2 * H * dk], x[:, 2 * H * dk + dv:2 * H * dk + 2 * dv]   # of head 1
+    if what == "state":
+        k[at, 5], v[at, 130], v[at, 131] = 1.3e30, 1.7e30, -1.1e30
+    elif what == "q.k":
+        q[at, 5], k[at - 3, 5], v[at - 3, 130], v[at - 3, 131] = 1.3e18, 1.7e18, 1.1e30, -1.3e30
+    elif what == "output":
+        k[at - 20, 5], v[at - 20, 130], v[at - 20, 131], q[at, 5] = 1.3e15, 1.7e15, -1.1e15, 1.3e30
+    else:                                      # (a state that the token's weight leaves out)
+        at = at // 64 * 64
+        k[at - 1, 5], v[at - 1, 130], v[at - 1, 131], q[at + 43, 5] = 1.3e15, 1.7e15, -1.1e15, 1.3e30
+    gates = torch.cat([torch.randn(T, H, device=dev), -0.1 * torch.rand(T, H, device=dev)], 1).contiguous()
+    if what == "faded":
+        gates[:, H:] = -3.0
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, got = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    for proj in (x, x.contiguous()):           # (rows off the 16-byte boundaries: multiply-adds)
+        s = torch.zeros(1, H, ops.mlstm_state_size(dk, dv), device=dev)
+        o = torch.zeros(T, H * dv, device=dev)
+        ops.mlstm_scan(proj, gates, s, qs, slots, o, 1, H, dk, dv, dk ** -0.5, err, max_q=T, chunked=True)
+        got.append(torch.cat([o.flatten(), s.flatten()]))
+    want, have = got
+    assert bool(want.isfinite().all()) == (what == "faded")
+    assert torch.equal(have.isnan(), want.isnan()) and torch.equal(have.isinf(), want.isinf())
+    assert torch.equal(have[have.isinf()], want[have.isinf()])
+    fin = want.isfinite()
+    assert float((have - want)[fin].abs().max() / want[fin].abs().max()) < 1e-5
+
+
 # ------------------------------------------- latent attention with keys and values expanded
 # portions below, at and above a key tile of 64, a query tile of 128 and a block of 256, from the
 # start and behind cached keys; the rows of two portions and a single token's row in one buffer
