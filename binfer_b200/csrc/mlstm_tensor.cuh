@@ -14,10 +14,11 @@
 //
 // A product of a float and a bfloat16 number is three products of terms.  The tensor core's sums cut
 // where arithmetic rounds, so the leading terms' products are summed 32 at a time, apart from the
-// smaller terms', and the sums are added in rounded float.  Operands that have no terms (infinities,
-// NaN) are zero in the products, and the results that they reach are computed by multiply-adds; so are
-// sums that are not finite (where finite operands' product leaves float's range, that of a smaller term may
-// overflow with a sign of its own).
+// smaller terms', and the sums are added in rounded float.  Floats are multiplied by 2^24 before they are
+// taken apart, so that their terms hold them whatever their size (split_utils.cuh), and the sums by 2^-24.
+// Operands that have no terms (infinities, NaN, floats from 2^104 on) are zero in the products, and the
+// results that they reach are computed by multiply-adds; so are sums that are not finite (where finite
+// operands' product leaves float's range, that of a smaller term may overflow with a sign of its own).
 //
 // 2,048 tokens, 8 heads of 256 x 512: mt_state 72 us (cs_state and cs_prefix 177), mt_out 92 (cs_out 168).
 // What bounds them: mt_state the issue slots (a chunk's keys and values to take apart, its sums, its states
@@ -71,6 +72,12 @@ __device__ __forceinline__ void mt_take(uint32_t at, unsigned long long (&u)[4])
   }
 }
 
+__device__ __forceinline__ unsigned long long mt_down(unsigned long long x) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(cs_pair(SPLIT_DOWN, SPLIT_DOWN)));
+  return r;
+}
+
 // Sixteen bytes on their way into shared memory
 __device__ __forceinline__ void mt_fetch(uint8_t* to, const void* from) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to)), "l"(from));
@@ -91,10 +98,12 @@ __device__ __forceinline__ MtEight mt_bf16s(const uint4& u) {
   }
   return x;
 }
-// Their terms to `at`, a term's tile `bytes` behind the one before.  `left` stays finite where all
-// have terms.
-__device__ __forceinline__ void mt_put(uint8_t* at, int bytes, const MtEight& x, float2& left) {
+// Their terms, times SPLIT_UP, to `at`, a term's tile `bytes` behind the one before.  `left` stays finite
+// where all have terms.
+__device__ __forceinline__ void mt_put(uint8_t* at, int bytes, MtEight x, float2& left) {
   uint4 hi, mid, lo;
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) split_up(x.v[i], x.v[i + 1]);
   split3(x.v[0], x.v[1], hi.x, mid.x, lo.x, left);
   split3(x.v[2], x.v[3], hi.y, mid.y, lo.y, left);
   split3(x.v[4], x.v[5], hi.z, mid.z, lo.z, left);
@@ -109,12 +118,14 @@ __device__ __forceinline__ bool mt_bad(const uint4& u) {
   auto two = [](uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; };
   return two(u.x) || two(u.y) || two(u.z) || two(u.w);
 }
-// zero in the place of what has no terms: a bit for each
-__device__ __forceinline__ int mt_clean(MtEight& x) {
+// zero in the place of what has no terms: a bit for each.  What is an infinity or a NaN among bfloat16
+// numbers; among floats what is beyond the largest of those once it is multiplied.
+constexpr uint32_t MT_NO_TERMS = 0x7f7f8000u, MT_NO_TERMS_UP = MT_NO_TERMS - (24u << 23);
+__device__ __forceinline__ int mt_clean(MtEight& x, uint32_t from) {
   int bad = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    if ((__float_as_uint(x.v[i]) & 0x7fffffffu) >= 0x7f7f8000u) {
+    if ((__float_as_uint(x.v[i]) & 0x7fffffffu) >= from) {
       bad |= 1 << i;
       x.v[i] = 0.f;
     }
@@ -327,7 +338,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_state_kernel(
 #pragma unroll 1
       for (int x = 0; x < 3; ++x) {
         MtEight e = x < 2 ? value(i, x) : mt_bf16s(k);
-        const int bad = mt_clean(e);
+        const int bad = mt_clean(e, x < 2 ? MT_NO_TERMS_UP : MT_NO_TERMS);
         for (int j = 0; j < 8; ++j)
           if (bad >> j & 1) (x < 2 ? odd_v[i % 3] + 8 * vq : odd_k[i % 3] + 8 * kq)[j] = i;
         if (x < 2) mt_put(tile + v_spot + x * 4096, MT_TILE, e, left);
@@ -390,7 +401,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_state_kernel(
       mt_take(at + (uint32_t)((i & 1) * 3 * MT_C + 2 * j0), u);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        S[j0 + j] = cs_fma2(dx2, S[j0 + j], cs_fma2(dy2, S[j0 + j], u[j]));
+        S[j0 + j] = cs_fma2(dx2, S[j0 + j], cs_fma2(dy2, S[j0 + j], mt_down(u[j])));
         zero = cs_fma2(u[j], 0ull, zero);
       }
     }
@@ -625,13 +636,13 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
 #pragma unroll 1
         for (int x = 0; x < 2; ++x) {
           MtEight e = eight(mr + 32 * x, MT_M, mq);
-          const int bad = mt_clean(e);
+          const int bad = mt_clean(e, MT_NO_TERMS_UP);
           for (int j = 0; j < 8; ++j)
             if (bad >> j & 1) tb.odd_m[8 * mq + j] = 0;
           mt_put(tm + x * 4096, MT_TILE, e, left);
         }
         MtEight f = mt_bf16s(qv);
-        if (mt_clean(f)) tb.odd_t[tr] = 1;
+        if (mt_clean(f, MT_NO_TERMS)) tb.odd_t[tr] = 1;
         *reinterpret_cast<uint4*>(tt) = mt_pack(f);
         tb.odd = 1;
       }
@@ -642,7 +653,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
       uint4 v = raw(x);
       if (mt_bad(v)) {
         MtEight f = mt_bf16s(v);
-        const int bad = mt_clean(f);
+        const int bad = mt_clean(f, MT_NO_TERMS);
         for (int j = 0; j < 8; ++j)
           if (bad >> j & 1) atomicMin(tb.odd_m + 8 * mq + j, mr + 32 * x);
         v = mt_pack(f);
@@ -666,7 +677,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
           (((w.v[0] + w.v[1]) + (w.v[2] + w.v[3])) + ((w.v[4] + w.v[5]) + (w.v[6] + w.v[7])));
     mt_put(tt, MT_TOK, w, left);
     if (mt_bad(left)) {
-      mt_clean(w);
+      mt_clean(w, MT_NO_TERMS_UP);
       tb.odd_t[tr] = 1;
       tb.odd = 1;
       mt_put(tt, MT_TOK, w, left);
@@ -675,7 +686,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
     for (int o = 1; o < 8; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
     if (tq == 0) tb.den[tr] = tr < c.n ? fmaxf(fabsf(den), E[(size_t)c.h * p.T + c.t0 + tr]) + 1e-6f : 1.f;
   };
-  unsigned long long sum[8];
+  unsigned long long sum[8];                     // (times SPLIT_UP)
   auto finish = [&](const MtTable& tb, int step, int i) {
     mt_done(sh, i);
 #pragma unroll
@@ -704,8 +715,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
       float a, b;
       cs_unpair(sum[j], a, b);
       lost |= (fabsf(a) < INFINITY ? 0u : 1u << 2 * j) | (fabsf(b) < INFINITY ? 0u : 2u << 2 * j);
-      if (2 * j < n) dst[0] = a / tb.den[group * 16 + 2 * j];
-      if (2 * j + 1 < n) dst[row] = b / tb.den[group * 16 + 2 * j + 1];
+      if (2 * j < n) dst[0] = a * SPLIT_DOWN / tb.den[group * 16 + 2 * j];
+      if (2 * j + 1 < n) dst[row] = b * SPLIT_DOWN / tb.den[group * 16 + 2 * j + 1];
       dst += 2 * row;
     }
     if (!tb.odd && !lost) return;

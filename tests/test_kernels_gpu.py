@@ -1595,6 +1595,58 @@ def test_mlstm_chunks_on_tensor_cores_keep_infinities_apart(cuda_device, what, a
         assert torch.equal(out[:, 1, :130], clean[:, 1, :130]) and torch.equal(out[:, 1, 131:], clean[:, 1, 131:])
 
 
+def _mlstm_f64(proj, gates, s0, H, dk, dv, scale):
+    """One request's outputs and last S, n, m in float64, token by token."""
+    x = proj.double()
+    q, k = x[:, :H * dk].view(-1, H, dk) * scale, x[:, H * dk:2 * H * dk].view(-1, H, dk)
+    v = x[:, 2 * H * dk:2 * H * dk + H * dv].view(-1, H, dv)
+    s0, g = s0.double(), gates.double()
+    S, n, m = s0[:, :dk * dv].view(H, dk, dv), s0[:, dk * dv:dk * dv + dk], s0[:, dk * dv + dk]
+    o = torch.empty_like(v)
+    for t in range(x.shape[0]):
+        m_new = torch.maximum(g[t, H:] + m, g[t, :H])
+        da, db = torch.exp(g[t, H:] + m - m_new), torch.exp(g[t, :H] - m_new)
+        S = S * da[:, None, None] + (k[t] * db[:, None])[:, :, None] * v[t][:, None, :]
+        n, m = da[:, None] * n + db[:, None] * k[t], m_new
+        den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + 1e-6
+        o[t] = (q[t][:, None, :] @ S)[:, 0] / den[:, None]
+    return o, S, n, m
+
+
+# small and large: states, weighted values, weighted products of q and k, and bfloat16 numbers themselves
+@pytest.mark.parametrize("what", ["values", "products", "keys", "queries", "large"])
+def test_mlstm_chunks_on_tensor_cores_hold_floats_of_every_size(cuda_device, what):
+    """Nothing that multiply-adds over chunks hold is lost in terms: relative errors against float64, no
+    further off.  (The walk is no measure: of keys or queries of 1e-39 its q . k are there in as many
+    bits as they are multiplied, over chunks in those that a float of that size has.)"""
+    from binfer_b200.csrc import ops
+    dev, T, H, dk, dv = cuda_device, 333, 2, 128, 256
+    torch.manual_seed(9)
+    size = {"values": (1, 1, 1e-35), "products": (1e-18, 1e-17, 1), "keys": (1, 1e-39, 1e28),
+            "queries": (1e-39, 1, 1e28), "large": (1, 1, 1e33)}[what]
+    x = torch.cat([c * torch.randn(T, n, device=dev) for c, n in zip(
+        size, (H * dk, H * dk, H * dv))] + [torch.zeros(T, H * dv, device=dev)], 1).to(BF16)
+    gates = torch.cat([2 * torch.randn(T, H, device=dev), torch.nn.functional.logsigmoid(
+        3 + torch.randn(T, H, device=dev))], 1).contiguous()
+    state = torch.randn(1, H, ops.mlstm_state_size(dk, dv), device=dev)
+    state[:, :, :dk * dv] *= size[1] * size[2]
+    state[:, :, dk * dv:dk * dv + dk] *= size[1]
+    state[:, :, dk * dv + dk:] = 0.0
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, off = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), []
+    want = _mlstm_f64(x, gates, state[0], H, dk, dv, dk ** -0.5)
+    for off16 in (4, 0):                       # (rows off the 16-byte boundaries: multiply-adds)
+        proj = torch.zeros(T, x.shape[1] + 8, device=dev, dtype=BF16)[:, off16:off16 + x.shape[1]].copy_(x)
+        s, o = state.clone(), torch.full((T, H * dv), 7.0, device=dev)
+        ops.mlstm_scan(proj, gates, s, qs, slots, o, 1, H, dk, dv, dk ** -0.5, err, max_q=T, chunked=True)
+        g = s[0].double()
+        off.append([float((a - b).norm() / b.norm()) for a, b in zip(
+            (o.double().view(-1, H, dv), g[:, :dk * dv].reshape(H, dk, dv),
+             g[:, dk * dv:dk * dv + dk], g[:, dk * dv + dk]), want)])
+    for adds, products in zip(*off):
+        assert products <= 1.5 * adds + 2e-7, off
+
+
 @pytest.mark.parametrize("at", [64, 140, 255])
 @pytest.mark.parametrize("what", ["state", "q.k", "output", "faded"])
 def test_mlstm_chunks_on_tensor_cores_with_products_that_overflow(cuda_device, at, what):
