@@ -1202,7 +1202,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles), 128, 0, stream>>>(qk, p, q_start,
                                                                                  qkm, nullptr);
   if constexpr (MLSTM) {
-    if (mt_takes(p, qk) && (long long)l.chunks * p.H * (p.dv / MT_M) < 0x7fffffff)
+    if (mt_takes(p, qk, l.chunks))
       return mt_launch(qk, p, l.chunks, q_start, state, slot_stride, state_size, state_slots, n_slots, G, Hs, g0,
                        Wl, E, qkm, U, Un, o_raw, err, stream);
   }
@@ -1258,6 +1258,13 @@ BF_EXPORT int bf_chunk_scan_mlstm(const void* proj, long long stride, const floa
   return cs_launch<__nv_bfloat16, __nv_bfloat16, true>(
       x, x, p, nullptr, nullptr, gates, state, slot_stride, state_size, q_start, state_slots,
       n_slots, o_raw, (char*)scratch, err, stream);
+}
+
+// How many kernels bf_chunk_scan_mlstm launches: four on the tensor cores, five of multiply-adds.
+BF_EXPORT int bf_chunk_scan_mlstm_kernels(const void* proj, long long stride, int T, int B, int H, int dk,
+                                          int dv, int C, int n_min) {
+  const CsIn p = {0, (long long)H * dk, 2LL * H * dk, stride, stride, H, H, dk, dv, C, T, B, n_min, 1.f};
+  return mt_takes(p, proj, cs_most_chunks(T, B, C, n_min)) ? 4 : 5;
 }
 
 // The gated delta rule.  Scratch: F (G and H are the same array), g0, Wl | qkm | kkm | W | Y |

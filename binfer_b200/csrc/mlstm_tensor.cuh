@@ -820,8 +820,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
 }
 
 // Chunks of 64 (tokens), keys in whole steps, values in whole tiles, rows on 16-byte boundaries.
-static bool mt_takes(const CsIn& p, const void* proj) {
-  return p.C == MT_C && p.dk % MT_C == 0 && p.dk <= MT_WORK && p.dv % MT_M == 0 && p.qk_stride % 8 == 0 &&
+static bool mt_takes(const CsIn& p, const void* proj, int chunks) {
+  return (long long)chunks * p.H * (p.dv / MT_M) < 0x7fffffff && p.C == MT_C && p.dk % MT_C == 0 && p.dk <= MT_WORK && p.dv % MT_M == 0 && p.qk_stride % 8 == 0 &&
          p.q_off % 8 == 0 && p.k_off % 8 == 0 && p.v_off % 8 == 0 && ((uintptr_t)proj & 15) == 0;
 }
 static int mt_launch(const mt_bf16* proj, const CsIn& p, int chunks, const int* q_start, float* state,

@@ -1492,7 +1492,9 @@ def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
              _c_float(q_scale), _c_int(CHUNK_SCAN_TOKENS),
              _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _ptr(err), _stream())
         global _launches
-        _launches += 4          # five kernels
+        _launches += lib().bf_chunk_scan_mlstm_kernels(
+            _ptr(proj), _c_ll(proj.stride(0)), _c_int(T), _c_int(B), _c_int(heads), _c_int(dk),
+            _c_int(dv), _c_int(CHUNK_SCAN_TOKENS), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN))) - 1
         if _walk_limit(scratch, B, CHUNK_SCAN_MIN) < 0:
             return
     _run("mlstm_scan", lib().bf_mlstm_scan, _ptr(proj), _c_ll(proj.stride(0)), _ptr(gates),

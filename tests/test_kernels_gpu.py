@@ -1613,6 +1613,75 @@ def _mlstm_f64(proj, gates, s0, H, dk, dv, scale):
     return o, S, n, m
 
 
+# tiles by the hundred, so that a CTA goes from tile to tile (an even and an odd number of steps a tile),
+# behind requests that are walked and, with a bad slot, past chunks that are left out
+@pytest.mark.parametrize("dk,dv,H", [(64, 384, 6), (128, 512, 4), (192, 256, 8)])
+@pytest.mark.parametrize("bad", [False, True])
+def test_mlstm_chunks_on_tensor_cores_tile_after_tile(cuda_device, dk, dv, H, bad):
+    """More than three tiles an SM, against float64 and no further off than the walking kernel."""
+    from binfer_b200.csrc import ops
+    dev, lens = cuda_device, [700, 1, 449, 30, 962, 161]
+    torch.manual_seed(dk)
+    T, B = sum(lens), len(lens)
+    assert sum(-(-n // 64) for n in lens if n > 160) * H * (dv // 128) > 3 * 148
+    proj = torch.randn(T, 2 * H * (dk + dv), device=dev).to(BF16)
+    gates = torch.cat([2 * torch.randn(T, H, device=dev), torch.nn.functional.logsigmoid(
+        3 + torch.randn(T, H, device=dev))], 1).contiguous()
+    state = 0.1 * torch.randn(B + 1, H, ops.mlstm_state_size(dk, dv), device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev).flip(0).contiguous()
+    if bad:
+        slots[2] = B + 1
+    ends = [0] + list(torch.tensor(lens).cumsum(0))
+    qs, err = torch.tensor(ends, dtype=torch.int32, device=dev), _err(dev)
+    got = {}
+    for chunked in (False, True):
+        s, o = state.clone(), torch.full((T, H * dv), 7.0, device=dev)
+        before = ops.launches()
+        ops.mlstm_scan(proj, gates, s, qs, slots, o, B, H, dk, dv, dk ** -0.5, err, max_q=max(lens),
+                       chunked=chunked)
+        assert ops.launches() - before == (5 if chunked else 1)      # (four on the tensor cores, and the walk)
+        assert int(err.item()) == (2 if bad else 0)
+        err.zero_()
+        got[chunked] = (o, s)
+    for b in range(B):
+        a, e, at = int(ends[b]), int(ends[b + 1]), int(slots[b])
+        if bad and b == 2:
+            assert bool((got[True][0][a:e] == 7.0).all())
+            continue
+        want = _mlstm_f64(proj[a:e], gates[a:e], state[at], H, dk, dv, dk ** -0.5)
+        off = []
+        for o, s in got.values():
+            g = s[at].double()
+            off.append([float((x - y).norm() / y.norm()) for x, y in zip(
+                (o[a:e].double().view(-1, H, dv), g[:, :dk * dv].reshape(H, dk, dv),
+                 g[:, dk * dv:dk * dv + dk], g[:, dk * dv + dk]), want)])
+        for walk, products in zip(*off):
+            assert products <= 1.5 * walk + 2e-7, (b, off)
+    assert torch.equal(got[True][1][B], state[B])
+
+
+# (sizes and offsets that the tensor cores take; a key size, a value size and rows that they do not)
+@pytest.mark.parametrize("dk,dv,off,kernels", [(64, 128, 0, 4), (256, 512, 8, 4), (96, 128, 0, 5), (64, 192, 0, 5),
+                                               (64, 128, 4, 5)])
+def test_mlstm_chunks_run_on_the_kernels_for_their_sizes(cuda_device, dk, dv, off, kernels):
+    """The kernels by name, as the profiler saw them, and their number, as the counter has it."""
+    from binfer_b200.csrc import ops
+    dev, T, H = cuda_device, 200, 2
+    proj = torch.randn(T, 2 * H * (dk + dv) + 8, device=dev).to(BF16)[:, off:off + 2 * H * (dk + dv)]
+    gates = torch.cat([torch.randn(T, H, device=dev), -torch.rand(T, H, device=dev)], 1).contiguous()
+    state = torch.zeros(1, H, ops.mlstm_state_size(dk, dv), device=dev)
+    qs, slots = torch.tensor([0, T], dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    out, before = torch.empty(T, H * dv, device=dev), ops.launches()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.mlstm_scan(proj, gates, state, qs, slots, out, 1, H, dk, dv, dk ** -0.5, _err(dev), max_q=T,
+                       chunked=True)
+        torch.cuda.synchronize()
+    assert ops.launches() - before == kernels
+    names = {n for e in prof.events() for n in ("mt_state", "mt_out", "cs_state", "cs_prefix", "cs_out")
+             if n + "_kernel" in e.name}
+    assert names == ({"mt_state", "mt_out"} if kernels == 4 else {"cs_state", "cs_prefix", "cs_out"}), names
+
+
 # small and large: states, weighted values, weighted products of q and k, and bfloat16 numbers themselves
 @pytest.mark.parametrize("what", ["values", "products", "keys", "queries", "large"])
 def test_mlstm_chunks_on_tensor_cores_hold_floats_of_every_size(cuda_device, what):
