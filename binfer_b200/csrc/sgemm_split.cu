@@ -164,12 +164,22 @@ __device__ __forceinline__ void sp_store_columns(uint32_t taddr, const float* t)
 // The plain sum, where that of the terms does not stand for it: in the order of sgemm_f32.cu, ascending
 // runs of 64 terms.  (Once NaN, always NaN.)
 __device__ __forceinline__ bool sp_finite(float v) { return fabsf(v) < INFINITY; }
+template <bool VEC>
 __device__ __noinline__ float sp_plain(const float* a, const float* w, int K) {
   float total = 0.f;
   for (int k0 = 0; k0 < K && total == total; k0 += 64) {
     float s = 0.f;
+    const int e = min(K, k0 + 64);
+    if (VEC) {
 #pragma unroll 8
-    for (int k = k0; k < min(K, k0 + 64); ++k) s = fmaf(a[k], w[k], s);
+      for (int k = k0; k < e; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s))));
+      }
+    } else {
+#pragma unroll 8
+      for (int k = k0; k < e; ++k) s = fmaf(a[k], w[k], s);
+    }
     total += s;
   }
   return total;
@@ -480,15 +490,18 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
   if (parts == 1) {
     const int f = f0 + quarter * 32 + lane;
     if (sums && f < p.N) {
+      unsigned long long lost = 0;
 #pragma unroll
       for (int i = 0; i < MINE; ++i) {
         const int t = group * MINE + i;
         if (m0 + t < p.M) {
-          float v = total[i] * (SPLIT_DOWN * SPLIT_DOWN);
-          if (!sp_finite(v))
-            v = sp_plain(A + (size_t)(m0 + t) * p.lda, W + (size_t)f * p.ldw, p.K);
-          C[(size_t)(m0 + t) * p.ldc + f] = v;
+          C[(size_t)(m0 + t) * p.ldc + f] = total[i] * (SPLIT_DOWN * SPLIT_DOWN);
+          if (!sp_finite(total[i])) lost |= 1ull << i;
         }
+      }
+      for (; lost; lost &= lost - 1) {
+        const int t = m0 + group * MINE + __ffsll(lost) - 1;
+        C[(size_t)t * p.ldc + f] = sp_plain<VEC>(A + (size_t)t * p.lda, W + (size_t)f * p.ldw, p.K);
       }
     }
   } else {
@@ -520,7 +533,7 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const SplitParams 
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             if (!sp_finite(*e[j]) && f + j < p.N)
-              *e[j] = sp_plain(A + (size_t)(m0 + t) * p.lda, W + (size_t)(f + j) * p.ldw, p.K);
+              *e[j] = sp_plain<VEC>(A + (size_t)(m0 + t) * p.lda, W + (size_t)(f + j) * p.ldw, p.K);
         }
         float* dst = C + (size_t)(m0 + t) * p.ldc + f;
         if (vec) {
