@@ -1982,11 +1982,11 @@ def _sgemm_split(a, w, out, M, N, K, batch, lda, ldw, ldc, batch_a, batch_w, bat
     err = error_word(a.device)
     for b, nb, m0, m in _sgemm_split_calls(M, K, batch):
         x, v, y = (a[m0:], w, out[m0:]) if a.dim() == 2 else (a[m0:, b:], w[b:], out[m0:, b:])
-        n = fn(_c_int(m), _c_int(N), _c_int(K), _c_int(nb), _c_int(0))
+        n = fn(_c_int(m), _c_int(N), _c_int(K), _c_int(nb), _c_int(batch), _c_int(0))
         scratch = torch.empty(n, dtype=torch.uint8, device=a.device) if n else None
         _run("sgemm_split", lib().bf_sgemm_split, _ptr(x), _ptr(v), _ptr(y), _c_int(m),
-             _c_int(N), _c_int(K), _c_ll(lda), _c_ll(ldw), _c_ll(ldc), _c_int(nb), _c_ll(batch_a),
-             _c_ll(batch_w), _c_ll(batch_c), _c_int(0), _ptr(scratch), _ptr(err), _stream())
+             _c_int(N), _c_int(K), _c_ll(lda), _c_ll(ldw), _c_ll(ldc), _c_int(nb), _c_int(batch),
+             _c_ll(batch_a), _c_ll(batch_w), _c_ll(batch_c), _c_int(0), _ptr(scratch), _ptr(err), _stream())
         _launches += n > 0           # two kernels: the rows' terms and the product
 
 

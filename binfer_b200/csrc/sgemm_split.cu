@@ -9,7 +9,7 @@
 // every dense product is a cuBLAS bf16 call with float accumulation
 // (cuda/kernels/gemm.cu:244-267).
 //
-// Every output is summed in an order that depends on N and K alone, whatever M, the tile or the
+// Every output is summed in an order that depends on N, K and the number of products alone, whatever M, the tile or the
 // alignment, so a token's result does not depend on which other tokens share the batch.
 //
 // A CTA computes 128 features x NT token rows over its share of K:
@@ -21,8 +21,8 @@
 //                as the tiles lie in shared memory (up to 16 rows: warps 0-7 do those too);
 //   warp 26      one thread fetches the features' floats (TMA) into a ring of its own.  (Rows off
 //                the 16-byte boundaries: warps 0-7 read them term by term.)
-// Weights of few features have too few tiles for the chip: the CTAs of a cluster (2 or 4, by N and
-// K alone) then share a tile along K and their sums are added in ascending order through
+// Weights of few features have too few tiles for the chip: the CTAs of a cluster (2 or 4, by N, K and the
+// number of products alone) then share a tile along K and their sums are added in ascending order through
 // distributed shared memory.
 //
 // Both operands are multiplied by 2^24 before they are taken apart, so that their terms hold floats of every
@@ -74,8 +74,11 @@ struct SplitParams {
   int* err;
 };
 
-int sp_parts(int N) {
-  const int tiles = (N + SP_F - 1) / SP_F;
+// of: the products side by side in the whole call (which may be cut into several).  From eight on their tiles
+// count together: 32 of 512 features and terms for one row took 38.9 us with a cluster of four a
+// tile, the multiply-adds 30.7.
+int sp_parts(int N, int of) {
+  const long long tiles = (long long)((N + SP_F - 1) / SP_F) * (of >= 8 ? of : 1);
   return tiles > 74 ? 1 : tiles > 18 ? 2 : 4;
 }
 
@@ -603,8 +606,8 @@ int sp_launch(const CUtensorMap& map, SplitParams p, int batch, uint8_t* scratch
 }
 
 // Token rows of a tile.
-int sp_tile(int M, int N, int batch) {
-  const long long cols = (long long)((N + SP_F - 1) / SP_F) * sp_parts(N) * batch;
+int sp_tile(int M, int N, int batch, int of) {
+  const long long cols = (long long)((N + SP_F - 1) / SP_F) * sp_parts(N, of) * batch;
   if (M <= SP_FEW) return SP_FEW;
   // a step of K took 0.74 us in tiles of 112 rows and 0.85 in tiles of 176 (one tile an SM)
   auto waves = [&](int n) { return (cols * ((M + n - 1) / n) + 147) / 148; };
@@ -614,25 +617,26 @@ int sp_tile(int M, int N, int batch) {
 }  // namespace
 
 // Bytes of scratch that bf_sgemm_split needs for these sizes (may be 0).
-BF_EXPORT long long bf_sgemm_split_scratch(int M, int N, int K, int batch, int nt) {
+BF_EXPORT long long bf_sgemm_split_scratch(int M, int N, int K, int batch, int of, int nt) {
   if (M <= SP_FEW) return 0;
-  if (!nt) nt = sp_tile(M, N, batch);
+  if (!nt) nt = sp_tile(M, N, batch, of);
   const long long rows = (long long)((M + nt - 1) / nt) * nt, steps = (K + SP_K - 1) / SP_K;
   return batch * steps * 3 * rows * 64;
 }
 
-// C[M, N] = A[M, K] * W[N, K]^T, `batch` of them (bf_sgemm_nt_batched's strides).  nt: token rows of
-// a tile (0: chosen here).  M up to 65,535 tiles.
+// C[M, N] = A[M, K] * W[N, K]^T, `batch` of them (bf_sgemm_nt_batched's strides), of `of` that the
+// caller has (the order of sums depends on those).  nt: token rows of a tile (0: chosen here).  M up to
+// 65,535 tiles.
 BF_EXPORT int bf_sgemm_split(const float* A, const float* W, float* C, int M, int N, int K,
-                             long long lda, long long ldw, long long ldc, int batch,
+                             long long lda, long long ldw, long long ldc, int batch, int of,
                              long long batch_a, long long batch_w, long long batch_c, int nt,
                              void* scratch, int* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
-  if (!nt) nt = sp_tile(M, N, batch);
+  if (!nt) nt = sp_tile(M, N, batch, of);
   if (K <= 0 || batch > 65535 || (M + nt - 1) / nt > 65535 || ((uintptr_t)scratch & 15) ||
       (nt > SP_FEW && !scratch))
     return (int)cudaErrorInvalidValue;
-  SplitParams p = {A, W, C, nullptr, 0, M, N, K, K < 512 ? 1 : sp_parts(N), 0, 0, lda, ldw, ldc,
+  SplitParams p = {A, W, C, nullptr, 0, M, N, K, K < 512 ? 1 : sp_parts(N, of), 0, 0, lda, ldw, ldc,
                    batch_a, batch_w, batch_c, err};
   CUtensorMap map = {};
   bool vec = ((K | lda | ldw | batch_a | batch_w) & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 &&

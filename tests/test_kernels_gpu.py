@@ -174,7 +174,7 @@ def test_sgemm_of_terms(cuda_device, M, N, K):
     assert int(ops.error_word(cuda_device).item()) == 0
 
 
-@pytest.mark.parametrize("M,N,K,batch", [(1241, 130, 1024, 1), (300, 40, 600, 5), (40, 8, 2048, 7)])
+@pytest.mark.parametrize("M,N,K,batch", [(1241, 130, 1024, 1), (300, 40, 600, 5), (40, 8, 2048, 7), (30, 300, 512, 9)])
 def test_sgemm_of_terms_in_several_calls(cuda_device, monkeypatch, M, N, K, batch):
     """A product whose rows' terms pass the limit, cut by rows and by products: the same bits."""
     from binfer_b200.csrc import ops
@@ -193,6 +193,24 @@ def test_sgemm_of_terms_in_several_calls(cuda_device, monkeypatch, M, N, K, batc
         assert ops.launches() - before == sum(1 + (m > 16) for _, _, _, m in calls)
     assert len(calls) > 1
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+# products side by side: each cluster size, tiles of 16 and of more rows
+@pytest.mark.parametrize("batch,N,K", [(16, 128, 512), (9, 300, 520), (40, 512, 544)])
+def test_sgemm_of_terms_many_products(cuda_device, batch, N, K):
+    """Against float64 with test_sgemm_of_terms' bound; a row's bits alone and in company."""
+    from binfer_b200.csrc import ops
+    a = torch.randn(130, batch, K, device=cuda_device)
+    w = torch.randn(batch, N, K, device=cuda_device)
+    outs = []
+    for M in (130, 16, 1):
+        outs.append(torch.full((M, batch, N), 7.0, device=cuda_device))
+        ops.sgemm_nt_batched(a[:M], w, outs[-1])
+    ref, size = (torch.einsum("mbk,bnk->mbn", x, y) for x, y in (
+        (a.double(), w.double()), (a.double().abs(), w.double().abs())))
+    bound = (12 * 2 + 8 + K / 256 + 4 + 1) * 2.0 ** -24 * size
+    assert bool(((outs[0].double() - ref).abs() <= bound).all())
+    assert torch.equal(outs[1], outs[0][:16]) and torch.equal(outs[2], outs[0][:1])
 
 
 # tiles of 16, 176 and 112 rows, features shared by clusters of 4 and 2 CTAs and not

@@ -18,7 +18,7 @@ def test_scratch_of_a_call_stays_within_its_limit(K, batch):
             assert not rows & seen and nb > 0 and b + nb <= batch and m0 + m <= M
             seen |= rows
             for N in (8, 4096, 151936):
-                n = scratch(m, N, K, nb, 0)
+                n = scratch(m, N, K, nb, batch, 0)
                 assert n <= ops.SGEMM_SPLIT_MAX_BYTES or (nb == 1 and m <= 112), (M, m, nb, n)
         starts = {m0: m for _, _, m0, m in ops._sgemm_split_calls(M, K, batch)}
         assert sum(starts.values()) == M and len(seen) == batch * len(starts)
