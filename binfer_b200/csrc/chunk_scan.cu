@@ -1185,7 +1185,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
                      const float* tok_decay, const float* gates, float* state,
                      long long slot_stride, int state_size, const int* q_start,
                      const int* state_slots, int n_slots, float* o_raw, char* scratch, int* err,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, bool tensor = false) {
   const CsLayout l = cs_layout(p.T, p.B, p.H, p.QH, p.dk, p.dv, p.C, MLSTM, p.n_min);
   double* G = (double*)(scratch + l.G);
   double* Hs = (double*)(scratch + l.Hs);
@@ -1202,7 +1202,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles), 128, 0, stream>>>(qk, p, q_start,
                                                                                  qkm, nullptr);
   if constexpr (MLSTM) {
-    if (mt_takes(p, qk, l.chunks))
+    if (tensor)
       return mt_launch(qk, p, l.chunks, q_start, state, slot_stride, state_size, state_slots, n_slots, G, Hs, g0,
                        Wl, E, qkm, U, Un, o_raw, err, stream);
   }
@@ -1242,12 +1242,13 @@ BF_EXPORT int bf_chunk_scan_linear(const float* qk, const float* vf, const float
                                         (char*)scratch, err, stream);
 }
 
-// proj rows [q: H dk | k: H dk | v: H dv | ...] in bfloat16, gates and state as in bf_mlstm_scan.
+// proj rows [q: H dk | k: H dk | v: H dv | ...] in bfloat16, gates and state as in bf_mlstm_scan; max_q and
+// min_ctas: mlstm_tensor.cuh, mt_takes.
 BF_EXPORT int bf_chunk_scan_mlstm(const void* proj, long long stride, const float* gates,
                                   float* state, long long slot_stride, int state_size,
                                   const int* q_start, const int* state_slots, int n_slots,
                                   float* o_raw, void* scratch, int T, int B, int H, int dk, int dv,
-                                  float q_scale, int C, int n_min, int* err,
+                                  float q_scale, int C, int n_min, int max_q, int min_ctas, int* err,
                                   cudaStream_t stream) {
   CsIn p = {0, (long long)H * dk, 2LL * H * dk, stride, stride, H, H, dk, dv, C, T, B, n_min,
             q_scale};
@@ -1257,14 +1258,15 @@ BF_EXPORT int bf_chunk_scan_mlstm(const void* proj, long long stride, const floa
   const __nv_bfloat16* x = (const __nv_bfloat16*)proj;
   return cs_launch<__nv_bfloat16, __nv_bfloat16, true>(
       x, x, p, nullptr, nullptr, gates, state, slot_stride, state_size, q_start, state_slots,
-      n_slots, o_raw, (char*)scratch, err, stream);
+      n_slots, o_raw, (char*)scratch, err, stream,
+      mt_takes(p, proj, cs_most_chunks(T, B, C, n_min), max_q, min_ctas));
 }
 
 // How many kernels bf_chunk_scan_mlstm launches: four on the tensor cores, five of multiply-adds.
 BF_EXPORT int bf_chunk_scan_mlstm_kernels(const void* proj, long long stride, int T, int B, int H, int dk,
-                                          int dv, int C, int n_min) {
+                                          int dv, int C, int n_min, int max_q, int min_ctas) {
   const CsIn p = {0, (long long)H * dk, 2LL * H * dk, stride, stride, H, H, dk, dv, C, T, B, n_min, 1.f};
-  return mt_takes(p, proj, cs_most_chunks(T, B, C, n_min)) ? 4 : 5;
+  return mt_takes(p, proj, cs_most_chunks(T, B, C, n_min), max_q, min_ctas) ? 4 : 5;
 }
 
 // The gated delta rule.  Scratch: F (G and H are the same array), g0, Wl | qkm | kkm | W | Y |

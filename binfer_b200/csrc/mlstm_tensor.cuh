@@ -819,9 +819,18 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
   mt_end(sh, tmem, err);
 }
 
-// Chunks of 64 (tokens), keys in whole steps, values in whole tiles, rows on 16-byte boundaries.
-static bool mt_takes(const CsIn& p, const void* proj, int chunks) {
-  return (long long)chunks * p.H * (p.dv / MT_M) < 0x7fffffff && p.C == MT_C && p.dk % MT_C == 0 && p.dk <= MT_WORK && p.dv % MT_M == 0 && p.qk_stride % 8 == 0 &&
+// Chunks of 64 (tokens), keys in whole steps, values in whole tiles, rows on 16-byte boundaries.  And CTAs
+// for the chip: mt_state goes from chunk to chunk with one for 64 x 128 elements of a state, where cs_state
+// has one for every chunk, too.  On the tensor cores / multiply-adds, 2,048 tokens: 48 CTAs 175 / 194 and
+// 185 / 202 us, 32 CTAs 161 / 149, 165 / 153 and 192 / 200, 16 CTAs 149 / 116 and 157 / 122, one 124 / 67;
+// 8,192 tokens, 48: 576 / 650, 16: 470 / 302.  Up to five chunks the former are no slower whatever the CTAs
+// (200 tokens: 52 to 77 us against 52 to 89).  `min_ctas`: 40.  max_q: the step's longest portion (0: not
+// known); requests of up to n_min tokens have no chunks.
+static bool mt_takes(const CsIn& p, const void* proj, int chunks, int max_q, int min_ctas) {
+  const int longs = max_q > 0 ? 1 + (p.T > max_q ? p.T - max_q : 0) / (p.n_min + 1) : p.T / (p.n_min + 1);
+  const long long ctas = (long long)(p.dk / MT_C) * (p.dv / MT_M) * p.H * (p.B < longs ? p.B : longs);
+  return (ctas >= min_ctas || chunks <= 5) &&
+         (long long)chunks * p.H * (p.dv / MT_M) < 0x7fffffff && p.C == MT_C && p.dk % MT_C == 0 && p.dk <= MT_WORK && p.dv % MT_M == 0 && p.qk_stride % 8 == 0 &&
          p.q_off % 8 == 0 && p.k_off % 8 == 0 && p.v_off % 8 == 0 && ((uintptr_t)proj & 15) == 0;
 }
 static int mt_launch(const mt_bf16* proj, const CsIn& p, int chunks, const int* q_start, float* state,

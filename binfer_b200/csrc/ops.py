@@ -1457,6 +1457,9 @@ def mlstm_gates(h: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
 
 
 MLSTM_MAX_QK_DIM = 256
+# Chunks on the tensor cores: CTAs of a state's 64 x 128 elements, over heads and requests, from which
+# (mlstm_tensor.cuh, mt_takes: 32 and 48 measured on either side)
+MLSTM_TENSOR_MIN_CTAS = 40
 
 
 def mlstm_state_size(dk: int, dv: int) -> int:
@@ -1490,11 +1493,13 @@ def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
              _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]), _ptr(o_raw),
              _ptr(scratch), _c_int(T), _c_int(B), _c_int(heads), _c_int(dk), _c_int(dv),
              _c_float(q_scale), _c_int(CHUNK_SCAN_TOKENS),
-             _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _ptr(err), _stream())
+             _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _c_int(max_q), _c_int(MLSTM_TENSOR_MIN_CTAS),
+             _ptr(err), _stream())
         global _launches
         _launches += lib().bf_chunk_scan_mlstm_kernels(
             _ptr(proj), _c_ll(proj.stride(0)), _c_int(T), _c_int(B), _c_int(heads), _c_int(dk),
-            _c_int(dv), _c_int(CHUNK_SCAN_TOKENS), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN))) - 1
+            _c_int(dv), _c_int(CHUNK_SCAN_TOKENS), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)),
+            _c_int(max_q), _c_int(MLSTM_TENSOR_MIN_CTAS)) - 1
         if _walk_limit(scratch, B, CHUNK_SCAN_MIN) < 0:
             return
     _run("mlstm_scan", lib().bf_mlstm_scan, _ptr(proj), _c_ll(proj.stride(0)), _ptr(gates),

@@ -1556,6 +1556,7 @@ def test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv):
                                           ([193, 320], 3, 128, 384), ([170, 3, 449], 2, 192, 256)])
 def test_mlstm_chunks_on_tensor_cores(cuda_device, monkeypatch, lens, H, dk, dv):
     from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "MLSTM_TENSOR_MIN_CTAS", 0)
     test_mlstm_scan_in_chunks(cuda_device, lens, H, dk, dv)
     # rows off the 16-byte boundaries take the multiply-adds: the same but for the order of sums
     dev, T, B = cuda_device, sum(lens), len(lens)
@@ -1586,10 +1587,11 @@ def test_mlstm_chunks_on_tensor_cores(cuda_device, monkeypatch, lens, H, dk, dv)
 @pytest.mark.parametrize("what", ["q", "k", "v"])
 @pytest.mark.parametrize("at", [64, 140, 255])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-def test_mlstm_chunks_on_tensor_cores_keep_infinities_apart(cuda_device, what, at, bad):
+def test_mlstm_chunks_on_tensor_cores_keep_infinities_apart(cuda_device, monkeypatch, what, at, bad):
     """What is not a number shows where the multiply-adds show it, and nowhere else changes a bit of the
     tokens before it and of the other head."""
     from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "MLSTM_TENSOR_MIN_CTAS", 0)
     dev, T, H, dk, dv = cuda_device, 300, 2, 128, 256
     torch.manual_seed(6)
     proj = torch.randn(T, 2 * H * (dk + dv), device=dev).to(BF16)
@@ -1678,23 +1680,28 @@ def test_mlstm_chunks_on_tensor_cores_tile_after_tile(cuda_device, dk, dv, H, ba
     assert torch.equal(got[True][1][B], state[B])
 
 
-# (sizes and offsets that the tensor cores take; a key size, a value size and rows that they do not)
-@pytest.mark.parametrize("dk,dv,off,kernels", [(64, 128, 0, 4), (256, 512, 8, 4), (96, 128, 0, 5), (64, 192, 0, 5),
-                                               (64, 128, 4, 5)])
-def test_mlstm_chunks_run_on_the_kernels_for_their_sizes(cuda_device, dk, dv, off, kernels):
+# sizes and offsets that the tensor cores take; a key size, a value size and rows that they do not; few chunks
+# of few heads and many; heads for the chip; single tokens beside a portion, which have no chunks
+@pytest.mark.parametrize("T,H,dk,dv,off,singles,kernels", [
+    (200, 2, 64, 128, 0, 0, 4), (200, 2, 256, 512, 8, 0, 4), (200, 2, 96, 128, 0, 0, 5), (200, 2, 64, 192, 0, 0, 5),
+    (200, 2, 64, 128, 4, 0, 5), (319, 1, 64, 128, 0, 0, 4), (320, 39, 64, 128, 0, 0, 5), (320, 40, 64, 128, 0, 0, 4),
+    (2000, 2, 256, 512, 0, 0, 5), (700, 3, 256, 512, 0, 0, 4), (700, 8, 128, 256, 0, 9, 5), (700, 8, 128, 256, 0, 0, 5)])
+def test_mlstm_chunks_run_on_the_kernels_for_their_sizes(cuda_device, T, H, dk, dv, off, singles, kernels):
     """The kernels by name, as the profiler saw them, and their number, as the counter has it."""
     from binfer_b200.csrc import ops
-    dev, T, H = cuda_device, 200, 2
+    dev, B, n = cuda_device, 1 + singles, T
+    T = T + singles
     proj = torch.randn(T, 2 * H * (dk + dv) + 8, device=dev).to(BF16)[:, off:off + 2 * H * (dk + dv)]
     gates = torch.cat([torch.randn(T, H, device=dev), -torch.rand(T, H, device=dev)], 1).contiguous()
-    state = torch.zeros(1, H, ops.mlstm_state_size(dk, dv), device=dev)
-    qs, slots = torch.tensor([0, T], dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    state = torch.zeros(B, H, ops.mlstm_state_size(dk, dv), device=dev)
+    qs = torch.tensor([0] + list(range(n, T + 1)), dtype=torch.int32, device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev)
     out, before = torch.empty(T, H * dv, device=dev), ops.launches()
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        ops.mlstm_scan(proj, gates, state, qs, slots, out, 1, H, dk, dv, dk ** -0.5, _err(dev), max_q=T,
+        ops.mlstm_scan(proj, gates, state, qs, slots, out, B, H, dk, dv, dk ** -0.5, _err(dev), max_q=n,
                        chunked=True)
         torch.cuda.synchronize()
-    assert ops.launches() - before == kernels
+    assert ops.launches() - before == kernels + (B > 1)           # (the walk serves the single tokens)
     names = {n for e in prof.events() for n in ("mt_state", "mt_out", "cs_state", "cs_prefix", "cs_out")
              if n + "_kernel" in e.name}
     assert names == ({"mt_state", "mt_out"} if kernels == 4 else {"cs_state", "cs_prefix", "cs_out"}), names
@@ -1702,11 +1709,12 @@ def test_mlstm_chunks_run_on_the_kernels_for_their_sizes(cuda_device, dk, dv, of
 
 # small and large: states, weighted values, weighted products of q and k, and bfloat16 numbers themselves
 @pytest.mark.parametrize("what", ["values", "products", "keys", "queries", "large"])
-def test_mlstm_chunks_on_tensor_cores_hold_floats_of_every_size(cuda_device, what):
+def test_mlstm_chunks_on_tensor_cores_hold_floats_of_every_size(cuda_device, monkeypatch, what):
     """Nothing that multiply-adds over chunks hold is lost in terms: relative errors against float64, no
     further off.  (The walk is no measure: of keys or queries of 1e-39 its q . k are there in as many
     bits as they are multiplied, over chunks in those that a float of that size has.)"""
     from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "MLSTM_TENSOR_MIN_CTAS", 0)
     dev, T, H, dk, dv = cuda_device, 333, 2, 128, 256
     torch.manual_seed(9)
     size = {"values": (1, 1, 1e-35), "products": (1e-18, 1e-17, 1), "keys": (1, 1e-39, 1e28),
@@ -1736,9 +1744,10 @@ def test_mlstm_chunks_on_tensor_cores_hold_floats_of_every_size(cuda_device, wha
 
 @pytest.mark.parametrize("at", [64, 140, 255])
 @pytest.mark.parametrize("what", ["state", "q.k", "output", "faded"])
-def test_mlstm_chunks_on_tensor_cores_with_products_that_overflow(cuda_device, at, what):
+def test_mlstm_chunks_on_tensor_cores_with_products_that_overflow(cuda_device, monkeypatch, at, what):
     """Finite operands whose products leave float's range: the infinities and NaN of the multiply-adds."""
     from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "MLSTM_TENSOR_MIN_CTAS", 0)
     dev, T, H, dk, dv = cuda_device, 300, 2, 128, 256
     torch.manual_seed(6)
     wide = torch.randn(T, 2 * H * (dk + dv) + 4, device=dev).to(BF16)
