@@ -1959,8 +1959,10 @@ def diff_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
 # The float32 product: terms of K from which it runs on the tensor cores with its operands in three
 # bfloat16 terms (sgemm_split.cu), below them as plain multiply-adds (sgemm_f32.cu).  By K alone, so
 # that a row's sums do not depend on the rows beside it.  Measured, 1 to 2,048 rows and 8 to 12,288
-# outputs: with 512 terms faster at every size (1.0 to 3.6 times; 13.9 against 8.1 us for one row
-# and 1,024 outputs), with 256 slower for few rows or outputs (7.6 against 9.0 us).
+# outputs, 1 to 128 products side by side: with 512 terms faster at every size (1.1 to 4.1 times; 13.9
+# against 8.1 us for one row and 1,024 outputs), with 256 slower for few rows or outputs (7.6 against 9.0 us).
+# (Slower: up to 16 rows of 151,936 outputs and 1,025 terms, rows off the 16-byte boundaries: 356 to 377
+# against 336 to 356 us; on them 1.3 times as fast.)
 SGEMM_SPLIT_MIN_K = 512
 SGEMM_SPLIT_MAX_BYTES = 256 << 20     # scratch of a call; more rows or products go in several
 
@@ -1969,11 +1971,14 @@ def _sgemm_split_calls(M: int, K: int, batch: int):
     """``(first product, products, first row, rows)`` of the calls that a product takes: as few as keep
     the rows' terms (six bytes an element, in whole tiles of 112 or 176 rows) within
     ``SGEMM_SPLIT_MAX_BYTES``, or a tile a call where one takes more."""
+    row = 192 * -(-K // 32)
+    # (sixteen rows need no scratch; whole tiles are at most 175 rows more)
+    if M <= 16 or batch * (M + 175) * row <= SGEMM_SPLIT_MAX_BYTES:
+        return [(0, batch, 0, M)]
+
     def padded(m):
         return max(-(-m // 112) * 112, -(-m // 176) * 176)
-    if M <= 16:                                              # (these rows need no scratch)
-        return [(0, batch, 0, M)]
-    most = SGEMM_SPLIT_MAX_BYTES // (192 * -(-K // 32))      # rows of a call
+    most = SGEMM_SPLIT_MAX_BYTES // row                      # rows of a call
     rows = M if padded(M) <= most else max(most // 1232 * 1232, 112)     # (1,232: whole tiles of both)
     products = max(1, min(batch, most // padded(rows)))
     return [(b, min(products, batch - b), m, min(rows, M - m))
