@@ -8,7 +8,7 @@
 //   warp 8      TMA producer: the Q tile once; per key tile one cp.async.bulk.tensor copy
 //               per (page, 64 columns) of K and of V into 128-byte-swizzled shared memory,
 //               two key tiles in flight;
-//   warp 9      one thread issues tcgen05.mma: S = Q K^T (M = 128 queries, N = 64 keys,
+//   warp 9      issues tcgen05.mma (one elected lane): S = Q K^T (M = 128 queries, N = 64 keys,
 //               K = head size) into one of two S buffers in tensor memory, and, once the
 //               probabilities are written, O += P V (M = 128, N = head size, K = 64 keys;
 //               V is read as stored, an MN-major operand).  O stays in tensor memory over

@@ -332,10 +332,9 @@ prefill_attention_umma2_kernel(const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp >= A2_MMA_WARP) {
     // ----------------------------------------------------------------- MMA issuers
-    // One warp per query tile, converged, one elected lane issuing: out of a branch of one lane a
-    // tcgen05.mma cost 55 to 100 cycles whatever its size (operands moved into uniform registers
-    // one lane at a time).  The two warps' products touch disjoint tensor memory; they share the
-    // K and V tiles, which are released when both have arrived.
+    // One warp per query tile, converged, one elected lane issuing (umma_utils.cuh).  The two warps'
+    // products touch disjoint tensor memory; they share the K and V tiles, which are released when
+    // both have arrived.
     const int grp = warp - A2_MMA_WARP;
     const int my_tiles = grp == 0 ? tiles_a : (active_b ? tiles : 0);
     {

@@ -11,7 +11,8 @@
 // mLSTM m_t = F_t - G_t.  F, G and H are double, so a difference of two of them is good to a
 // float's last bit; its exponential is a float and what is left of it (cs_exp), the products of q and k
 // (and of k and k) inside a chunk are summed in double and rounded once, every other product is float
-// (FP32 multiply-adds, no tensor-core mode), every sum of one order.  Per chunk of `C` tokens and head:
+// (FP32 multiply-adds; the mLSTM's on the tensor cores where mlstm_tensor.cuh takes its sizes: exact
+// products of bfloat16 terms, added in float), every sum of one order.  Per chunk of `C` tokens and head:
 //
 //   cs_gates   F, G, H of every token, its weight behind its chunk; one block per (head, request)
 //   cs_qk      Q K^T of a chunk, once per q/k head (several heads may share them), in double
@@ -26,7 +27,7 @@
 //
 // GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads 208 / 467 us (cs_out 99,
 // cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8); 8 heads of 128 x 256 124 / 270; mLSTM, 8 heads of 256 x
-// 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 208).  What bounds them: cs_state and cs_out shared-memory reads (the
+// 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them: cs_state and cs_out shared-memory reads (the
 // pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
 // expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
 // further from 64 bits than the walk where decays are fast.

@@ -9,7 +9,7 @@
 //               up to 128 token rows x 64 K and one of BN feature rows x 64 K (128-byte
 //               swizzle) into a ring of shared-memory stages, completion on an
 //               mbarrier per stage;
-//   warp 1      one thread issues tcgen05.mma (M = 128, N = BN, K = 16, four per stage)
+//   warp 1      issues tcgen05.mma (one elected lane; M = 128, N = BN, K = 16, four per stage)
 //               with the accumulator in tensor memory; tcgen05.commit hands the stage
 //               back to the producer.  The warp also owns the TMEM allocation: two
 //               accumulators, so the epilogue of one tile overlaps the products of the

@@ -294,9 +294,8 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_x,
     }
   } else if (warp == 1 || warp == 3) {
     // Two issuing warps, an accumulator each (summed by the epilogue in a fixed order).  Each is
-    // converged with one elected lane issuing: out of a branch of one lane a tcgen05.mma cost 55 to
-    // 100 cycles whatever its size (four layers of width 4,096 at one row: 560 -> 546 us).  One
-    // issuing warp is slower still: 558 us.
+    // converged with one elected lane issuing: four layers of width 4,096 at one row took 560 us with
+    // the products issued from a branch of one lane, 546 so, and 558 with one such warp.
     // A ring slot belongs to one issuer for good (slot s to issuer s % 2), so that the thread
     // waits for every fill of its slots in turn.  An mbarrier's phase is one bit: with the K
     // steps dealt out in turn and an odd number of slots, a thread met only every second fill

@@ -16,7 +16,7 @@
 //   warp 0      TMA producer in both CTAs: its own token rows and its own half of the
 //               feature rows, completion on the LEADER's (cluster rank 0) mbarrier of the
 //               stage (cp.async.bulk.tensor ... .cta_group::2), which expects both CTAs' bytes;
-//   warp 1      in the leader one thread issues the products and commits with
+//   warp 1      in the leader issues the products (one elected lane) and commits with
 //               .multicast::cluster to both CTAs' barriers (stage free; accumulator complete);
 //               in both CTAs the warp owns the tensor-memory allocation (two accumulators);
 //   warps 2-5   epilogue in both CTAs: tcgen05.ld of the own 128 rows, conversion (or the

@@ -20,7 +20,7 @@
 // results that they reach are computed by multiply-adds; so are sums that are not finite (where finite
 // operands' product leaves float's range, that of a smaller term may overflow with a sign of its own).
 //
-// 2,048 tokens, 8 heads of 256 x 512: mt_state 72 us (cs_state and cs_prefix 177), mt_out 92 (cs_out 168).
+// 2,048 tokens, 8 heads of 256 x 512: mt_state 73 us (cs_state and cs_prefix 177), mt_out 95 (cs_out 168).
 // What bounds them: mt_state the issue slots (a chunk's keys and values to take apart, its sums, its states
 // to store: some 4,000 cycles for 600 of products), mt_out the same (a step 2,500 cycles) and the start
 // and the end of a tile (4,000).  Relative errors against 64 bits, this / those, at 2,048 tokens (four inputs):

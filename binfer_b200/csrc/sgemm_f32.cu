@@ -1,7 +1,8 @@
 // True 32-bit matrix product for the float32 engine: C[M,N] = A[M,K] * W[N,K]^T, for sums of
-// fewer than 512 terms (longer ones: sgemm_split.cu).
+// fewer than 512 terms (longer ones: sgemm_split.cu), and for sums of any length where the float32 engine
+// checks the tensor cores' paths and should share nothing with them (ops.sgemm_nt, multiply_adds).
 //
-// Plain FP32 FMAs on the CUDA cores.
+// Plain FP32 FMAs on the CUDA cores; no tensor-core mode of any kind.
 // The reference has no 32-bit product at all: every dense product is a cuBLAS
 // bf16 call with float accumulation (cuda/kernels/gemm.cu:244-267); the operand
 // layout here is the same (weights as stored, [out, in] row-major).

@@ -36,12 +36,13 @@
 // operands (a step of 32 terms in 0.74 us for 112 token rows, 0.85 for 176; the products alone 0.36
 // and 0.56), and waves of tiles that do not fill the chip.  In us against plain multiply-adds:
 //   rows x outputs x terms       1      333             2,048
-//   4,096 x 2,048        50 -> 26   186 ->  37     798 -> 201
-//   2,048 x 2,048        49 -> 16   133 ->  25     409 -> 134
-//   12,288 x 2,048       83 -> 45   460 -> 109   2,331 -> 552
-// (2,048 rows: 1,120 TFLOP/s of bfloat16 products.)  Relative error against 64 bits over random
+//   4,096 x 2,048        49 -> 24   186 ->  36     797 -> 200
+//   2,048 x 2,048        49 -> 15   133 ->  24     409 -> 130
+//   12,288 x 2,048       84 -> 43   460 -> 111   2,331 -> 602
+// (2,048 rows: 1,030 TFLOP/s of bfloat16 products, at the power limit.)  Without the operands' scaling the last
+// line's 333 rows take 109.  Relative error against 64 bits over random
 // operands: 0.94e-7 at 2,048 terms and 1.03e-7 at 6,144 (multiply-adds in runs of 64: 1.8e-7, 2.3e-7);
-// positive ones: 0.63e-7 (0.82e-7).  On the way here: features' floats into registers instead of by
+// positive ones: 0.68e-7 and 0.63e-7 (0.82e-7).  On the way here: features' floats into registers instead of by
 // TMA 152 us for the third line's 333 rows, products issued from a branch of one lane 122.
 #include <cuda.h>
 

@@ -99,10 +99,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   const bool ok = mbar_wait(bar, parity, abort);
   return __all_sync(0xffffffffu, ok);
 }
-// tcgen05.mma and tcgen05.commit by one lane of a CONVERGED warp.  All lanes compute the operands, so that
-// these stay in uniform registers; from a branch of one lane each product first has to move its six operands
-// there, some 55 to 100 cycles a product, which held every kernel whose products are small (a 32-bit
-// product of 333 rows 122 -> 107 us, decode products and attention: see there).
+// tcgen05.mma and tcgen05.commit by one lane of a CONVERGED warp, all lanes with the same operands.  Out
+// of a branch of one lane every kernel whose products are small was slower: a 32-bit product of 333 rows
+// took 122 us and takes 107 so, four decode layers of width 4,096 560 and 546.  Why was not measured.
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc,
                                           uint32_t idesc, uint32_t accumulate) {
   asm volatile(
