@@ -11,8 +11,8 @@
 // mLSTM m_t = F_t - G_t.  F, G and H are double, so a difference of two of them is good to a
 // float's last bit; its exponential is a float and what is left of it (cs_exp), the products of q and k
 // (and of k and k) inside a chunk are summed in double and rounded once, every other product is float
-// (FP32 multiply-adds; the mLSTM's on the tensor cores where mlstm_tensor.cuh takes its sizes: exact
-// products of bfloat16 terms, added in float), every sum of one order.  Per chunk of `C` tokens and head:
+// (FP32 multiply-adds; on the tensor cores where those files take the sizes: exact products of bfloat16 terms, added
+// in float), every sum of one order.  Per chunk of `C` tokens and head:
 //
 //   cs_gates   F, G, H of every token, its weight behind its chunk; one block per (head, request)
 //   cs_qk      Q K^T of a chunk, once per q/k head (several heads may share them), in double
@@ -23,10 +23,11 @@
 //              C terms, the weights applied as its operands are stored into shared memory
 //
 // The mLSTM with keys in whole steps of 64 and values in whole tiles of 128 runs its products on the tensor
-// cores (mlstm_tensor.cuh: the last three kernels become two).
+// cores (mlstm_tensor.cuh: the last three kernels become two), and so do the linear scan with keys in whole steps of
+// 128, values of 64 or whole tiles of 128 and CTAs enough, and the delta rule's cs_out (chunk_tensor.cuh).
 //
-// GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads 208 / 467 us (cs_out 99,
-// cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8); 8 heads of 128 x 256 124 / 270; mLSTM, 8 heads of 256 x
+// GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads by multiply-adds 208 / 467 us (cs_out
+// 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 138; 8 heads of 128 x 256 124 / 270 (83); mLSTM, 8 heads of 256 x
 // 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them: cs_state and cs_out shared-memory reads (the
 // pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
 // expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
@@ -66,6 +67,7 @@
 // depends on where a step's portions begin, so the float32 engine, whose results must not depend
 // on the cut, does not use these kernels.
 #include "common.cuh"
+#include "split_utils.cuh"
 
 #define CS_THREADS 128
 #define CS_T 64            // tile edge
@@ -418,20 +420,78 @@ __device__ __forceinline__ void cs_dmma(double (&c)[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
+// q and k in three bfloat16 terms on the way, for the products on the tensor cores (chunk_tensor.cuh; chunks of 64,
+// sizes in whole steps of 64): X[chunk][qh][dk / 64] tiles of three terms of 64 tokens x 64 sizes, a token's sizes
+// in a row of 128 bytes with the 128-byte swizzle, rows beyond the chunk's tokens zero.  Numbers without terms
+// (split_utils.cuh) are zero; odd[chunk][qh][q | k]: a bit for every token that has one.
+struct CsTerms {
+  uint8_t *q, *k;              // (null: not asked for)
+  unsigned long long* odd;
+};
+#define CS_TERMS_TERM (64 * 128)
+#define CS_TERMS_TILE (3 * CS_TERMS_TERM)
+// the first float that has none, times 2^24, as bits
+constexpr uint32_t CS_NO_TERMS_UP = 0x7f7f8000u - (24u << 23);
+// Two blocks beside those of a chunk and head's products, which the double tensor pipe bounds, where these are
+// bound by memory: q's terms (what 0) and k's.
+template <int THREADS>
+__device__ __forceinline__ void cs_terms(const float* __restrict__ qk, const CsIn& p, const CsChunk& c, int what,
+                                         const CsTerms& out) {
+  __shared__ unsigned long long odd;
+  if (threadIdx.x == 0) odd = 0ull;
+  __syncthreads();
+  const int at = c.index * 64, n = min(64, c.n - at), pieces = p.dk / 8;
+  const float* rows = qk + (size_t)(c.t0 + at) * p.qk_stride + (what ? p.k_off : p.q_off) + (size_t)blockIdx.y * p.dk;
+  const size_t head = (size_t)blockIdx.x * p.QH + blockIdx.y;
+  uint8_t* X = (what ? out.k : out.q) + head * (p.dk / 64) * CS_TERMS_TILE;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < 64 * pieces; i += THREADS) {
+    const int t = i / pieces, pc = i % pieces;
+    float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (t < n) {
+      const float4 a = *reinterpret_cast<const float4*>(rows + (size_t)t * p.qk_stride + 8 * pc);
+      const float4 b = *reinterpret_cast<const float4*>(rows + (size_t)t * p.qk_stride + 8 * pc + 4);
+      x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    }
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if ((__float_as_uint(x[j]) & 0x7fffffffu) >= CS_NO_TERMS_UP) {
+        bad = true;
+        x[j] = 0.f;
+      }
+    if (bad) atomicOr(&odd, 1ull << t);
+    uint4 hi, mid, lo;
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) split_up(x[j], x[j + 1]);
+    split3(x[0], x[1], hi.x, mid.x, lo.x);
+    split3(x[2], x[3], hi.y, mid.y, lo.y);
+    split3(x[4], x[5], hi.z, mid.z, lo.z);
+    split3(x[6], x[7], hi.w, mid.w, lo.w);
+    uint8_t* to = X + (size_t)(pc >> 3) * CS_TERMS_TILE + t * 128 + (((pc & 7) ^ (t & 7)) << 4);
+    *reinterpret_cast<uint4*>(to) = hi;
+    *reinterpret_cast<uint4*>(to + CS_TERMS_TERM) = mid;
+    *reinterpret_cast<uint4*>(to + 2 * CS_TERMS_TERM) = lo;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) out.odd[head * 2 + what] = odd;
+}
+
 template <typename A, bool KK>
 __global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
     const A* __restrict__ qk, CsIn p, const int* __restrict__ q_start, float* __restrict__ qkm,
-    float* __restrict__ kkm) {
+    float* __restrict__ kkm, CsTerms x_out) {
   constexpr int THREADS = KK ? 256 : 128, PIECES = 128 * (CS_QS / 4) / THREADS;
   __shared__ __align__(16) double rows_s[128][CS_QP];      // 64 rows of q, 64 of k
   const int tiles = p.C / CS_T;
   const int rt = blockIdx.z / tiles, ct = blockIdx.z % tiles;
-  if (ct > rt) return;
   const CsChunk c = cs_find(q_start, p.B, p.C, p.n_min, blockIdx.x, -1);
-  if (c.b < 0) return;
   const int at = c.index * p.C;                  // the chunk's first token inside the request
   const int n = min(p.C, c.n - at);
-  if (rt * CS_T >= n) return;
+  if constexpr (sizeof(A) == 4) {
+    if (rt >= tiles && c.b >= 0) cs_terms<THREADS>(qk, p, c, blockIdx.z - tiles * tiles, x_out);
+  }
+  if (ct > rt || c.b < 0 || rt * CS_T >= n || rt >= tiles) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hq = blockIdx.y;
   const A* q = qk + (size_t)(c.t0 + at) * p.qk_stride + p.q_off + (size_t)hq * p.dk;
@@ -814,13 +874,6 @@ __global__ void __launch_bounds__(CS_THREADS, 4) cs_out_kernel(
 
 #include "mlstm_tensor.cuh"
 
-// ------------------------------------------------------------------- the gated delta rule
-#define DS_C 64            // tokens a chunk
-#define DS_D 128           // most key and value sizes
-#define DS_P (DS_D + 4)
-#define DS_NS 32           // columns of the state a CTA of ds_walk keeps
-#define DS_PREP_THREADS 256
-
 struct DsIn {
   const float* qkv;        // [T][C]: q (G heads of dk), k, v (H heads of dv)
   const float* gates;      // [T][2][H]: beta, decay
@@ -834,10 +887,20 @@ __device__ __forceinline__ void ds_cp16(float* smem, const float* gmem, bool ok)
                "r"(ok ? 16 : 0));
 }
 
+#include "chunk_tensor.cuh"
+
+// ------------------------------------------------------------------- the gated delta rule
+#define DS_C 64            // tokens a chunk
+#define DS_D 128           // most key and value sizes
+#define DS_P (DS_D + 4)
+#define DS_NS 32           // columns of the state a CTA of ds_walk keeps
+#define DS_PREP_THREADS 256
+
 // grid (chunks, H): W [chunk][H][64][dk], Y [chunk][H][64][dv]
 __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     DsIn p, const int* __restrict__ q_start, const double* __restrict__ F,
-    const float* __restrict__ KKm, float* __restrict__ W, float* __restrict__ Y) {
+    const float* __restrict__ KKm, float* __restrict__ W, float* __restrict__ Y,
+    const float* __restrict__ qkm, CtHead* __restrict__ Ww) {
   extern __shared__ __align__(16) float ds_smem[];
   float* Ks = ds_smem;                           // [64][DS_P]
   float* Vs = Ks + DS_C * DS_P;                  // [64][DS_P]
@@ -862,6 +925,9 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
   asm volatile("cp.async.commit_group;" ::);
   const double* f = F + (size_t)h * p.T + c.t0 + at;
   const double f0 = c.index ? f[-1] : 0.0;
+  if (Ww)                                        // (its tables lie where L and T will)
+    ct_weights(f, f, f0, n, 1.f, qkm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C,
+               *reinterpret_cast<CtWeights*>(Ls), Ww + (size_t)blockIdx.x * p.H + h);
   if (tid < DS_C) {
     fs[tid] = tid < n ? f[tid] - f0 : 0.0;
     beta[tid] = tid < n ? p.gates[(size_t)(c.t0 + at + tid) * 2 * p.H + h] : 0.f;
@@ -981,7 +1047,8 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
   }
 }
 
-// grid (column slices of 32, H, B): u [T][H][dv], Sc [chunk][H][dk][dv] (the state before each chunk).
+// grid (column slices of 32, H, B): u [T][H][dv], Sc [chunk][H][dk][dv] (the state before each chunk; tiled:
+// as ct_state's U).
 // 128 threads with 4 x 4 outputs of U and 8 x 4 of the state each: what a thread reads from shared
 // memory (at 128 bytes a cycle and SM) is about what its multiply-adds take.  1,111 and 694 tokens of
 // 16 heads of 128: 115 us; 256 threads with half of that 130, and the state's columns in the lanes'
@@ -991,7 +1058,7 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
     float* __restrict__ state, long long slot_stride, const double* __restrict__ F,
     const float2* __restrict__ Wl, const float* __restrict__ W, const float* __restrict__ Y,
     float* __restrict__ u,
-    float* __restrict__ Sc, int* __restrict__ err) {
+    float* __restrict__ Sc, bool tiled, int* __restrict__ err) {
   extern __shared__ __align__(16) float ds_smem[];
   constexpr int PS = DS_NS + 4;
   float* Ws = ds_smem;                           // [2][64][DS_P]
@@ -1053,7 +1120,8 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
 #pragma unroll
       for (int r = 0; r < 8; ++r)
         if (ty * 8 + r < p.dk)
-          *reinterpret_cast<float4*>(Sc + (chunk * p.dk + ty * 8 + r) * p.dv + col) =
+          *reinterpret_cast<float4*>(tiled ? Sc + (chunk * p.dv + col0) * p.dk + (ty * 8 + r) * DS_NS + ((tx ^ r) << 2)
+                                           : Sc + (chunk * p.dk + ty * 8 + r) * p.dv + col) =
               *reinterpret_cast<const float4*>(Ss + (ty * 8 + r) * PS + 4 * tx);
     }
     // U = Y - W S, in runs of 16 terms
@@ -1144,9 +1212,9 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
 
 // -------------------------------------------------------------------------------- launches
 // Scratch (bytes, each part on a 256-byte boundary): G, Hs, g0, Wl | E (mLSTM) | qkm | U | Un
-// (mLSTM).
+// (mLSTM) | Xq, Xk, odd, W (`terms`: chunk_tensor.cuh).
 struct CsLayout {
-  size_t G, Hs, g0, Wl, E, qkm, U, Un, total;
+  size_t G, Hs, g0, Wl, E, qkm, U, Un, Xq, Xk, odd, W, total;
   int chunks;
 };
 // The most chunks of C tokens that a step's portions of more than n_min tokens can have.
@@ -1155,7 +1223,7 @@ static int cs_most_chunks(int T, int B, int C, int n_min) {
   return T / C + (B < long_ones ? B : long_ones);
 }
 static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, int mlstm,
-                          int n_min) {
+                          int n_min, bool terms) {
   CsLayout l;
   size_t at = 0;
   auto take = [&](size_t bytes) {
@@ -1172,13 +1240,19 @@ static CsLayout cs_layout(int T, int B, int H, int QH, int dk, int dv, int C, in
   l.qkm = take((size_t)l.chunks * QH * C * C * 4);
   l.U = take((size_t)l.chunks * H * dk * dv * 4);
   l.Un = take(mlstm ? (size_t)l.chunks * H * dk * 4 : 0);
+  l.Xq = take(terms ? ct_terms_bytes(l.chunks, QH, dk) : 0);
+  l.Xk = take(terms ? ct_terms_bytes(l.chunks, QH, dk) : 0);
+  l.odd = take(terms ? (size_t)l.chunks * QH * 16 : 0);
+  l.W = take(terms ? (size_t)l.chunks * H * sizeof(CtHead) : 0);
   l.total = at;
   return l;
 }
 
+// terms: with the room that a linear scan's products on the tensor cores need (0 where none takes the sizes)
 BF_EXPORT long long bf_chunk_scan_scratch(int T, int B, int H, int QH, int dk, int dv, int C,
-                                          int mlstm, int n_min) {
-  return (long long)cs_layout(T, B, H, QH, dk, dv, C, mlstm, n_min).total;
+                                          int mlstm, int n_min, int terms) {
+  if (terms && (mlstm || !ct_takes(H, QH, dk, dv, C, cs_most_chunks(T, B, C, n_min)))) return 0;
+  return (long long)cs_layout(T, B, H, QH, dk, dv, C, mlstm, n_min, terms).total;
 }
 
 template <typename A, typename V, bool MLSTM>
@@ -1187,7 +1261,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
                      long long slot_stride, int state_size, const int* q_start,
                      const int* state_slots, int n_slots, float* o_raw, char* scratch, int* err,
                      cudaStream_t stream, bool tensor = false) {
-  const CsLayout l = cs_layout(p.T, p.B, p.H, p.QH, p.dk, p.dv, p.C, MLSTM, p.n_min);
+  const CsLayout l = cs_layout(p.T, p.B, p.H, p.QH, p.dk, p.dv, p.C, MLSTM, p.n_min, !MLSTM && tensor);
   double* G = (double*)(scratch + l.G);
   double* Hs = (double*)(scratch + l.Hs);
   double* g0 = (double*)(scratch + l.g0);
@@ -1200,12 +1274,23 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   cs_gates_kernel<MLSTM><<<dim3(p.H, p.B), CS_GATE_THREADS, 0, stream>>>(
       decays, tok_decay, gates, state, slot_stride, state_size, q_start, state_slots, n_slots, G,
       Hs, E, g0, Wl, p.C, p.T, p.H, p.dk * p.dv, p.dk, p.n_min, p.H);
-  cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles), 128, 0, stream>>>(qk, p, q_start,
-                                                                                 qkm, nullptr);
+  CsTerms x = {nullptr, nullptr, nullptr};
+  if (!MLSTM && tensor)
+    x = {(uint8_t*)scratch + l.Xq, (uint8_t*)scratch + l.Xk, (unsigned long long*)(scratch + l.odd)};
+  cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)), 128, 0, stream>>>(qk, p, q_start, qkm,
+                                                                                                 nullptr, x);
   if constexpr (MLSTM) {
     if (tensor)
       return mt_launch(qk, p, l.chunks, q_start, state, slot_stride, state_size, state_slots, n_slots, G, Hs, g0,
                        Wl, E, qkm, U, Un, o_raw, err, stream);
+  } else if (tensor) {
+    if (const int e = ct_configure()) return e;
+    CtHead* W = (CtHead*)(scratch + l.W);
+    ct_weights_kernel<<<dim3(l.chunks, p.H), 256, 0, stream>>>(p, q_start, G, Hs, g0, qkm, W);
+    ct_state_kernel<<<dim3(p.dv / CT_SV * (p.dk / 128), p.H, p.B), CT_S_THREADS, CT_S_SMEM, stream>>>(
+        qk, v, p, q_start, state, slot_stride, state_slots, n_slots, G, Wl, x.k, x.odd, U, err);
+    ct_out_launch(qk, v, p, l.chunks, q_start, state_slots, n_slots, G, Hs, W, qkm, x.q, x.odd, U, o_raw, err, stream);
+    return bf_launch_status();
   }
   cs_state_kernel<A, V, MLSTM><<<dim3(l.chunks, p.H, tk * tv), CS_THREADS, 0, stream>>>(
       qk, v, p, q_start, Wl, U, Un);
@@ -1226,21 +1311,23 @@ static bool cs_sizes_ok(const CsIn& p, const void* state, long long slot_stride,
 }
 
 // qk [T][2][QH][dk] (q, then k), vf [T][H][dv], float; a decay per head or per (token, head).
-// State and o_raw as in bf_linear_scan; requests of at most n_min tokens are left alone.
+// State and o_raw as in bf_linear_scan; requests of at most n_min tokens are left alone.  terms: `scratch` has
+// the room for the products on the tensor cores (chunk_tensor.cuh), which then run there.
 BF_EXPORT int bf_chunk_scan_linear(const float* qk, const float* vf, const float* decays,
                                    const float* tok_decay, float* state, long long slot_stride,
                                    const int* q_start, const int* state_slots, int n_slots,
                                    float* o_raw, void* scratch, int T, int B, int H, int QH,
-                                   int dk, int dv, int C, int n_min, int* err,
+                                   int dk, int dv, int C, int n_min, int terms, int* err,
                                    cudaStream_t stream) {
   CsIn p = {0, (long long)QH * dk, 0, 2LL * QH * dk, (long long)H * dv, H, QH, dk, dv, C, T, B,
             n_min, 1.f};
   if (!cs_sizes_ok(p, state, slot_stride, o_raw) || (!decays && !tok_decay) || !scratch ||
-      (((uintptr_t)qk | (uintptr_t)vf) & 15))
+      (((uintptr_t)qk | (uintptr_t)vf) & 15) ||
+      (terms && !ct_takes(H, QH, dk, dv, C, cs_most_chunks(T, B, C, n_min))))
     return (int)cudaErrorInvalidValue;
   return cs_launch<float, float, false>(qk, vf, p, decays, tok_decay, nullptr, state, slot_stride,
                                         dk * dv, q_start, state_slots, n_slots, o_raw,
-                                        (char*)scratch, err, stream);
+                                        (char*)scratch, err, stream, terms);
 }
 
 // proj rows [q: H dk | k: H dk | v: H dv | ...] in bfloat16, gates and state as in bf_mlstm_scan; max_q and
@@ -1273,10 +1360,10 @@ BF_EXPORT int bf_chunk_scan_mlstm_kernels(const void* proj, long long stride, in
 // The gated delta rule.  Scratch: F (G and H are the same array), g0, Wl | qkm | kkm | W | Y |
 // u | Sc.
 struct DsLayout {
-  size_t F, g0, Wl, qkm, kkm, W, Y, u, Sc, total;
+  size_t F, g0, Wl, qkm, kkm, W, Y, u, Sc, Xq, odd, Ww, total;
   int chunks;
 };
-static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min) {
+static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min, bool terms) {
   DsLayout l;
   size_t at = 0;
   auto take = [&](size_t bytes) {
@@ -1294,13 +1381,18 @@ static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min)
   l.Y = take((size_t)l.chunks * H * DS_C * dv * 4);
   l.u = take((size_t)T * H * dv * 4);
   l.Sc = take((size_t)l.chunks * H * dk * dv * 4);
+  l.Xq = take(terms ? ct_terms_bytes(l.chunks, G, dk) : 0);
+  l.odd = take(terms ? (size_t)l.chunks * G * 16 : 0);
+  l.Ww = take(terms ? (size_t)l.chunks * H * sizeof(CtHead) : 0);
   l.total = at;
   return l;
 }
 
+// terms: as for bf_chunk_scan_scratch
 BF_EXPORT long long bf_chunk_scan_delta_scratch(int T, int B, int H, int G, int dk, int dv,
-                                                int n_min) {
-  return (long long)ds_layout(T, B, H, G, dk, dv, n_min).total;
+                                                int n_min, int terms) {
+  if (terms && !ct_takes(H, G, dk, dv, DS_C, cs_most_chunks(T, B, DS_C, n_min))) return 0;
+  return (long long)ds_layout(T, B, H, G, dk, dv, n_min, terms).total;
 }
 
 // qkv, gates, state and o_raw as in bf_delta_scan (keys and values of at most 128, multiples of 4);
@@ -1308,14 +1400,15 @@ BF_EXPORT long long bf_chunk_scan_delta_scratch(int T, int B, int H, int G, int 
 BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* state,
                                   long long slot_stride, const int* q_start,
                                   const int* state_slots, int n_slots, float* o_raw, void* scratch,
-                                  int T, int B, int H, int G, int dk, int dv, int n_min, int* err,
-                                  cudaStream_t stream) {
+                                  int T, int B, int H, int G, int dk, int dv, int n_min, int terms,
+                                  int* err, cudaStream_t stream) {
   const long long C = 2LL * G * dk + (long long)H * dv;
   if (T <= 0 || B <= 0 || B > 65535 || H <= 0 || H > 65535 || G <= 0 || H % G || dk <= 0 ||
       n_min < 0 || dv <= 0 || dk > DS_D || dv > DS_D || dk % 4 || dv % 4 || !scratch ||
-      (((uintptr_t)qkv | (uintptr_t)o_raw) & 15))
+      (((uintptr_t)qkv | (uintptr_t)o_raw) & 15) ||
+      (terms && !ct_takes(H, G, dk, dv, DS_C, cs_most_chunks(T, B, DS_C, n_min))))
     return (int)cudaErrorInvalidValue;
-  const DsLayout l = ds_layout(T, B, H, G, dk, dv, n_min);
+  const DsLayout l = ds_layout(T, B, H, G, dk, dv, n_min, terms);
   char* base = (char*)scratch;
   double* F = (double*)(base + l.F);
   double* g0 = (double*)(base + l.g0);
@@ -1326,6 +1419,9 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
   float* Y = (float*)(base + l.Y);
   float* u = (float*)(base + l.u);
   float* Sc = (float*)(base + l.Sc);
+  uint8_t* Xq = terms ? (uint8_t*)base + l.Xq : nullptr;
+  unsigned long long* odd = (unsigned long long*)(base + l.odd);
+  CtHead* Ww = (CtHead*)(base + l.Ww);
   const DsIn d = {qkv, gates, C, H, G, dk, dv, T, B, n_min};
   // (the decays are the second rows of gates: [T][2][H])
   const CsIn p = {0, (long long)G * dk, 0, C, (long long)H * dv, H, G, dk, dv, DS_C, T, B, n_min,
@@ -1343,15 +1439,22 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
     if (e != cudaSuccess) return (int)e;
     done = true;
   }
+  if (terms) {
+    if (const int e = ct_configure()) return e;
+  }
   cs_gates_kernel<false><<<dim3(H, B), CS_GATE_THREADS, 0, stream>>>(
       nullptr, gates + H, nullptr, state, slot_stride, dk * dv, q_start, state_slots, n_slots, F, F,
       nullptr, g0, Wl, DS_C, T, H, dk * dv, dk, n_min, 2 * H);
-  cs_qk_kernel<float, true><<<dim3(l.chunks, G, 1), 256, 0, stream>>>(qkv, p, q_start, qkm, kkm);
+  const CsTerms x = {Xq, nullptr, odd};
+  cs_qk_kernel<float, true><<<dim3(l.chunks, G, x.q ? 2 : 1), 256, 0, stream>>>(qkv, p, q_start, qkm, kkm, x);
   ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, kkm, W,
-                                                                            Y);
+                                                                            Y, qkm, terms ? Ww : nullptr);
   ds_walk_kernel<<<dim3((dv + DS_NS - 1) / DS_NS, H, B), 128, smem_walk, stream>>>(
-      d, q_start, state_slots, n_slots, state, slot_stride, F, Wl, W, Y, u, Sc, err);
-  cs_out_kernel<float, float, false, true>
+      d, q_start, state_slots, n_slots, state, slot_stride, F, Wl, W, Y, u, Sc, terms, err);
+  if (terms)
+    ct_out_launch(qkv, u, p, l.chunks, q_start, state_slots, n_slots, F, F, Ww, qkm, Xq, odd, Sc, o_raw, err, stream);
+  else
+    cs_out_kernel<float, float, false, true>
       <<<dim3(l.chunks, H, (dv + CS_T - 1) / CS_T), CS_THREADS, 0, stream>>>(
           qkv, u, p, q_start, state_slots, n_slots, F, F, g0, nullptr, qkm, Sc, nullptr, o_raw);
   return bf_launch_status();

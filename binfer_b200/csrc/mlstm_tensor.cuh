@@ -26,10 +26,8 @@
 // and the end of a tile (4,000).  Relative errors against 64 bits, this / those, at 2,048 tokens (four inputs):
 // outputs 5.7 7.1 6.4 5.5 / 5.5 8.8 7.5 5.8 e-7, states 0.85 1.2 0.94 0.98 / 1.4 1.5 1.4 1.3 e-7.
 //
-// The recurrences whose operands are floats stay on cs_state, cs_prefix and cs_out: with six products and both
-// operands to take apart these kernels took 90 + 144 us where those take 188 (2,000 tokens, 64 heads of
-// 128 x 64) and 66 + 48 against 105 (8 heads of 128 x 256): what a chunk's sums cost outside of
-// the products, for every element of a state, outweighs the multiply-adds that they replace.
+// The recurrences whose operands are floats have kernels of their own (chunk_tensor.cuh): with six products and
+// both operands to take apart these took 90 + 144 us where multiply-adds took 188 (2,000 tokens, 64 heads of 128 x 64).
 //
 // Included by chunk_scan.cu behind its helpers.
 #pragma once

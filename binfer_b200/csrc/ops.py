@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -744,6 +744,14 @@ CHUNK_SCAN_TOKENS = 64
 CHUNK_SCAN_MAX_BYTES = 768 << 20
 
 
+# Fewest CTAs of a request (a head's 128 key x 32 value sizes each) for a linear scan's chunks on the tensor
+# cores, where ct_state goes from chunk to chunk and cs_state has CTAs for every chunk.  Tensor cores / multiply-adds
+# in us at 500, 2,000 and 8,192 tokens: 16 CTAs 50 / 48, 72 / 65, 220 / 204; 32 50 / 52, 84 / 90, 270 / 312; 64 51 / 56,
+# 99 / 130, 310 / 464; 128 58 / 77, 140 / 224, 441 / 823 (what shares the step does not count: a request's results
+# have the same bits beside others).
+LINEAR_TENSOR_MIN_CTAS = 32
+
+
 def chunk_scan_pays(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bool:
     """Whether a step's linear scan is the faster one in chunks: ``tokens`` of all requests, of which
     the longest brings ``max_q``.  The walk is a chain over the longest portion until the portions'
@@ -761,20 +769,24 @@ def chunk_scan_pays(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bo
 
 def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_heads: int, dk: int,
                    dv: int, state: torch.Tensor, mlstm: int,
-                   *buffers: torch.Tensor) -> Optional[torch.Tensor]:
+                   *buffers: torch.Tensor) -> Tuple[Optional[torch.Tensor], int]:
     """Scratch for the products over chunks, or None where a step's recurrence is walked: single
     tokens and short portions, and sizes or addresses (of the state and of ``buffers``, float)
-    that are no whole 16-byte pieces."""
+    that are no whole 16-byte pieces.  And 1 where it has the room for a linear scan's products on the
+    tensor cores (``chunk_tensor.cuh``), which are taken where their sizes and the limit allow."""
     if (not chunked or max_q <= CHUNK_SCAN_MIN or dk % 4 or dv % 4 or state.stride(0) % 4
             or any(t.data_ptr() % 16 for t in (state, *buffers)) or B > 65535 or heads > 65535):
-        return None
+        return None, 0
     fn = lib().bf_chunk_scan_scratch
     fn.restype = _c_ll
-    n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
-           _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)))
-    if n > CHUNK_SCAN_MAX_BYTES:
-        return None
-    return torch.empty(n, dtype=torch.uint8, device=state.device)
+    few = heads * (dk // 128) * (dv // 32) < LINEAR_TENSOR_MIN_CTAS
+    for terms in (0,) if few else (1, 0):
+        n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
+               _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)),
+               _c_int(terms))
+        if 0 < n <= CHUNK_SCAN_MAX_BYTES:
+            return torch.empty(n, dtype=torch.uint8, device=state.device), terms
+    return None, 0
 
 
 def _chunk_limit(B: int, n_min: int) -> int:
@@ -789,12 +801,12 @@ def _walk_limit(scratch: Optional[torch.Tensor], B: int, n_min: int) -> int:
 
 
 def _chunk_scan_linear(name, qk, vf, decays, tok_decay, state, q_start, state_slots, o_raw, scratch,
-                       B, heads, qk_heads, dk, dv, err) -> None:
+                       terms, B, heads, qk_heads, dk, dv, err) -> None:
     _run(name + "_chunks", lib().bf_chunk_scan_linear, _ptr(qk), _ptr(vf), _ptr(decays),
          _ptr(tok_decay), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
          _c_int(state.shape[0]), _ptr(o_raw), _ptr(scratch), _c_int(vf.shape[0]), _c_int(B),
          _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv), _c_int(CHUNK_SCAN_TOKENS),
-         _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _ptr(err), _stream())
+         _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)), _c_int(terms), _ptr(err), _stream())
     global _launches
     _launches += 4          # five kernels
 
@@ -833,8 +845,7 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
     # two kernels
     qk = torch.empty((T, 2, heads, dk), dtype=torch.float32, device=proj.device)
     vf = torch.empty((T, heads, dv), dtype=torch.float32, device=proj.device)
-    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, heads, dk, dv, state, 0,
-                             o_raw)
+    scratch, terms = _chunk_scratch(chunked, max_q or T, T, B, heads, heads, dk, dv, state, 0, o_raw)
     _run("retention_scan", lib().bf_retention_scan, _ptr(proj), _c_ll(proj.stride(0)),
          _c_ll(q_off), _c_ll(k_off), _c_ll(v_off), _ptr(decays), _ptr(inv_freq), _c_int(rot_half),
          _ptr(positions), _ptr(state), _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots),
@@ -845,7 +856,7 @@ def retention_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay
     _launches += 1          # two kernels: the rotation and the scan
     if scratch is not None:
         _chunk_scan_linear("retention_scan", qk, vf, decays, None, state, q_start, state_slots,
-                           o_raw, scratch, B, heads, heads, dk, dv, err)
+                           o_raw, scratch, terms, B, heads, heads, dk, dv, err)
 
 
 def linear_scan(qk: torch.Tensor, vf: torch.Tensor, tok_decay: torch.Tensor, state: torch.Tensor,
@@ -871,11 +882,11 @@ def linear_scan(qk: torch.Tensor, vf: torch.Tensor, tok_decay: torch.Tensor, sta
     if (state.dtype != torch.float32 or state.stride(1) != 1
             or state.shape[1] != heads * dk * dv):
         raise KernelError("linear_scan: state must be float32 [slots, heads * dk * dv]")
-    scratch = _chunk_scratch(chunked, max_q or T, T, B, heads, qk_heads, dk, dv, state, 0,
-                             qk, vf, o_raw)
+    scratch, terms = _chunk_scratch(chunked, max_q or T, T, B, heads, qk_heads, dk, dv, state, 0,
+                                    qk, vf, o_raw)
     if scratch is not None:
         _chunk_scan_linear("linear_scan", qk, vf, None, tok_decay, state, q_start, state_slots,
-                           o_raw, scratch, B, heads, qk_heads, dk, dv, err)
+                           o_raw, scratch, terms, B, heads, qk_heads, dk, dv, err)
         if _walk_limit(scratch, B, CHUNK_SCAN_MIN) < 0:
             return
     _run("linear_scan", lib().bf_linear_scan, _ptr(qk), _ptr(vf), _ptr(tok_decay), _ptr(state),
@@ -1111,21 +1122,24 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
     if (state.dtype != torch.float32 or state.stride(1) != 1
             or state.shape[1] != heads * dk * dv or dk > DELTA_MAX_QK_DIM):
         raise KernelError("delta_scan: state must be float32 [slots, heads * dk * dv]")
-    scratch = None
+    scratch, terms = None, 0
     if (chunked and (max_q or T) > DELTA_CHUNK_MIN and dk <= 128 and dv <= 128 and dk % 4 == 0
             and dv % 4 == 0 and B <= 65535 and heads <= 65535 and qkv.is_contiguous()
             and gates.is_contiguous() and qkv.data_ptr() % 16 == 0 and o_raw.data_ptr() % 16 == 0):
         fn = lib().bf_chunk_scan_delta_scratch
         fn.restype = _c_ll
-        n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
-               _c_int(_chunk_limit(B, DELTA_CHUNK_MIN)))
-        if n <= CHUNK_SCAN_MAX_BYTES:
-            scratch = torch.empty(n, dtype=torch.uint8, device=state.device)
+        for terms in (1, 0):             # (as in _chunk_scratch)
+            n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
+                   _c_int(_chunk_limit(B, DELTA_CHUNK_MIN)), _c_int(terms))
+            if 0 < n <= CHUNK_SCAN_MAX_BYTES:
+                scratch = torch.empty(n, dtype=torch.uint8, device=state.device)
+                break
     if scratch is not None:
         _run("delta_scan_chunks", lib().bf_chunk_scan_delta, _ptr(qkv), _ptr(gates), _ptr(state),
              _c_ll(state.stride(0)), _ptr(q_start), _ptr(state_slots), _c_int(state.shape[0]),
              _ptr(o_raw), _ptr(scratch), _c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads),
-             _c_int(dk), _c_int(dv), _c_int(_chunk_limit(B, DELTA_CHUNK_MIN)), _ptr(err), _stream())
+             _c_int(dk), _c_int(dv), _c_int(_chunk_limit(B, DELTA_CHUNK_MIN)), _c_int(terms), _ptr(err),
+             _stream())
         global _launches
         _launches += 4          # five kernels
         if _walk_limit(scratch, B, DELTA_CHUNK_MIN) < 0:
@@ -1486,7 +1500,7 @@ def mlstm_scan(proj: torch.Tensor, gates: torch.Tensor, state: torch.Tensor,
     T = proj.shape[0]
     takes = (chunked and proj.dtype == torch.bfloat16 and proj.stride(0) % 4 == 0
              and proj.data_ptr() % 8 == 0 and state.stride(1) == state.shape[2])
-    scratch = _chunk_scratch(takes, max_q or T, T, B, heads, heads, dk, dv, state, 1, o_raw)
+    scratch, _ = _chunk_scratch(takes, max_q or T, T, B, heads, heads, dk, dv, state, 1, o_raw)
     if scratch is not None:
         _run("mlstm_scan_chunks", lib().bf_chunk_scan_mlstm, _ptr(proj), _c_ll(proj.stride(0)),
              _ptr(gates), _ptr(state), _c_ll(state.stride(0)), _c_int(state.shape[2]),

@@ -1332,6 +1332,146 @@ def test_linear_scan_in_chunks(cuda_device, lens, H, G, dk, dv, decays):
     err.zero_()
 
 
+# the same on the tensor cores: two heads of 64 a tile and one of 128 or more, requests of odd lengths beside
+# walked ones, more tiles than SMs; the multiply-adds beside them
+@pytest.mark.parametrize("lens,H,G,dk,dv,decays", [
+    ([161, 1, 192, 160, 257], 4, 2, 128, 64, "spread"), ([193, 320], 4, 1, 256, 64, "zeros"),
+    ([300], 2, 2, 128, 128, "slow"), ([170, 3, 700], 16, 8, 128, 256, "slow")])
+def test_linear_chunks_on_tensor_cores(cuda_device, monkeypatch, lens, H, G, dk, dv, decays):
+    """Bound as in test_linear_scan_in_chunks; and no further from float64 than the multiply-adds with slow
+    decays, half a unit in the last place more with others (a sum of few terms is cut where that one rounds)."""
+    from binfer_b200.csrc import ops
+    torch.manual_seed(len(lens) + dk)
+    T, B, dev = sum(lens), len(lens), cuda_device
+    qk, v = torch.randn(T, 2, G, dk, device=dev), torch.randn(T, H, dv, device=dev)
+    d = torch.rand(T, H, device=dev)
+    if decays == "slow":
+        d = 1.0 - 0.01 * d
+    elif decays == "zeros":
+        d[torch.rand(T, H, device=dev) < 0.1] = 0.0
+    state = torch.randn(B + 1, H * dk * dv, device=dev)
+    slots = torch.arange(B, dtype=torch.int32, device=dev).flip(0).contiguous()
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    got, err = [], _err(dev)
+    for ctas in (0, 1 << 30):
+        monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", ctas)
+        _, terms = ops._chunk_scratch(True, max(lens), T, B, H, G, dk, dv, state, 0, qk)
+        assert terms == (ctas == 0)
+        s, o = state.clone(), torch.full((T, H * dv), 7.0, device=dev)
+        ops.linear_scan(qk, v, d, s, qs, slots, o, B, H, G, dk, dv, err, max_q=max(lens), chunked=True)
+        assert int(err.item()) == 0 and torch.equal(s[B], state[B])
+        got.append((o, s))
+    off = [[0.0, 0.0], [0.0, 0.0]]
+    for b in range(B):
+        a, e, at = int(qs[b]), int(qs[b + 1]), int(slots[b])
+        q, k = (qk[a:e, i].double().repeat_interleave(H // G, 1) for i in (0, 1))
+        S0 = state[at].double().view(H, dv, dk).transpose(1, 2)
+        o, S = _walk64(q, k, v[a:e].double(), d[a:e].double(), S0)
+        bound_o, bound_S = _walk64(q.abs(), k.abs(), v[a:e].double().abs(), d[a:e].double(), S0.abs())
+        c = (64 + 4 * len(lens)) * 2.0 ** -24
+        for i, (go, gs) in enumerate(got):
+            oo = go[a:e].view(-1, H, dv).double()
+            SS = gs[at].double().view(H, dv, dk).transpose(1, 2)
+            assert bool(((oo - o).abs() <= c * bound_o + 1e-30).all())
+            assert bool(((SS - S).abs() <= c * bound_S + 1e-30).all())
+            if e - a > ops.CHUNK_SCAN_MIN:
+                for j, (x, y) in enumerate(((oo, o), (SS, S))):
+                    off[i][j] = max(off[i][j], float((x - y).norm() / y.norm()))
+    for tensor, adds in zip(*off):
+        assert tensor <= adds + (0.0 if decays == "slow" else 2.0 ** -25), off
+    bad, keep, o = slots.clone(), got[0][1].clone(), got[0][0].clone()
+    bad[0] = B + 5
+    monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", 0)
+    ops.linear_scan(qk, v, d, keep, qs, bad, o, B, H, G, dk, dv, err, max_q=max(lens), chunked=True)
+    assert int(err.item()) == 2 and torch.equal(keep[int(slots[0])], got[0][1][int(slots[0])])
+    err.zero_()
+
+
+# (the delta rule's own sums leave float's range before these do)
+@pytest.mark.parametrize("kind,dv,what", [
+    (*k, w) for k in (("linear", 64), ("linear", 128), ("delta", 128))
+    for w in ("v", "k", "q", "decay", "state", "large v", "small", "products", "all v")
+    if k[0] == "linear" or w not in ("large v", "products", "state")])
+def test_chunks_on_tensor_cores_take_floats_of_every_size(cuda_device, monkeypatch, kind, dv, what):
+    """Infinities, NaN, floats that have no terms, products that leave float's range: numbers where the
+    multiply-adds have numbers, the same ones but for rounding; the bits of the tokens before are the clean
+    call's."""
+    from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN", 160)
+    dev, T, H, G, dk, at = cuda_device, 330, 4, 2, 128, 140
+    torch.manual_seed(11)
+    unit = lambda x: torch.nn.functional.normalize(x, dim=-1)
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err, outs = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev), {}
+    clean = (unit(torch.randn(T, 2, G, dk, device=dev)), torch.randn(T, H, dv, device=dev),
+             1 - 0.1 * torch.rand(T, H, device=dev), 0.1 * torch.randn(1, H * dk * dv, device=dev))
+    for bad in (False, True):
+        x, v, d, s0 = (t.clone() for t in clean)
+        if bad and what == "v":
+            v[at, 1, 5] = float("inf")
+        elif bad and what == "all v":
+            v[:] = float("inf")
+        elif bad and what == "k":
+            x[at, 1, 0, 77] = float("-inf")
+        elif bad and what == "q":
+            x[at, 0, 1, 3] = float("nan")
+        elif bad and what == "decay":
+            d[at, 2] = float("nan")
+        elif bad and what == "state":
+            s0[0, 5000] = float("inf")
+        elif bad and what == "large v":
+            v[at:, 1] *= 3e37
+        elif bad and what == "small":
+            v *= 1e-33
+            s0 *= 1e-33
+        elif bad and what == "products":
+            v[at:, 1], x[at:, 1, 0] = v[at:, 1] * 1e24, x[at:, 1, 0] * 1e24
+        for ctas in (0, 1 << 30):
+            monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", ctas)
+            monkeypatch.setattr(ops, "CHUNK_SCAN_MAX_BYTES", 768 << 20)
+            if kind == "delta" and ctas:         # (the limit between the two calls' scratch)
+                fn = ops.lib().bf_chunk_scan_delta_scratch
+                args = [ops._c_int(z) for z in (T, 1, H, G, dk, dv, 0, 0)]
+                monkeypatch.setattr(ops, "CHUNK_SCAN_MAX_BYTES", fn(*args))
+            s, o = s0.clone(), torch.empty(T, H * dv, device=dev)
+            if kind == "linear":
+                ops.linear_scan(x, v, d, s, qs, slots, o, 1, H, G, dk, dv, err, max_q=T, chunked=True)
+            else:
+                qkv = torch.cat([x[:, 0].reshape(T, -1), x[:, 1].reshape(T, -1), v.reshape(T, -1)], 1).contiguous()
+                ops.delta_scan(qkv, torch.stack([d / 2, d], 1).contiguous(), s, qs, slots, o, 1, H, G, dk, dv, err,
+                               max_q=T, chunked=True)
+            outs[bad, ctas == 0] = (o.view(T, H, dv), s)
+    assert int(err.item()) == 0
+    for mine, adds in zip(outs[True, True], outs[True, False]):
+        assert torch.equal(mine.isfinite(), adds.isfinite())
+        fin = mine.isfinite()
+        if bool(fin.any()):
+            scale = adds[fin].abs().max()
+            assert float(((mine - adds)[fin] / scale).abs().max()) <= 1e-5
+    if what not in ("state", "small", "all v"):
+        assert torch.equal(outs[True, True][0][:at], outs[False, True][0][:at])
+
+
+def test_linear_chunks_on_tensor_cores_of_many_tiles(cuda_device, monkeypatch):
+    """More tiles than one CTA an SM has room for in its list: the multiply-adds' results."""
+    from binfer_b200.csrc import ops
+    dev, T, H, dk, dv = cuda_device, 9700, 64, 128, 128
+    torch.manual_seed(12)
+    qk = torch.nn.functional.normalize(torch.randn(T, 2, 8, dk, device=dev), dim=-1)
+    v, d = torch.randn(T, H, dv, device=dev), 1 - 0.05 * torch.rand(T, H, device=dev)
+    qs, slots = torch.tensor([0, T], dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    got, err = [], _err(dev)
+    monkeypatch.setattr(ops, "CHUNK_SCAN_MAX_BYTES", 2 << 30)
+    for ctas in (0, 1 << 30):
+        monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", ctas)
+        s, o = torch.zeros(1, H * dk * dv, device=dev), torch.empty(T, H * dv, device=dev)
+        ops.linear_scan(qk, v, d, s, qs, slots, o, 1, H, 8, dk, dv, err, max_q=T, chunked=True)
+        got.append((o, s))
+    assert int(err.item()) == 0
+    for a, b in zip(*got):
+        assert float((a - b).norm() / b.norm()) <= 5e-7
+
+
 def test_retention_part_walks_decays_below_zero(cuda_device, monkeypatch):
     """A portion long enough for chunks and the same tokens in two that are walked."""
     from types import SimpleNamespace
