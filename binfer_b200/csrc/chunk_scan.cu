@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(CS_GATE_THREADS) cs_gates_kernel(
     double* __restrict__ g0, float2* __restrict__ Wl, int C, int T, int H, int dkdv, int dk, int n_min,
     int decay_stride) {
   __shared__ double sh[CS_GATE_THREADS / 32];
+  bf_pdl_trigger();                              // (cs_qk reads nothing of these: it runs beside them)
   const int h = blockIdx.x, b = blockIdx.y;
   const int t0 = q_start[b], n = q_start[b + 1] - t0;
   if (n <= n_min) return;
@@ -491,7 +492,10 @@ __global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
   if constexpr (sizeof(A) == 4) {
     if (rt >= tiles && c.b >= 0) cs_terms<THREADS>(qk, p, c, blockIdx.z - tiles * tiles, x_out);
   }
-  if (ct > rt || c.b < 0 || rt * CS_T >= n || rt >= tiles) return;
+  if (ct > rt || c.b < 0 || rt * CS_T >= n || rt >= tiles) {
+    bf_pdl_wait();                               // (on every path: this grid's end is that of cs_gates, too)
+    return;
+  }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hq = blockIdx.y;
   const A* q = qk + (size_t)(c.t0 + at) * p.qk_stride + p.q_off + (size_t)hq * p.dk;
@@ -549,6 +553,7 @@ __global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
         *reinterpret_cast<float2*>(
             dst + (size_t)(rt * CS_T + block * 16 + 8 * i + (lane >> 2)) * p.C + ct * CS_T + 8 * j +
             (lane & 3) * 2) = make_float2((float)(acc[i][j][0] * scale), (float)(acc[i][j][1] * scale));
+  bf_pdl_wait();
 }
 
 // ------------------------------------------------------------------------------- cs_state
@@ -1277,8 +1282,9 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   CsTerms x = {nullptr, nullptr, nullptr};
   if (!MLSTM && tensor)
     x = {(uint8_t*)scratch + l.Xq, (uint8_t*)scratch + l.Xk, (unsigned long long*)(scratch + l.odd)};
-  cs_qk_kernel<A, false><<<dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)), 128, 0, stream>>>(qk, p, q_start, qkm,
-                                                                                                 nullptr, x);
+  if (const int e = bf_launch_pdl(cs_qk_kernel<A, false>, dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)), dim3(128), 0, stream,
+                                  qk, p, q_start, qkm, (float*)nullptr, x))
+    return e;
   if constexpr (MLSTM) {
     if (tensor)
       return mt_launch(qk, p, l.chunks, q_start, state, slot_stride, state_size, state_slots, n_slots, G, Hs, g0,
@@ -1446,7 +1452,9 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
       nullptr, gates + H, nullptr, state, slot_stride, dk * dv, q_start, state_slots, n_slots, F, F,
       nullptr, g0, Wl, DS_C, T, H, dk * dv, dk, n_min, 2 * H);
   const CsTerms x = {Xq, nullptr, odd};
-  cs_qk_kernel<float, true><<<dim3(l.chunks, G, x.q ? 2 : 1), 256, 0, stream>>>(qkv, p, q_start, qkm, kkm, x);
+  if (const int e = bf_launch_pdl(cs_qk_kernel<float, true>, dim3(l.chunks, G, x.q ? 2 : 1), dim3(256), 0, stream, qkv, p, q_start,
+                                  qkm, kkm, x))
+    return e;
   ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, kkm, W,
                                                                             Y, qkm, terms ? Ww : nullptr);
   ds_walk_kernel<<<dim3((dv + DS_NS - 1) / DS_NS, H, B), 128, smem_walk, stream>>>(
