@@ -24,7 +24,7 @@
 //
 // The mLSTM with keys in whole steps of 64 and values in whole tiles of 128 runs its products on the tensor
 // cores (mlstm_tensor.cuh: the last three kernels become two), and so do the linear scan with keys in whole steps of
-// 128, values of 64 or whole tiles of 128 and CTAs enough, and the delta rule's cs_out (chunk_tensor.cuh).
+// 128, values of 64 or whole tiles of 128 and CTAs enough, and the delta rule with keys of 128 (chunk_tensor.cuh).
 //
 // GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads by multiply-adds 208 / 467 us (cs_out
 // 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 138; 8 heads of 128 x 256 124 / 270 (83); mLSTM, 8 heads of 256 x
@@ -55,8 +55,8 @@
 //              32 columns) in parallel
 //   cs_out     as above, on U
 //
-// 2,048 tokens of 16 heads of 128: 341 us (ds_walk 187, cs_out 54, ds_prep 48, cs_qk 42) against the walk's
-// 563; 1,000 tokens 168 and 277, three portions of 1,000 381 and 431.  Errors against 64 bits, walk / chunks:
+// 2,048 tokens of 16 heads of 128: 341 us (ds_walk 187, cs_out 54, ds_prep 48, cs_qk 42) by multiply-adds against the
+// walk's 563; 1,000 tokens 168 and 277, three portions of 1,000 381 and 431.  Errors against 64 bits, walk / chunks:
 // keys at random, decays of 0.98 to 1: o 2.3e-7 / 1.6e-7, state 2.3e-7 / 1.8e-7; keys of a cosine of 0.9
 // 2.6e-7 / 2.6e-7 and 2.5e-7 / 2.5e-7; fast decays o 1.1e-7 / 7.8e-8, state 6.2e-8 / 7.1e-8.  (What the walk
 // has and a chunk's inverse has not is that a token's u answers to the rounding of the one before it:
@@ -433,6 +433,28 @@ struct CsTerms {
 #define CS_TERMS_TILE (3 * CS_TERMS_TERM)
 // the first float that has none, times 2^24, as bits
 constexpr uint32_t CS_NO_TERMS_UP = 0x7f7f8000u - (24u << 23);
+// four sizes of a token; true where one has no terms
+__device__ __forceinline__ bool cs_put_terms(uint8_t* X, int token, int size, float4 v) {
+  float x[4] = {v.x, v.y, v.z, v.w};
+  bool bad = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if ((__float_as_uint(x[i]) & 0x7fffffffu) >= CS_NO_TERMS_UP) {
+      bad = true;
+      x[i] = 0.f;
+    }
+  uint2 hi, mid, lo;
+  split_up(x[0], x[1]);
+  split_up(x[2], x[3]);
+  split3(x[0], x[1], hi.x, mid.x, lo.x);
+  split3(x[2], x[3], hi.y, mid.y, lo.y);
+  uint8_t* to = X + (size_t)(size >> 6) * CS_TERMS_TILE + token * 128 + ((((size >> 3) & 7) ^ (token & 7)) << 4) +
+                (size & 4) * 2;
+  *reinterpret_cast<uint2*>(to) = hi;
+  *reinterpret_cast<uint2*>(to + CS_TERMS_TERM) = mid;
+  *reinterpret_cast<uint2*>(to + 2 * CS_TERMS_TERM) = lo;
+  return bad;
+}
 // Two blocks beside those of a chunk and head's products, which the double tensor pipe bounds, where these are
 // bound by memory: q's terms (what 0) and k's.
 template <int THREADS>
@@ -905,8 +927,10 @@ __device__ __forceinline__ void ds_cp16(float* smem, const float* gmem, bool ok)
 __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     DsIn p, const int* __restrict__ q_start, const double* __restrict__ F,
     const float* __restrict__ KKm, float* __restrict__ W, float* __restrict__ Y,
-    const float* __restrict__ qkm, CtHead* __restrict__ Ww) {
+    const float* __restrict__ qkm, CtHead* __restrict__ Ww, uint8_t* __restrict__ Xw,
+    unsigned long long* __restrict__ odd_w) {
   extern __shared__ __align__(16) float ds_smem[];
+  __shared__ unsigned long long odd;
   float* Ks = ds_smem;                           // [64][DS_P]
   float* Vs = Ks + DS_C * DS_P;                  // [64][DS_P]
   float* Ls = Vs + DS_C * DS_P;                  // [64][68]
@@ -933,6 +957,7 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
   if (Ww)                                        // (its tables lie where L and T will)
     ct_weights(f, f, f0, n, 1.f, qkm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C,
                *reinterpret_cast<CtWeights*>(Ls), Ww + (size_t)blockIdx.x * p.H + h);
+  if (tid == 0) odd = 0ull;
   if (tid < DS_C) {
     fs[tid] = tid < n ? f[tid] - f0 : 0.0;
     beta[tid] = tid < n ? p.gates[(size_t)(c.t0 + at + tid) * 2 * p.H + h] : 0.f;
@@ -1048,12 +1073,18 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
         cs_unpair(acc[i][j][0], r.x, r.y);
         cs_unpair(acc[i][j][1], r.z, r.w);
         *reinterpret_cast<float4*>(dst + (size_t)(ty * 4 + i) * width + col) = r;
+        // W in terms, too, for dt_walk
+        if (Xw && !what && cs_put_terms(Xw + ((size_t)blockIdx.x * p.H + h) * 2 * CS_TERMS_TILE, ty * 4 + i, col, r))
+          atomicOr(&odd, 1ull << (ty * 4 + i));
       }
+  }
+  if (Xw) {
+    __syncthreads();
+    if (tid == 0) odd_w[(size_t)blockIdx.x * p.H + h] = odd;
   }
 }
 
-// grid (column slices of 32, H, B): u [T][H][dv], Sc [chunk][H][dk][dv] (the state before each chunk; tiled:
-// as ct_state's U).
+// grid (column slices of 32, H, B): u [T][H][dv], Sc [chunk][H][dk][dv] (the state before each chunk).
 // 128 threads with 4 x 4 outputs of U and 8 x 4 of the state each: what a thread reads from shared
 // memory (at 128 bytes a cycle and SM) is about what its multiply-adds take.  1,111 and 694 tokens of
 // 16 heads of 128: 115 us; 256 threads with half of that 130, and the state's columns in the lanes'
@@ -1063,7 +1094,7 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
     float* __restrict__ state, long long slot_stride, const double* __restrict__ F,
     const float2* __restrict__ Wl, const float* __restrict__ W, const float* __restrict__ Y,
     float* __restrict__ u,
-    float* __restrict__ Sc, bool tiled, int* __restrict__ err) {
+    float* __restrict__ Sc, int* __restrict__ err) {
   extern __shared__ __align__(16) float ds_smem[];
   constexpr int PS = DS_NS + 4;
   float* Ws = ds_smem;                           // [2][64][DS_P]
@@ -1125,8 +1156,7 @@ __global__ void __launch_bounds__(128) ds_walk_kernel(
 #pragma unroll
       for (int r = 0; r < 8; ++r)
         if (ty * 8 + r < p.dk)
-          *reinterpret_cast<float4*>(tiled ? Sc + (chunk * p.dv + col0) * p.dk + (ty * 8 + r) * DS_NS + ((tx ^ r) << 2)
-                                           : Sc + (chunk * p.dk + ty * 8 + r) * p.dv + col) =
+          *reinterpret_cast<float4*>(Sc + (chunk * p.dk + ty * 8 + r) * p.dv + col) =
               *reinterpret_cast<const float4*>(Ss + (ty * 8 + r) * PS + 4 * tx);
     }
     // U = Y - W S, in runs of 16 terms
@@ -1366,7 +1396,7 @@ BF_EXPORT int bf_chunk_scan_mlstm_kernels(const void* proj, long long stride, in
 // The gated delta rule.  Scratch: F (G and H are the same array), g0, Wl | qkm | kkm | W | Y |
 // u | Sc.
 struct DsLayout {
-  size_t F, g0, Wl, qkm, kkm, W, Y, u, Sc, Xq, odd, Ww, total;
+  size_t F, g0, Wl, qkm, kkm, W, Y, u, Sc, Xq, Xk, odd, Ww, Xw, odd_w, total;
   int chunks;
 };
 static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min, bool terms) {
@@ -1388,6 +1418,9 @@ static DsLayout ds_layout(int T, int B, int H, int G, int dk, int dv, int n_min,
   l.u = take((size_t)T * H * dv * 4);
   l.Sc = take((size_t)l.chunks * H * dk * dv * 4);
   l.Xq = take(terms ? ct_terms_bytes(l.chunks, G, dk) : 0);
+  l.Xk = take(terms ? ct_terms_bytes(l.chunks, G, dk) : 0);
+  l.Xw = take(terms ? ct_terms_bytes(l.chunks, H, dk) : 0);
+  l.odd_w = take(terms ? (size_t)l.chunks * H * 8 : 0);
   l.odd = take(terms ? (size_t)l.chunks * G * 16 : 0);
   l.Ww = take(terms ? (size_t)l.chunks * H * sizeof(CtHead) : 0);
   l.total = at;
@@ -1451,18 +1484,23 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
   cs_gates_kernel<false><<<dim3(H, B), CS_GATE_THREADS, 0, stream>>>(
       nullptr, gates + H, nullptr, state, slot_stride, dk * dv, q_start, state_slots, n_slots, F, F,
       nullptr, g0, Wl, DS_C, T, H, dk * dv, dk, n_min, 2 * H);
-  const CsTerms x = {Xq, nullptr, odd};
-  if (const int e = bf_launch_pdl(cs_qk_kernel<float, true>, dim3(l.chunks, G, x.q ? 2 : 1), dim3(256), 0, stream, qkv, p, q_start,
+  const CsTerms x = {Xq, terms ? (uint8_t*)base + l.Xk : nullptr, odd};
+  uint8_t* Xw = terms ? (uint8_t*)base + l.Xw : nullptr;
+  unsigned long long* odd_w = (unsigned long long*)(base + l.odd_w);
+  if (const int e = bf_launch_pdl(cs_qk_kernel<float, true>, dim3(l.chunks, G, x.q ? 3 : 1), dim3(256), 0, stream, qkv, p, q_start,
                                   qkm, kkm, x))
     return e;
   ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, kkm, W,
-                                                                            Y, qkm, terms ? Ww : nullptr);
-  ds_walk_kernel<<<dim3((dv + DS_NS - 1) / DS_NS, H, B), 128, smem_walk, stream>>>(
-      d, q_start, state_slots, n_slots, state, slot_stride, F, Wl, W, Y, u, Sc, terms, err);
-  if (terms)
+                                                                            Y, qkm, terms ? Ww : nullptr, Xw, odd_w);
+  if (terms) {
+    dt_walk_kernel<<<dim3(dv / CT_SV, H, B), DT_THREADS, DT_SMEM, stream>>>(
+        d, q_start, state_slots, n_slots, state, slot_stride, F, Wl, W, Y, Xw, odd_w, x.k, odd, u, Sc, err);
     ct_out_launch(qkv, u, p, l.chunks, q_start, state_slots, n_slots, F, F, Ww, qkm, Xq, odd, Sc, o_raw, err, stream);
-  else
-    cs_out_kernel<float, float, false, true>
+    return bf_launch_status();
+  }
+  ds_walk_kernel<<<dim3((dv + DS_NS - 1) / DS_NS, H, B), 128, smem_walk, stream>>>(
+      d, q_start, state_slots, n_slots, state, slot_stride, F, Wl, W, Y, u, Sc, err);
+  cs_out_kernel<float, float, false, true>
       <<<dim3(l.chunks, H, (dv + CS_T - 1) / CS_T), CS_THREADS, 0, stream>>>(
           qkv, u, p, q_start, state_slots, n_slots, F, F, g0, nullptr, qkm, Sc, nullptr, o_raw);
   return bf_launch_status();

@@ -6,6 +6,7 @@
 //   ct_weights q . k with the weights of a head's tokens
 //   ct_state   what cs_state and cs_prefix compute: a CTA keeps 128 key x 32 value sizes of a head's state in
 //              registers and goes from chunk to chunk; the states between the chunks are written once
+//   dt_walk    what ds_walk computes, the delta rule's chain
 //   ct_out     what cs_out computes: 128 value sizes (of one head, or of two heads of 64) x 64 tokens a tile,
 //              a CTA an SM goes from tile to tile
 //
@@ -25,14 +26,15 @@
 // Operands that have no terms (infinities, NaN, floats from 2^104 on) are zero in the products, and what they
 // reach is computed by multiply-adds in cs_state's and cs_out's order; so are sums that are not finite.
 //
-// 2,000 tokens of 64 heads of 128 x 64 over 8: ct_state 35 us (cs_state and cs_prefix 87), ct_weights 15, ct_out 56
-// (cs_out 100); 1,300 and 812 tokens of 8 heads of 128 x 256: 24 (47), 5, 29 (58); the delta rule's 1,111 and 694 of
-// 16 heads of 128: ct_out 29 (cs_out 53), ds_prep 51 (47).  What bounds them is the rate at which their warps get
-// instructions (0.45 a cycle and scheduler): ct_out's time changes by 0 to 3 us without its stores, with loads that
-// always hit, with half of the products or without taking the operands apart.
-// Relative errors against 64 bits (outputs, states), these / multiply-adds, e-7: decays of 0.98 to 1 0.88 0.69 / 1.37
-// 1.29, a state space layer's 0.67 0.51 / 0.68 0.59; decays spread over 0 to 1 0.62 0.59 / 0.50 0.42 (there one or
-// two tokens make up a sum, which the tensor core cuts where a multiply-add rounds).
+// 2,000 tokens of 64 heads of 128 x 64 over 8: ct_state 39 us (cs_state and cs_prefix 87), ct_weights 15, ct_out 58
+// (cs_out 100); 1,300 and 812 tokens of 8 heads of 128 x 256: 27 (47), 5, 30 (58); the delta rule's 1,111 and 694 of
+// 16 heads of 128: dt_walk 70 (ds_walk 108), ct_out 30 (cs_out 53), ds_prep 54 (47).  What bounds ct_out is the rate
+// at which its warps get instructions (0.45 a cycle and scheduler): its time changes by 0 to 3 us without its
+// stores, with loads that always hit, with half of the products or without taking the operands apart.  ct_state and
+// dt_walk are bound by their chains: some 2,300 and 7,000 cycles a chunk.
+// Relative errors against 64 bits (outputs, states), these / multiply-adds, e-7: decays of 0.98 to 1 0.79 0.66 / 1.37
+// 1.29, a state space layer's 0.55 0.46 / 0.68 0.59, spread over 0 to 1 0.51 0.42 / 0.50 0.42; the delta rule's 0.97
+// 0.86 / 1.63 1.80, 0.66 0.59 / 0.77 0.68, 0.58 0.55 / 0.57 0.48.
 //
 // Included by chunk_scan.cu behind mlstm_tensor.cuh.
 #pragma once
@@ -41,6 +43,7 @@
 #define CT_TERM CS_TERMS_TERM         // a term of a tile: 64 rows (tokens) of 64 numbers
 #define CT_TILE CS_TERMS_TILE         // 64 tokens x 64 sizes of q or k
 constexpr float CT_DOWN = SPLIT_DOWN * SPLIT_DOWN;
+constexpr float CT_CUT = 1.f / 33554432.f;               // 2^-25
 
 __device__ __forceinline__ unsigned long long ct_mul2(unsigned long long x, unsigned long long y) {
   unsigned long long r;
@@ -76,9 +79,13 @@ __device__ __forceinline__ void ct_products(uint32_t d, uint32_t a, uint32_t ter
   }
 }
 
-// Eight columns of such a step's four places, added up
+// Eight columns of such a step's four places: the sums of the leading products' 32 terms that come last (`second`:
+// the second 32), and of all others.  Where decays are fast the last terms make up the result, so they are added
+// last; and their sum, which the tensor core cuts, is half a unit too small on average: 2^-25 of it is added to the
+// others (less than half a unit, so that a sum that is exact stays so).
 template <int N>
-__device__ __forceinline__ void ct_take(uint32_t at, unsigned long long (&u)[4]) {
+__device__ __forceinline__ void ct_take(uint32_t at, bool second, unsigned long long (&last)[4],
+                                        unsigned long long (&rest)[4]) {
   uint32_t r[32];
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%32];\n\t"
@@ -91,7 +98,7 @@ __device__ __forceinline__ void ct_take(uint32_t at, unsigned long long (&u)[4])
         "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
         "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
         "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(at), "r"(at + N), "r"(at + 2 * N), "r"(at + 3 * N)
+      : "r"(second ? at : at + 3 * N), "r"(at + N), "r"(at + 2 * N), "r"(second ? at + 3 * N : at)
       : "memory");
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -99,7 +106,8 @@ __device__ __forceinline__ void ct_take(uint32_t at, unsigned long long (&u)[4])
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       x[k] = cs_pair(__uint_as_float(r[8 * k + 2 * i]), __uint_as_float(r[8 * k + 2 * i + 1]));
-    u[i] = cs_add2(cs_add2(x[0], x[3]), cs_add2(x[1], x[2]));
+    last[i] = x[3];
+    rest[i] = cs_add2(x[0], cs_fma2(x[3], cs_pair(CT_CUT, CT_CUT), cs_add2(x[1], x[2])));
   }
 }
 
@@ -499,15 +507,20 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       ct_wait(sh.done + (i & 1), (i >> 1) & 1, &sh.abort);
       __syncwarp();
       tc_fence_after();
-      unsigned long long u[CT_SV / 2], zero = 0ull;      // (NaN where some sum is not finite)
+      // S <- last + (decay S + rest): where decays are fast the last tokens make up the state, rounded once
+      unsigned long long was[CT_SV / 2], zero = 0ull;    // zero: NaN where some sum is not finite
+      const bool second = c.n - i * CT_C > 32;
+      const unsigned long long dx2 = cs_pair(dx, dx), dy2 = cs_pair(dy, dy), down = cs_pair(CT_DOWN, CT_DOWN);
 #pragma unroll
       for (int j0 = 0; j0 < CT_SV / 2; j0 += 4) {
-        unsigned long long x[4];
-        ct_take<CT_SV>(from + (uint32_t)((i & 1) * 4 * CT_SV + 2 * j0), x);
+        unsigned long long last[4], rest[4];
+        ct_take<CT_SV>(from + (uint32_t)((i & 1) * 4 * CT_SV + 2 * j0), second, last, rest);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          zero = cs_fma2(x[j], 0ull, zero);
-          u[j0 + j] = ct_mul2(x[j], CT_DOWN);
+          zero = cs_fma2(cs_add2(last[j], rest[j]), 0ull, zero);
+          const unsigned long long before = S[j0 + j];
+          was[j0 + j] = before;
+          S[j0 + j] = cs_fma2(last[j], down, cs_fma2(dx2, before, cs_fma2(dy2, before, ct_mul2(rest[j], down))));
         }
       }
       tc_fence_before();
@@ -524,16 +537,16 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
                        min(CT_C, c.n - i * CT_C), again);
 #pragma unroll
         for (int j = 0; j < CT_SV / 2; ++j) {
-          float a, e;
-          cs_unpair(u[j], a, e);
-          if (bad_now || (odd_cols >> (2 * j) & 1) || !(fabsf(a) < INFINITY)) a = again[2 * j];
-          if (bad_now || (odd_cols >> (2 * j + 1) & 1) || !(fabsf(e) < INFINITY)) e = again[2 * j + 1];
-          u[j] = cs_pair(a, e);
+          float x[2], b[2];
+          cs_unpair(S[j], x[0], x[1]);
+          cs_unpair(was[j], b[0], b[1]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (bad_now || (odd_cols >> (2 * j + e) & 1) || !(fabsf(x[e]) < INFINITY))
+              x[e] = fmaf(dx, b[e], fmaf(dy, b[e], again[2 * j + e]));
+          S[j] = cs_pair(x[0], x[1]);
         }
       }
-      const unsigned long long dx2 = cs_pair(dx, dx), dy2 = cs_pair(dy, dy);
-#pragma unroll
-      for (int j = 0; j < CT_SV / 2; ++j) S[j] = cs_fma2(dx2, S[j], cs_fma2(dy2, S[j], u[j]));
     }
 #pragma unroll
     for (int j = 0; j < CT_SV / 2; ++j) {
@@ -901,21 +914,21 @@ __global__ void __launch_bounds__(CT_O_THREADS, 1) ct_out_kernel(
         if (s < steps) {
 #pragma unroll
           for (int j0 = 0; j0 < 16; j0 += 4) {
-            unsigned long long v[4];
-            ct_take<CT_C>(from + (uint32_t)((is & 1) * 4 * CT_C + 2 * j0), v);
+            unsigned long long last[4], rest[4];
+            ct_take<CT_C>(from + (uint32_t)((is & 1) * 4 * CT_C + 2 * j0), t_first > 0, last, rest);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sum[j0 + j] = cs_add2(sum[j0 + j], v[j]);
+            for (int j = 0; j < 4; ++j) sum[j0 + j] = cs_add2(sum[j0 + j], cs_add2(last[j], rest[j]));
           }
         } else if (s - steps == own) {                   // (the weights were there before that step's q . k)
 #pragma unroll
           for (int j0 = 0; j0 < 16; j0 += 4) {
-            unsigned long long v[4];
-            ct_take<CT_C>(from + (uint32_t)((is & 1) * 4 * CT_C + 2 * j0), v);
+            unsigned long long last[4], rest[4];
+            ct_take<CT_C>(from + (uint32_t)((is & 1) * 4 * CT_C + 2 * j0), t_first > 0, last, rest);
 #pragma unroll
             for (int j = j0; j < j0 + 4; ++j) {
               const unsigned long long w = *reinterpret_cast<const unsigned long long*>(at + 2 * j);
               const unsigned long long wl = *reinterpret_cast<const unsigned long long*>(at + CT_C + 2 * j);
-              sum[j] = cs_add2(cs_fma2(sum[j], w, ct_mul2(sum[j], wl)), v[j - j0]);
+              sum[j] = cs_add2(cs_add2(cs_fma2(sum[j], w, ct_mul2(sum[j], wl)), rest[j - j0]), last[j - j0]);
               float a, b;
               cs_unpair(ct_mul2(sum[j], CT_DOWN), a, b);
               if (2 * j < n) dst[(size_t)(2 * j) * row] = a;
@@ -962,6 +975,332 @@ __global__ void __launch_bounds__(CT_O_THREADS, 1) ct_out_kernel(
   ct_end<CT_O_COLS>(sh, tmem, warp, 20, err);
 }
 
+// -------------------------------------------------------------------------------- dt_walk
+// The delta rule's chain from chunk to chunk (ds_walk) with keys of 128: U = Y - W S, S <- exp(F_C) S + K^T
+// (exp(F_C - F) U).  grid (32 value sizes, H, B).  Four warps keep 128 x 32 of the state, a row a thread, and take
+// each product's operand apart as the other's sums come; one warp issues products, one asks for W's and K's tiles
+// (X: W in terms, chunk and head by chunk and head).  The state before a chunk leaves as ct_state's does.
+//
+// W S: 64 tokens x 32 columns over 128 terms, leading terms' products summed 32 at a time (four places), the
+// others' in two; a warp reads its 16 rows in the shape of a fragment, rows lane / 4 and eight further, so that
+// neighbouring tokens, which lie side by side in the next operand, are one exchange away.
+#define DT_TERM (CT_SV * 128)                            // 32 columns x 64 terms
+#define DT_SMEM (1024 + 2 * CT_S_KEYS + 9 * DT_TERM + 128 * CT_SV * 4 + CT_C * CT_SV * 4)
+#define DT_THREADS 192
+#define DT_SUMS 192                                      // columns of W S's places; K^T U's four of 32 behind them
+
+// rows' terms K-major (two tiles of 64 sizes) times columns' (two tiles of 32 x 64)
+__device__ __forceinline__ void dt_products(uint32_t d, uint32_t a, uint32_t b) {
+  constexpr uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(64 >> 4) << 24);
+  constexpr uint32_t one = base | ((uint32_t)(32 >> 3) << 17), two = base | ((uint32_t)(64 >> 3) << 17),
+                     three = base | ((uint32_t)(96 >> 3) << 17);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t ak = a + (k >> 2) * CT_TILE + (k & 3) * 32, bk = b + (k >> 2) * 3 * DT_TERM + (k & 3) * 32;
+    const uint64_t hi = umma_desc_k_sw128(ak), mid = umma_desc_k_sw128(ak + CT_TERM),
+                   lo = umma_desc_k_sw128(ak + 2 * CT_TERM), bh = umma_desc_k_sw128(bk),
+                   bm = umma_desc_k_sw128(bk + DT_TERM);
+    if (k < 2) {
+      umma_bf16(d, hi, bh, three, k > 0);
+    } else {
+      umma_bf16(d + 64 + (k >> 1) * 32, hi, bh, one, k & 1);
+      umma_bf16(d + 32, hi, bm, two, 1);
+    }
+    umma_bf16(d + 32, mid, bh, two, 1);
+    umma_bf16(d + 64, lo, bh, one, 1);
+  }
+}
+__device__ __forceinline__ void dt_load(uint32_t at, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(at));
+}
+// Two neighbouring numbers of a row of terms, times SPLIT_UP, to `at` (a term's tile DT_TERM behind the one
+// before); numbers without terms as zeros, and true
+__device__ __forceinline__ bool dt_put(uint8_t* at, float a, float b) {
+  const bool bad_a = (__float_as_uint(a) & 0x7fffffffu) >= CS_NO_TERMS_UP,
+             bad_b = (__float_as_uint(b) & 0x7fffffffu) >= CS_NO_TERMS_UP;
+  if (bad_a) a = 0.f;
+  if (bad_b) b = 0.f;
+  uint32_t hi, mid, lo;
+  split_up(a, b);
+  split3(a, b, hi, mid, lo);
+  *reinterpret_cast<uint32_t*>(at) = hi;
+  *reinterpret_cast<uint32_t*>(at + DT_TERM) = mid;
+  *reinterpret_cast<uint32_t*>(at + 2 * DT_TERM) = lo;
+  return bad_a || bad_b;
+}
+// W S of two rows and their eight columns (8 c + col, + 1) by multiply-adds, in ds_walk's order
+__device__ __noinline__ void dt_again_ws(const float* w0, const float* w1, const float* kept, int col, float* out) {
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int k0 = 0; k0 < 128; k0 += 16) {
+      float run[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int k = k0; k < k0 + 16; ++k) {
+        const int v = 8 * c + col;
+        const float2 x = *reinterpret_cast<const float2*>(kept + k * CT_SV + (((v >> 2) ^ (k & 7)) << 2) + (v & 3));
+        run[0] = fmaf(w0[k], x.x, run[0]);
+        run[1] = fmaf(w0[k], x.y, run[1]);
+        run[2] = fmaf(w1[k], x.x, run[2]);
+        run[3] = fmaf(w1[k], x.y, run[3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] += run[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[4 * c + j] = o[j];
+  }
+}
+// a row of the state behind the chunk by multiply-adds, one chain a number
+__device__ __noinline__ void dt_again_state(const float* k, long long k_stride, const float* us, int n, float2 g,
+                                            const float* was, float* out) {
+#pragma unroll 1
+  for (int j = 0; j < CT_SV; ++j) {
+    float x = cs_times(was[j], g);
+#pragma unroll 4
+    for (int s = 0; s < n; ++s) x = fmaf(k[(size_t)s * k_stride], us[s * CT_SV + j], x);
+    out[j] = x;
+  }
+}
+
+__global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
+    DsIn p, const int* __restrict__ q_start, const int* __restrict__ state_slots, int n_slots,
+    float* __restrict__ state, long long slot_stride, const double* __restrict__ F,
+    const float2* __restrict__ Wl, const float* __restrict__ W, const float* __restrict__ Y,
+    const uint8_t* __restrict__ Xw, const unsigned long long* __restrict__ odd_w, const uint8_t* __restrict__ Xk,
+    const unsigned long long* __restrict__ odd_rows, float* __restrict__ u, float* __restrict__ Sc,
+    int* __restrict__ err) {
+  extern __shared__ __align__(16) uint8_t ct_raw[];
+  __shared__ CtShared sh;                                // full, free: W's and K's tiles; put, done: S's and U's operands
+  __shared__ int odd_s[2];                               // of S and of U: chunk + 1 where a number has no terms
+  uint8_t* w_tile = ct_raw + ((1024u - (smem_u32(ct_raw) & 1023u)) & 1023u);
+  uint8_t* k_tile = w_tile + CT_S_KEYS;
+  uint8_t* s_op = k_tile + CT_S_KEYS;                    // two tiles of three terms
+  uint8_t* u_op = s_op + 6 * DT_TERM;
+  float* kept = reinterpret_cast<float*>(u_op + 3 * DT_TERM);            // [128][32]
+  float* us = kept + 128 * CT_SV;                        // [64][32]
+  const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * CT_SV;
+  const CsChunk c = cs_find(q_start, p.B, CT_C, p.n_min, 0, b);
+  if (c.n <= p.n_min) return;
+  const int slot = state_slots[b];
+  if (slot < 0 || slot >= n_slots) {
+    if (threadIdx.x == 0) atomicOr(err, BF_ERR_SLOT);
+    return;
+  }
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int hq = h / (p.H / p.G), chunks = (c.n + CT_C - 1) / CT_C;
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(sh.full + i, 1);
+      mbar_init(sh.free + i, 1);
+      mbar_init(sh.put + i, 4);
+      mbar_init(sh.done + i, 1);
+      odd_s[i] = 0;
+    }
+    mbar_init(&sh.drain, 2);
+    sh.abort = 0;
+  }
+  const uint32_t tmem = ct_begin<512>(sh, warp, 4);
+
+  if (warp == 5) {                                       // ---- tiles; (also of the second warp that ct_end expects)
+    if (lane == 0) {
+      uint32_t phase = 0;
+      bool ok = true;
+      int asked = 0;                                     // fills of both places in turn
+      for (int i = 0; i < chunks && ok; ++i, phase ^= 1u) {
+        const size_t chunk = (size_t)(c.first + i);
+        for (int x = 0; x < 2 && ok; ++x) {
+          ok = i == 0 || ct_wait(sh.free + x, phase ^ 1u, &sh.abort);
+          if (!ok) break;
+          mbar_expect_tx(sh.full + x, CT_S_KEYS);
+          bf_bulk_load(x ? k_tile : w_tile, x ? Xk + (chunk * p.G + hq) * CT_S_KEYS : Xw + (chunk * p.H + h) * CT_S_KEYS,
+                       CT_S_KEYS, sh.full + x);
+          ++asked;
+        }
+      }
+      if (*(volatile int*)&sh.abort) mbar_drain(sh.full, 2, asked & 1, (uint32_t)(asked >> 1) & 1u);
+    }
+    __syncwarp();
+  } else if (warp == 4) {                                // ---- products
+    for (int i = 0; i < chunks; ++i) {
+      ct_wait_warp(sh.full, i & 1, &sh.abort);
+      ct_wait_warp(sh.put, i & 1, &sh.abort);
+      ct_fence();
+      tc_fence_after();
+      dt_products(tmem, smem_u32(w_tile), smem_u32(s_op));
+      umma_commit(sh.done);
+      umma_commit(sh.free);
+      ct_wait_warp(sh.full + 1, i & 1, &sh.abort);
+      ct_wait_warp(sh.put + 1, i & 1, &sh.abort);
+      ct_fence();
+      tc_fence_after();
+      ct_products<CT_SV>(tmem + DT_SUMS, smem_u32(k_tile), CT_TERM, CT_TILE, smem_u32(u_op));
+      umma_commit(sh.done + 1);
+      umma_commit(sh.free + 1);
+    }
+  } else {
+    float* st = state + (size_t)slot * slot_stride + ((size_t)h * p.dv + col0) * 128 + tid;
+    const double* f = F + (size_t)h * p.T + c.t0;
+    const float2* wl = Wl + (size_t)h * p.T + c.t0;
+    const uint32_t from = tmem + ((uint32_t)(warp * 32) << 16);
+    const int r = lane >> 2, q = 2 * (lane & 3);         // of W S: rows 16 warp + r, + 8, columns 8 c + q, + 1
+    const int t_own = 16 * warp + r;
+    float S[CT_SV];
+#pragma unroll
+    for (int j = 0; j < CT_SV; ++j) S[j] = st[(size_t)j * 128];
+    double before = 0.0;
+    for (int i = 0; i < chunks; ++i) {
+      const int n = min(CT_C, c.n - i * CT_C);
+      const size_t chunk = (size_t)(c.first + i) * p.H + h;
+      const float* y_at = Y + (chunk * CT_C + t_own) * p.dv + col0 + q;
+      float2 y[2][4], g_t[2];                            // (asked for ahead of the products that need them)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[x][j] = *reinterpret_cast<const float2*>(y_at + (size_t)(8 * x) * p.dv + 8 * j);
+        const int t = t_own + 8 * x;
+        g_t[x] = t < n ? wl[i * CT_C + t] : make_float2(0.f, 0.f);
+      }
+      const unsigned long long bad_w = odd_w[chunk], bad_k = odd_rows[((size_t)(c.first + i) * p.G + hq) * 2 + 1];
+      const double last = f[i * CT_C + n - 1];
+      // ---- the state: as it is, and in terms
+      if (tid == 0) bf_bulk_wait_read<0>();
+      asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+#pragma unroll
+      for (int x = 0; x < CT_SV / 4; ++x)
+        *reinterpret_cast<float4*>(kept + tid * CT_SV + ((x ^ (tid & 7)) << 2)) =
+            make_float4(S[4 * x], S[4 * x + 1], S[4 * x + 2], S[4 * x + 3]);
+      {
+        // keys tid and its neighbour: the even one takes the first sixteen columns of both
+        const bool second = tid & 1;
+        uint8_t* to = s_op + (tid >> 6) * 3 * DT_TERM + (tid & 6) * 2;
+        const int piece = (tid & 63) >> 3;
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < CT_SV / 2; ++j) {
+          const float keep = second ? S[j + CT_SV / 2] : S[j], give = second ? S[j] : S[j + CT_SV / 2];
+          const float got = __shfl_xor_sync(0xffffffffu, give, 1);
+          const int v = j + (second ? CT_SV / 2 : 0);
+          bad |= dt_put(to + v * 128 + ((piece ^ (j & 7)) << 4), second ? got : keep, second ? keep : got);
+        }
+        if (bad) odd_s[0] = i + 1;
+      }
+      ct_arrive(sh.put);
+      asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+      if (tid == 0) {
+        ct_fence();
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                         Sc + (chunk * p.dv + col0) * 128),
+                     "r"(smem_u32(kept)), "r"(128 * CT_SV * 4)
+                     : "memory");
+        bf_bulk_commit();
+      }
+      const float2 g = cs_exp(last - before);
+      before = last;
+      // ---- U
+      ct_wait(sh.done, i & 1, &sh.abort);
+      __syncwarp();
+      tc_fence_after();
+      float a[16];                                       // [column block][row, column]: rows t_own, + 8
+      {
+        uint32_t x0[16], x1[16], x2[16], x3[16], x4[16], x5[16];
+        dt_load(from, x0);
+        dt_load(from + 96, x1);
+        dt_load(from + 128, x2);
+        dt_load(from + 160, x3);
+        dt_load(from + 32, x4);
+        dt_load(from + 64, x5);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float lead = (__uint_as_float(x0[j]) + __uint_as_float(x1[j])) +
+                             (__uint_as_float(x2[j]) + __uint_as_float(x3[j]));
+          a[j] = (lead + (__uint_as_float(x4[j]) + __uint_as_float(x5[j]))) * CT_DOWN;
+        }
+      }
+      float zero = 0.f;                                  // (NaN where some sum is not finite)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) zero = fmaf(a[j], 0.f, zero);
+      const bool odd = *(volatile int*)&odd_s[0] == i + 1;
+      if (odd || (bad_w >> t_own & 0x101ull) || zero != 0.f) {
+        float again[16];
+        dt_again_ws(W + (chunk * CT_C + t_own) * 128, W + (chunk * CT_C + t_own + 8) * 128, kept, q, again);
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (odd || (bad_w >> (t_own + (j & 2) * 4) & 1ull) || !(fabsf(a[j]) < INFINITY)) a[j] = again[j];
+      }
+      bool bad = false;
+      {
+        // tokens t_own and its neighbour (lane ^ 4): the even one takes the first column of both
+        const bool second = r & 1;
+        float* u_at = u + ((size_t)(c.t0 + i * CT_C + t_own) * p.H + h) * p.dv + col0 + q;
+        uint8_t* to = u_op + ((q + second) & 7) * 128 + (r & 6) * 2;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 uv = make_float2(y[x][j].x - a[4 * j + 2 * x], y[x][j].y - a[4 * j + 2 * x + 1]);
+            if (t_own + 8 * x < n)
+              *reinterpret_cast<float2*>(u_at + (size_t)(8 * x) * p.H * p.dv + 8 * j) = uv;
+            const float2 w = make_float2(cs_times(uv.x, g_t[x]), cs_times(uv.y, g_t[x]));
+            *reinterpret_cast<float2*>(us + (t_own + 8 * x) * CT_SV + 8 * j + q) = w;
+            const float keep = second ? w.y : w.x, got = __shfl_xor_sync(0xffffffffu, second ? w.x : w.y, 4);
+            bad |= dt_put(to + 8 * j * 128 + (((2 * warp + x) ^ ((q + second) & 7)) << 4), second ? got : keep,
+                          second ? keep : got);
+          }
+        if (bad) odd_s[1] = i + 1;
+      }
+      tc_fence_before();
+      ct_arrive(sh.put + 1);
+      // ---- the state behind the chunk
+      ct_wait(sh.done + 1, i & 1, &sh.abort);
+      __syncwarp();
+      tc_fence_after();
+      float now[CT_SV], z = 0.f;                         // z: NaN where some sum is not finite
+#pragma unroll
+      for (int j0 = 0; j0 < CT_SV / 2; j0 += 4) {
+        unsigned long long x[4], y[4];
+        ct_take<CT_SV>(from + DT_SUMS + (uint32_t)(2 * j0), n > 32, x, y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float l[2], m[2];
+          cs_unpair(x[j], l[0], l[1]);
+          cs_unpair(ct_mul2(y[j], CT_DOWN), m[0], m[1]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {                  // (as in ct_state)
+            const float was = S[2 * (j0 + j) + e];
+            now[2 * (j0 + j) + e] = fmaf(l[e], CT_DOWN, fmaf(g.x, was, fmaf(g.y, was, m[e])));
+            z = fmaf(l[e] + m[e], 0.f, z);
+          }
+        }
+      }
+      tc_fence_before();
+      if (*(volatile int*)&odd_s[1] == i + 1 || bad_k || z != 0.f) {
+        // (all rows of us are there: their products are)
+        float was[CT_SV], again[CT_SV];
+#pragma unroll
+        for (int j = 0; j < CT_SV; ++j) was[j] = S[j];
+        dt_again_state(p.qkv + (size_t)(c.t0 + i * CT_C) * p.stride + (size_t)(p.G + hq) * 128 + tid, p.stride, us, n,
+                       g, was, again);
+#pragma unroll
+        for (int j = 0; j < CT_SV; ++j) now[j] = again[j];
+      }
+#pragma unroll
+      for (int j = 0; j < CT_SV; ++j) S[j] = now[j];
+    }
+#pragma unroll
+    for (int j = 0; j < CT_SV; ++j) st[(size_t)j * 128] = S[j];
+    if (tid == 0) bf_bulk_wait_read<0>();
+  }
+  ct_end<512>(sh, tmem, warp, 4, err);
+}
+
 // Chunks of 64, keys in whole steps of 128, values of 64 or in whole tiles of 128 (two heads of 64 share a
 // tile: an even number of them, reading the same q).
 static bool ct_takes(int H, int QH, int dk, int dv, int C, int chunks) {
@@ -979,6 +1318,8 @@ static int ct_configure() {
                                          CT_S_SMEM);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(ct_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_O_SMEM);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(dt_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_SMEM);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
