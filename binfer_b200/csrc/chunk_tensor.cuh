@@ -318,15 +318,15 @@ __global__ void __launch_bounds__(256) ct_weights_kernel(CsIn p, const int* __re
 #define CT_S_VALS (3 * CT_SV * 128)                      // the values' terms
 #define CT_S_RAW (CT_C * CT_SV * 4)                      // and as they come
 #define CT_S_SMEM (1024 + CT_S_RING * CT_S_KEYS + 2 * CT_S_VALS + 128 * CT_SV * 4 + 4 * (CT_S_RAW + CT_C * 8))
-#define CT_S_THREADS 352             // four warps that add, four that convert, one that copies, two for products
+#define CT_S_THREADS 480             // eight warps that add, four that convert, one that copies, two for products
 #define CT_S_COLS 256                                    // tensor memory: two places of 4 x 32 columns
 
-// the chunk's share of 32 elements of the state by multiply-adds, as cs_state sums it
+// the chunk's share of 16 elements of the state by multiply-adds, as cs_state sums it
 __device__ __noinline__ void ct_state_again(const float* __restrict__ k, long long k_stride,
                                             const float* __restrict__ v, long long v_stride,
                                             const float2* __restrict__ wl, int n, float* u) {
 #pragma unroll 1
-  for (int j0 = 0; j0 < CT_SV; j0 += 8) {
+  for (int j0 = 0; j0 < CT_SV / 2; j0 += 8) {
     float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int s = 0; s < n; ++s) {
@@ -376,15 +376,15 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
     for (int i = 0; i < 2; ++i) {
       mbar_init(sh.put + i, 4);
       mbar_init(sh.done + i, 1);
-      mbar_init(sh.taken + i, 4);
+      mbar_init(sh.taken + i, 8);
     }
     mbar_init(&sh.drain, 2);
     sh.abort = 0;
   }
   if (tid < 4 * CT_SV) odd_v[tid / CT_SV][tid % CT_SV] = 0;
-  const uint32_t tmem = ct_begin<CT_S_COLS>(sh, warp, 9);
+  const uint32_t tmem = ct_begin<CT_S_COLS>(sh, warp, 13);
 
-  if (warp == 8) {                                       // ---- k's tiles
+  if (warp == 12) {                                      // ---- k's tiles
     if (lane == 0) {
       int place = 0;
       uint32_t phase = 0;
@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       if (*(volatile int*)&sh.abort) mbar_drain(sh.full, CT_S_RING, place, phase);
     }
     __syncwarp();
-  } else if (warp >= 9) {                                // ---- products: chunks in turn
-    for (int i = warp - 9; i < chunks; i += 2) {
+  } else if (warp >= 13) {                               // ---- products: chunks in turn
+    for (int i = warp - 13; i < chunks; i += 2) {
       const int place = i % CT_S_RING;
       ct_wait_warp(sh.full + place, (i / CT_S_RING) & 1, &sh.abort);
       ct_wait_warp(sh.put + (i & 1), (i >> 1) & 1, &sh.abort);
@@ -412,9 +412,9 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       umma_commit(sh.free + place);
       umma_commit(sh.done + (i & 1));
     }
-  } else if (warp >= 4) {                                // ---- the values, weighted: lane = value size
+  } else if (warp >= 8) {                                // ---- the values, weighted: lane = value size
     // (this warp's tokens of a chunk: two runs of eight, w and w + 4)
-    const int w = warp - 4;
+    const int w = warp - 8;
     uint8_t* mine = raw + w * (CT_S_RAW / 4);
     float2* mine_w = raw_w + w * 16;
     auto token = [&](int r) { return 8 * w + (r & 7) + (r >> 3) * 32; };
@@ -466,16 +466,18 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       ct_arrive(sh.put + (i & 1));
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else {                                               // ---- the state: key size k0 + tid, 32 value sizes
+  } else {                                               // ---- the state: key size k0 + own, 16 value sizes
+    const int own = tid & 127, half = tid >> 7;
     const double* g = G + (size_t)h * p.T + c.t0;
-    float* st = state + (size_t)slot * slot_stride + (size_t)h * p.dv * p.dk + (size_t)v0 * p.dk + k0 + tid;
+    float* st = state + (size_t)slot * slot_stride + (size_t)h * p.dv * p.dk +
+                (size_t)(v0 + 16 * half) * p.dk + k0 + own;
     const unsigned long long* odd_k = odd_rows + ((size_t)c.first * p.QH + hq) * 2 + 1;
     float* to = U + (((size_t)c.first * p.H + h) * p.dv + v0) * p.dk + (size_t)k0 * CT_SV;
     const size_t step = (size_t)p.H * p.dv * p.dk;
-    const uint32_t from = tmem + ((uint32_t)(warp * 32) << 16);
-    unsigned long long S[CT_SV / 2];
+    const uint32_t from = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(16 * half);
+    unsigned long long S[CT_SV / 4];
 #pragma unroll
-    for (int j = 0; j < CT_SV / 2; ++j) S[j] = cs_pair(st[(size_t)(2 * j) * p.dk], st[(size_t)(2 * j + 1) * p.dk]);
+    for (int j = 0; j < CT_SV / 4; ++j) S[j] = cs_pair(st[(size_t)(2 * j) * p.dk], st[(size_t)(2 * j + 1) * p.dk]);
     float2 dec = make_float2(0.f, 0.f);                  // (lane l: over chunk l of the current 32)
     unsigned long long bad_k = odd_k[0];
     for (int i = 0; i < chunks; ++i) {
@@ -486,15 +488,15 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       const float dx = __shfl_sync(0xffffffffu, dec.x, i & 31), dy = __shfl_sync(0xffffffffu, dec.y, i & 31);
       // the state before the chunk leaves
       if (tid == 0) bf_bulk_wait_read<0>();
-      asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+      asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
 #pragma unroll
-      for (int q = 0; q < CT_SV / 4; ++q) {
+      for (int q = 0; q < CT_SV / 8; ++q) {
         float4 x;
         cs_unpair(S[2 * q], x.x, x.y);
         cs_unpair(S[2 * q + 1], x.z, x.w);
-        *reinterpret_cast<float4*>(kept + tid * CT_SV + ((q ^ (tid & 7)) << 2)) = x;
+        *reinterpret_cast<float4*>(kept + own * CT_SV + (((q + 4 * half) ^ (own & 7)) << 2)) = x;
       }
-      asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+      asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
       if (tid == 0) {
         ct_fence();
         asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(to + i * step),
@@ -508,11 +510,11 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       __syncwarp();
       tc_fence_after();
       // S <- last + (decay S + rest): where decays are fast the last tokens make up the state, rounded once
-      unsigned long long was[CT_SV / 2], zero = 0ull;    // zero: NaN where some sum is not finite
+      unsigned long long was[CT_SV / 4], zero = 0ull;    // zero: NaN where some sum is not finite
       const bool second = c.n - i * CT_C > 32;
       const unsigned long long dx2 = cs_pair(dx, dx), dy2 = cs_pair(dy, dy), down = cs_pair(CT_DOWN, CT_DOWN);
 #pragma unroll
-      for (int j0 = 0; j0 < CT_SV / 2; j0 += 4) {
+      for (int j0 = 0; j0 < CT_SV / 4; j0 += 4) {
         unsigned long long last[4], rest[4];
         ct_take<CT_SV>(from + (uint32_t)((i & 1) * 4 * CT_SV + 2 * j0), second, last, rest);
 #pragma unroll
@@ -529,14 +531,14 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       cs_unpair(zero, z0, z1);
       const bool lost = z0 + z1 != 0.f;
       const bool odd = *(volatile int*)&odd_v[i & 3][lane] == i + 1;
-      const unsigned odd_cols = __ballot_sync(0xffffffffu, odd);
+      const unsigned odd_cols = __ballot_sync(0xffffffffu, odd) >> (16 * half) & 0xffffu;
       if (odd_cols || bad_now || lost) {
-        float again[CT_SV];
-        ct_state_again(qk + (size_t)(c.t0 + i * CT_C) * p.qk_stride + p.k_off + (size_t)hq * p.dk + k0 + tid,
-                       p.qk_stride, vp + (size_t)i * CT_C * p.v_stride, p.v_stride, wl + i * CT_C,
+        float again[CT_SV / 2];
+        ct_state_again(qk + (size_t)(c.t0 + i * CT_C) * p.qk_stride + p.k_off + (size_t)hq * p.dk + k0 + own,
+                       p.qk_stride, vp + (size_t)i * CT_C * p.v_stride + 16 * half, p.v_stride, wl + i * CT_C,
                        min(CT_C, c.n - i * CT_C), again);
 #pragma unroll
-        for (int j = 0; j < CT_SV / 2; ++j) {
+        for (int j = 0; j < CT_SV / 4; ++j) {
           float x[2], b[2];
           cs_unpair(S[j], x[0], x[1]);
           cs_unpair(was[j], b[0], b[1]);
@@ -549,7 +551,7 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
       }
     }
 #pragma unroll
-    for (int j = 0; j < CT_SV / 2; ++j) {
+    for (int j = 0; j < CT_SV / 4; ++j) {
       float a, e;
       cs_unpair(S[j], a, e);
       st[(size_t)(2 * j) * p.dk] = a;
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
     }
     if (tid == 0) bf_bulk_wait_read<0>();
   }
-  ct_end<CT_S_COLS>(sh, tmem, warp, 9, err);
+  ct_end<CT_S_COLS>(sh, tmem, warp, 13, err);
 }
 
 // ---------------------------------------------------------------------------------- ct_out
@@ -977,7 +979,7 @@ __global__ void __launch_bounds__(CT_O_THREADS, 1) ct_out_kernel(
 
 // -------------------------------------------------------------------------------- dt_walk
 // The delta rule's chain from chunk to chunk (ds_walk) with keys of 128: U = Y - W S, S <- exp(F_C) S + K^T
-// (exp(F_C - F) U).  grid (32 value sizes, H, B).  Four warps keep 128 x 32 of the state, a row a thread, and take
+// (exp(F_C - F) U).  grid (32 value sizes, H, B).  Eight warps keep 128 x 32 of the state, half a row a thread, and take
 // each product's operand apart as the other's sums come; one warp issues products, one asks for W's and K's tiles
 // (X: W in terms, chunk and head by chunk and head).  The state before a chunk leaves as ct_state's does.
 //
@@ -986,7 +988,7 @@ __global__ void __launch_bounds__(CT_O_THREADS, 1) ct_out_kernel(
 // neighbouring tokens, which lie side by side in the next operand, are one exchange away.
 #define DT_TERM (CT_SV * 128)                            // 32 columns x 64 terms
 #define DT_SMEM (1024 + 2 * CT_S_KEYS + 9 * DT_TERM + 128 * CT_SV * 4 + CT_C * CT_SV * 4)
-#define DT_THREADS 192
+#define DT_THREADS 320
 #define DT_SUMS 192                                      // columns of W S's places; K^T U's four of 32 behind them
 
 // rows' terms K-major (two tiles of 64 sizes) times columns' (two tiles of 32 x 64)
@@ -1010,13 +1012,10 @@ __device__ __forceinline__ void dt_products(uint32_t d, uint32_t a, uint32_t b) 
     umma_bf16(d + 64, lo, bh, one, 1);
   }
 }
-__device__ __forceinline__ void dt_load(uint32_t at, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(at));
+__device__ __forceinline__ void dt_load(uint32_t at, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(at));
 }
 // Two neighbouring numbers of a row of terms, times SPLIT_UP, to `at` (a term's tile DT_TERM behind the one
 // before); numbers without terms as zeros, and true
@@ -1033,10 +1032,10 @@ __device__ __forceinline__ bool dt_put(uint8_t* at, float a, float b) {
   *reinterpret_cast<uint32_t*>(at + 2 * DT_TERM) = lo;
   return bad_a || bad_b;
 }
-// W S of two rows and their eight columns (8 c + col, + 1) by multiply-adds, in ds_walk's order
+// W S of two rows and their four columns (8 c + col, + 1) by multiply-adds, in ds_walk's order
 __device__ __noinline__ void dt_again_ws(const float* w0, const float* w1, const float* kept, int col, float* out) {
 #pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < 2; ++c) {
     float o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int k0 = 0; k0 < 128; k0 += 16) {
@@ -1057,11 +1056,11 @@ __device__ __noinline__ void dt_again_ws(const float* w0, const float* w1, const
     for (int j = 0; j < 4; ++j) out[4 * c + j] = o[j];
   }
 }
-// a row of the state behind the chunk by multiply-adds, one chain a number
+// half a row of the state behind the chunk by multiply-adds, one chain a number
 __device__ __noinline__ void dt_again_state(const float* k, long long k_stride, const float* us, int n, float2 g,
                                             const float* was, float* out) {
 #pragma unroll 1
-  for (int j = 0; j < CT_SV; ++j) {
+  for (int j = 0; j < CT_SV / 2; ++j) {
     float x = cs_times(was[j], g);
 #pragma unroll 4
     for (int s = 0; s < n; ++s) x = fmaf(k[(size_t)s * k_stride], us[s * CT_SV + j], x);
@@ -1099,16 +1098,16 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
     for (int i = 0; i < 2; ++i) {
       mbar_init(sh.full + i, 1);
       mbar_init(sh.free + i, 1);
-      mbar_init(sh.put + i, 4);
+      mbar_init(sh.put + i, 8);
       mbar_init(sh.done + i, 1);
       odd_s[i] = 0;
     }
     mbar_init(&sh.drain, 2);
     sh.abort = 0;
   }
-  const uint32_t tmem = ct_begin<512>(sh, warp, 4);
+  const uint32_t tmem = ct_begin<512>(sh, warp, 8);
 
-  if (warp == 5) {                                       // ---- tiles; (also of the second warp that ct_end expects)
+  if (warp == 9) {                                       // ---- tiles; (also of the second warp that ct_end expects)
     if (lane == 0) {
       uint32_t phase = 0;
       bool ok = true;
@@ -1127,7 +1126,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       if (*(volatile int*)&sh.abort) mbar_drain(sh.full, 2, asked & 1, (uint32_t)(asked >> 1) & 1u);
     }
     __syncwarp();
-  } else if (warp == 4) {                                // ---- products
+  } else if (warp == 8) {                                // ---- products
     for (int i = 0; i < chunks; ++i) {
       ct_wait_warp(sh.full, i & 1, &sh.abort);
       ct_wait_warp(sh.put, i & 1, &sh.abort);
@@ -1145,25 +1144,26 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       umma_commit(sh.free + 1);
     }
   } else {
-    float* st = state + (size_t)slot * slot_stride + ((size_t)h * p.dv + col0) * 128 + tid;
+    const int own = tid & 127, half = tid >> 7, quarter = warp & 3;        // key size; columns 16 half ..
+    float* st = state + (size_t)slot * slot_stride + ((size_t)h * p.dv + col0 + 16 * half) * 128 + own;
     const double* f = F + (size_t)h * p.T + c.t0;
     const float2* wl = Wl + (size_t)h * p.T + c.t0;
-    const uint32_t from = tmem + ((uint32_t)(warp * 32) << 16);
-    const int r = lane >> 2, q = 2 * (lane & 3);         // of W S: rows 16 warp + r, + 8, columns 8 c + q, + 1
-    const int t_own = 16 * warp + r;
-    float S[CT_SV];
+    const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(16 * half);
+    // of W S: rows 16 quarter + r, + 8, columns q + 8 c, + 1
+    const int r = lane >> 2, q = 16 * half + 2 * (lane & 3), t_own = 16 * quarter + r;
+    float S[CT_SV / 2];
 #pragma unroll
-    for (int j = 0; j < CT_SV; ++j) S[j] = st[(size_t)j * 128];
+    for (int j = 0; j < CT_SV / 2; ++j) S[j] = st[(size_t)j * 128];
     double before = 0.0;
     for (int i = 0; i < chunks; ++i) {
       const int n = min(CT_C, c.n - i * CT_C);
       const size_t chunk = (size_t)(c.first + i) * p.H + h;
       const float* y_at = Y + (chunk * CT_C + t_own) * p.dv + col0 + q;
-      float2 y[2][4], g_t[2];                            // (asked for ahead of the products that need them)
+      float2 y[2][2], g_t[2];                            // (asked for ahead of the products that need them)
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) y[x][j] = *reinterpret_cast<const float2*>(y_at + (size_t)(8 * x) * p.dv + 8 * j);
+        for (int j = 0; j < 2; ++j) y[x][j] = *reinterpret_cast<const float2*>(y_at + (size_t)(8 * x) * p.dv + 8 * j);
         const int t = t_own + 8 * x;
         g_t[x] = t < n ? wl[i * CT_C + t] : make_float2(0.f, 0.f);
       }
@@ -1171,28 +1171,28 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       const double last = f[i * CT_C + n - 1];
       // ---- the state: as it is, and in terms
       if (tid == 0) bf_bulk_wait_read<0>();
-      asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+      asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
 #pragma unroll
-      for (int x = 0; x < CT_SV / 4; ++x)
-        *reinterpret_cast<float4*>(kept + tid * CT_SV + ((x ^ (tid & 7)) << 2)) =
+      for (int x = 0; x < CT_SV / 8; ++x)
+        *reinterpret_cast<float4*>(kept + own * CT_SV + (((x + 4 * half) ^ (own & 7)) << 2)) =
             make_float4(S[4 * x], S[4 * x + 1], S[4 * x + 2], S[4 * x + 3]);
       {
-        // keys tid and its neighbour: the even one takes the first sixteen columns of both
-        const bool second = tid & 1;
-        uint8_t* to = s_op + (tid >> 6) * 3 * DT_TERM + (tid & 6) * 2;
-        const int piece = (tid & 63) >> 3;
+        // keys own and its neighbour: the even one takes the first eight columns of both
+        const bool second = own & 1;
+        uint8_t* to = s_op + (own >> 6) * 3 * DT_TERM + (own & 6) * 2 + 16 * half * 128;
+        const int piece = (own & 63) >> 3;
         bool bad = false;
 #pragma unroll
-        for (int j = 0; j < CT_SV / 2; ++j) {
-          const float keep = second ? S[j + CT_SV / 2] : S[j], give = second ? S[j] : S[j + CT_SV / 2];
+        for (int j = 0; j < 8; ++j) {
+          const float keep = second ? S[j + 8] : S[j], give = second ? S[j] : S[j + 8];
           const float got = __shfl_xor_sync(0xffffffffu, give, 1);
-          const int v = j + (second ? CT_SV / 2 : 0);
+          const int v = j + (second ? 8 : 0);
           bad |= dt_put(to + v * 128 + ((piece ^ (j & 7)) << 4), second ? got : keep, second ? keep : got);
         }
         if (bad) odd_s[0] = i + 1;
       }
       ct_arrive(sh.put);
-      asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+      asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
       if (tid == 0) {
         ct_fence();
         asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
@@ -1207,9 +1207,9 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       ct_wait(sh.done, i & 1, &sh.abort);
       __syncwarp();
       tc_fence_after();
-      float a[16];                                       // [column block][row, column]: rows t_own, + 8
+      float a[8];                                        // [column block][row, column]: rows t_own, + 8
       {
-        uint32_t x0[16], x1[16], x2[16], x3[16], x4[16], x5[16];
+        uint32_t x0[8], x1[8], x2[8], x3[8], x4[8], x5[8];
         dt_load(from, x0);
         dt_load(from + 96, x1);
         dt_load(from + 128, x2);
@@ -1218,7 +1218,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
         dt_load(from + 64, x5);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < 8; ++j) {
           const float lead = (__uint_as_float(x0[j]) + __uint_as_float(x1[j])) +
                              (__uint_as_float(x2[j]) + __uint_as_float(x3[j]));
           a[j] = (lead + (__uint_as_float(x4[j]) + __uint_as_float(x5[j]))) * CT_DOWN;
@@ -1226,13 +1226,13 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       }
       float zero = 0.f;                                  // (NaN where some sum is not finite)
 #pragma unroll
-      for (int j = 0; j < 16; ++j) zero = fmaf(a[j], 0.f, zero);
+      for (int j = 0; j < 8; ++j) zero = fmaf(a[j], 0.f, zero);
       const bool odd = *(volatile int*)&odd_s[0] == i + 1;
       if (odd || (bad_w >> t_own & 0x101ull) || zero != 0.f) {
-        float again[16];
+        float again[8];
         dt_again_ws(W + (chunk * CT_C + t_own) * 128, W + (chunk * CT_C + t_own + 8) * 128, kept, q, again);
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
+        for (int j = 0; j < 8; ++j)
           if (odd || (bad_w >> (t_own + (j & 2) * 4) & 1ull) || !(fabsf(a[j]) < INFINITY)) a[j] = again[j];
       }
       bool bad = false;
@@ -1240,18 +1240,18 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
         // tokens t_own and its neighbour (lane ^ 4): the even one takes the first column of both
         const bool second = r & 1;
         float* u_at = u + ((size_t)(c.t0 + i * CT_C + t_own) * p.H + h) * p.dv + col0 + q;
-        uint8_t* to = u_op + ((q + second) & 7) * 128 + (r & 6) * 2;
+        uint8_t* to = u_op + (q + second) * 128 + (r & 6) * 2;
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < 2; ++j) {
             const float2 uv = make_float2(y[x][j].x - a[4 * j + 2 * x], y[x][j].y - a[4 * j + 2 * x + 1]);
             if (t_own + 8 * x < n)
               *reinterpret_cast<float2*>(u_at + (size_t)(8 * x) * p.H * p.dv + 8 * j) = uv;
             const float2 w = make_float2(cs_times(uv.x, g_t[x]), cs_times(uv.y, g_t[x]));
             *reinterpret_cast<float2*>(us + (t_own + 8 * x) * CT_SV + 8 * j + q) = w;
             const float keep = second ? w.y : w.x, got = __shfl_xor_sync(0xffffffffu, second ? w.x : w.y, 4);
-            bad |= dt_put(to + 8 * j * 128 + (((2 * warp + x) ^ ((q + second) & 7)) << 4), second ? got : keep,
+            bad |= dt_put(to + 8 * j * 128 + (((2 * quarter + x) ^ ((q + second) & 7)) << 4), second ? got : keep,
                           second ? keep : got);
           }
         if (bad) odd_s[1] = i + 1;
@@ -1262,9 +1262,9 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       ct_wait(sh.done + 1, i & 1, &sh.abort);
       __syncwarp();
       tc_fence_after();
-      float now[CT_SV], z = 0.f;                         // z: NaN where some sum is not finite
+      float now[CT_SV / 2], z = 0.f;                         // z: NaN where some sum is not finite
 #pragma unroll
-      for (int j0 = 0; j0 < CT_SV / 2; j0 += 4) {
+      for (int j0 = 0; j0 < CT_SV / 4; j0 += 4) {
         unsigned long long x[4], y[4];
         ct_take<CT_SV>(from + DT_SUMS + (uint32_t)(2 * j0), n > 32, x, y);
 #pragma unroll
@@ -1283,22 +1283,23 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
       tc_fence_before();
       if (*(volatile int*)&odd_s[1] == i + 1 || bad_k || z != 0.f) {
         // (all rows of us are there: their products are)
-        float was[CT_SV], again[CT_SV];
+        float was[CT_SV / 2], again[CT_SV / 2];
 #pragma unroll
-        for (int j = 0; j < CT_SV; ++j) was[j] = S[j];
-        dt_again_state(p.qkv + (size_t)(c.t0 + i * CT_C) * p.stride + (size_t)(p.G + hq) * 128 + tid, p.stride, us, n,
+        for (int j = 0; j < CT_SV / 2; ++j) was[j] = S[j];
+        dt_again_state(p.qkv + (size_t)(c.t0 + i * CT_C) * p.stride + (size_t)(p.G + hq) * 128 + own, p.stride,
+                       us + 16 * half, n,
                        g, was, again);
 #pragma unroll
-        for (int j = 0; j < CT_SV; ++j) now[j] = again[j];
+        for (int j = 0; j < CT_SV / 2; ++j) now[j] = again[j];
       }
 #pragma unroll
-      for (int j = 0; j < CT_SV; ++j) S[j] = now[j];
+      for (int j = 0; j < CT_SV / 2; ++j) S[j] = now[j];
     }
 #pragma unroll
-    for (int j = 0; j < CT_SV; ++j) st[(size_t)j * 128] = S[j];
+    for (int j = 0; j < CT_SV / 2; ++j) st[(size_t)j * 128] = S[j];
     if (tid == 0) bf_bulk_wait_read<0>();
   }
-  ct_end<512>(sh, tmem, warp, 4, err);
+  ct_end<512>(sh, tmem, warp, 8, err);
 }
 
 // Chunks of 64, keys in whole steps of 128, values of 64 or in whole tiles of 128 (two heads of 64 share a
