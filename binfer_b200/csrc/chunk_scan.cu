@@ -409,9 +409,10 @@ struct CsIn {
 // sums of up to 64 of them behind it show an error that is one of |q| |k|, however small q . k is
 // itself.  In float, in runs of 16, outputs were 1.2 to 1.7 times as far from 64 bits as the walk's (fast
 // decays; the delta rule's keys alike), at 12 us instead of 14 (2,048 tokens, 8 q/k heads of 128) and 21
-// instead of 42 (16 heads, K K^T too, which ds_prep then computed itself in another 5).  Warp w takes 16
-// rows; with K's rows behind Q's the blocks run the other way, so that every scheduler has the same
-// share of the triangle.
+// instead of 42 (16 heads, K K^T too, which ds_prep then computed itself in another 5).  A warp takes 16
+// rows; of Q alone two warps share a block of 16 rows, every other eight columns each (2,048 tokens of 8 heads of
+// 256 33 us with one warp a block, 28 so); the second four warps' blocks run the other way, so that every scheduler
+// has the same share of the triangle.
 #define CS_QS 32            // sizes a stage
 #define CS_QP (CS_QS + 4)   // pitch: eight rows of four neighbouring sizes on different banks
 
@@ -501,10 +502,10 @@ __device__ __forceinline__ void cs_terms(const float* __restrict__ qk, const CsI
 }
 
 template <typename A, bool KK>
-__global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
+__global__ void __launch_bounds__(256) cs_qk_kernel(
     const A* __restrict__ qk, CsIn p, const int* __restrict__ q_start, float* __restrict__ qkm,
     float* __restrict__ kkm, CsTerms x_out) {
-  constexpr int THREADS = KK ? 256 : 128, PIECES = 128 * (CS_QS / 4) / THREADS;
+  constexpr int THREADS = 256, PIECES = 128 * (CS_QS / 4) / THREADS, SHARES = KK ? 1 : 2, COLS = 8 / SHARES;
   __shared__ __align__(16) double rows_s[128][CS_QP];      // 64 rows of q, 64 of k
   const int tiles = p.C / CS_T;
   const int rt = blockIdx.z / tiles, ct = blockIdx.z % tiles;
@@ -522,14 +523,15 @@ __global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
   const int hq = blockIdx.y;
   const A* q = qk + (size_t)(c.t0 + at) * p.qk_stride + p.q_off + (size_t)hq * p.dk;
   const A* k = qk + (size_t)(c.t0 + at) * p.qk_stride + p.k_off + (size_t)hq * p.dk;
-  const int block = warp >= 4 ? 7 - warp : !KK && (blockIdx.x & 1) ? 3 - warp : warp;
-  const int row0 = (warp >= 4 ? 64 : 0) + block * 16;
-  const int cols = ct < rt ? 8 : 2 * (block + 1);          // blocks of eight columns
-  double acc[2][8][2];
+  const bool of_k = KK && warp >= 4;             // rows of K against K
+  const int share = KK ? 0 : warp >> 2, block = warp >= 4 ? 7 - warp : warp;
+  const int row0 = (of_k ? 64 : 0) + block * 16;
+  const int cols = ct < rt ? 8 : 2 * (block + 1);          // blocks of eight columns: this warp's shares of them
+  double acc[2][COLS][2];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < COLS; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   float4 f[PIECES];
   auto fetch = [&](int k0) {
 #pragma unroll
@@ -556,24 +558,24 @@ __global__ void __launch_bounds__(KK ? 256 : 128) cs_qk_kernel(
       const double a0 = rows_s[row0 + (lane >> 2)][kk + (lane & 3)];
       const double a1 = rows_s[row0 + 8 + (lane >> 2)][kk + (lane & 3)];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (j < cols) {
-          const double b = rows_s[64 + 8 * j + (lane >> 2)][kk + (lane & 3)];
+      for (int j = 0; j < COLS; ++j)
+        if (SHARES * j + share < cols) {
+          const double b = rows_s[64 + 8 * (SHARES * j + share) + (lane >> 2)][kk + (lane & 3)];
           cs_dmma(acc[0][j], a0, b);
           cs_dmma(acc[1][j], a1, b);
         }
     }
     __syncthreads();
   }
-  const double scale = warp >= 4 ? 1.0 : (double)p.q_scale;
-  float* dst = (warp >= 4 ? kkm : qkm) + ((size_t)blockIdx.x * p.QH + hq) * p.C * p.C;
+  const double scale = of_k ? 1.0 : (double)p.q_scale;
+  float* dst = (of_k ? kkm : qkm) + ((size_t)blockIdx.x * p.QH + hq) * p.C * p.C;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < cols)
+    for (int j = 0; j < COLS; ++j)
+      if (SHARES * j + share < cols)
         *reinterpret_cast<float2*>(
-            dst + (size_t)(rt * CS_T + block * 16 + 8 * i + (lane >> 2)) * p.C + ct * CS_T + 8 * j +
+            dst + (size_t)(rt * CS_T + block * 16 + 8 * i + (lane >> 2)) * p.C + ct * CS_T + 8 * (SHARES * j + share) +
             (lane & 3) * 2) = make_float2((float)(acc[i][j][0] * scale), (float)(acc[i][j][1] * scale));
   bf_pdl_wait();
 }
@@ -1312,7 +1314,7 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   CsTerms x = {nullptr, nullptr, nullptr};
   if (!MLSTM && tensor)
     x = {(uint8_t*)scratch + l.Xq, (uint8_t*)scratch + l.Xk, (unsigned long long*)(scratch + l.odd)};
-  if (const int e = bf_launch_pdl(cs_qk_kernel<A, false>, dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)), dim3(128), 0, stream,
+  if (const int e = bf_launch_pdl(cs_qk_kernel<A, false>, dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)), dim3(256), 0, stream,
                                   qk, p, q_start, qkm, (float*)nullptr, x))
     return e;
   if constexpr (MLSTM) {
