@@ -20,7 +20,7 @@
 // results that they reach are computed by multiply-adds; so are sums that are not finite (where finite
 // operands' product leaves float's range, that of a smaller term may overflow with a sign of its own).
 //
-// 2,048 tokens, 8 heads of 256 x 512: mt_state 73 us (cs_state and cs_prefix 177), mt_out 95 (cs_out 168).
+// 2,048 tokens, 8 heads of 256 x 512: mt_state 73 us (cs_state and cs_prefix 177), mt_out 91 (cs_out 168).
 // What bounds them: mt_state the issue slots (a chunk's keys and values to take apart, its sums, its states
 // to store: some 4,000 cycles for 600 of products), mt_out the same (a step 2,500 cycles) and the start
 // and the end of a tile (4,000).  Relative errors against 64 bits, this / those, at 2,048 tokens (four inputs):
@@ -166,7 +166,7 @@ __device__ __forceinline__ void mt_products(uint32_t d, uint32_t a, uint32_t b) 
 }
 
 struct MtShared {
-  uint64_t done[2], drain, got;  // a step's products are complete (even and odd steps); all are; a copy is here
+  uint64_t done[2], drain, got[2];  // a step's products are complete (even and odd steps); all are; a copy is here
   uint32_t tmem;
   int abort;
 };
@@ -175,7 +175,8 @@ __device__ __forceinline__ uint32_t mt_begin(MtShared& s) {
     mbar_init(s.done, 1);
     mbar_init(s.done + 1, 1);
     mbar_init(&s.drain, 1);
-    mbar_init(&s.got, 1);
+    mbar_init(s.got, 1);
+    mbar_init(s.got + 1, 1);
     s.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -482,8 +483,11 @@ struct MtTable {                 // of a tile
   float den[MT_C];
   int odd_t[MT_C], odd_m[MT_M], odd;   // the token's operands have no terms; from which token on the row's
 };                                     // some have none; any
-#define MT_OUT_STAGE (3 * (MT_TILE + MT_TOK))
-#define MT_OUT_SMEM (1024 + 2 * MT_OUT_STAGE + MT_C * MT_M * 4 + MT_WORK * 32)
+// a stage: the rows' three terms and q (one term), or the values (one term) and q . k in three; what a step's
+// operands are made from, for two steps (with one place, asked for behind the step before, 95 us; so 91)
+#define MT_OUT_STAGE (3 * MT_TILE + MT_TOK)
+#define MT_OUT_RAW (MT_C * MT_M * 4 + MT_WORK * 16)
+#define MT_OUT_SMEM (1024 + 2 * MT_OUT_STAGE + 2 * MT_OUT_RAW)
 __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
     const mt_bf16* __restrict__ proj, CsIn p, int n_chunks, const int* __restrict__ q_start,
     const int* __restrict__ state_slots, int n_slots, const double* __restrict__ G,
@@ -494,7 +498,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
   __shared__ MtShared sh;
   __shared__ MtTable table[2];
   __shared__ MtUnit next_s;                      // the tile after the one in work, found by the issuing warp
-  __shared__ __align__(16) float n_s[MT_C];      // n's sizes of the step
+  __shared__ __align__(16) float n_s[2][MT_C];   // n's sizes of the step
   uint8_t* ring = mt_raw + ((1024u - (smem_u32(mt_raw) & 1023u)) & 1023u);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m_tiles = p.dv / MT_M, steps = p.dk / MT_C;
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
         const uint32_t tm = smem_u32(ring) + (uint32_t)((i & 1) * MT_OUT_STAGE);
         const uint32_t d = tmem + (uint32_t)((i & 1) * 3 * MT_C);
         if (step < steps) mt_products<3, 1, false>(d, tm, tm + 3 * MT_TILE);
-        else mt_products<1, 3, false>(d, tm, tm + 3 * MT_TILE);
+        else mt_products<1, 3, false>(d, tm, tm + MT_TILE);
         umma_commit(sh.done + (i & 1));
         if (step == 0) more = next();            // (read by the others behind a later step's barrier)
       }
@@ -550,53 +554,56 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
   const int m = quarter * 32 + lane;
   const uint32_t from = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(group * 16);
   // a step's floats (the state's 64 rows of 128, or q . k) come in one copy, q's or the values' rows in
-  // pieces of sixteen bytes that the same thread reads
+  // pieces of sixteen bytes that the same thread reads behind them
   uint8_t* block = ring + 2 * MT_OUT_STAGE;
-  uint8_t* mine = block + MT_C * MT_M * 4 + tid * 16;
-  auto eight = [&](int row, int width, int piece) {
-    const float4* at = reinterpret_cast<const float4*>(block) + row * (width / 4) + 2 * piece;
+  auto place = [&](int i) { return block + (i & 1) * MT_OUT_RAW; };
+  auto eight = [&](int i, int row, int width, int piece) {
+    const float4* at = reinterpret_cast<const float4*>(place(i)) + row * (width / 4) + 2 * piece;
     const float4 a = at[0], b = at[1];
     MtEight e = {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
     return e;
   };
-  auto raw = [&](int x) { return *reinterpret_cast<const uint4*>(mine + x * 16 * MT_WORK); };
+  auto mine = [&](int i, bool values) { return place(i) + (values ? MT_C * MT_C * 4 : MT_C * MT_M * 4) + tid * 16; };
 
-  MtUnit c = {};                                 // the tile whose operands are fetched
-  OnePlace copies;                               // (of thread 0)
+  MtUnit c = {};                                 // the tile in work
+  OnePlace copies[2];                            // (of thread 0)
   auto gave_up = [&]() { return *(volatile int*)&sh.abort != 0; };
-  // (all have read the step before; rows beyond the last repeat it: q's results are not stored, values'
-  // weights are zero)
-  auto fetch = [&](int step) {
+  // step `i` of all, a tile's `step` (all have read the step before last; rows beyond the last repeat it: q's
+  // results are not stored, values' weights are zero)
+  auto fetch = [&](const MtUnit& c, int step, int i) {
     const size_t head = (size_t)c.chunk * p.H + c.h;
+    uint8_t* to = place(i);
+    uint64_t* got = sh.got + (i & 1);
     if (step < steps) {
       if (tid == 0) {
-        copies.fill(gave_up(), [&]() {
-          mbar_expect_tx(&sh.got, MT_C * MT_M * 4 + MT_C * 4);
-          bf_bulk_load(n_s, Un + head * p.dk + step * MT_C, MT_C * 4, &sh.got);
-          bf_bulk_load(block, U + head * p.dk * p.dv + (size_t)c.m0 * p.dk + step * MT_C * MT_M,
-                       MT_C * MT_M * 4, &sh.got);
+        copies[i & 1].fill(gave_up(), [&]() {
+          mbar_expect_tx(got, MT_C * MT_M * 4 + MT_C * 4);
+          bf_bulk_load(n_s[i & 1], Un + head * p.dk + step * MT_C, MT_C * 4, got);
+          bf_bulk_load(to, U + head * p.dk * p.dv + (size_t)c.m0 * p.dk + step * MT_C * MT_M, MT_C * MT_M * 4, got);
         });
       }
-      mt_fetch(mine, proj + (size_t)(c.t0 + min(tr, c.n - 1)) * p.qk_stride + p.q_off + (size_t)c.h * p.dk +
-                         step * MT_C + 8 * tq);
+      mt_fetch(mine(i, false), proj + (size_t)(c.t0 + min(tr, c.n - 1)) * p.qk_stride + p.q_off +
+                                   (size_t)c.h * p.dk + step * MT_C + 8 * tq);
     } else {
       if (tid == 0) {
-        copies.fill(gave_up(), [&]() {
-          mbar_expect_tx(&sh.got, MT_C * MT_C * 4);
-          bf_bulk_load(block, qkm + head * MT_C * MT_C, MT_C * MT_C * 4, &sh.got);
+        copies[i & 1].fill(gave_up(), [&]() {
+          mbar_expect_tx(got, MT_C * MT_C * 4);
+          bf_bulk_load(to, qkm + head * MT_C * MT_C, MT_C * MT_C * 4, got);
         });
       }
       const mt_bf16* v = proj + (size_t)c.t0 * p.v_stride + p.v_off + (size_t)c.h * p.dv + c.m0 + 8 * mq;
-      mt_fetch(mine, v + (size_t)min(mr, c.n - 1) * p.v_stride);
-      mt_fetch(mine + 16 * MT_WORK, v + (size_t)min(mr + 32, c.n - 1) * p.v_stride);
+      uint8_t* at = mine(i, true);
+      mt_fetch(at, v + (size_t)min(mr, c.n - 1) * p.v_stride);
+      mt_fetch(at + 16 * MT_WORK, v + (size_t)min(mr + 32, c.n - 1) * p.v_stride);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // q . k with its weight: row t sees the chunk's tokens up to itself
-  auto weighted = [&](const MtTable& tb) {
+  auto weighted = [&](const MtTable& tb, int i) {
     const int t = tr, s = 8 * tq, last = t < c.n ? t : -1, b = s >> 4;
     MtEight e = {};
     if (s > last) return e;
-    e = eight(t, MT_C, tq);
+    e = eight(i, t, MT_C, tq);
     if (b < t >> 4) {
       const float2 r = tb.row[b][t];
 #pragma unroll
@@ -614,26 +621,31 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
   float den = 0.f;                               // n_t . q_t, this thread's share of row tr
   auto convert = [&](MtTable& tb, int step, int i) {
     uint8_t* tm = ring + (i & 1) * MT_OUT_STAGE + m_spot;
-    uint8_t* tt = ring + (i & 1) * MT_OUT_STAGE + 3 * MT_TILE + t_spot;
+    uint8_t* tt = ring + (i & 1) * MT_OUT_STAGE + (step < steps ? 3 : 1) * MT_TILE + t_spot;
     float2 left = make_float2(0.f, 0.f);
-    mt_fetched();
-    mbar_wait(&sh.got, i & 1, &sh.abort);
+    // (two steps are asked for; of tiles of two steps, whose next is known late, both or none)
+    if (steps > 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    mbar_wait(sh.got + (i & 1), (i >> 1) & 1, &sh.abort);
+    auto raw = [&](int x) {
+      return *reinterpret_cast<const uint4*>(mine(i, step == steps) + x * 16 * MT_WORK);
+    };
     if (step < steps) {
 #pragma unroll
-      for (int x = 0; x < 2; ++x) mt_put(tm + x * 4096, MT_TILE, eight(mr + 32 * x, MT_M, mq), left);
+      for (int x = 0; x < 2; ++x) mt_put(tm + x * 4096, MT_TILE, eight(i, mr + 32 * x, MT_M, mq), left);
       const uint4 qv = raw(0);
       *reinterpret_cast<uint4*>(tt) = qv;
       {
         const MtEight f = mt_bf16s(qv);
-        const float4 a = *reinterpret_cast<const float4*>(n_s + 8 * tq);
-        const float4 b = *reinterpret_cast<const float4*>(n_s + 8 * tq + 4);
+        const float4 a = *reinterpret_cast<const float4*>(n_s[i & 1] + 8 * tq);
+        const float4 b = *reinterpret_cast<const float4*>(n_s[i & 1] + 8 * tq + 4);
         den += ((f.v[0] * a.x + f.v[1] * a.y) + (f.v[2] * a.z + f.v[3] * a.w)) +
                ((f.v[4] * b.x + f.v[5] * b.y) + (f.v[6] * b.z + f.v[7] * b.w));
       }
       if (mt_bad(left) || mt_bad(qv)) {
 #pragma unroll 1
         for (int x = 0; x < 2; ++x) {
-          MtEight e = eight(mr + 32 * x, MT_M, mq);
+          MtEight e = eight(i, mr + 32 * x, MT_M, mq);
           const int bad = mt_clean(e, MT_NO_TERMS_UP);
           for (int j = 0; j < 8; ++j)
             if (bad >> j & 1) tb.odd_m[8 * mq + j] = 0;
@@ -659,7 +671,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
       }
       *reinterpret_cast<uint4*>(tm + x * 4096) = v;
     }
-    MtEight w = weighted(tb);
+    MtEight w = weighted(tb, i);
     // n_t . q_t: the state's share with the token's weight, and the row's sum
     den = cs_times(den, tb.at[tr]);
     if (!(fabsf(den) < INFINITY) && tr < c.n) {  // (the weight on q: it may keep the products finite)
@@ -749,19 +761,20 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
 
   int i = 0, tab = 0;
   double gn = 0.0, hn = 0.0, before = 0.0;       // of the next tile's token tid
-  auto ahead = [&]() {
-    c = next_s;
-    if (c.b < 0) return;
-    fetch(0);
-    if (tid < MT_C) {
-      const size_t t = (size_t)c.h * p.T + c.t0;
-      before = c.index ? G[t - 1] : g0[(size_t)c.b * p.H + c.h];
-      gn = G[t + min(tid, c.n - 1)];
-      hn = Hs[t + min(tid, c.n - 1)];
-    }
+  auto sums = [&](const MtUnit& c) {             // a tile's token tid
+    if (c.b < 0 || tid >= MT_C) return;
+    const size_t t = (size_t)c.h * p.T + c.t0;
+    before = c.index ? G[t - 1] : g0[(size_t)c.b * p.H + c.h];
+    gn = G[t + min(tid, c.n - 1)];
+    hn = Hs[t + min(tid, c.n - 1)];
   };
   __syncthreads();                               // (the first tile is found)
-  ahead();
+  c = next_s;
+  sums(c);
+  if (c.b >= 0) {
+    fetch(c, 0, 0);
+    fetch(c, 1, 1);
+  }
   while (c.b >= 0) {
     // ---- the tile's tables (the tile before last, whose place they take, is finished)
     MtTable& tb = table[tab];
@@ -801,19 +814,29 @@ __global__ void __launch_bounds__(MT_THREADS, 1) mt_out_kernel(
         tb.col[t] = cs_exp(tb.g[t | 15] - tb.h[t]);
       }
     }
+    MtUnit after = {};                           // the tile behind it: known from its second step on
     for (int step = 0; step <= steps; ++step, ++i) {
       convert(tb, step, i);
       mt_stored();
-      if (step < steps) fetch(step + 1);
-      else ahead();
+      if (step == 1) after = next_s;
+      if (step + 2 <= steps) {
+        fetch(c, step + 2, i + 2);
+      } else if (step > 0 && after.b >= 0) {
+        if (steps == 1) fetch(after, 0, i + 1);
+        fetch(after, step + 1 - steps, i + 2);
+      } else {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      }
+      if (step == steps) sums(after);
       if (step) finish(tb, step - 1, i - 1);
       else if (i) finish(table[tab ^ 1], steps, i - 1);
     }
     tab ^= 1;
+    c = after;
   }
   if (i) finish(table[tab ^ 1], steps, i - 1);
   if (tid == 0 && gave_up())                     // (a copy that this thread did not see land)
-    copies.drain([&](int, unsigned parity) { mbar_drain_one(&sh.got, parity); });
+    for (int x = 0; x < 2; ++x) copies[x].drain([&](int, unsigned parity) { mbar_drain_one(sh.got + x, parity); });
   mt_end(sh, tmem, err);
 }
 
