@@ -26,12 +26,13 @@
 // Operands that have no terms (infinities, NaN, floats from 2^104 on) are zero in the products, and what they
 // reach is computed by multiply-adds in cs_state's and cs_out's order; so are sums that are not finite.
 //
-// 2,000 tokens of 64 heads of 128 x 64 over 8: ct_state 39 us (cs_state and cs_prefix 87), ct_weights 15, ct_out 58
-// (cs_out 100); 1,300 and 812 tokens of 8 heads of 128 x 256: 27 (47), 5, 30 (58); the delta rule's 1,111 and 694 of
-// 16 heads of 128: dt_walk 70 (ds_walk 108), ct_out 30 (cs_out 53), ds_prep 54 (47).  What bounds ct_out is the rate
+// 2,000 tokens of 64 heads of 128 x 64 over 8: ct_state 36 us (cs_state and cs_prefix 87), ct_weights 15, ct_out 58
+// (cs_out 100); 1,300 and 812 tokens of 8 heads of 128 x 256: 25 (47), 5, 30 (58); the delta rule's 1,111 and 694 of
+// 16 heads of 128: dt_walk 59 (ds_walk 108), ct_out 31 (cs_out 53), ds_prep 54 (47).  What bounds ct_out is the rate
 // at which its warps get instructions (0.45 a cycle and scheduler): its time changes by 0 to 3 us without its
 // stores, with loads that always hit, with half of the products or without taking the operands apart.  ct_state and
-// dt_walk are bound by their chains: some 2,300 and 7,000 cycles a chunk.
+// dt_walk are bound by their chains: some 1,850 and 4,600 cycles a chunk.  (With a row of the state a thread, half
+// as many warps, they were 39 and 70 us.)
 // Relative errors against 64 bits (outputs, states), these / multiply-adds, e-7: decays of 0.98 to 1 0.79 0.66 / 1.37
 // 1.29, a state space layer's 0.55 0.46 / 0.68 0.59, spread over 0 to 1 0.51 0.42 / 0.50 0.42; the delta rule's 0.97
 // 0.86 / 1.63 1.80, 0.66 0.59 / 0.77 0.68, 0.58 0.55 / 0.57 0.48.
@@ -141,9 +142,10 @@ __device__ __forceinline__ bool ct_wait_warp(uint64_t* bar, uint32_t parity, vol
   return __all_sync(0xffffffffu, ok);
 }
 
-// What other threads stored ahead of a barrier that this one has passed is there for the products.  (By the
-// warp that issues them and not by those that store: the fence waits for a thread's loads too, and theirs are for the
-// step behind: 1,400 of 4,500 cycles a step.)
+// What other threads stored ahead of a barrier that this one has passed is there for the products: a proxy fence
+// anywhere on the way from a write to the other proxy's read orders them.  (By the warp that issues the products and
+// not by those that store: there it waits for a thread's loads, too, and theirs are for the step behind; ct_out 61 us
+// so, 58 here.)
 __device__ __forceinline__ void ct_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void ct_arrive(uint64_t* bar) {      // by a warp: its writes are done
   __syncwarp();

@@ -760,7 +760,9 @@ def chunk_scan_pays(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bo
     33 / 39, 46 / 46, two 41 / 48, 49 / 49, 72 / 58; 64 heads of 128 x 64, one 42 / 46, 51 / 50, 72 / 56, two
     64 / 65, 76 / 70, 111 / 88.  Heads of 64 x 64 and less fill half of a tile's terms: 32 of them, one portion
     of 260 tokens 36 / 36, six of 400 98 / 101.  (``tokens / max_q`` stands for the number of portions: single
-    tokens beside them hardly count.)"""
+    tokens beside them hardly count.)  Chunks by multiply-adds; on the tensor cores they are faster (256 tokens: 8 heads
+    of 128 x 256 45 / 44, two portions 68 / 52), but a whole layer of width 2,048 waits for the host there and a line
+    at 176 tokens and 248 cost it 8 to 15 %."""
     if dk * dv < 8192:
         return max_q > 448
     elements = tokens * heads * dk * dv / max(1, max_q)
@@ -1095,8 +1097,9 @@ DELTA_CHUNK_MIN = 384
 
 
 def delta_chunks_pay(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bool:
-    """Whether a step's gated delta rule is the faster one in chunks (arguments as for
-    :func:`chunk_scan_pays`), whose chain has a block per portion, head and 32 columns, one an SM (148) and
+    """Whether a step's gated delta rule is the faster one in chunks (arguments and the chunks' kernels as for
+    :func:`chunk_scan_pays`; on the tensor cores 384 tokens of 16 heads 113 / 79, but two portions of
+    370 and 231 tokens through a layer of width 2,048 at 0.79 of the walk's speed), whose chain has a block per portion, head and 32 columns, one an SM (148) and
     built for keys of 128.  Walk / chunks in us, 16 heads of 128, portions of 400 and 500 tokens: one
     113 / 97, 140 / 103, two 144 / 116, 180 / 124, three (192 blocks, a second round of 44) 174 / 200, 217 / 218,
     six 342 / 308, 428 / 342.  16 heads of 64: one 96 / 77, 119 / 82, three 96 / 110, 119 / 117, six (the walk has
