@@ -27,8 +27,8 @@
 // 128, values of 64 or whole tiles of 128 and CTAs enough, and the delta rule with keys of 128 (chunk_tensor.cuh).
 //
 // GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads by multiply-adds 208 / 467 us (cs_out
-// 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 138; 8 heads of 128 x 256 124 / 270 (83); mLSTM, 8 heads of 256 x
-// 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them: cs_state and cs_out shared-memory reads (the
+// 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 138; 8 heads of 128 x 256 124 / 270 (83);
+// mLSTM, 8 heads of 256 x 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them: cs_state and cs_out shared-memory reads (the
 // pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
 // expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
 // further from 64 bits than the walk where decays are fast.
@@ -1314,8 +1314,8 @@ static int cs_launch(const A* qk, const V* v, const CsIn& p, const float* decays
   CsTerms x = {nullptr, nullptr, nullptr};
   if (!MLSTM && tensor)
     x = {(uint8_t*)scratch + l.Xq, (uint8_t*)scratch + l.Xk, (unsigned long long*)(scratch + l.odd)};
-  if (const int e = bf_launch_pdl(cs_qk_kernel<A, false>, dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)), dim3(256), 0, stream,
-                                  qk, p, q_start, qkm, (float*)nullptr, x))
+  if (const int e = bf_launch_pdl(cs_qk_kernel<A, false>, dim3(l.chunks, p.QH, tiles * tiles + (x.q ? 2 : 0)),
+                                  dim3(256), 0, stream, qk, p, q_start, qkm, (float*)nullptr, x))
     return e;
   if constexpr (MLSTM) {
     if (tensor)
@@ -1489,8 +1489,8 @@ BF_EXPORT int bf_chunk_scan_delta(const float* qkv, const float* gates, float* s
   const CsTerms x = {Xq, terms ? (uint8_t*)base + l.Xk : nullptr, odd};
   uint8_t* Xw = terms ? (uint8_t*)base + l.Xw : nullptr;
   unsigned long long* odd_w = (unsigned long long*)(base + l.odd_w);
-  if (const int e = bf_launch_pdl(cs_qk_kernel<float, true>, dim3(l.chunks, G, x.q ? 3 : 1), dim3(256), 0, stream, qkv, p, q_start,
-                                  qkm, kkm, x))
+  if (const int e = bf_launch_pdl(cs_qk_kernel<float, true>, dim3(l.chunks, G, x.q ? 3 : 1), dim3(256), 0, stream,
+                                  qkv, p, q_start, qkm, kkm, x))
     return e;
   ds_prep_kernel<<<dim3(l.chunks, H), DS_PREP_THREADS, smem_prep, stream>>>(d, q_start, F, kkm, W,
                                                                             Y, qkm, terms ? Ww : nullptr, Xw, odd_w);

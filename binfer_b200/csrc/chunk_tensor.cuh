@@ -290,7 +290,8 @@ __device__ __forceinline__ void ct_weights(const double* g, const double* hs, do
         return j + at <= last ? cs_times(a, f) : 0.f;
       };
       *reinterpret_cast<float4*>(&to->P[t][s + j]) =
-          make_float4(one(v.x, hi.x, lo.x, 0), one(v.y, hi.y, lo.y, 1), one(v.z, hi.z, lo.z, 2), one(v.w, hi.w, lo.w, 3));
+          make_float4(one(v.x, hi.x, lo.x, 0), one(v.y, hi.y, lo.y, 1), one(v.z, hi.z, lo.z, 2),
+                      one(v.w, hi.w, lo.w, 3));
     }
   }
 }
@@ -569,12 +570,12 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
 // are value sizes, their columns the chunk's tokens: first the state times q over dk, a step of 64 at a time,
 // times the token's weight, then the values times the weighted q . k; two heads of 64 have a step each there,
 // whose sums only the lanes of that head add.
-//
 #define CT_O_A (3 * 2 * CT_TERM)                         // 64 terms x 128 value sizes in three terms
 #define CT_O_SMEM (1024 + 2 * CT_O_A + 2 * CT_TILE + 2 * CT_TILE)
 #define CT_O_COLS 512                                    // two places of 4 x 64 columns
-// eight warps that add (a quarter of the lanes, half of the tokens each), eight that convert, four that X registers a thread at the
-// start, 96, 80, 80 and 48 from then on.
+// eight warps that add (a quarter of the lanes, half of the tokens each), eight that convert the states and values,
+// four the weighted q . k, two that issue products and one that copies: 80 registers a thread at the start, 96, 80,
+// 80 and 48 from then on.
 // What every role does for a step is written once, rare paths are functions of their own: five roles' code,
 // unrolled, was 158 KB, and warps waited for instructions most of their time (125 us).
 #define CT_O_THREADS 768
@@ -981,9 +982,9 @@ __global__ void __launch_bounds__(CT_O_THREADS, 1) ct_out_kernel(
 
 // -------------------------------------------------------------------------------- dt_walk
 // The delta rule's chain from chunk to chunk (ds_walk) with keys of 128: U = Y - W S, S <- exp(F_C) S + K^T
-// (exp(F_C - F) U).  grid (32 value sizes, H, B).  Eight warps keep 128 x 32 of the state, half a row a thread, and take
-// each product's operand apart as the other's sums come; one warp issues products, one asks for W's and K's tiles
-// (X: W in terms, chunk and head by chunk and head).  The state before a chunk leaves as ct_state's does.
+// (exp(F_C - F) U).  grid (32 value sizes, H, B).  Eight warps keep 128 x 32 of the state, half a row a thread, and
+// take each product's operand apart as the other's sums come; one warp issues products, one asks for W's and K's
+// tiles (X: W in terms, chunk and head by chunk and head).  The state before a chunk leaves as ct_state's does.
 //
 // W S: 64 tokens x 32 columns over 128 terms, leading terms' products summed 32 at a time (four places), the
 // others' in two; a warp reads its 16 rows in the shape of a fragment, rows lane / 4 and eight further, so that
@@ -1078,7 +1079,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
     const unsigned long long* __restrict__ odd_rows, float* __restrict__ u, float* __restrict__ Sc,
     int* __restrict__ err) {
   extern __shared__ __align__(16) uint8_t ct_raw[];
-  __shared__ CtShared sh;                                // full, free: W's and K's tiles; put, done: S's and U's operands
+  __shared__ CtShared sh;                                // full, free: W's and K's tiles; put, done: S's, U's
   __shared__ int odd_s[2];                               // of S and of U: chunk + 1 where a number has no terms
   uint8_t* w_tile = ct_raw + ((1024u - (smem_u32(ct_raw) & 1023u)) & 1023u);
   uint8_t* k_tile = w_tile + CT_S_KEYS;
@@ -1120,8 +1121,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
           ok = i == 0 || ct_wait(sh.free + x, phase ^ 1u, &sh.abort);
           if (!ok) break;
           mbar_expect_tx(sh.full + x, CT_S_KEYS);
-          bf_bulk_load(x ? k_tile : w_tile, x ? Xk + (chunk * p.G + hq) * CT_S_KEYS : Xw + (chunk * p.H + h) * CT_S_KEYS,
-                       CT_S_KEYS, sh.full + x);
+          bf_bulk_load(x ? k_tile : w_tile,
+                       x ? Xk + (chunk * p.G + hq) * CT_S_KEYS : Xw + (chunk * p.H + h) * CT_S_KEYS, CT_S_KEYS, sh.full + x);
           ++asked;
         }
       }

@@ -1099,8 +1099,8 @@ DELTA_CHUNK_MIN = 384
 def delta_chunks_pay(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bool:
     """Whether a step's gated delta rule is the faster one in chunks (arguments and the chunks' kernels as for
     :func:`chunk_scan_pays`; on the tensor cores 384 tokens of 16 heads 113 / 79, but two portions of
-    370 and 231 tokens through a layer of width 2,048 at 0.79 of the walk's speed), whose chain has a block per portion, head and 32 columns, one an SM (148) and
-    built for keys of 128.  Walk / chunks in us, 16 heads of 128, portions of 400 and 500 tokens: one
+    370 and 231 tokens through a layer of width 2,048 at 0.79 of the walk's speed), whose chain has a block per
+    portion, head and 32 columns, one an SM (148) and built for keys of 128.  Walk / chunks in us, 16 heads of 128, portions of 400 and 500 tokens: one
     113 / 97, 140 / 103, two 144 / 116, 180 / 124, three (192 blocks, a second round of 44) 174 / 200, 217 / 218,
     six 342 / 308, 428 / 342.  16 heads of 64: one 96 / 77, 119 / 82, three 96 / 110, 119 / 117, six (the walk has
     a quarter of the work) 123 / 189, 153 / 212 and 303 / 385 at 1,000."""
