@@ -28,8 +28,8 @@
 //
 // GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads by multiply-adds 208 / 467 us (cs_out
 // 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 138; 8 heads of 128 x 256 124 / 270 (83);
-// mLSTM, 8 heads of 256 x 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them: cs_state and cs_out shared-memory reads (the
-// pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
+// mLSTM, 8 heads of 256 x 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them:
+// cs_state and cs_out shared-memory reads (the pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
 // expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
 // further from 64 bits than the walk where decays are fast.
 //
@@ -55,7 +55,7 @@
 //              32 columns) in parallel
 //   cs_out     as above, on U
 //
-// 2,048 tokens of 16 heads of 128: 341 us (ds_walk 187, cs_out 54, ds_prep 48, cs_qk 42) by multiply-adds against the
+// 2,048 tokens of 16 heads of 128: 333 us (ds_walk 187, cs_out 54, ds_prep 40, cs_qk 42) by multiply-adds against the
 // walk's 563; 1,000 tokens 168 and 277, three portions of 1,000 381 and 431.  Errors against 64 bits, walk / chunks:
 // keys at random, decays of 0.98 to 1: o 2.3e-7 / 1.6e-7, state 2.3e-7 / 1.8e-7; keys of a cosine of 0.9
 // 2.6e-7 / 2.6e-7 and 2.5e-7 / 2.5e-7; fast decays o 1.1e-7 / 7.8e-8, state 6.2e-8 / 7.1e-8.  (What the walk
@@ -120,20 +120,29 @@ __device__ __forceinline__ float4 cs_times(float4 v, float2 w) {
 // eighth is below 2^-27) on top of 1 + r, whose rounding is kept.  One conversion: those and the double
 // operations are what it costs.  (The weights of tokens hang together in every result: with expf, up to two units
 // off in the last place, an output of keys and queries alike was four times as far from 64 bits as
-// the walk's.)
+// the walk's.)  FINE: with what r's float leaves of it and the eighth power, good to some 2^-27 (2^-29.6 and not
+// 2^-27.4 in the mean), for factors: a product of two is then no further off than one exponential.
+template <bool FINE = false>
 __device__ __forceinline__ float2 cs_exp(double x) {
   if (!(x > -104.0)) return make_float2(x != x ? NAN : 0.f, 0.f);
   if (x > 89.0) return make_float2(INFINITY, 0.f);
   const double whole = 6755399441055744.0;            // 1.5 2^52
   const double t = fma(x, 1.4426950408889634, whole);
   const int n = __double2loint(t);
-  const float rh = (float)fma(t - whole, -0.69314718055994531, x);
-  float q = fmaf(rh, 1.f / 5040.f, 1.f / 720.f);
+  const double r = fma(t - whole, -0.69314718055994531, x);
+  const float rh = (float)r;
+  float q = fmaf(rh, FINE ? fmaf(rh, 1.f / 40320.f, 1.f / 5040.f) : 1.f / 5040.f, 1.f / 720.f);
   q = fmaf(rh, q, 1.f / 120.f);
   q = fmaf(rh, q, 1.f / 24.f);
   q = fmaf(rh, q, 1.f / 6.f);
   q = fmaf(rh, q, 0.5f);
-  const float s = 1.f + rh, rest = fmaf(rh * rh, q, rh - (s - 1.f));
+  const float s = 1.f + rh;
+  float below = rh - (s - 1.f);
+  if (FINE) {
+    const float rl = (float)(r - (double)rh);
+    below += fmaf(rl, rh, rl);
+  }
+  const float rest = fmaf(rh * rh, q, below);
   const float hi = s + rest, lo = rest - (hi - s);
   // (two factors: n may lie below the smallest normal exponent)
   const int n1 = n >> 1;
@@ -926,6 +935,11 @@ __device__ __forceinline__ void ds_cp16(float* smem, const float* gmem, bool ok)
 #define DS_PREP_THREADS 256
 
 // grid (chunks, H): W [chunk][H][64][dk], Y [chunk][H][64][dv]
+// 1,111 and 694 tokens of 16 heads of 128: 39 us, 54 before (without terms and weights, 16 heads of
+// 64: 35, 46).  A block's phases follow one another (26,000 cycles, two blocks an SM), so it is the length of each that
+// counts: L's exponentials as products of the factors that the outputs' weights have anyway 7,400 -> 2,200 cycles; T's
+// rows with a thread at one row and column of each block, loops unrolled, 9,700 -> 3,100; the decays asked for ahead of
+// keys and values 3 us; W and Y with even shares for the schedulers 4,900 -> 4,100.
 __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     DsIn p, const int* __restrict__ q_start, const double* __restrict__ F,
     const float* __restrict__ KKm, float* __restrict__ W, float* __restrict__ Y,
@@ -947,6 +961,10 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const float* k = p.qkv + (size_t)(c.t0 + at) * p.stride + (size_t)(p.G + hq) * p.dk;
   const float* v = p.qkv + (size_t)(c.t0 + at) * p.stride + 2 * (size_t)p.G * p.dk + (size_t)h * p.dv;
+  // (the few numbers that are waited for first are asked for first)
+  const double* f = F + (size_t)h * p.T + c.t0 + at;
+  const double f0 = c.index ? f[-1] : 0.0, f_t = tid < n ? f[tid] : 0.0;
+  const float beta_t = tid < n ? p.gates[(size_t)(c.t0 + at + tid) * 2 * p.H + h] : 0.f;
   for (int i = tid; i < DS_C * (DS_D / 4); i += DS_PREP_THREADS) {
     const int r = i / (DS_D / 4), e = i % (DS_D / 4) * 4;
     const bool ok_k = r < n && e < p.dk, ok_v = r < n && e < p.dv;
@@ -954,36 +972,41 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     ds_cp16(Vs + r * DS_P + e, ok_v ? v + (size_t)r * p.stride + e : p.qkv, ok_v);
   }
   asm volatile("cp.async.commit_group;" ::);
-  const double* f = F + (size_t)h * p.T + c.t0 + at;
-  const double f0 = c.index ? f[-1] : 0.0;
-  if (Ww)                                        // (its tables lie where L and T will)
-    ct_weights(f, f, f0, n, 1.f, qkm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C,
-               *reinterpret_cast<CtWeights*>(Ls), Ww + (size_t)blockIdx.x * p.H + h);
-  if (tid == 0) odd = 0ull;
   if (tid < DS_C) {
-    fs[tid] = tid < n ? f[tid] - f0 : 0.0;
-    beta[tid] = tid < n ? p.gates[(size_t)(c.t0 + at + tid) * 2 * p.H + h] : 0.f;
-    grow[tid] = cs_times(beta[tid], cs_exp(fs[tid]));
+    fs[tid] = f_t;
+    beta[tid] = beta_t;
+    grow[tid] = cs_times(beta_t, cs_exp(tid < n ? f_t - f0 : 0.0));
   }
+  if (tid == 0) odd = 0ull;
+  __syncthreads();
+  // exp(F_t - F_s) for L, and for the outputs' weights; the tables lie where T will
+  static_assert(sizeof(CtWeights) <= DS_C * 68 * sizeof(float), "");
+  CtWeights& tab = *reinterpret_cast<CtWeights*>(Ts);
+  CtHead* head = Ww ? Ww + (size_t)blockIdx.x * p.H + h : nullptr;
+  ct_factors(fs, fs, f0, n, 1.f, tab, head ? head->at : nullptr);
+  if (head) ct_weights(tab, n, qkm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C, head);
+  const float* kk = KKm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C;
+  float4 kt[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) kt[i] = *reinterpret_cast<const float4*>(kk + (ty * 4 + i) * DS_C + 4 * tx);
   asm volatile("cp.async.wait_group 0;" ::);
   __syncthreads();
   // L: rows 4 ty .., columns 4 tx .., rounded once (keys alike make it hang on every bit)
-  const float* kk = KKm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int t = ty * 4 + i;
-    const float4 x = *reinterpret_cast<const float4*>(kk + t * DS_C + 4 * tx);
-    const float xs[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int s = 4 * tx + j;
-      float l = 0.f;
-      if (s < t && t < n) {
-        const float2 w = cs_exp(fs[t] - fs[s]);
-        l = (float)((double)beta[t] * ((double)w.x + (double)w.y) * (double)xs[j]);
-      }
-      Ls[t * 68 + s] = l;
-    }
+    const float4 x = kt[i];
+    const int bl = tx >> 2;                      // the block of 16 that s is in
+    const bool own = bl == t >> 4, some = 4 * tx < t && t < n;
+    const float4 hi = *reinterpret_cast<const float4*>(own ? &tab.near[0][t][4 * tx & 15] : &tab.col[0][4 * tx % 48]);
+    const float4 lo = *reinterpret_cast<const float4*>(own ? &tab.near[1][t][4 * tx & 15] : &tab.col[1][4 * tx % 48]);
+    const double by = (double)beta[t] * (own || !some ? 1.0 : (double)tab.row[0][bl][t] + (double)tab.row[1][bl][t]);
+    auto one = [&](float k2, float whi, float wlo, int j) {
+      return some && 4 * tx + j < t ? (float)(by * ((double)whi + (double)wlo) * (double)k2) : 0.f;
+    };
+    *reinterpret_cast<float4*>(Ls + t * 68 + 4 * tx) =
+        make_float4(one(x.x, hi.x, lo.x, 0), one(x.y, hi.y, lo.y, 1), one(x.z, hi.z, lo.z, 2),
+                    one(x.w, hi.w, lo.w, 3));
   }
   __syncthreads();
   // T = (I + L)^-1 by blocks of 16: the diagonal blocks, a thread a column ...
@@ -996,35 +1019,63 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     for (int t = 0; t < 16; ++t) {
       float r = t == j ? 1.f : 0.f;
 #pragma unroll
-      for (int s = 0; s < t; ++s) r = fmaf(-Ls[(o + t) * 68 + o + s], col[s], r);
+      for (int s = 0; s < t; s += 4) {
+        const float4 l = *reinterpret_cast<const float4*>(Ls + (o + t) * 68 + o + s);
+        r = fmaf(-l.x, col[s], r);
+        if (s + 1 < t) r = fmaf(-l.y, col[s + 1], r);
+        if (s + 2 < t) r = fmaf(-l.z, col[s + 2], r);
+        if (s + 3 < t) r = fmaf(-l.w, col[s + 3], r);
+      }
       col[t] = r;
       Ts[(o + t) * 68 + o + j] = r;
     }
   }
   __syncthreads();
-  // ... then block row by block row: T_i* = -T_ii (sum_k L_ik T_k*)
+  // ... then block row by block row: T_i* = -T_ii (sum_k L_ik T_k*), a thread row ty, column tx of each block
+#pragma unroll
   for (int i = 1; i < 4; ++i) {
-    const int cols = 16 * i;
-    for (int e = tid; e < 16 * cols; e += DS_PREP_THREADS) {
-      const int r = e / cols, j = e % cols;
-      float a0 = 0.f, a1 = 0.f;
-      for (int s = j & ~15; s < cols; s += 2) {
-        a0 = fmaf(Ls[(16 * i + r) * 68 + s], Ts[s * 68 + j], a0);
-        a1 = fmaf(Ls[(16 * i + r) * 68 + s + 1], Ts[(s + 1) * 68 + j], a1);
+    const float* l = Ls + (16 * i + ty) * 68;
+    float a0[3] = {0.f, 0.f, 0.f}, a1[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < 16 * i; s += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(l + s);
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        if (16 * b > s) continue;                // (T is zero there, but x may be infinite)
+        const float* t = Ts + s * 68 + 16 * b + tx;
+        a0[b] = fmaf(x.x, t[0], a0[b]);
+        a1[b] = fmaf(x.y, t[68], a1[b]);
+        a0[b] = fmaf(x.z, t[2 * 68], a0[b]);
+        a1[b] = fmaf(x.w, t[3 * 68], a1[b]);
       }
-      Rs[r * 52 + j] = a0 + a1;
     }
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (b < i) Rs[ty * 52 + 16 * b + tx] = a0[b] + a1[b];
     __syncthreads();
-    for (int e = tid; e < 16 * cols; e += DS_PREP_THREADS) {
-      const int r = e / cols, j = e % cols;
-      float a = 0.f;
-      // (row s of the block reaches the rows from s on alone, also where it is not finite)
-      for (int s = 0; s <= r; ++s) a = fmaf(Ts[(16 * i + r) * 68 + 16 * i + s], Rs[s * 52 + j], a);
-      Ts[(16 * i + r) * 68 + j] = -a;
+    float a[3] = {0.f, 0.f, 0.f};
+    float* t = Ts + (16 * i + ty) * 68;
+#pragma unroll
+    for (int s4 = 0; s4 < 16; s4 += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(t + 16 * i + s4);
+      const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // (row s of the block reaches the rows from s on alone, also where it is not finite)
+        if (s4 + j > ty) continue;
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+          if (b < i) a[b] = fmaf(xs[j], Rs[(s4 + j) * 52 + 16 * b + tx], a[b]);
+      }
     }
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (b < i) t[16 * b + tx] = -a[b];
     __syncthreads();
   }
-  // W = T (beta e^F K), Y = T (beta V): rows 4 ty .., columns 4 tx + 64 j
+  // W = T (beta e^F K), Y = T (beta V): rows 4 r4 .., columns 4 tx + 64 j.  (Row block r4 has r4 + 1 of 16 terms:
+  // warps w and w + 4, of one scheduler, have 34 between them whatever w is)
+  const int r4 = ty < 8 ? ty : 23 - ty;
 #pragma unroll 1
   for (int what = 0; what < 2; ++what) {
     const float* B = what ? Vs : Ks;
@@ -1041,7 +1092,7 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
       float4 tr[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        tr[i] = *reinterpret_cast<const float4*>(Ts + (ty * 4 + i) * 68 + s);
+        tr[i] = *reinterpret_cast<const float4*>(Ts + (r4 * 4 + i) * 68 + s);
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         const float fsc = sc[s + x];
@@ -1062,8 +1113,8 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
         }
       }
     };
-    for (int s = 0; s < ty * 4; s += 4) four(s, false);
-    four(ty * 4, true);
+    for (int s = 0; s < r4 * 4; s += 4) four(s, false);
+    four(r4 * 4, true);
     float* dst = (what ? Y : W) + ((size_t)blockIdx.x * p.H + h) * DS_C * width;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -1074,10 +1125,10 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
         float4 r;
         cs_unpair(acc[i][j][0], r.x, r.y);
         cs_unpair(acc[i][j][1], r.z, r.w);
-        *reinterpret_cast<float4*>(dst + (size_t)(ty * 4 + i) * width + col) = r;
+        *reinterpret_cast<float4*>(dst + (size_t)(r4 * 4 + i) * width + col) = r;
         // W in terms, too, for dt_walk
-        if (Xw && !what && cs_put_terms(Xw + ((size_t)blockIdx.x * p.H + h) * 2 * CS_TERMS_TILE, ty * 4 + i, col, r))
-          atomicOr(&odd, 1ull << (ty * 4 + i));
+        if (Xw && !what && cs_put_terms(Xw + ((size_t)blockIdx.x * p.H + h) * 2 * CS_TERMS_TILE, r4 * 4 + i, col, r))
+          atomicOr(&odd, 1ull << (r4 * 4 + i));
       }
   }
   if (Xw) {

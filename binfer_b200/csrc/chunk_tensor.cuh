@@ -28,7 +28,7 @@
 //
 // 2,000 tokens of 64 heads of 128 x 64 over 8: ct_state 36 us (cs_state and cs_prefix 87), ct_weights 15, ct_out 58
 // (cs_out 100); 1,300 and 812 tokens of 8 heads of 128 x 256: 25 (47), 5, 30 (58); the delta rule's 1,111 and 694 of
-// 16 heads of 128: dt_walk 59 (ds_walk 108), ct_out 31 (cs_out 53), ds_prep 54 (47).  What bounds ct_out is the rate
+// 16 heads of 128: dt_walk 59 (ds_walk 108), ct_out 31 (cs_out 53), ds_prep 39 (47).  What bounds ct_out is the rate
 // at which its warps get instructions (0.45 a cycle and scheduler): its time changes by 0 to 3 us without its
 // stores, with loads that always hit, with half of the products or without taking the operands apart.  ct_state and
 // dt_walk are bound by their chains: some 1,850 and 4,600 cycles a chunk.  (With a row of the state a thread, half
@@ -214,15 +214,19 @@ struct CtWeights {
   float col[2][48];                                      // exp(that - H_s)
 };
 
-// By a block of 256 threads; g, hs: G and H of the chunk's n tokens, before: G of the token ahead of them, pm: the
-// chunk's q . k.  Where s lies in an earlier block of 16 tokens than t, exp(G_t - H_s) is two factors (at most 1)
-// by the block's last G, each a float and what is left of it: some 700 exponentials and not 2,080.
-__device__ __forceinline__ void ct_weights(const double* g, const double* hs, double before, int n, float q_scale,
-                                           const float* __restrict__ pm, CtWeights& w, CtHead* __restrict__ to) {
+// By a block of 256 threads; g, hs: G and H of the chunk's n tokens, before: G of the token ahead of them, at: CtHead's
+// or null.  Where s lies in an earlier block of 16 tokens than t, exp(G_t - H_s) is two factors (at most 1) by the
+// block's last G, each a float and what is left of it: some 700 exponentials and not 2,080.
+__device__ __forceinline__ void ct_factors(const double* g, const double* hs, double before, int n, float q_scale,
+                                           CtWeights& w, float (*__restrict__ at)[CT_C]) {
   const int tid = threadIdx.x;
   if (tid < 2 * CT_C) (tid < CT_C ? w.g : w.h)[tid % CT_C] = tid % CT_C < n ? (tid < CT_C ? g : hs)[tid % CT_C] : 0.0;
   __syncthreads();
-  // (rows q and 15 - q of a block have 17 columns up to the diagonal; 48, 32 and 16 rows behind blocks 0, 1, 2)
+  // (rows q and 15 - q of a block have 17 columns up to the diagonal; 48, 32 and 16 rows behind blocks 0, 1, 2.
+  // A thread's three exponentials side by side: ds_prep 2 us less)
+  double d[3];
+  float *to[3], *left[3];
+  bool scaled = false;
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
     const int i = tid + 256 * x;
@@ -248,25 +252,37 @@ __device__ __forceinline__ void ct_weights(const double* g, const double* hs, do
       from = w.h[c];
       dst = &w.col[0][c];
       rest = &w.col[1][c];
-    } else if (i < 32 * 17 + 144 + CT_C) {
+    } else if (at && i < 32 * 17 + 144 + CT_C) {
       gi = i - 32 * 17 - 144;
       from = before;
-      dst = &to->at[0][gi];
-      rest = &to->at[1][gi];
-    } else {
-      continue;
+      dst = &at[0][gi];
+      rest = &at[1][gi];
+      scaled = x == 2;
     }
-    float2 e = make_float2(0.f, 0.f);
-    if (gi < n) e = cs_exp(w.g[gi] - from);
-    if (i >= 32 * 17 + 144) {                            // (the product's roundings are part of what is left)
-      const float f = e.x * q_scale;
-      e = make_float2(f, fmaf(e.x, q_scale, -f) + e.y * q_scale);
-      if (!(fabsf(f) < INFINITY)) e.y = 0.f;
-    }
-    *dst = e.x;
-    *rest = e.y;
+    d[x] = gi < n ? w.g[gi] - from : -INFINITY;          // (0 for rows that are not there)
+    to[x] = dst;
+    left[x] = rest;
+  }
+  float2 e[3];
+#pragma unroll
+  for (int x = 0; x < 3; ++x) e[x] = cs_exp<true>(d[x]);
+  if (scaled) {                                          // (the product's roundings are part of what is left)
+    const float f = e[2].x * q_scale;
+    e[2] = make_float2(f, fmaf(e[2].x, q_scale, -f) + e[2].y * q_scale);
+    if (!(fabsf(f) < INFINITY)) e[2].y = 0.f;
+  }
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    if (!to[x]) continue;
+    *to[x] = e[x].x;
+    *left[x] = e[x].y;
   }
   __syncthreads();
+}
+// pm: the chunk's q . k
+__device__ __forceinline__ void ct_weights(const CtWeights& w, int n, const float* __restrict__ pm,
+                                           CtHead* __restrict__ to) {
+  const int tid = threadIdx.x;
   // row tid / 4, octets tid % 4 and four further
   const int t = tid >> 2;
 #pragma unroll
@@ -306,8 +322,10 @@ __global__ void __launch_bounds__(256) ct_weights_kernel(CsIn p, const int* __re
   if (c.b < 0) return;
   const int at = c.index * CT_C, h = blockIdx.y, hq = h / (p.H / p.QH);
   const double* g = G + (size_t)h * p.T + c.t0 + at;
-  ct_weights(g, Hs + (g - G), c.index ? g[-1] : g0[(size_t)c.b * p.H + h], min(CT_C, c.n - at), p.q_scale,
-             qkm + ((size_t)blockIdx.x * p.QH + hq) * CT_C * CT_C, w, W + (size_t)blockIdx.x * p.H + h);
+  const int n = min(CT_C, c.n - at);
+  CtHead* to = W + (size_t)blockIdx.x * p.H + h;
+  ct_factors(g, Hs + (g - G), c.index ? g[-1] : g0[(size_t)c.b * p.H + h], n, p.q_scale, w, to->at);
+  ct_weights(w, n, qkm + ((size_t)blockIdx.x * p.QH + hq) * CT_C * CT_C, to);
 }
 
 // -------------------------------------------------------------------------------- ct_state
@@ -1122,7 +1140,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) dt_walk_kernel(
           if (!ok) break;
           mbar_expect_tx(sh.full + x, CT_S_KEYS);
           bf_bulk_load(x ? k_tile : w_tile,
-                       x ? Xk + (chunk * p.G + hq) * CT_S_KEYS : Xw + (chunk * p.H + h) * CT_S_KEYS, CT_S_KEYS, sh.full + x);
+                       x ? Xk + (chunk * p.G + hq) * CT_S_KEYS : Xw + (chunk * p.H + h) * CT_S_KEYS, CT_S_KEYS,
+                       sh.full + x);
           ++asked;
         }
       }

@@ -2378,6 +2378,40 @@ def test_chunks_are_as_close_to_64_bits_as_the_walk(cuda_device, kind, decays, a
         assert products <= max(1.1 * walk, 2.0 ** -24), off
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("rest", [1, 15, 16, 17, 33, 48, 63])
+def test_delta_chunks_weights_by_factors(cuda_device, rest, d):
+    """A last chunk that ends at and beside each block of 16 tokens, decays of zero among slow ones (a
+    factor of an earlier block is zero, or both of its sides are): relative errors of outputs and state
+    against float64, with the bound that the chunks have beside the walk (half as much again, and three
+    half units in the last place for the matrix products' sums)."""
+    from binfer_b200.csrc import ops
+    T, H, dev = 7 * 64 + rest, 2, cuda_device
+    torch.manual_seed(rest)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, H, d, device=dev), dim=-1) for _ in range(2))
+    v, beta = torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    g = (1 - 0.1 * torch.rand(T, H, device=dev)) * (torch.rand(T, H, device=dev) > 0.02)
+    s0 = torch.randn(1, H * d * d, device=dev)
+    S, want = s0.double().view(H, d, d).transpose(1, 2), []
+    for qt, kt, vt, gt, bt in zip(*(x.double() for x in (q, k, v, g, beta))):
+        S = S * gt[:, None, None]
+        S = S + kt[:, :, None] * (bt[:, None] * (vt - (kt[:, None] @ S)[:, 0]))[:, None]
+        want.append((qt[:, None] @ S)[:, 0])
+    want, off = torch.stack(want), []
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev)
+    for chunked in (False, True):
+        s, o = s0.clone(), torch.empty(T, H * d, device=dev)
+        ops.delta_scan(torch.cat([x.reshape(T, -1) for x in (q, k, v)], 1).contiguous(),
+                       torch.stack([beta, g], 1).contiguous(), s, qs, slots, o, 1, H, H, d, d, err,
+                       max_q=T, chunked=chunked)
+        off.append([float((x - y).norm() / y.norm()) for x, y in
+                    ((o.double().view(T, H, d), want), (s.double().view(H, d, d).transpose(1, 2), S))])
+    for walk, products in zip(*off):
+        assert products <= 1.5 * walk + 2e-7, off
+    assert int(err.item()) == 0
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("lens", [[1], [3, 1, 9, 2, 17], [1] * 5, [700, 1, 1, 643]])
