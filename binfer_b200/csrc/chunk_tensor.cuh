@@ -546,12 +546,13 @@ __global__ void __launch_bounds__(CT_S_THREADS, 1) ct_state_kernel(
           S[j0 + j] = cs_fma2(last[j], down, cs_fma2(dx2, before, cs_fma2(dy2, before, ct_mul2(rest[j], down))));
         }
       }
+      // (ahead of the arrival: behind it the products of chunk i + 2 may be done and chunk i + 4's flag be put here)
+      const bool odd = *(volatile int*)&odd_v[i & 3][lane] == i + 1;
       tc_fence_before();
       ct_arrive(sh.taken + (i & 1));
       float z0, z1;
       cs_unpair(zero, z0, z1);
       const bool lost = z0 + z1 != 0.f;
-      const bool odd = *(volatile int*)&odd_v[i & 3][lane] == i + 1;
       const unsigned odd_cols = __ballot_sync(0xffffffffu, odd) >> (16 * half) & 0xffffu;
       if (odd_cols || bad_now || lost) {
         float again[CT_SV / 2];

@@ -1,5 +1,7 @@
-"""Which recurrences run as products over chunks: the rule alone, without a GPU."""
+"""The recurrences as products over chunks, without a GPU: which ones run so, and the order of what no run shows."""
 import math
+import os
+import re
 
 import pytest
 import torch
@@ -121,3 +123,15 @@ def test_retention_wants_a_position_per_row(monkeypatch, positions):
         ops.retention_scan(torch.zeros(4, 24), 0, 8, 16, torch.zeros(1), None, positions,
                            torch.zeros(1, 64), one, one, torch.zeros(4, 8), 1, 1, 8, 8, 1.0, one)
     assert not seen
+
+
+def test_a_chunks_flags_are_read_before_its_place_is_given_back():
+    """ct_state's summing warps give a chunk's sums back by an arrival, and that is all that the flags of the chunk
+    four further, in the same place, wait for: what is read behind it may be theirs.  (A run hardly ever shows it.)"""
+    from binfer_b200.csrc import build
+    with open(os.path.join(build.HERE, "chunk_tensor.cuh")) as f:
+        kernel = f.read().split("ct_state_kernel(", 1)[1].split("\n}\n", 1)[0]
+    sums = kernel[kernel.index("the state: key size"):]
+    reads = [m.start() for m in re.finditer(r"odd_v\[", sums)]
+    assert reads and sums.count("ct_arrive(sh.taken") == 1
+    assert max(reads) < sums.index("ct_arrive(sh.taken")

@@ -1452,6 +1452,35 @@ def test_chunks_on_tensor_cores_take_floats_of_every_size(cuda_device, monkeypat
         assert torch.equal(outs[True, True][0][:at], outs[False, True][0][:at])
 
 
+@pytest.mark.parametrize("dv", [64, 128])
+def test_numbers_without_terms_four_chunks_apart(cuda_device, monkeypatch, dv):
+    """One value size has a float without terms in every fourth chunk, and a decay of zero forgets it: the flags of
+    those chunks share a place.  Between the zeros the results are the multiply-adds' but for rounding (chains of at
+    most 700 + 128 sums, twice: 2^-24 each, a tenth of that where they err at random)."""
+    from binfer_b200.csrc import ops
+    dev, T, H, G, dk = cuda_device, 700, 4, 2, 128
+    torch.manual_seed(13)
+    qk = torch.nn.functional.normalize(torch.randn(T, 2, G, dk, device=dev), dim=-1)
+    v, d = torch.randn(T, H, dv, device=dev), 1 - 0.1 * torch.rand(T, H, device=dev)
+    for at in (70, 326, 582):                    # in chunks 1, 5 and 9
+        v[at, 1, 5], d[at + 40, 1] = 3e31, 0.0
+    qs, slots = torch.tensor([0, T], dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    got, err = [], _err(dev)
+    for ctas in (0, 1 << 30):
+        monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", ctas)
+        s, o = torch.zeros(1, H * dk * dv, device=dev), torch.empty(T, H * dv, device=dev)
+        assert ops._chunk_scratch(True, T, T, 1, H, G, dk, dv, s, 0, qk)[1] == (ctas == 0)
+        ops.linear_scan(qk, v, d, s, qs, slots, o, 1, H, G, dk, dv, err, max_q=T, chunked=True)
+        got.append((o.view(T, H, dv), s))
+    assert int(err.item()) == 0
+    for a, e in ((0, 70), (70, 110), (110, 326), (326, 366), (366, 582), (582, 622), (622, T)):
+        x, y = (o[a:e] for o, _ in got)
+        for part in ((slice(None), 1, 5), (slice(None), 0), (slice(None), 1, slice(6, None))):
+            assert bool(y[part].isfinite().all()) and float(y[part].norm()) > 0
+            assert float((x[part] - y[part]).norm() / y[part].norm()) <= 1e-5, (a, part)
+    assert float((got[0][1] - got[1][1]).norm() / got[1][1].norm()) <= 1e-5
+
+
 def test_linear_chunks_on_tensor_cores_of_many_tiles(cuda_device, monkeypatch):
     """More tiles than one CTA an SM has room for in its list: the multiply-adds' results."""
     from binfer_b200.csrc import ops
