@@ -934,6 +934,16 @@ __device__ __forceinline__ void ds_cp16(float* smem, const float* gmem, bool ok)
 #define DS_NS 32           // columns of the state a CTA of ds_walk keeps
 #define DS_PREP_THREADS 256
 
+// four of L's numbers, all left of the diagonal, with exponentials of their own
+__device__ __noinline__ void ds_again_L(const double* fs, float beta, int t, int s, float4 kk, float* out) {
+  const float xs[4] = {kk.x, kk.y, kk.z, kk.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 w = cs_exp(fs[t] - fs[s + j]);
+    out[j] = (float)((double)beta * ((double)w.x + (double)w.y) * (double)xs[j]);
+  }
+}
+
 // grid (chunks, H): W [chunk][H][64][dk], Y [chunk][H][64][dv]
 // 1,111 and 694 tokens of 16 heads of 128: 39 us, 54 before (without terms and weights, 16 heads of
 // 64: 35, 46).  A block's phases follow one another (26,000 cycles, two blocks an SM), so it is the length of each that
@@ -983,8 +993,8 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
   static_assert(sizeof(CtWeights) <= DS_C * 68 * sizeof(float), "");
   CtWeights& tab = *reinterpret_cast<CtWeights*>(Ts);
   CtHead* head = Ww ? Ww + (size_t)blockIdx.x * p.H + h : nullptr;
-  ct_factors(fs, fs, f0, n, 1.f, tab, head ? head->at : nullptr);
-  if (head) ct_weights(tab, n, qkm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C, head);
+  const bool above = ct_factors(fs, fs, f0, n, 1.f, tab, head ? head->at : nullptr);
+  if (head) ct_weights(tab, n, above, qkm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C, head);
   const float* kk = KKm + ((size_t)blockIdx.x * p.G + hq) * DS_C * DS_C;
   float4 kt[4];
 #pragma unroll
@@ -1004,6 +1014,10 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
     auto one = [&](float k2, float whi, float wlo, int j) {
       return some && 4 * tx + j < t ? (float)(by * ((double)whi + (double)wlo) * (double)k2) : 0.f;
     };
+    if (above && !own && some) {
+      ds_again_L(fs, beta[t], t, 4 * tx, x, Ls + t * 68 + 4 * tx);
+      continue;
+    }
     *reinterpret_cast<float4*>(Ls + t * 68 + 4 * tx) =
         make_float4(one(x.x, hi.x, lo.x, 0), one(x.y, hi.y, lo.y, 1), one(x.z, hi.z, lo.z, 2),
                     one(x.w, hi.w, lo.w, 3));

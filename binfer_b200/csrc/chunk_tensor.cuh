@@ -215,9 +215,11 @@ struct CtWeights {
 };
 
 // By a block of 256 threads; g, hs: G and H of the chunk's n tokens, before: G of the token ahead of them, at: CtHead's
-// or null.  Where s lies in an earlier block of 16 tokens than t, exp(G_t - H_s) is two factors (at most 1) by the
-// block's last G, each a float and what is left of it: some 700 exponentials and not 2,080.
-__device__ __forceinline__ void ct_factors(const double* g, const double* hs, double before, int n, float q_scale,
+// or null.  Where s lies in an earlier block of 16 tokens than t, exp(G_t - H_s) is two factors by the block's last G,
+// each a float and what is left of it: some 700 exponentials and not 2,080.  Returns true where a factor is above 1,
+// as decays above 1 make it: the other one may then lie below the normal floats while the product does not, and
+// whoever asks takes the exponential itself.
+__device__ __forceinline__ bool ct_factors(const double* g, const double* hs, double before, int n, float q_scale,
                                            CtWeights& w, float (*__restrict__ at)[CT_C]) {
   const int tid = threadIdx.x;
   if (tid < 2 * CT_C) (tid < CT_C ? w.g : w.h)[tid % CT_C] = tid % CT_C < n ? (tid < CT_C ? g : hs)[tid % CT_C] : 0.0;
@@ -226,7 +228,7 @@ __device__ __forceinline__ void ct_factors(const double* g, const double* hs, do
   // A thread's three exponentials side by side: ds_prep 2 us less)
   double d[3];
   float *to[3], *left[3];
-  bool scaled = false;
+  bool scaled = false, above = false;
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
     const int i = tid + 256 * x;
@@ -260,6 +262,7 @@ __device__ __forceinline__ void ct_factors(const double* g, const double* hs, do
       scaled = x == 2;
     }
     d[x] = gi < n ? w.g[gi] - from : -INFINITY;          // (0 for rows that are not there)
+    above |= i >= 32 * 17 && i < 32 * 17 + 144 && d[x] > 0.0;
     to[x] = dst;
     left[x] = rest;
   }
@@ -277,10 +280,17 @@ __device__ __forceinline__ void ct_factors(const double* g, const double* hs, do
     *to[x] = e[x].x;
     *left[x] = e[x].y;
   }
-  __syncthreads();
+  return __syncthreads_or(above);
 }
-// pm: the chunk's q . k
-__device__ __forceinline__ void ct_weights(const CtWeights& w, int n, const float* __restrict__ pm,
+// the weights of a row's octet as exponentials of their own
+__device__ __noinline__ void ct_weights_again(const CtWeights& w, int t, int s, int n, const float* __restrict__ pm,
+                                              CtHead* __restrict__ to) {
+#pragma unroll 1
+  for (int c = s; c < s + 8; ++c)
+    to->P[t][c] = t < n && c <= t ? cs_times(pm[t * CT_C + c], cs_exp(w.g[t] - w.h[c])) : 0.f;
+}
+// pm: the chunk's q . k, above: ct_factors'
+__device__ __forceinline__ void ct_weights(const CtWeights& w, int n, bool above, const float* __restrict__ pm,
                                            CtHead* __restrict__ to) {
   const int tid = threadIdx.x;
   // row tid / 4, octets tid % 4 and four further
@@ -290,6 +300,10 @@ __device__ __forceinline__ void ct_weights(const CtWeights& w, int n, const floa
     const int s = 8 * ((tid & 3) + 4 * x), cb = s >> 4;
     if (cb > t >> 4) continue;
     const bool own = cb == t >> 4;
+    if (above && !own) {
+      ct_weights_again(w, t, s, n, pm, to);
+      continue;
+    }
     const float rx = own ? 0.f : w.row[0][cb][t], ry = own ? 0.f : w.row[1][cb][t];
     const int last = t < n ? t - s : -1;
 #pragma unroll
@@ -324,8 +338,9 @@ __global__ void __launch_bounds__(256) ct_weights_kernel(CsIn p, const int* __re
   const double* g = G + (size_t)h * p.T + c.t0 + at;
   const int n = min(CT_C, c.n - at);
   CtHead* to = W + (size_t)blockIdx.x * p.H + h;
-  ct_factors(g, Hs + (g - G), c.index ? g[-1] : g0[(size_t)c.b * p.H + h], n, p.q_scale, w, to->at);
-  ct_weights(w, n, qkm + ((size_t)blockIdx.x * p.QH + hq) * CT_C * CT_C, to);
+  const bool above =
+      ct_factors(g, Hs + (g - G), c.index ? g[-1] : g0[(size_t)c.b * p.H + h], n, p.q_scale, w, to->at);
+  ct_weights(w, n, above, qkm + ((size_t)blockIdx.x * p.QH + hq) * CT_C * CT_C, to);
 }
 
 // -------------------------------------------------------------------------------- ct_state

@@ -2441,6 +2441,50 @@ def test_delta_chunks_weights_by_factors(cuda_device, rest, d):
     assert int(err.item()) == 0
 
 
+@pytest.mark.parametrize("grows,first", [(60, 1e17), (84, 1e9)])
+@pytest.mark.parametrize("kind,d", [("linear", 128), ("delta", 64), ("delta", 128)])
+def test_chunks_of_decays_above_one(cuda_device, monkeypatch, kind, d, grows, first):
+    """Twelve tokens of a block of 16 make the state e^grows times larger, thirty behind them e^100 times smaller:
+    the tokens ahead of them (of values so large that they still count) have weights that are floats, one of whose
+    two factors by the block's end is not, or without most of its bits.  (The delta rule's tokens between leave the
+    state alone: its own u are of no use where weights leave the floats.)  Every token's result within the bound of
+    its sums (d products of q and S, 64 weighted tokens, as many in u: 2^-24 each)."""
+    from binfer_b200.csrc import ops
+    T, H, dev = 500, 2, cuda_device
+    torch.manual_seed(grows)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, H, d, device=dev), dim=-1) for _ in range(2))
+    v, beta = 1e-30 * torch.randn(T, H, d, device=dev), torch.rand(T, H, device=dev)
+    v[128:132] *= first
+    beta[132:176] = 0.0
+    g = 1 - 0.02 * torch.rand(T, H, device=dev)
+    g[132:144], g[146:176] = math.exp(grows / 12), math.exp(-100 / 30)
+    s0 = 1e-30 * torch.randn(1, H * d * d, device=dev)
+    S, want = s0.double().view(H, d, d).transpose(1, 2), []
+    for qt, kt, vt, gt, bt in zip(*(x.double() for x in (q, k, v, g, beta))):
+        S = S * gt[:, None, None]
+        u = bt[:, None] * (vt - (kt[:, None] @ S)[:, 0]) if kind == "delta" else vt
+        S = S + kt[:, :, None] * u[:, None]
+        want.append((qt[:, None] @ S)[:, 0])
+    want = torch.stack(want)
+    qs = torch.tensor([0, T], dtype=torch.int32, device=dev)
+    slots, err = torch.zeros(1, dtype=torch.int32, device=dev), _err(dev)
+    monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", 0)
+    s, o = s0.clone(), torch.empty(T, H * d, device=dev)
+    if kind == "linear":
+        qk = torch.stack([q, k], 1).contiguous()
+        assert ops._chunk_scratch(True, T, T, 1, H, H, d, d, s, 0, qk, v, o)[1]
+        ops.linear_scan(qk, v, g, s, qs, slots, o, 1, H, H, d, d, err, max_q=T, chunked=True)
+    else:
+        ops.delta_scan(torch.cat([x.reshape(T, -1) for x in (q, k, v)], 1).contiguous(),
+                       torch.stack([beta, g], 1).contiguous(), s, qs, slots, o, 1, H, H, d, d, err,
+                       max_q=T, chunked=True)
+    c = (d + 128) * 2.0 ** -24
+    off = (o.double().view(T, H, d) - want).norm(dim=2) / want.norm(dim=2)
+    assert float(off.max()) <= c, (int(off.max(1)[0].argmax()), float(off.max()))
+    assert float((s.double().view(H, d, d).transpose(1, 2) - S).norm() / S.norm()) <= c
+    assert int(err.item()) == 0
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("lens", [[1], [3, 1, 9, 2, 17], [1] * 5, [700, 1, 1, 643]])
