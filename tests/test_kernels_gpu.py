@@ -1433,6 +1433,8 @@ def test_chunks_on_tensor_cores_take_floats_of_every_size(cuda_device, monkeypat
                 fn = ops.lib().bf_chunk_scan_delta_scratch
                 args = [ops._c_int(z) for z in (T, 1, H, G, dk, dv, 0, 0)]
                 monkeypatch.setattr(ops, "CHUNK_SCAN_MAX_BYTES", fn(*args))
+            assert (_delta_on_tensor_cores(T, 1, H, G, dk, dv) if kind == "delta" else
+                    ops._chunk_scratch(True, T, T, 1, H, G, dk, dv, s0, 0)[1]) == (ctas == 0)
             s, o = s0.clone(), torch.empty(T, H * dv, device=dev)
             if kind == "linear":
                 ops.linear_scan(x, v, d, s, qs, slots, o, 1, H, G, dk, dv, err, max_q=T, chunked=True)
@@ -1494,6 +1496,7 @@ def test_linear_chunks_on_tensor_cores_of_many_tiles(cuda_device, monkeypatch):
     for ctas in (0, 1 << 30):
         monkeypatch.setattr(ops, "LINEAR_TENSOR_MIN_CTAS", ctas)
         s, o = torch.zeros(1, H * dk * dv, device=dev), torch.empty(T, H * dv, device=dev)
+        assert ops._chunk_scratch(True, T, T, 1, H, 8, dk, dv, s, 0)[1] == (ctas == 0)
         ops.linear_scan(qk, v, d, s, qs, slots, o, 1, H, 8, dk, dv, err, max_q=T, chunked=True)
         got.append((o, s))
     assert int(err.item()) == 0
@@ -2307,14 +2310,27 @@ def test_attention_f32_keys_that_a_row_does_not_see(cuda_device, window):
     _close(out[fin].cpu(), want[fin].cpu(), F32)
 
 
+def _delta_on_tensor_cores(T, B, H, G, dk, dv):
+    """Whether ``ops.delta_scan`` runs a step's chunks on the tensor cores: they take the sizes, and their scratch is
+    within the limit."""
+    from binfer_b200.csrc import ops
+    fn = ops.lib().bf_chunk_scan_delta_scratch
+    fn.restype = ops._c_ll
+    return 0 < fn(*(ops._c_int(x) for x in (T, B, H, G, dk, dv, ops._chunk_limit(B, ops.DELTA_CHUNK_MIN), 1))) <= (
+        ops.CHUNK_SCAN_MAX_BYTES)
+
+
 @pytest.mark.parametrize("lens,H,G,dk,dv", [([161, 1, 192, 160, 257], 4, 2, 32, 24),
-                                            ([300], 2, 1, 128, 128), ([193, 3], 3, 3, 68, 100)])
+                                            ([300], 2, 1, 128, 128), ([193, 3], 3, 3, 68, 100),
+                                            ([161, 1, 192, 160, 257], 4, 2, 128, 128),
+                                            ([193, 320], 4, 2, 128, 64)])
 def test_delta_scan_in_chunks(cuda_device, monkeypatch, lens, H, G, dk, dv):
     """Against the walking kernel and both against float64: the products are no further off."""
     from binfer_b200.csrc import ops
     monkeypatch.setattr(ops, "DELTA_CHUNK_MIN", 160)
     torch.manual_seed(len(lens) + dk)
     T, B, dev = sum(lens), len(lens), cuda_device
+    assert _delta_on_tensor_cores(T, B, H, G, dk, dv) == (dk == 128)
     q, k = (torch.nn.functional.normalize(torch.randn(T, G, dk, device=dev), dim=-1)
             for _ in range(2))
     # neighbouring keys alike, so that a chunk's writes hang together
@@ -2357,6 +2373,42 @@ def test_delta_scan_in_chunks(cuda_device, monkeypatch, lens, H, G, dk, dv):
     ops.delta_scan(qkv, gates, keep, qs, bad, o, B, H, G, dk, dv, err, max_q=max(lens), chunked=True)
     assert int(err.item()) == 2 and torch.equal(keep[int(slots[0])], got[True][1][int(slots[0])])
     err.zero_()
+
+
+@pytest.mark.parametrize("what", ["v", "k", "q", "state"])
+@pytest.mark.parametrize("dv", [64, 128])
+def test_delta_chunks_keep_to_their_portion(cuda_device, monkeypatch, dv, what):
+    """An infinity in the last of three portions, with a single token beside them: the numbers of that portion alone
+    are not finite, the same ones as by multiply-adds, and the others' bits are the clean call's."""
+    from binfer_b200.csrc import ops
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN", 160)
+    lens, H, G, dk, dev = [193, 1, 320, 260], 4, 2, 128, cuda_device
+    T, B, at = sum(lens), len(lens), sum(lens[:3]) + 70
+    torch.manual_seed(17)
+    q, k = (torch.nn.functional.normalize(torch.randn(T, G, dk, device=dev), dim=-1) for _ in range(2))
+    v, s0 = torch.randn(T, H, dv, device=dev), torch.randn(B, H * dk * dv, device=dev)
+    gates = torch.stack([torch.rand(T, H, device=dev), 1 - 0.05 * torch.rand(T, H, device=dev)], 1).contiguous()
+    qs = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=dev)
+    slots, err, got = torch.arange(B, dtype=torch.int32, device=dev), _err(dev), {}
+    room = ops.CHUNK_SCAN_MAX_BYTES
+    fn = ops.lib().bf_chunk_scan_delta_scratch
+    fn.restype = ops._c_ll
+    without = fn(*(ops._c_int(x) for x in (T, B, H, G, dk, dv, ops._chunk_limit(B, 160), 0)))
+    for bad, tensor in ((False, True), (True, True), (True, False)):
+        monkeypatch.setattr(ops, "CHUNK_SCAN_MAX_BYTES", room if tensor else without)
+        assert _delta_on_tensor_cores(T, B, H, G, dk, dv) == tensor
+        x = {"q": q.clone(), "k": k.clone(), "v": v.clone(), "state": s0.clone()}
+        if bad:
+            {"q": x["q"][at, 1], "k": x["k"][at, 0], "v": x["v"][at, 2], "state": x["state"][3]}[what][9] = math.inf
+        qkv = torch.cat([x[n].reshape(T, -1) for n in "qkv"], 1).contiguous()
+        o = torch.empty(T, H * dv, device=dev)
+        ops.delta_scan(qkv, gates, x["state"], qs, slots, o, B, H, G, dk, dv, err, max_q=max(lens), chunked=True)
+        got[bad, tensor] = (o, x["state"])
+    assert int(err.item()) == 0
+    (o0, clean), (o, s), (o_adds, s_adds) = got[False, True], got[True, True], got[True, False]
+    assert bool(o0.isfinite().all()) and not bool(o.isfinite().all())
+    assert torch.equal(o.isfinite(), o_adds.isfinite()) and torch.equal(s.isfinite(), s_adds.isfinite())
+    assert torch.equal(o[:sum(lens[:3])], o0[:sum(lens[:3])]) and torch.equal(s[:3], clean[:3])
 
 
 # keys at random, alike by a half and nearly the same; decays that forget in a few tokens and slow ones
@@ -2412,8 +2464,9 @@ def test_chunks_are_as_close_to_64_bits_as_the_walk(cuda_device, kind, decays, a
 def test_delta_chunks_weights_by_factors(cuda_device, rest, d):
     """A last chunk that ends at and beside each block of 16 tokens, decays of zero among slow ones (a
     factor of an earlier block is zero, or both of its sides are): relative errors of outputs and state
-    against float64, with the bound that the chunks have beside the walk (half as much again, and three
-    half units in the last place for the matrix products' sums)."""
+    against float64, beside the walk's 0.9 to 1.3e-7.  A chunk rounds the state once where the walk rounds it
+    with every token: the products have 0.73 to 0.84 of the walk's errors with keys of 64 and 0.55 to 0.67 on the
+    tensor cores, and weights that are half a unit in the last place off on one side would add more than is left."""
     from binfer_b200.csrc import ops
     T, H, dev = 7 * 64 + rest, 2, cuda_device
     torch.manual_seed(rest)
@@ -2437,7 +2490,7 @@ def test_delta_chunks_weights_by_factors(cuda_device, rest, d):
         off.append([float((x - y).norm() / y.norm()) for x, y in
                     ((o.double().view(T, H, d), want), (s.double().view(H, d, d).transpose(1, 2), S))])
     for walk, products in zip(*off):
-        assert products <= 1.5 * walk + 2e-7, off
+        assert products <= (0.75 if d == 128 else 0.9) * walk, off
     assert int(err.item()) == 0
 
 
