@@ -781,8 +781,8 @@ def _chunk_scratch(chunked: bool, max_q: int, T: int, B: int, heads: int, qk_hea
         return None, 0
     fn = lib().bf_chunk_scan_scratch
     fn.restype = _c_ll
-    few = heads * (dk // 128) * (dv // 32) < LINEAR_TENSOR_MIN_CTAS
-    for terms in (0,) if few else (1, 0):
+    with_terms = not mlstm and heads * (dk // 128) * (dv // 32) >= LINEAR_TENSOR_MIN_CTAS
+    for terms in (1, 0) if with_terms else (0,):
         n = fn(_c_int(T), _c_int(B), _c_int(heads), _c_int(qk_heads), _c_int(dk), _c_int(dv),
                _c_int(CHUNK_SCAN_TOKENS), _c_int(mlstm), _c_int(_chunk_limit(B, CHUNK_SCAN_MIN)),
                _c_int(terms))

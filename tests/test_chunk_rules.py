@@ -76,6 +76,24 @@ def test_scans_off_16_byte_boundaries_are_walked(monkeypatch):
             assert seen and not any(n.endswith("_chunks") for n in seen), (call, off)
 
 
+def test_the_matrix_memory_asks_for_its_scratch_once(monkeypatch):
+    """The room for a linear scan's terms is none of its business."""
+    from binfer_b200.csrc import ops
+    lib, asked = FakeLibrary(), []
+
+    def entry(*args):
+        asked.append(args[-1].value)
+        return lib.scratch
+
+    lib.bf_chunk_scan_scratch = entry
+    monkeypatch.setattr(ops, "lib", lambda: lib)
+    state = torch.zeros(1, 8, 256 * 512 + 512)
+    for mlstm, want in ((1, [0]), (0, [1])):
+        asked.clear()
+        scratch, terms = ops._chunk_scratch(True, 2048, 2048, 1, 8, 8, 256, 512, state, mlstm)
+        assert asked == want and terms == want[0] and scratch.numel() == 4096
+
+
 # us on a B200: (heads, dk, dv, portions, tokens of each): (walk, products over chunks)
 LINEAR_US = {
     (64, 128, 64, 1, 161): (42, 46), (64, 128, 64, 1, 200): (51, 50), (64, 128, 64, 1, 260): (64, 55),
