@@ -7,8 +7,8 @@
 //
 // With F_t the sum of the log decays up to token t, H_s = F_s - i_s and G_t = min(-m_0, min_{s <= t}
 // H_s) (linear: i = m = 0 and G = H = F), token s reaches token t with the weight exp(G_t - H_s)
-// <= 1 and the state before a chunk whose last earlier token is c with exp(G_t - G_c); for the
-// mLSTM m_t = F_t - G_t.  F, G and H are double, so a difference of two of them is good to a
+// (at most 1 unless a decay is above it) and the state before a chunk whose last earlier token is c with
+// exp(G_t - G_c); for the mLSTM m_t = F_t - G_t.  F, G and H are double, so a difference of two of them is good to a
 // float's last bit; its exponential is a float and what is left of it (cs_exp), the products of q and k
 // (and of k and k) inside a chunk are summed in double and rounded once, every other product is float
 // (FP32 multiply-adds; on the tensor cores where those files take the sizes: exact products of bfloat16 terms, added
@@ -27,16 +27,16 @@
 // 128, values of 64 or whole tiles of 128 and CTAs enough, and the delta rule with keys of 128 (chunk_tensor.cuh).
 //
 // GPU time at 2,048 tokens, chunks / walk: 64 heads of 128 x 64 over 8 q/k heads by multiply-adds 208 / 467 us (cs_out
-// 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 138; 8 heads of 128 x 256 124 / 270 (83);
+// 99, cs_state 62, cs_prefix 25, cs_qk 14, cs_gates 8), on the tensor cores 133; 8 heads of 128 x 256 117 / 288 (87);
 // mLSTM, 8 heads of 256 x 512, 392 / 979 (171, 123, 55, 32, 11; on the tensor cores 212).  What bounds them:
-// cs_state and cs_out shared-memory reads (the pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double tensor pipe, cs_prefix memory.  With
-// expf, float products of q and k and the states' sums in runs of 16 these were 204, 119 and 381 us, and
-// further from 64 bits than the walk where decays are fast.
+// cs_state and cs_out shared-memory reads (the pipe is 0.61 to 0.64 busy, the multiply-adds 0.3), cs_qk the double
+// tensor pipe, cs_prefix memory.  With expf, float products of q and k and the states' sums in runs of 16 these were
+// 204, 119 and 381 us, and further from 64 bits than the walk where decays are fast.
 //
-// Relative errors against 64 bits over 777 tokens, walk / chunks: decays of 0.98 to 1: o 1.9e-7 / 1.4e-7,
-// state 1.8e-7 / 1.3e-7; spread over 0 to 1: o 8.3e-8 / 5.0e-8, state 4.0e-8 / 4.2e-8 (half a unit in the
-// last place is up to 6.0e-8); mLSTM, gates that forget in a few tokens and in twenty: o 4.8e-7 / 2.3e-7 and
-// 1.3e-5 / 1.2e-6, state 2.9e-8 / 3.7e-8 and 2.3e-7 / 1.0e-7.
+// Relative errors against 64 bits over 777 tokens, walk / chunks by multiply-adds (chunk_tensor.cuh has those of the
+// tensor cores): decays of 0.98 to 1: o 1.9e-7 / 1.4e-7, state 1.8e-7 / 1.3e-7; spread over 0 to 1: o 8.3e-8 /
+// 5.0e-8, state 4.0e-8 / 4.2e-8 (half a unit in the last place is up to 6.0e-8); mLSTM, gates that forget in a few
+// tokens and in twenty: o 4.8e-7 / 2.3e-7 and 1.3e-5 / 1.2e-6, state 2.9e-8 / 3.7e-8 and 2.3e-7 / 1.0e-7.
 //
 // Why: the walk has heads x dk x dv independent elements and a chain of multiply-adds from token to
 // token, so it left the FP32 pipes at 15 to 20 % (see those files); the products have no chain and
@@ -55,8 +55,8 @@
 //              32 columns) in parallel
 //   cs_out     as above, on U
 //
-// 2,048 tokens of 16 heads of 128: 333 us (ds_walk 187, cs_out 54, ds_prep 40, cs_qk 42) by multiply-adds against the
-// walk's 563; 1,000 tokens 168 and 277, three portions of 1,000 381 and 431.  Errors against 64 bits, walk / chunks:
+// 2,048 tokens of 16 heads of 128: 320 us by multiply-adds, 225 on the tensor cores against the walk's 565; 1,000
+// tokens 169, 117 and 279, three portions of 1,000 387, 286 and 432.  Errors against 64 bits, walk / multiply-adds:
 // keys at random, decays of 0.98 to 1: o 2.3e-7 / 1.6e-7, state 2.3e-7 / 1.8e-7; keys of a cosine of 0.9
 // 2.6e-7 / 2.6e-7 and 2.5e-7 / 2.5e-7; fast decays o 1.1e-7 / 7.8e-8, state 6.2e-8 / 7.1e-8.  (What the walk
 // has and a chunk's inverse has not is that a token's u answers to the rounding of the one before it:
@@ -1154,8 +1154,9 @@ __global__ void __launch_bounds__(DS_PREP_THREADS, 2) ds_prep_kernel(
 // grid (column slices of 32, H, B): u [T][H][dv], Sc [chunk][H][dk][dv] (the state before each chunk).
 // 128 threads with 4 x 4 outputs of U and 8 x 4 of the state each: what a thread reads from shared
 // memory (at 128 bytes a cycle and SM) is about what its multiply-adds take.  1,111 and 694 tokens of
-// 16 heads of 128: 115 us; 256 threads with half of that 130, and the state's columns in the lanes'
-// registers, W and K read by all lanes alike, 133.
+// 16 heads of 64: 86 us.  (By 16 heads of 128, which dt_walk takes unless its scratch is too much: 108 us; the
+// choices were made there, at 115: 256 threads with half of that 130, and the state's columns in the lanes'
+// registers, W and K read by all lanes alike, 133.)
 __global__ void __launch_bounds__(128) ds_walk_kernel(
     DsIn p, const int* __restrict__ q_start, const int* __restrict__ state_slots, int n_slots,
     float* __restrict__ state, long long slot_stride, const double* __restrict__ F,

@@ -10,10 +10,11 @@
 //   ct_out     what cs_out computes: 128 value sizes (of one head, or of two heads of 64) x 64 tokens a tile,
 //              a CTA an SM goes from tile to tile
 //
-// Both have a warp that asks for the terms' tiles, warps that weight the other operand, take it apart and store
-// its terms, a warp that issues the products and warps that take the sums out of tensor memory and add;
-// each goes ahead as far as rings of two to four places let it.  (One set of warps that did all of it in
-// turn spent three quarters of its time waiting for its own copies and sums.)
+// ct_state and ct_out have a warp that asks for the terms' tiles, warps that weight the other operand, take it apart
+// and store its terms, two warps that issue the products in turn and warps that take the sums out of tensor memory and
+// add; each goes ahead as far as rings of two to four places let it.  (One set of warps that did all of it in
+// turn spent three quarters of its time waiting for its own copies and sums.)  dt_walk's two products a chunk wait
+// for one another, so the warps that keep the state do both there.
 //
 // A step has 64 terms.  Products of a leading term with all three of the other side go out as one instruction
 // of three times the columns, so a step's rows are read from shared memory three times and not six:
@@ -31,11 +32,16 @@
 // 16 heads of 128: dt_walk 59 (ds_walk 108), ct_out 31 (cs_out 53), ds_prep 39 (47).  What bounds ct_out is the rate
 // at which its warps get instructions (0.45 a cycle and scheduler): its time changes by 0 to 3 us without its
 // stores, with loads that always hit, with half of the products or without taking the operands apart.  ct_state and
-// dt_walk are bound by their chains: some 1,850 and 4,600 cycles a chunk.  (With a row of the state a thread, half
-// as many warps, they were 39 and 70 us.)
-// Relative errors against 64 bits (outputs, states), these / multiply-adds, e-7: decays of 0.98 to 1 0.79 0.66 / 1.37
-// 1.29, a state space layer's 0.55 0.46 / 0.68 0.59, spread over 0 to 1 0.51 0.42 / 0.50 0.42; the delta rule's 0.97
-// 0.86 / 1.63 1.80, 0.66 0.59 / 0.77 0.68, 0.58 0.55 / 0.57 0.48.
+// dt_walk are bound by their chains: some 1,460 (25 of its 35 us at 32 chunks; the rest is its start and end) and
+// 4,600 cycles a chunk.  (With a row of the state a thread, half as many warps, they were 39 and 70 us.)
+// Relative errors against 64 bits (outputs, states), these / multiply-adds, e-7: decays of 0.98 to 1 0.78 0.66 / 1.32
+// 1.28, a state space layer's 0.55 0.46 / 0.68 0.59, spread over 0 to 1 0.51 0.43 / 0.54 0.42, a tenth of those zero
+// 0.50 0.42 / 0.51 0.37; the delta rule's 0.91 0.85 / 1.61 1.80, 0.66 0.59 / 0.77 0.68, 0.60 0.56 / 0.66 0.50, 0.58
+// 0.52 / 0.64 0.46.  Where a state is made up of a few tokens, as with the last two, it is up to 0.06e-7 further
+// off (half a unit in the last place is 0.6e-7): its last terms' sum is cut, one more loss of the size of a rounding.
+// More or less than ct_take's 2^-25 is no way out (delta, spread and zeros: none 0.66 0.55, half of it 0.59 0.51,
+// three quarters 0.57 0.51), nor are the products of terms that are left out (0.557 0.514, and 5 us more of 139) or
+// both roundings of the last additions kept (no change).
 //
 // Included by chunk_scan.cu behind mlstm_tensor.cuh.
 #pragma once

@@ -747,8 +747,10 @@ CHUNK_SCAN_MAX_BYTES = 768 << 20
 # Fewest CTAs of a request (a head's 128 key x 32 value sizes each) for a linear scan's chunks on the tensor
 # cores, where ct_state goes from chunk to chunk and cs_state has CTAs for every chunk.  Tensor cores / multiply-adds
 # in us at 500, 2,000 and 8,192 tokens: 16 CTAs 50 / 48, 72 / 65, 220 / 204; 32 50 / 52, 84 / 90, 270 / 312; 64 51 / 56,
-# 99 / 130, 310 / 464; 128 58 / 77, 140 / 224, 441 / 823 (what shares the step does not count: a request's results
-# have the same bits beside others).
+# 99 / 130, 310 / 464; 128 58 / 77, 140 / 224, 441 / 823.  This line counts a request's CTAs and not the step's; the
+# scratch limit and chunk_scan_pays do look at the whole step, so what shares it can change which kernels run.  (The
+# delta rule has no such line: with 1 and 2 heads of 128 400 to 4,000 tokens take 66 to 244 us there and 88 to 393 by
+# multiply-adds.)
 LINEAR_TENSOR_MIN_CTAS = 32
 
 
@@ -1097,13 +1099,15 @@ DELTA_CHUNK_MIN = 384
 
 
 def delta_chunks_pay(tokens: int, max_q: int, heads: int, dk: int, dv: int) -> bool:
-    """Whether a step's gated delta rule is the faster one in chunks (arguments and the chunks' kernels as for
-    :func:`chunk_scan_pays`; on the tensor cores 384 tokens of 16 heads 113 / 79, but two portions of
-    370 and 231 tokens through a layer of width 2,048 at 0.79 of the walk's speed), whose chain has a block per
-    portion, head and 32 columns, one an SM (148) and built for keys of 128.  Walk / chunks in us, 16 heads of 128, portions of 400 and 500 tokens: one
-    113 / 97, 140 / 103, two 144 / 116, 180 / 124, three (192 blocks, a second round of 44) 174 / 200, 217 / 218,
-    six 342 / 308, 428 / 342.  16 heads of 64: one 96 / 77, 119 / 82, three 96 / 110, 119 / 117, six (the walk has
-    a quarter of the work) 123 / 189, 153 / 212 and 303 / 385 at 1,000."""
+    """Whether a step's gated delta rule is the faster one in chunks (arguments as for :func:`chunk_scan_pays`),
+    whose chain has a block per portion, head and 32 columns, one an SM (148) and built for keys of 128.  The lines
+    are those of the chunks by multiply-adds.  Walk / multiply-adds / tensor cores in us, 16 heads of 128, portions
+    of 400 and 500 tokens: one 114 / 88 / 65, 142 / 96 / 69, two 146 / 118 / 91, 181 / 129 / 97, three (192 blocks, a
+    second round of 44) 176 / 198 / 143, 218 / 215 / 152, six 344 / 309 / 234, 430 / 349 / 265: on the tensor cores
+    (keys of 128) chunks are the faster ones between 148 and 220 blocks, too; through a layer of width 2,048 three
+    portions of 390 tokens take 213 us so, walked 247.  Below the shortest portion two of 370 and 231 tokens were at
+    0.79 of the walk's speed there.  16 heads of 64, walk / multiply-adds: one 96 / 70, 121 / 76, three 97 / 103, 121 /
+    111, six (the walk has a quarter of the work) 125 / 184, 154 / 209 and 305 / 376 at 1,000."""
     blocks = tokens * heads * -(-dv // 32) / max(1, max_q)
     if dk * dv < 14_000:
         return blocks <= 148 and max_q > (DELTA_CHUNK_MIN if blocks <= 74 else 520)

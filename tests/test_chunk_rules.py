@@ -94,7 +94,8 @@ def test_the_matrix_memory_asks_for_its_scratch_once(monkeypatch):
         assert asked == want and terms == want[0] and scratch.numel() == 4096
 
 
-# us on a B200: (heads, dk, dv, portions, tokens of each): (walk, products over chunks)
+# us on a B200: (heads, dk, dv, portions, tokens of each): (walk, products over chunks by multiply-adds, which the
+# lines were laid by)
 LINEAR_US = {
     (64, 128, 64, 1, 161): (42, 46), (64, 128, 64, 1, 200): (51, 50), (64, 128, 64, 1, 260): (64, 55),
     (64, 128, 64, 1, 1000): (232, 112), (64, 128, 64, 2, 161): (64, 65), (64, 128, 64, 2, 200): (76, 70),
